@@ -186,6 +186,39 @@ def test_gemm_f32_is_true_32_bit(m, n, k):
     assert torch.equal(alone[0], out[m - 1])
 
 
+@pytest.mark.parametrize("n,k", [(7, 63), (9, 65), (129, 1024), (128, 1025), (1024, 2052), (40, 6148)])
+def test_gemm_f32_edges_of_segments_rounds_tiles_and_parts(n, k):
+    """Both kernels (up to 16 rows, and tiles) at the edges of their cuts, with operands on and off 16-byte borders."""
+    g = torch.Generator().manual_seed(n + k)
+    wide, w, b = torch.randn(130, k + 1, generator=g), torch.randn(n, k, generator=g), torch.randn(n, generator=g)
+    w_d, b_d = w.to(DEV), b.to(DEV)
+    # a result is chains of 64 fused multiply-adds, a sum over k / 64 chains, one over at most 8 parts, and the bias
+    steps = 64 + (k + 63) // 64 + 8 + 1
+    for columns in (slice(0, k), slice(1, k + 1)):
+        x = wide[:, columns].double()
+        want = x @ w.double().T + b.double()
+        bound = steps * 2.0 ** -24 * (x.abs() @ w.double().abs().T + b.double().abs())
+        rows = wide.to(DEV)[:, columns]
+        whole = ops.linear(rows, w_d, b_d)
+        assert bool(((whole.cpu().double() - want).abs() <= bound).all())
+        for m in (1, 2, 3, 8, 9, 16, 17, 64, 65):
+            assert torch.equal(ops.linear(rows[130 - m:], w_d, b_d), whole[130 - m:]), (m, columns)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n_q,n_kv,d,page", [(4, 2, 128, 16), (1, 1, 20, 8), (3, 1, 18, 8), (12, 2, 64, 4)])
+def test_generic_attention_by_fours_and_one_by_one(dtype, n_q, n_kv, d, page):
+    """Rows that move four elements at a time (sizes in groups of four, pools on their borders) and one at a time."""
+    case = paged_case(dtype, n_q, n_kv, d, page, (33, 1, 130), (2, 1, 1), None, seed=7)
+    want = expected_attention(case, 1.0 / math.sqrt(d))
+    for split in (0, 64):
+        close(run_attention(case, 1.0 / math.sqrt(d), split), want, dtype, f"split {split}")
+    for name in ("k_pool", "v_pool"):                       # one element off: the pools start on no border
+        pool = case[name]
+        case[name] = torch.cat([pool.new_zeros(1), pool.reshape(-1)])[1:].view(pool.shape)
+    close(run_attention(case, 1.0 / math.sqrt(d), 0), want, dtype, "pools off the border")
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n_q,n_kv,d,rot,inter", [(4, 2, 16, 16, False), (5, 1, 48, 48, False), (3, 3, 128, 64, False),
                                                   (2, 1, 80, 80, True), (8, 2, 256, 256, False)])
