@@ -141,20 +141,52 @@ __device__ __forceinline__ int row_split_count(const AttnParams& p, int pos) {
   return pos / p.split_size - first + 1 + srb_kept_pieces(p.keep_first, p.split_size, first);
 }
 
-template <typename T, int DIM_PER_LANE>
-__global__ void paged_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_pool,
-                                       const T* __restrict__ v_pool, T* __restrict__ out,
-                                       float* __restrict__ part_acc, float* __restrict__ part_ml,
-                                       AttnParams p) {
-  extern __shared__ float smem[];
+// Four neighbouring elements, 32-bit.
+__device__ __forceinline__ float4 load_four(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load_four(const __nv_bfloat16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// The rows of a key block into a tile with `pitch` floats a row: a warp takes whole rows, four at a time, so that a lane
+// has four loads in flight and no index needs a division.  `offset`: of the keys' rows, in rows of `width`; -1: zeros.
+template <typename T>
+__device__ __forceinline__ void load_rows(float* tile, int pitch, const T* pool, int width, const long long* offset) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  for (int e = lane * 4; e < width; e += 128) {
+    for (int first = warp * 4; first < KEY_BLOCK; first += warps * 4) {
+      float4 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const long long at = offset[first + i];
+        v[i] = at < 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : load_four(pool + at * width + e);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(tile + (first + i) * pitch + e) = v[i];
+    }
+  }
+}
+
+// WIDE: rows of keys and values are multiples of four elements and start on four elements' borders: they move four
+// elements at a time, and a score is four chains of additions (entries 0, 4, .. / 1, 5, .. / 2, 6, .. / 3, 7, ..).  Moved one
+// element at a time with two divisions each, a tile of 32 keys of 128 took 85 us in a block of 64 threads.
+// A warp per query head that shares the kv head: up to 32 of them, 15 where values are wider than 512 entries (registers).
+template <typename T, int DIM_PER_LANE, bool WIDE>
+__global__ void __launch_bounds__(DIM_PER_LANE <= 16 ? 1024 : 480)
+paged_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const T* __restrict__ v_pool, T* __restrict__ out,
+                       float* __restrict__ part_acc, float* __restrict__ part_ml, AttnParams p) {
+  extern __shared__ __align__(16) float smem[];
   const int d = p.head_dim, vd = p.value_dim;
   const int groups = p.n_q / p.n_kv;
-  float* k_tile = smem;                                  // [32][d + 1]
-  float* v_tile = k_tile + KEY_BLOCK * (d + 1);          // [32][vd], or the key tile itself
+  const int k_pitch = d + (WIDE ? 4 : 1);                // a lane per key: neighbouring keys on different banks
+  float* k_tile = smem;                                  // [32][k_pitch]
+  float* v_tile = k_tile + KEY_BLOCK * k_pitch;          // [32][vd], or the key tile itself
   float* q_tile = v_tile + (p.shared_values ? 0 : KEY_BLOCK * vd);   // [heads_per_block][d]
-  const int v_stride = p.shared_values ? d + 1 : vd;
+  const int v_stride = p.shared_values ? k_pitch : vd;
   if (p.shared_values) v_tile = k_tile;
-  __shared__ long long key_offset[KEY_BLOCK];            // element offset of each key's row, -1 = masked
+  __shared__ long long key_offset[KEY_BLOCK];            // which row of the pool each key's is, -1 = masked
 
   const int row = blockIdx.z, kv_head = blockIdx.y / p.head_chunks, chunk = blockIdx.y % p.head_chunks;
   const int split = blockIdx.x;
@@ -202,31 +234,44 @@ __global__ void paged_attention_kernel(const T* __restrict__ q, const T* __restr
         if (page < 0 || page >= p.num_pages) {
           atomicOr(p.error_word, SRB_FLAG_BAD_PAGE);
         } else {
-          offset = (((long long)page * p.n_kv + kv_head) * p.page_size + key % p.page_size) * d;
+          offset = ((long long)page * p.n_kv + kv_head) * p.page_size + key % p.page_size;
         }
       }
       key_offset[threadIdx.x] = offset;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < KEY_BLOCK * d; i += blockDim.x) {
-      const int key = i / d, e = i - key * d;
-      const long long offset = key_offset[key];
-      k_tile[key * (d + 1) + e] = offset < 0 ? 0.f : srb_to_float(k_pool[offset + e]);
-    }
-    if (!p.shared_values) {
-      for (int i = threadIdx.x; i < KEY_BLOCK * vd; i += blockDim.x) {
-        const int key = i / vd, e = i - key * vd;
-        const long long offset = key_offset[key];          // in elements of a key row: rows are d or vd wide
-        v_tile[key * vd + e] = offset < 0 ? 0.f : srb_to_float(v_pool[offset / d * vd + e]);
-      }
-    }
-    __syncthreads();
-
-    // one key per lane: the dot product runs over the head in index order
     float s = 0.f;
     const float* qv = q_tile + (live ? warp : 0) * d;
-    const float* kv = k_tile + lane * (d + 1);
-    for (int e = e_begin; e < e_end; ++e) s += qv[e] * kv[e];
+    const float* kv = k_tile + lane * k_pitch;
+    if (WIDE) {
+      load_rows(k_tile, k_pitch, k_pool, d, key_offset);
+      if (!p.shared_values) load_rows(v_tile, vd, v_pool, vd, key_offset);
+      __syncthreads();
+      // one key per lane
+      float s4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+      for (int e = e_begin; e < e_end; e += 4) {
+        const float4 x = load_four(qv + e), y = load_four(kv + e);
+        s4[0] += x.x * y.x; s4[1] += x.y * y.y; s4[2] += x.z * y.z; s4[3] += x.w * y.w;
+      }
+      s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+    } else {
+      for (int i = threadIdx.x; i < KEY_BLOCK * d; i += blockDim.x) {
+        const int key = i / d, e = i - key * d;
+        const long long offset = key_offset[key];
+        k_tile[key * k_pitch + e] = offset < 0 ? 0.f : srb_to_float(k_pool[offset * d + e]);
+      }
+      if (!p.shared_values) {
+        for (int i = threadIdx.x; i < KEY_BLOCK * vd; i += blockDim.x) {
+          const int key = i / vd, e = i - key * vd;
+          const long long offset = key_offset[key];
+          v_tile[key * vd + e] = offset < 0 ? 0.f : srb_to_float(v_pool[offset * vd + e]);
+        }
+      }
+      __syncthreads();
+      // one key per lane: the dot product runs over the head in index order
+      for (int e = e_begin; e < e_end; ++e) s += qv[e] * kv[e];
+    }
     s *= p.scale;
     if (p.softcap > 0.f) s = srb_capped(s / p.softcap, p.softcap);
     if (key_offset[lane] < 0) s = -INFINITY;
@@ -238,6 +283,7 @@ __global__ void paged_attention_kernel(const T* __restrict__ q, const T* __restr
     m = m_new;
 #pragma unroll
     for (int j = 0; j < DIM_PER_LANE; ++j) acc[j] *= correction;
+#pragma unroll 8
     for (int key = 0; key < KEY_BLOCK; ++key) {
       const float pk = __shfl_sync(0xffffffffu, prob, key);
 #pragma unroll
@@ -314,15 +360,22 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_acc, con
 template <typename T, int DIM_PER_LANE>
 static int launch_attention(const void* q, const void* k_pool, const void* v_pool, void* out, float* part_acc,
                             float* part_ml, const AttnParams& p, int rows, cudaStream_t s) {
-  const size_t smem = ((size_t)KEY_BLOCK * (p.head_dim + 1) + (p.shared_values ? 0 : (size_t)KEY_BLOCK * p.value_dim) +
-                       (size_t)p.heads_per_block * p.head_dim) * sizeof(float);
+  auto bytes = [&p](int extra) {
+    return ((size_t)KEY_BLOCK * (p.head_dim + extra) + (p.shared_values ? 0 : (size_t)KEY_BLOCK * p.value_dim) +
+            (size_t)p.heads_per_block * p.head_dim) * sizeof(float);
+  };
+  // rows of whole groups of four elements on four elements' borders (each half of a key row of two maps too)
+  const size_t group = 4 * sizeof(T);
+  const bool wide = p.head_dim % (p.maps == 2 ? 8 : 4) == 0 && p.value_dim % 4 == 0 &&
+                    ((uintptr_t)k_pool | (uintptr_t)v_pool) % group == 0 && bytes(4) <= 227 * 1024;
+  const size_t smem = bytes(wide ? 4 : 1);
   if (smem > 227 * 1024) SRB_FAIL("paged_attention: %zu bytes of shared memory exceed 232448", smem);
-  if (smem > 48 * 1024)
-    SRB_CUDA_CALL(cudaFuncSetAttribute(paged_attention_kernel<T, DIM_PER_LANE>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  auto kernel = wide ? paged_attention_kernel<T, DIM_PER_LANE, true> : paged_attention_kernel<T, DIM_PER_LANE, false>;
+  if (smem > 48 * 1024) SRB_CUDA_CALL(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid(p.split_size == 0 ? 1 : p.max_splits, p.n_kv * p.head_chunks, rows);
   if (grid.y > 65535) SRB_FAIL("paged_attention: %d blocks along the heads exceed 65535", (int)grid.y);
-  paged_attention_kernel<T, DIM_PER_LANE><<<grid, p.heads_per_block * 32, smem, s>>>(
+  // at least four warps bring the rows, whatever the number of heads that share them
+  kernel<<<grid, (p.heads_per_block < 4 ? 4 : p.heads_per_block) * 32, smem, s>>>(
       (const T*)q, (const T*)k_pool, (const T*)v_pool, (T*)out, part_acc, part_ml, p);
   SRB_LAUNCH_CHECK("paged_attention");
   if (p.split_size != 0) {
