@@ -1,25 +1,31 @@
-// Y = X W^T in bfloat16 for many tokens (prompt portions): tiles of 256 features x 256 tokens computed
+// Y = X W^T in bfloat16 for many tokens (prompt portions): tiles of 256 tokens x 256 weight rows computed
 // by pairs of CTAs on neighbouring SMs with tcgen05.mma.cta_group::2, in a persistent loop.
 //
-// The pair is a thread-block cluster of two.  CTA r of the pair brings 128 rows of W (its half of the
-// M side) and 128 tokens of X (its half of the N side) into its own shared memory by TMA; one thread of
-// the even CTA issues the products for both, and each CTA's tensor memory receives the 128 x 256
-// accumulator of its own W rows.  Per product step a CTA reads 8 KB of operands from shared memory and
-// the pair asks L2 for 1 byte per 131 FLOP (a single CTA with a 128 x 256 tile: 12 KB and 1 byte per
-// 85 FLOP).  The kernel is persistent: 74 pairs walk the tiles, the accumulator has two buffers in
-// tensor memory, and the epilogue of a tile (tensor memory -> registers -> shared memory -> 16-byte
-// stores, 128 tokens at a time) runs while the products of the next tile are issued.  Six stages of
-// 32 KB keep 160 KB of operands in flight per CTA.
+// The pair is a thread-block cluster of two.  The tokens are the M side: CTA r of the pair brings 128 tokens of X and
+// 128 rows of W (its half of the N side) into its own shared memory by TMA; one thread of the even CTA issues the
+// products for both, and each CTA's tensor memory receives the accumulator of its own tokens, a token per lane.  Per
+// product step a CTA reads 8 KB of operands from shared memory and the pair asks L2 for 1 byte per 131 FLOP (a single
+// CTA with a 128 x 256 tile: 12 KB and 1 byte per 85 FLOP).  The kernel is persistent: 74 pairs walk the tiles, the
+// accumulator has two buffers in tensor memory, and the epilogue of a tile runs while the products of the next one are
+// issued.  Six stages of 32 KB keep 160 KB of operands in flight per CTA.
+//
+// A token per lane is what the epilogue wants: in the gated mode the even CTA brings gate rows and the odd one the up
+// rows of the same features, so a lane finds both in its own columns, and a lane's results are neighbours in the output
+// row.  Eight epilogue warps (a quarter of the lanes and half of the columns each) work on their own: tensor memory ->
+// registers -> a swizzled 4 KB tile of 32 tokens x 128 bytes -> one TMA store, no barrier between warps.  With the weight
+// rows in the lanes (gate and up 64 lanes apart) they met through shared memory behind a barrier every 32 tokens and half
+// of the four warps computed: 19 us a tile, twice what its products take at K = 2,048.
 //
 // Warps of each CTA: 0 copies (TMA), 1 issues products (even CTA only) and owns the tensor memory,
-// 2-5 epilogue.  Barriers: full[s] lives in the even CTA and counts the bytes of both CTAs' copies;
+// 2-9 epilogue.  Barriers: full[s] lives in the even CTA and counts the bytes of both CTAs' copies;
 // empty[s] and acc_full[b] live in both and are signalled by tcgen05.commit with a multicast to the
 // pair; acc_empty[b] lives in the even CTA and is signalled by the epilogue warps of both.
 // Every wait is bounded; a wait that runs out flags SRB_FLAG_WAIT_TIMEOUT and every role leaves its
 // loop.  No TMA load uses multicast.
 //
-// Modes: bfloat16 store; SiLU(gate) * up where a CTA's 128 weight rows are 64 gate rows over the 64 up
-// rows of the same features (as in gemm_bf16.cu).
+// Modes: bfloat16 store, with an activation or without; float store; act(gate) * up.  Each of them also over grouped rows
+// (routed experts, GROUPED): the rows of X are slots in the order of their experts, a tile is up to 256 slots of one expert
+// (moe_plan_kernel's list) and its weight rows are that expert's.
 #include "common.cuh"
 #include "tcgen05_helpers.cuh"
 #include "activations.cuh"
@@ -27,24 +33,31 @@
 #include <mutex>
 
 SRB_DEFINE_LAST_ERROR()
+SRB_DEFINE_PDL_SWITCH()
 
-#define PAIR_F 128            // weight rows per CTA (256 per pair)
+#define PAIR_ROWS 128         // tokens, and weight rows, per CTA (256 of each per pair)
 #define PAIR_T 256            // tokens per tile (128 copied by each CTA)
 #define PAIR_K 64
 #define PAIR_STAGES 6
-#define PAIR_OUT_T 128         // tokens of a tile that are staged for the stores at a time
-#define PAIR_THREADS 192
+#define PAIR_EPILOGUE_WARPS 8
+#define PAIR_THREADS (64 + 32 * PAIR_EPILOGUE_WARPS)
+#define PAIR_BOX_BYTES 4096   // a warp's piece of the output on its way: 32 tokens x 128 bytes, swizzled
 #define PAIR_EPI_BF16 0
+#define PAIR_EPI_F32 1
 #define PAIR_EPI_SILU 2
 #define PAIR_EPI_ACT 5        // out = activation(x w^T): the plain kernel with an activation in its epilogue
 
 struct PairArgs {
-  __nv_bfloat16* out;
+  void* out;                 // bfloat16, or float (PAIR_EPI_F32)
   int tokens, features, k, ldo, up_row_offset;
   float act_param;           // the activation's parameter, for those that have one
   int activation;            // which SRB_ACT_* the gated mode applies to the gate half, or the plain mode to its result (-1: none)
-  int tiles_t, tiles_f, num_tiles;
+  int tiles_t, tiles_f;
   int* error_word;
+  // GROUPED: [number of row tiles, first slot of every expert (experts + 1), then (expert, first slot) per row tile]
+  const int* plan;
+  int experts, expert_rows;
+  const float* slot_weight;  // a factor on the input of every slot (its sums are multiplied by it), or null
 };
 
 // ---- the cta_group::2 forms of the instructions
@@ -80,20 +93,60 @@ __device__ __forceinline__ void mbar_arrive_remote(unsigned bar, unsigned rank) 
 
 __host__ __device__ constexpr unsigned pair_idesc() {
   // D float, A and B bfloat16, both K-major, M = 256 (the pair), N = 256
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(PAIR_T >> 3) << 17) | ((unsigned)(256 >> 4) << 24);
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(2 * PAIR_ROWS >> 3) << 17) | ((unsigned)(PAIR_T >> 4) << 24);
 }
 
-template <int EPI>
+// A tile of 32 rows x 128 bytes of shared memory to the tensor of `map`; rows and columns beyond its extents are not written.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, unsigned src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void tma_stores_have_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ unsigned pack_bf16(float low, float high) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(low, high);
+  return *reinterpret_cast<const unsigned*>(&v);
+}
+
+// What a tile is, the same in every role of both CTAs.
+struct PairTile {
+  int feature0, token0;      // the first output feature; the first token (or slot)
+  int limit;                 // tokens (or slots of the expert) end here
+  int w_row0;                // the expert's first weight row, or 0
+};
+
+template <int EPI, bool GROUPED>
+__device__ __forceinline__ PairTile pair_tile(const PairArgs& args, int tile) {
+  constexpr int FEATURES = EPI == PAIR_EPI_SILU ? PAIR_ROWS : 2 * PAIR_ROWS;
+  PairTile t;
+  if (GROUPED) {
+    // the features of one row tile follow one another: its rows stay in L2, and an expert's weights are streamed once
+    const int* first_slot = args.plan + 1;
+    const int* tiles = first_slot + args.experts + 1;
+    const int rt = tile / args.tiles_f;
+    const int expert = tiles[2 * rt];
+    t.feature0 = (tile % args.tiles_f) * FEATURES;
+    t.token0 = tiles[2 * rt + 1];
+    t.limit = min(t.token0 + PAIR_T, first_slot[expert + 1]);
+    t.w_row0 = expert * args.expert_rows;
+  } else {
+    t.feature0 = tile / args.tiles_t * FEATURES;
+    t.token0 = tile % args.tiles_t * PAIR_T;
+    t.limit = args.tokens;
+    t.w_row0 = 0;
+  }
+  return t;
+}
+
+template <int EPI, bool GROUPED>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                      PairArgs args) {
-  constexpr int A_BYTES = PAIR_F * PAIR_K * 2;               // 16 KB: this CTA's rows of W
-  constexpr int B_BYTES = (PAIR_T / 2) * PAIR_K * 2;         // 16 KB: this CTA's tokens of X
+                      const __grid_constant__ CUtensorMap map_out, PairArgs args) {
+  constexpr int A_BYTES = PAIR_ROWS * PAIR_K * 2;            // 16 KB: this CTA's tokens of X
+  constexpr int B_BYTES = PAIR_ROWS * PAIR_K * 2;            // 16 KB: this CTA's rows of W
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  constexpr int FEATURES_PER_CTA = EPI == PAIR_EPI_SILU ? PAIR_F / 2 : PAIR_F;
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_unaligned + 1023) & ~(uintptr_t)1023);
-  unsigned char* out_smem = smem + PAIR_STAGES * STAGE_BYTES;
   __shared__ __align__(8) unsigned long long full_bar[PAIR_STAGES], empty_bar[PAIR_STAGES], acc_full[2], acc_empty[2];
   __shared__ unsigned tmem_holder;
   __shared__ int abort_flag;
@@ -111,7 +164,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&acc_full[b]), 1);
-      mbar_init(smem_u32(&acc_empty[b]), 8);                 // one lane of each epilogue warp of both CTAs
+      mbar_init(smem_u32(&acc_empty[b]), 2 * PAIR_EPILOGUE_WARPS);      // one lane of each epilogue warp of both CTAs
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -120,16 +173,20 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
   srb_cluster_sync();                                        // both CTAs' barriers exist before anyone signals them
   tc_fence_after();
   const unsigned tmem_base = tmem_holder;
+  srb_launch_dependents();
+  srb_grid_dependency_wait();                                // x and the plan are written by kernels ahead
+  const int num_tiles = GROUPED ? args.plan[0] * args.tiles_f : args.tiles_t * args.tiles_f;
 
   if (warp == 0) {
     // copies: both CTAs, each its own halves, into its own stages; the bytes count on the even CTA's barrier
     int issued = 0;
     long long round = 0;
     bool ok = true;
-    for (int tile = pair; tile < args.num_tiles && ok; tile += num_pairs) {
-      const int ft = tile / args.tiles_t, tt = tile % args.tiles_t;
-      const int feature0 = ft * 2 * FEATURES_PER_CTA + (int)rank * FEATURES_PER_CTA;
-      const int token0 = tt * PAIR_T + (int)rank * (PAIR_T / 2);
+    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+      const PairTile t = pair_tile<EPI, GROUPED>(args, tile);
+      // gated: the even CTA brings the gate rows, the odd one the up rows of the same features
+      const int w_row = t.w_row0 + t.feature0 + (int)rank * (EPI == PAIR_EPI_SILU ? args.up_row_offset : PAIR_ROWS);
+      const int token = t.token0 + (int)rank * PAIR_ROWS;
       for (int kb = 0; kb < total_kb && ok; ++kb, ++round) {
         const int s = (int)(round % PAIR_STAGES);
         const unsigned phase = (unsigned)(round / PAIR_STAGES) & 1u;
@@ -140,13 +197,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         const int kx = kb * PAIR_K;
         if (elect_one()) {
           if (rank == 0) mbar_expect_tx(bar, 2 * STAGE_BYTES);
-          if (EPI == PAIR_EPI_SILU) {
-            tma_load_2d_pair(stage, &map_w, bar, kx, feature0);
-            tma_load_2d_pair(stage + A_BYTES / 2, &map_w, bar, kx, args.up_row_offset + feature0);
-          } else {
-            tma_load_2d_pair(stage, &map_w, bar, kx, feature0);
-          }
-          tma_load_2d_pair(stage + A_BYTES, &map_x, bar, kx, token0);
+          tma_load_2d_pair(stage, &map_x, bar, kx, token);
+          tma_load_2d_pair(stage + A_BYTES, &map_w, bar, kx, w_row);
         }
         ++issued;
       }
@@ -165,13 +217,13 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
       long long round = 0;
       int local_tile = 0;
       bool ok = true;
-      for (int tile = pair; tile < args.num_tiles && ok; tile += num_pairs, ++local_tile) {
+      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local_tile) {
         const int b = local_tile & 1;
         // the epilogue warps of both CTAs have read this accumulator buffer (two tiles ago)
         ok = mbar_wait_warp(smem_u32(&acc_empty[b]), (((unsigned)(local_tile >> 1)) & 1u) ^ 1u, &abort_flag);
         if (!ok) break;
         tc_fence_after();
-        const unsigned acc = tmem_base + b * PAIR_T;
+        const unsigned acc = tmem_base + b * 2 * PAIR_ROWS;
         for (int kb = 0; kb < total_kb && ok; ++kb, ++round) {
           const int s = (int)(round % PAIR_STAGES);
           const unsigned phase = (unsigned)(round / PAIR_STAGES) & 1u;
@@ -193,85 +245,95 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
       }
     }
   } else {
-    // epilogue: warp w reads TMEM lanes 32 * (w % 4) .. + 32 of its own CTA
-    const int quarter = warp & 3;
-    const int row_in_cta = quarter * 32 + lane;              // the W row (TMEM lane) this thread holds
+    // epilogue: warp w reads TMEM lanes 32 * (w % 4) .. + 32 of its own CTA, and one half of the columns
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
     const unsigned lane_address = tmem_base + ((unsigned)(quarter * 32) << 16);
-    __nv_bfloat16* staged = reinterpret_cast<__nv_bfloat16*>(out_smem);   // [token][FEATURES_PER_CTA]
+    unsigned char* box = smem + PAIR_STAGES * STAGE_BYTES + (warp - 2) * PAIR_BOX_BYTES;
+    constexpr int BOX_FEATURES = EPI == PAIR_EPI_F32 ? 32 : 64;         // 128 bytes of an output row
+    constexpr int HALF_FEATURES = EPI == PAIR_EPI_SILU ? PAIR_ROWS / 2 : PAIR_ROWS;
     int local_tile = 0;
-    bool ok = true;
-    for (int tile = pair; tile < args.num_tiles && ok; tile += num_pairs, ++local_tile) {
+    for (int tile = pair; tile < num_tiles; tile += num_pairs, ++local_tile) {
       const int b = local_tile & 1;
-      const int ft = tile / args.tiles_t, tt = tile % args.tiles_t;
-      const int feature0 = ft * 2 * FEATURES_PER_CTA + (int)rank * FEATURES_PER_CTA;
-      const int token_base = tt * PAIR_T;
-      ok = mbar_wait(smem_u32(&acc_full[b]), ((unsigned)(local_tile >> 1)) & 1u, &abort_flag);
-      if (!ok) break;
+      const PairTile t = pair_tile<EPI, GROUPED>(args, tile);
+      const int token = t.token0 + (int)rank * PAIR_ROWS + quarter * 32;                // of lane 0
+      const int live = min(t.limit - token, 32);
+      const float weight = GROUPED && EPI != PAIR_EPI_F32 && args.slot_weight && lane < live ? args.slot_weight[token + lane] : 1.0f;
+      if (!mbar_wait_warp(smem_u32(&acc_full[b]), ((unsigned)(local_tile >> 1)) & 1u, &abort_flag)) break;
       tc_fence_after();
-      // 128 tokens at a time: accumulator -> registers -> staging tile [token][feature] -> 16-byte stores
 #pragma unroll 1
-      for (int half = 0; half < PAIR_T / PAIR_OUT_T; ++half) {
-        if (EPI == PAIR_EPI_SILU) {
-          // lanes 0..63 hold gate, lanes 64..127 up of the same 64 features: up passes through shared
-          // memory, 32 tokens at a time, in two buffers that take turns (one barrier per round)
-          float* exchange = reinterpret_cast<float*>(out_smem + PAIR_OUT_T * FEATURES_PER_CTA * 2);   // [2][64][32] floats
-#pragma unroll 1
-          for (int c = 0; c < PAIR_OUT_T; c += 32) {
-            float acc[32];
-            tmem_load_32(lane_address + b * PAIR_T + half * PAIR_OUT_T + c, acc);
-            float* buffer = exchange + ((c >> 5) & 1) * 64 * 32;
-            if (quarter >= 2) {
+      for (int c = 0; c < HALF_FEATURES; c += BOX_FEATURES) {
+        const unsigned column = lane_address + b * 2 * PAIR_ROWS + half * HALF_FEATURES + c;
+        // the row's 128 bytes as eight pieces; a piece goes where the 128-byte swizzle of the store expects it
+        const unsigned row = smem_u32(box) + lane * 128;
+        const int turn = lane & 7;
 #pragma unroll
-              for (int j = 0; j < 32; ++j) buffer[j * 64 + (quarter & 1) * 32 + lane] = acc[j];
-            }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (quarter < 2) {
+        for (int part = 0; part < BOX_FEATURES; part += 32) {
+          float acc[32];
+          unsigned packed[16];
+          tmem_load_32(column + part, acc);
+          if (EPI == PAIR_EPI_SILU) {
+            float up[32];
+            tmem_load_32(column + PAIR_ROWS + part, up);
 #pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const float g = acc[j], u = buffer[j * 64 + (quarter & 1) * 32 + lane];
-                staged[(c + j) * FEATURES_PER_CTA + row_in_cta] = __float2bfloat16_rn(srb_gated<false>(args.activation, g, u, args.act_param));
-              }
+            for (int j = 0; j < 32; ++j) {
+              if (GROUPED) { acc[j] *= weight; up[j] *= weight; }
+              acc[j] = srb_gated<GROUPED>(args.activation, acc[j], up[j], args.act_param);
             }
+          } else if (EPI == PAIR_EPI_BF16 && args.activation >= 0) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              acc[j] = srb_gated<GROUPED>(args.activation, GROUPED ? acc[j] * weight : acc[j], 1.0f, args.act_param);
           }
-        } else {
-#pragma unroll 1
-          for (int c = 0; c < PAIR_OUT_T; c += 16) {
-            float acc[16];
-            tmem_load_16(lane_address + b * PAIR_T + half * PAIR_OUT_T + c, acc);
+          if (part == 0) {
+            // the store of the box before has read it
+            if (lane == 0) tma_stores_have_read();
+            __syncwarp();
+          }
+          if (EPI == PAIR_EPI_F32) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              staged[(c + j) * FEATURES_PER_CTA + row_in_cta] =
-                  __float2bfloat16_rn(args.activation >= 0 ? srb_gated<false>(args.activation, acc[j], 1.0f, args.act_param) : acc[j]);
+            for (int i = 0; i < 8; ++i)
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row + ((i ^ turn) << 4)), "r"(__float_as_uint(acc[4 * i])),
+                           "r"(__float_as_uint(acc[4 * i + 1])), "r"(__float_as_uint(acc[4 * i + 2])), "r"(__float_as_uint(acc[4 * i + 3])) : "memory");
+          } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) packed[j] = pack_bf16(acc[2 * j], acc[2 * j + 1]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row + (((part / 8 + i) ^ turn) << 4)), "r"(packed[4 * i]),
+                           "r"(packed[4 * i + 1]), "r"(packed[4 * i + 2]), "r"(packed[4 * i + 3]) : "memory");
           }
         }
-        if (half == PAIR_T / PAIR_OUT_T - 1) {
+        if (c + BOX_FEATURES >= HALF_FEATURES) {
           // the accumulator buffer is free for the tile after next
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_remote(smem_u32(&acc_empty[b]), 0);
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");        // the staged rows are complete
-        // 16-byte stores: a token's FEATURES_PER_CTA features are consecutive in the output
-        constexpr int CHUNKS = FEATURES_PER_CTA / 8;
-        for (int i = threadIdx.x - 64; i < PAIR_OUT_T * CHUNKS; i += 128) {
-          const int token = i / CHUNKS, chunk = i % CHUNKS;
-          const int feature = feature0 + chunk * 8;
-          const int out_token = token_base + half * PAIR_OUT_T + token;
-          if (out_token >= args.tokens || feature >= args.features) continue;
-          const uint4 value = *reinterpret_cast<const uint4*>(staged + token * FEATURES_PER_CTA + chunk * 8);
-          __nv_bfloat16* dst = args.out + (size_t)out_token * args.ldo + feature;
-          if (feature + 8 <= args.features) {
-            *reinterpret_cast<uint4*>(dst) = value;
-          } else {
-            const __nv_bfloat16* v = reinterpret_cast<const __nv_bfloat16*>(&value);
-            for (int e = 0; feature + e < args.features; ++e) dst[e] = v[e];
+        const int feature = t.feature0 + half * HALF_FEATURES + c;
+        if (feature >= args.features || live <= 0) continue;
+        if (!GROUPED || live == 32) {
+          fence_proxy_async_shared();
+          __syncwarp();
+          if (lane == 0) tma_store_2d(&map_out, smem_u32(box), feature, token);
+        } else {
+          // the rows behind the expert's last slot belong to the next one: only the live rows, 16 bytes a lane
+          __syncwarp();
+          constexpr int ELEMENT = EPI == PAIR_EPI_F32 ? 4 : 2;
+          const int piece = lane & 7;
+          for (int r = lane >> 3; r < live; r += 4) {
+            if (feature + piece * (16 / ELEMENT) >= args.features) continue;        // whole pieces: features are a multiple of 8
+            const uint4 v = *reinterpret_cast<const uint4*>(box + r * 128 + ((piece ^ (r & 7)) << 4));
+            *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(args.out) +
+                                      ((size_t)(token + r) * args.ldo + feature) * ELEMENT + piece * 16) = v;
           }
+          __syncwarp();
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");        // the staging tile may be written again
       }
     }
+    if (lane == 0) tma_stores_have_read();                   // before this block's shared memory goes
     tc_fence_before();
   }
+  __syncwarp();
   srb_cluster_sync();                                        // nobody leaves while the other CTA may still signal or read
   if (threadIdx.x == 0 && abort_flag) atomicOr(args.error_word, SRB_FLAG_WAIT_TIMEOUT);
   if (warp == 1) {
@@ -298,17 +360,31 @@ static EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-static int make_map(CUtensorMap* map, const void* base, long long rows, long long k, long long pitch, int box_rows) {
+// A row-major matrix [rows, columns] (row pitch in elements) cut into boxes of [box_rows, 128 bytes] with 128-byte swizzle.
+static int make_map(CUtensorMap* map, const void* base, long long rows, long long columns, long long pitch, int box_rows,
+                    bool floats = false) {
   EncodeTiledFn fn = encode_tiled();
   if (!fn) SRB_FAIL("gemm_bf16_pair: the driver does not offer cuTensorMapEncodeTiled");
-  const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)pitch * 2};
-  const cuuint32_t box[2] = {PAIR_K, (cuuint32_t)box_rows};
+  const cuuint64_t dims[2] = {(cuuint64_t)columns, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)pitch * (floats ? 4 : 2)};
+  const cuuint32_t box[2] = {(cuuint32_t)(floats ? 32 : 64), (cuuint32_t)box_rows};
   const cuuint32_t elem[2] = {1, 1};
-  const CUresult status = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box,
-                             elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+  const CUresult status = fn(map, floats ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base),
+                             dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (status != CUDA_SUCCESS) SRB_FAIL("gemm_bf16_pair: cuTensorMapEncodeTiled failed with %d", (int)status);
+  return SRB_OK;
+}
+
+template <int EPI, bool GROUPED>
+static int launch_pair(const CUtensorMap& map_w, const CUtensorMap& map_x, const CUtensorMap& map_out, const PairArgs& args,
+                       int max_tiles, cudaStream_t s) {
+  const int pairs = std::max(1, std::min(srb_sm_count() / 2, max_tiles));
+  // the stages, a box per epilogue warp, alignment
+  const size_t smem = (size_t)PAIR_STAGES * 2 * PAIR_ROWS * PAIR_K * 2 + PAIR_EPILOGUE_WARPS * PAIR_BOX_BYTES + 1024;
+  auto kernel = gemm_bf16_pair_kernel<EPI, GROUPED>;
+  SRB_CUDA_CALL(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  SRB_CUDA_CALL(srb_launch_clustered(kernel, dim3(2 * pairs), dim3(PAIR_THREADS), smem, s, dim3(2, 1, 1), map_w, map_x, map_out, args));
   return SRB_OK;
 }
 
@@ -331,33 +407,20 @@ extern "C" int srb_gemm_bf16_pair_param(const void* x, const void* w, void* out,
   if (mode == PAIR_EPI_SILU && up_row_offset + features > rows_of_w)
     SRB_FAIL("gemm_bf16_pair: the up rows lie outside the %d rows of w", rows_of_w);
   if (mode == PAIR_EPI_BF16 && features > rows_of_w) SRB_FAIL("gemm_bf16_pair: %d features exceed %d rows of w", features, rows_of_w);
-  CUtensorMap map_w, map_x;
-  if (make_map(&map_w, w, rows_of_w, k, ldw, mode == PAIR_EPI_SILU ? PAIR_F / 2 : PAIR_F) != SRB_OK) return SRB_ERR_INVALID;
-  if (make_map(&map_x, x, tokens, k, ldx, PAIR_T / 2) != SRB_OK) return SRB_ERR_INVALID;
-  const int features_per_pair = mode == PAIR_EPI_SILU ? PAIR_F : 2 * PAIR_F;
-  PairArgs args;
-  args.out = (__nv_bfloat16*)out; args.tokens = tokens; args.features = features; args.k = k; args.ldo = ldo;
+  CUtensorMap map_w, map_x, map_out;
+  if (make_map(&map_w, w, rows_of_w, k, ldw, PAIR_ROWS) != SRB_OK || make_map(&map_x, x, tokens, k, ldx, PAIR_ROWS) != SRB_OK ||
+      make_map(&map_out, out, tokens, features, ldo, 32) != SRB_OK)
+    return SRB_ERR_INVALID;
+  const int features_per_tile = mode == PAIR_EPI_SILU ? PAIR_ROWS : 2 * PAIR_ROWS;
+  PairArgs args = {};
+  args.out = out; args.tokens = tokens; args.features = features; args.k = k; args.ldo = ldo;
   args.up_row_offset = up_row_offset; args.activation = activation; args.act_param = act_param; args.error_word = error_word;
   args.tiles_t = (tokens + PAIR_T - 1) / PAIR_T;
-  args.tiles_f = (features + features_per_pair - 1) / features_per_pair;
-  args.num_tiles = args.tiles_t * args.tiles_f;
-  int device = 0, sms = 0;
-  SRB_CUDA_CALL(cudaGetDevice(&device));
-  SRB_CUDA_CALL(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  const int pairs = std::max(1, std::min(sms / 2, args.num_tiles));
-  // the stages, the staging tile of the stores (and in SiLU mode, inside it, the exchange of the up half), alignment
-  const size_t smem = (size_t)PAIR_STAGES * (PAIR_F * PAIR_K * 2 + (PAIR_T / 2) * PAIR_K * 2) + PAIR_OUT_T * PAIR_F * 2 + 1024;
+  args.tiles_f = (features + features_per_tile - 1) / features_per_tile;
+  const int tiles = args.tiles_t * args.tiles_f;
   cudaStream_t s = (cudaStream_t)stream;
-  if (mode == PAIR_EPI_SILU) {
-    SRB_CUDA_CALL(cudaFuncSetAttribute(gemm_bf16_pair_kernel<PAIR_EPI_SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    SRB_CUDA_CALL(srb_launch_clustered(gemm_bf16_pair_kernel<PAIR_EPI_SILU>, dim3(2 * pairs), dim3(PAIR_THREADS), smem, s,
-                                       dim3(2, 1, 1), map_w, map_x, args));
-  } else {
-    SRB_CUDA_CALL(cudaFuncSetAttribute(gemm_bf16_pair_kernel<PAIR_EPI_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    SRB_CUDA_CALL(srb_launch_clustered(gemm_bf16_pair_kernel<PAIR_EPI_BF16>, dim3(2 * pairs), dim3(PAIR_THREADS), smem, s,
-                                       dim3(2, 1, 1), map_w, map_x, args));
-  }
-  return SRB_OK;
+  if (mode == PAIR_EPI_SILU) return launch_pair<PAIR_EPI_SILU, false>(map_w, map_x, map_out, args, tiles, s);
+  return launch_pair<PAIR_EPI_BF16, false>(map_w, map_x, map_out, args, tiles, s);
 }
 
 extern "C" int srb_gemm_bf16_pair(const void* x, const void* w, void* out, int tokens, int features, int k, int ldx,
