@@ -24,8 +24,8 @@
 // loop.  No TMA load uses multicast.
 //
 // Modes: bfloat16 store, with an activation or without; float store; act(gate) * up.  Each of them also over grouped rows
-// (routed experts, GROUPED): the rows of X are slots in the order of their experts, a tile is up to 256 slots of one expert
-// (moe_plan_kernel's list) and its weight rows are that expert's.
+// (routed experts, GROUPED): the rows of X are slots in the order of their experts, a tile is up to `tile_slots` slots of one
+// expert (moe_plan_kernel's list, read on the device: pairs walk as many tiles as there are) and its weight rows are that expert's.
 #include "common.cuh"
 #include "tcgen05_helpers.cuh"
 #include "activations.cuh"
@@ -56,7 +56,7 @@ struct PairArgs {
   int* error_word;
   // GROUPED: [number of row tiles, first slot of every expert (experts + 1), then (expert, first slot) per row tile]
   const int* plan;
-  int experts, expert_rows;
+  int tile_slots, experts, expert_rows;
   const float* slot_weight;  // a factor on the input of every slot (its sums are multiplied by it), or null
 };
 
@@ -127,7 +127,7 @@ __device__ __forceinline__ PairTile pair_tile(const PairArgs& args, int tile) {
     const int expert = tiles[2 * rt];
     t.feature0 = (tile % args.tiles_f) * FEATURES;
     t.token0 = tiles[2 * rt + 1];
-    t.limit = min(t.token0 + PAIR_T, first_slot[expert + 1]);
+    t.limit = min(t.token0 + args.tile_slots, first_slot[expert + 1]);
     t.w_row0 = expert * args.expert_rows;
   } else {
     t.feature0 = tile / args.tiles_t * FEATURES;
@@ -430,4 +430,44 @@ extern "C" int srb_gemm_bf16_pair(const void* x, const void* w, void* out, int t
     SRB_FAIL("gemm_bf16_pair: an activation with a parameter comes with its parameter");
   return srb_gemm_bf16_pair_param(x, w, out, tokens, features, k, ldx, ldw, ldo, rows_of_w, up_row_offset, mode, activation, 0.f,
                                   error_word, stream);
+}
+
+// ---- grouped: one weight matrix per expert, rows grouped by expert ---------------------------------------------
+// x [slots, k]: the rows in slot order (the slots of an expert are consecutive); w [experts * expert_rows, k]; `plan` (device)
+// as in PairArgs, with row tiles of `tile_slots` slots (256 at most).  mode 1: out float [slots, ldo] = x w_e^T over `features`
+// rows of the expert's matrix; mode 2: the expert's matrix stacks gate rows [0, features) over up rows [up_row_offset,
+// + features), out bf16 [slots, ldo] = act(gate) * up; mode 5: out bf16 = act(x w_e^T).  `slot_weight` (float [slots], or
+// null): a factor on the input of every slot, taken on the 32-bit sums (modes 2 and 5).  The activations are computed with the
+// full-precision exponential.
+extern "C" int srb_gemm_bf16_pair_grouped(const void* x, const void* w, void* out, const int* plan, int tile_slots, int slots,
+                                          int experts, int expert_rows, int features, int k, int ldo, int up_row_offset, int mode,
+                                          int activation, float act_param, const float* slot_weight, int* error_word, void* stream) {
+  if (slots <= 0 || features <= 0) return SRB_OK;
+  if (tile_slots != 128 && tile_slots != 256) SRB_FAIL("gemm_bf16_pair_grouped: tiles of %d slots are not 128 or 256", tile_slots);
+  if (k <= 0 || k % 8 != 0 || features % 8 != 0 || ldo % 8 != 0)
+    SRB_FAIL("gemm_bf16_pair_grouped: the sizes %d, %d and the pitch %d must be positive multiples of 8", k, features, ldo);
+  if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15) SRB_FAIL("gemm_bf16_pair_grouped: operands must be 16-byte aligned");
+  if (mode != PAIR_EPI_F32 && mode != PAIR_EPI_SILU && mode != PAIR_EPI_ACT)
+    SRB_FAIL("gemm_bf16_pair_grouped: mode %d is not float, gated or activated", mode);
+  if (mode != PAIR_EPI_F32 && (activation < 0 || activation >= SRB_ACT_COUNT))
+    SRB_FAIL("gemm_bf16_pair_grouped: unknown activation %d", activation);
+  if (!plan || experts <= 0 || expert_rows <= 0) SRB_FAIL("gemm_bf16_pair_grouped: a plan and the experts' sizes are needed");
+  if ((mode == PAIR_EPI_SILU ? up_row_offset + features : features) > expert_rows)
+    SRB_FAIL("gemm_bf16_pair_grouped: %d features do not fit the %d rows of an expert", features, expert_rows);
+  if (ldo < features) SRB_FAIL("gemm_bf16_pair_grouped: output pitch %d is smaller than %d features", ldo, features);
+  CUtensorMap map_w, map_x, map_out;
+  if (make_map(&map_w, w, (long long)experts * expert_rows, k, k, PAIR_ROWS) != SRB_OK || make_map(&map_x, x, slots, k, k, PAIR_ROWS) != SRB_OK ||
+      make_map(&map_out, out, slots, features, ldo, 32, mode == PAIR_EPI_F32) != SRB_OK)
+    return SRB_ERR_INVALID;
+  const int features_per_tile = mode == PAIR_EPI_SILU ? PAIR_ROWS : 2 * PAIR_ROWS;
+  PairArgs args = {};
+  args.out = out; args.tokens = slots; args.features = features; args.k = k; args.ldo = ldo;
+  args.up_row_offset = up_row_offset; args.activation = activation; args.act_param = act_param; args.error_word = error_word;
+  args.plan = plan; args.tile_slots = tile_slots; args.experts = experts; args.expert_rows = expert_rows; args.slot_weight = slot_weight;
+  args.tiles_f = (features + features_per_tile - 1) / features_per_tile;
+  const int max_tiles = (slots / tile_slots + experts) * args.tiles_f;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (mode == PAIR_EPI_F32) return launch_pair<PAIR_EPI_F32, true>(map_w, map_x, map_out, args, max_tiles, s);
+  if (mode == PAIR_EPI_SILU) return launch_pair<PAIR_EPI_SILU, true>(map_w, map_x, map_out, args, max_tiles, s);
+  return launch_pair<PAIR_EPI_BF16, true>(map_w, map_x, map_out, args, max_tiles, s);
 }

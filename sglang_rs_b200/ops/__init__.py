@@ -909,7 +909,7 @@ def head_linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, gate: 
 # --------------------------------------------------------------------------- routed experts
 
 #: bfloat16 steps with many choices per expert run the experts' two products on the grouped mode of the tcgen05
-#: kernel (csrc/gemm_bf16.cu) over rows gathered into slot order; SRB_GROUPED_EXPERTS=0 keeps the mma.sync tiles
+#: kernel for many rows (csrc/gemm_bf16_pair.cu) over rows gathered into slot order; SRB_GROUPED_EXPERTS=0 keeps the mma.sync tiles
 GROUPED_EXPERTS = os.environ.get("SRB_GROUPED_EXPERTS", "1") not in ("0", "off", "false")
 #: from this many rows on the router's logits come from the product kernels (every block of the fused router kernel reads
 #: the whole router matrix: 94 us at 2,048 rows and 64 experts of width 2,048 against the product's few)
@@ -952,8 +952,8 @@ def routed_experts(h: torch.Tensor, router: torch.Tensor, w_gate_up: torch.Tenso
 
     The two products: float32 and odd sizes on FFMA or 64 x 64 mma tiles; bfloat16 on mma.sync tiles with asynchronous
     copies, or, where a step has many choices per expert (tiles of 128 slots), on tcgen05 tensor cores through the
-    grouped mode of :func:`gemm_bf16`'s kernel: the rows are gathered into slot order first, so that a tile's operand is
-    128 consecutive rows that TMA can fetch."""
+    grouped mode of :func:`gemm_bf16_pair`'s kernel: the rows are gathered into slot order first, so that a tile's operand is
+    consecutive rows that TMA can fetch."""
     _need(h, "h"); _need(router, "router", h.dtype); _need(w_gate_up, "w_gate_up", h.dtype); _need(w_down, "w_down", h.dtype)
     rows, width = h.shape
     experts, inner = w_gate_up.shape[0], w_gate_up.shape[1] // (2 if gated else 1)
@@ -1009,18 +1009,17 @@ def routed_experts(h: torch.Tensor, router: torch.Tensor, w_gate_up: torch.Tenso
     _check(lib, lib.srb_moe_plan_of(_ptr(chosen), rows, top, experts, tile_slots, _ptr(plan), _ptr(slot_row),
                                     _ptr(entry_slot), _ptr(weights), _ptr(slot_weight), _ptr(error_word), stream))
     if grouped:
-        product = load_library("gemm_bf16")
-        max_tiles = lib.srb_moe_max_tiles_of(rows, top, experts, tile_slots)
+        product = load_library("gemm_bf16_pair")
         gathered = torch.empty((entries, width), dtype=h.dtype, device=device)
         # the plan's last offset is the number of slots handed out (choices of experts without tensors get none)
         used = ctypes.c_void_p(plan.data_ptr() + 4 * (1 + experts))
         _check(lib, lib.srb_moe_gather_used(_ptr(h), _ptr(slot_row), entries, width, _ptr(gathered), used, code, stream))
-        _check(product, product.srb_gemm_bf16_grouped(
-            _ptr(gathered), _ptr(w_gate_up), _ptr(act), _ptr(plan), max_tiles, tile_slots, entries, experts,
+        _check(product, product.srb_gemm_bf16_pair_grouped(
+            _ptr(gathered), _ptr(w_gate_up), _ptr(act), _ptr(plan), tile_slots, entries, experts,
             (2 if gated else 1) * inner, inner, width, inner, inner if gated else 0, GEMM_MODES["gated" if gated else "act"],
             act_code, act_param, _ptr(slot_weight), _ptr(error_word), stream))
-        _check(product, product.srb_gemm_bf16_grouped(
-            _ptr(act), _ptr(w_down), _ptr(y), _ptr(plan), max_tiles, tile_slots, entries, experts, width, width, inner, width, 0,
+        _check(product, product.srb_gemm_bf16_pair_grouped(
+            _ptr(act), _ptr(w_down), _ptr(y), _ptr(plan), tile_slots, entries, experts, width, width, inner, width, 0,
             GEMM_MODES["f32"], 0, ctypes.c_float(0.0), None, _ptr(error_word), stream))
     else:
         element = h.element_size()

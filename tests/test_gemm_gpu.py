@@ -163,3 +163,44 @@ def test_gate_up_takes_the_kernel_of_its_row_count(tokens, activation):
     gate_up = pm.plain_linear(x.double(), w.double())
     want = GATED[activation](gate_up[:, :inner], gate_up[:, inner:])
     assert got.shape == (tokens, inner) and relative_error(got, want) < 1e-2
+
+
+@pytest.mark.parametrize("tile_slots", [128, 256])
+@pytest.mark.parametrize("features,k", [(136, 72), (264, 200), (1024, 64)])
+@pytest.mark.parametrize("mode", ["f32", "gated", "act"])
+def test_grouped_products_on_pairs_of_ctas(mode, features, k, tile_slots):
+    """One weight matrix per expert over slots in expert order, experts of every awkward size: none, one slot, a box of 32
+    and one more, a CTA's half, a tile and one more or less; only the experts' own slots are written."""
+    import ctypes
+    from sglang_rs_b200.csrc.build import load_library
+    counts = [0, 1, 32, 33, 127, 128, 129, 255, 256, 257, 0, 300, 5]
+    experts, slots = len(counts), sum(counts)
+    expert_rows = 2 * features if mode == "gated" else features
+    g = torch.Generator().manual_seed(features + k)
+    x = torch.randn(slots, k, generator=g).to(torch.bfloat16)
+    w = (torch.randn(experts, expert_rows, k, generator=g) * 0.5).to(torch.bfloat16)
+    weight = torch.rand(slots, generator=g) + 0.5
+    first = [sum(counts[:e]) for e in range(experts + 1)]
+    tiles = [(e, first[e] + t) for e in range(experts) for t in range(0, counts[e], tile_slots)]
+    plan = torch.tensor([len(tiles), *first, *[v for tile in tiles for v in tile]], dtype=torch.int32)
+    pitch = features + 8
+    out = torch.full((slots + 3, pitch), 7.0, dtype=torch.float32 if mode == "f32" else torch.bfloat16, device=DEV)
+    word, lib = ops.new_error_word(DEV), load_library("gemm_bf16_pair")
+    held = [t.to(DEV) for t in (x, w, plan, weight)]
+    address = [ctypes.c_void_p(t.data_ptr()) for t in held]
+    status = lib.srb_gemm_bf16_pair_grouped(
+        address[0], address[1], ctypes.c_void_p(out.data_ptr()), address[2], tile_slots, slots, experts, expert_rows, features, k,
+        pitch, features if mode == "gated" else 0, ops.GEMM_MODES[mode], 0, ctypes.c_float(0.0),
+        None if mode == "f32" else address[3], ctypes.c_void_p(word.data_ptr()), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert status == 0, lib.srb_last_error()
+    ops.raise_on_error_word(word)
+    want = torch.cat([x[first[e]:first[e + 1]].double() @ w[e].double().T for e in range(experts)])
+    if mode == "gated":
+        want = want * weight.double()[:, None]
+        want = GATED["silu"](want[:, :features], want[:, features:])
+    elif mode == "act":
+        want = want * weight.double()[:, None]
+        want = want * torch.sigmoid(want)
+    # 32-bit sums of exact products; bfloat16 results round to 2^-9 of themselves
+    assert relative_error(out[:slots, :features], want) < (1e-5 if mode == "f32" else 5e-3)
+    assert torch.all(out[slots:] == 7.0) and torch.all(out[:, features:] == 7.0)
