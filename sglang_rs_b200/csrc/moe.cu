@@ -244,23 +244,38 @@ __global__ void moe_plan_kernel(const int* __restrict__ chosen, int entries, int
   srb_grid_dependency_wait();
   for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
   __syncthreads();
+#pragma unroll 4
   for (int i = threadIdx.x; i < entries; i += blockDim.x) {
     const int e = chosen[i];
     if (e >= 0 && e < experts) atomicAdd(&count[e], 1);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  // running sums of the experts' slots and tiles by one warp, 32 experts at a time
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
     int slots = 0, tiles = 0;
-    for (int e = 0; e < experts; ++e) {
-      first[e] = slots;
-      tile_first[e] = tiles;
-      slots += count[e];
-      tiles += (count[e] + tile_rows - 1) / tile_rows;
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      const int mine = e0 + lane < experts ? count[e0 + lane] : 0;
+      const int mine_tiles = (mine + tile_rows - 1) / tile_rows;
+      int run = mine, run_tiles = mine_tiles;
+#pragma unroll
+      for (int offset = 1; offset < 32; offset <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, run, offset), b = __shfl_up_sync(0xffffffffu, run_tiles, offset);
+        if (lane >= offset) { run += a; run_tiles += b; }
+      }
+      if (e0 + lane < experts) {
+        first[e0 + lane] = slots + run - mine;
+        tile_first[e0 + lane] = tiles + run_tiles - mine_tiles;
+      }
+      slots += __shfl_sync(0xffffffffu, run, 31);
+      tiles += __shfl_sync(0xffffffffu, run_tiles, 31);
     }
-    first[experts] = slots;
-    tile_first[experts] = tiles;
-    plan[0] = tiles <= max_tiles ? tiles : max_tiles;
-    if (tiles > max_tiles) atomicOr(error_word, SRB_FLAG_BAD_SLOT);
+    if (lane == 0) {
+      first[experts] = slots;
+      tile_first[experts] = tiles;
+      plan[0] = tiles <= max_tiles ? tiles : max_tiles;
+      if (tiles > max_tiles) atomicOr(error_word, SRB_FLAG_BAD_SLOT);
+    }
   }
   __syncthreads();
   int* offsets = plan + 1;
@@ -278,6 +293,7 @@ __global__ void moe_plan_kernel(const int* __restrict__ chosen, int entries, int
     count[e] = 0;                       // becomes the number of the expert's slots handed out so far
   }
   __syncthreads();
+#pragma unroll 4
   for (int i = threadIdx.x; i < entries; i += blockDim.x) {
     const int e = chosen[i];
     if (e < 0 || e >= experts) { entry_slot[i] = -1; continue; }
@@ -629,15 +645,69 @@ extern "C" int srb_moe_down(const void* act, const void* w_down, const int* plan
 // it is the first term of the sum.  `chosen` and `input` (both or neither): a choice whose number is `experts` or more
 // names an expert that returns its input, so its term is weight * input[row] (such choices have no slot in the plan).
 // `base_gate` (float [rows], or null) multiplies the shared term; `weights` null: the results are summed as they are.
+//
+// Reads top rows of 32-bit results for every row it writes, so memory bounds it: rows of whole groups of four entries move 16 bytes
+// a thread, the slots and weights of a row are read once, and up to eight results are in flight before they are
+// added (in the order of the choices).
 template <typename T>
+__device__ __forceinline__ float4 moe_load_four(const T* p);
+template <>
+__device__ __forceinline__ float4 moe_load_four<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <>
+__device__ __forceinline__ float4 moe_load_four<__nv_bfloat16>(const __nv_bfloat16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+template <typename T, bool WIDE>
 __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ entry_slot,
                                    const float* __restrict__ weights, int top, int width, float* __restrict__ out,
                                    const float* __restrict__ base, const int* __restrict__ chosen, int experts,
                                    const T* __restrict__ input, const float* __restrict__ base_gate) {
+  constexpr int FLIGHT = 8;
+  __shared__ int s_slot[32];
+  __shared__ float s_weight[32];
   srb_launch_dependents();
   srb_grid_dependency_wait();
   const int row = blockIdx.x;
   const float gate = base_gate ? base_gate[row] : 1.0f;
+  if (WIDE) {
+    // -1: no slot and no term; -2: the expert returns its input
+    if (threadIdx.x < top) {
+      const size_t at = (size_t)row * top + threadIdx.x;
+      const int slot = entry_slot[at];
+      s_slot[threadIdx.x] = slot >= 0 ? slot : (input && chosen[at] >= experts ? -2 : -1);
+      s_weight[threadIdx.x] = weights ? weights[at] : 1.0f;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x * 4; i < width; i += blockDim.x * 4) {
+      float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (base) {
+        sum = moe_load_four(base + (size_t)row * width + i);
+        sum = make_float4(sum.x * gate, sum.y * gate, sum.z * gate, sum.w * gate);
+      }
+      for (int first = 0; first < top; first += FLIGHT) {
+        float4 v[FLIGHT];
+#pragma unroll
+        for (int k = 0; k < FLIGHT; ++k)
+          if (first + k < top) {
+            const int slot = s_slot[first + k];
+            if (slot >= 0) v[k] = moe_load_four(y + (size_t)slot * width + i);
+            else if (slot == -2) v[k] = moe_load_four(input + (size_t)row * width + i);
+          }
+#pragma unroll
+        for (int k = 0; k < FLIGHT; ++k)
+          if (first + k < top && s_slot[first + k] != -1) {
+            const float w = s_weight[first + k];
+            sum = make_float4(fmaf(w, v[k].x, sum.x), fmaf(w, v[k].y, sum.y), fmaf(w, v[k].z, sum.z), fmaf(w, v[k].w, sum.w));
+          }
+      }
+      *reinterpret_cast<float4*>(out + (size_t)row * width + i) = sum;
+    }
+    return;
+  }
   for (int i = threadIdx.x; i < width; i += blockDim.x) {
     float sum = base ? base[(size_t)row * width + i] * gate : 0.f;
     for (int k = 0; k < top; ++k) {
@@ -650,19 +720,31 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __res
   }
 }
 
+template <typename T>
+static cudaError_t launch_moe_combine(const float* y, const int* entry_slot, const float* weights, int rows, int top, int width,
+                                      float* out, const float* base, const int* chosen, int experts, const T* input,
+                                      const float* base_gate, cudaStream_t s) {
+  const bool wide = width % 4 == 0 && top <= 32 && (((uintptr_t)y | (uintptr_t)out | (uintptr_t)base) & 15) == 0 &&
+                    ((uintptr_t)input & (4 * sizeof(T) - 1)) == 0;
+  const dim3 block(width >= 1024 ? 256 : 128);
+  return wide ? srb_launch(moe_combine_kernel<T, true>, dim3(rows), block, 0, s, y, entry_slot, weights, top, width, out, base,
+                           chosen, experts, input, base_gate)
+              : srb_launch(moe_combine_kernel<T, false>, dim3(rows), block, 0, s, y, entry_slot, weights, top, width, out, base,
+                           chosen, experts, input, base_gate);
+}
+
 extern "C" int srb_moe_combine_identity(const float* y, const int* entry_slot, const float* weights, int rows, int top,
                                         int width, float* out, const float* base, const int* chosen, int experts,
                                         const void* input, const float* base_gate, int dtype, void* stream) {
   if (rows <= 0) return SRB_OK;
   if (!weights && input) SRB_FAIL("moe_combine: experts that return their input need the weights");
   if ((chosen == nullptr) != (input == nullptr)) SRB_FAIL("moe_combine: the choices and the experts' input come together");
-  const dim3 block(width >= 1024 ? 256 : 128);
   if (dtype == SRB_DTYPE_F32)
-    SRB_CUDA_CALL(srb_launch(moe_combine_kernel<float>, dim3(rows), block, 0, (cudaStream_t)stream, y, entry_slot, weights, top,
-                             width, out, base, chosen, experts, (const float*)input, base_gate));
+    SRB_CUDA_CALL(launch_moe_combine(y, entry_slot, weights, rows, top, width, out, base, chosen, experts, (const float*)input,
+                                     base_gate, (cudaStream_t)stream));
   else if (dtype == SRB_DTYPE_BF16)
-    SRB_CUDA_CALL(srb_launch(moe_combine_kernel<__nv_bfloat16>, dim3(rows), block, 0, (cudaStream_t)stream, y, entry_slot,
-                             weights, top, width, out, base, chosen, experts, (const __nv_bfloat16*)input, base_gate));
+    SRB_CUDA_CALL(launch_moe_combine(y, entry_slot, weights, rows, top, width, out, base, chosen, experts,
+                                     (const __nv_bfloat16*)input, base_gate, (cudaStream_t)stream));
   else
     SRB_FAIL("moe_combine: unknown dtype %d", dtype);
   SRB_LAUNCH_CHECK("moe_combine");
