@@ -80,33 +80,48 @@ __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_pick_kernel(const float* __restrict__ logits, int vocab, int stride, const float* __restrict__ temperature,
                    const float* __restrict__ uniform, const float* __restrict__ chunk_max,
                    const int* __restrict__ chunk_arg, const float* __restrict__ chunk_sum, int* __restrict__ out) {
-  __shared__ float part_sum[SAMPLE_THREADS];
+  __shared__ __align__(16) float part_sum[SAMPLE_THREADS];
+  __shared__ float part_max[SAMPLE_CHUNKS], chunk_mass[SAMPLE_CHUNKS];
+  __shared__ int part_arg[SAMPLE_CHUNKS];
   __shared__ float sh_max, sh_target, sh_prefix;
   __shared__ int sh_chunk;
   const int row = blockIdx.x;
   const float* l = logits + (size_t)row * stride;
   const float temp = temperature ? temperature[row] : 0.f;
   const size_t base = (size_t)row * SAMPLE_CHUNKS;
+  // One thread adds and compares in chunk order (the order decides the token); what it reads, the chunks' masses under the row's
+  // maximum among it, is brought and computed by a thread per chunk.  (By one thread, exponentials and all, the kernel
+  // took 25 us for 64 rows; 12 us now.)
+  if (threadIdx.x < SAMPLE_CHUNKS) {
+    part_max[threadIdx.x] = chunk_max[base + threadIdx.x];
+    part_arg[threadIdx.x] = chunk_arg[base + threadIdx.x];
+  }
+  __syncthreads();
+  float best = part_max[0];
+  int best_index = part_arg[0];
+#pragma unroll 16
+  for (int c = 1; c < SAMPLE_CHUNKS; ++c)
+    if (part_max[c] > best) {                     // chunks are in index order: ties keep the lower index
+      best = part_max[c];
+      best_index = part_arg[c];
+    }
+  if (temp > 0.f && threadIdx.x < SAMPLE_CHUNKS)
+    chunk_mass[threadIdx.x] = chunk_sum[base + threadIdx.x] * expf((part_max[threadIdx.x] - best) / temp);
+  __syncthreads();
   if (threadIdx.x == 0) {
-    float best = chunk_max[base];
-    int best_index = chunk_arg[base];
-    for (int c = 1; c < SAMPLE_CHUNKS; ++c)
-      if (chunk_max[base + c] > best) {           // chunks are in index order: ties keep the lower index
-        best = chunk_max[base + c];
-        best_index = chunk_arg[base + c];
-      }
     sh_max = best;
     sh_chunk = -1;
     if (!(temp > 0.f)) {
       out[row] = best_index == 0x7fffffff ? 0 : best_index;
     } else {
       float total = 0.f;
-      for (int c = 0; c < SAMPLE_CHUNKS; ++c) total += chunk_sum[base + c] * expf((chunk_max[base + c] - best) / temp);
+#pragma unroll 16
+      for (int c = 0; c < SAMPLE_CHUNKS; ++c) total += chunk_mass[c];
       const float target = uniform[row] * total;
       float running = 0.f;
       int owner = -1;
       for (int c = 0; c < SAMPLE_CHUNKS; ++c) {
-        const float mass = chunk_sum[base + c] * expf((chunk_max[base + c] - best) / temp);
+        const float mass = chunk_mass[c];
         if (target < running + mass) {
           owner = c;
           break;
@@ -137,12 +152,16 @@ sample_pick_kernel(const float* __restrict__ logits, int vocab, int stride, cons
   if (threadIdx.x == 0) {
     float running = sh_prefix;
     int owner = -1;
-    for (int t = 0; t < (int)blockDim.x; ++t) {
-      if (sh_target < running + part_sum[t]) {
-        owner = t;
-        break;
+    const float target = sh_target;
+    for (int t = 0; t < SAMPLE_THREADS && owner < 0; t += 4) {
+      const float4 four = *reinterpret_cast<const float4*>(part_sum + t);
+      const float part[4] = {four.x, four.y, four.z, four.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (owner >= 0) continue;
+        if (target < running + part[e]) owner = t + e;
+        else running += part[e];
       }
-      running += part_sum[t];
     }
     if (owner < 0) {                               // take the last token of the chunk that has p > 0
       int last = end - 1;
@@ -179,30 +198,34 @@ sample_pick_kernel(const float* __restrict__ logits, int vocab, int stride, cons
 // a probability tau and a number n: all items above tau and the first n, in index order, of
 // those equal to tau.  The item at which a running count or a running mass crosses a threshold
 // is found by a radix search over the bits of p (11 + 11 + 10 bits): the histogram of the first
-// 11 bits (counts and masses per bin) is built once per row, together with the p themselves,
-// which go to scratch memory; each search then refines inside one bin with two light passes
-// over the stored p.  The position among equal items follows by division.  Masses are integers
-// (p * 2^40, rounded), so sums do not depend on the order in which threads add them and a row's
-// token does not depend on timing.  Up to eight blocks per row (a thread-block cluster) share the
-// passes that build the first histogram; one of them does the searches.
+// 11 bits (counts and masses per bin) is built once per row, together with the p themselves;
+// each search then refines inside one bin with two light passes over p.  The position among equal
+// items follows by division.  Masses are integers (p * 2^40, rounded), so sums do not depend on the
+// order in which threads add them and a row's token does not depend on timing.
+//
+// The blocks of a row form a thread-block cluster (up to eight).  Each keeps its slice of the row's
+// probabilities in its own shared memory from the first pass to the last (a slice of a vocabulary too long for
+// eight blocks' memory lies in scratch memory instead), adds the slice to its own histograms, and reads the others'
+// histograms through the cluster, so every block knows every search's outcome and none waits for one that searches
+// for all.  Latency bounds it: 32 rows of 151,936 entries take 56 us without a cut and 67 to 82 us with one or two, where one
+// block searched alone over probabilities in scratch memory 153 to 179 us; a search is 14 us of cluster barriers and scans.
 #define FS_THREADS 1024
 #define FS_BINS 2048
 #define FS_BATCH 8          // loads of a thread in flight at once
-#define FS_QUADS 4          // the same for 16-byte loads of the stored probabilities
+#define FS_MAX_BLOCKS 8     // blocks of a row
 typedef unsigned long long u64;
 
 __device__ __forceinline__ u64 fs_mass(float p) { return __float2ull_rn(p * 1099511627776.0f); }   // p * 2^40
 
-struct FsShared {
+struct __align__(16) FsShared {
   u64 first_mass[FS_BINS];        // histogram of the first 11 bits of p: mass and count per bin
-  u64 mass[FS_BINS + 1];          // histogram of the level being refined; the last entry is a mailbox
-  u64 totals[99];
+  u64 mass[FS_BINS + 2];          // histogram of the level being refined; entry FS_BINS is a mailbox
+  u64 totals[100];
   unsigned first_count[FS_BINS];
   unsigned count[FS_BINS];
-  unsigned found[4];
+  unsigned found[4];              // what fs_scan found: the bin, the count above it, its own count; [3]: a mailbox
   float warp_max[FS_THREADS / 32];
   float slice_max;
-  int index;
 };
 
 // loads from the shared memory of another block of the cluster
@@ -212,12 +235,29 @@ __device__ __forceinline__ unsigned fs_peer_u32(const unsigned* mine, unsigned r
   asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(remote) : "memory");
   return v;
 }
-__device__ __forceinline__ u64 fs_peer_u64(const u64* mine, unsigned rank) {
-  unsigned local = (unsigned)__cvta_generic_to_shared(mine), remote;
-  u64 v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
-  asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(remote) : "memory");
-  return v;
+// two neighbouring bins of every block's histogram, all loads under way before the first sum
+__device__ __forceinline__ void fs_peer_bins(const unsigned* count, const u64* mass, int blocks, u64 (&c)[2], u64 (&m)[2]) {
+  const unsigned local_c = (unsigned)__cvta_generic_to_shared(count), local_m = (unsigned)__cvta_generic_to_shared(mass);
+  unsigned pc[FS_MAX_BLOCKS][2];
+  u64 pm[FS_MAX_BLOCKS][2];
+#pragma unroll
+  for (int b = 0; b < FS_MAX_BLOCKS; ++b) {
+    pc[b][0] = pc[b][1] = 0u;
+    pm[b][0] = pm[b][1] = 0ull;
+    if (b < blocks) {
+      unsigned remote;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_c), "r"(b));
+      asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];" : "=r"(pc[b][0]), "=r"(pc[b][1]) : "r"(remote));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_m), "r"(b));
+      asm volatile("ld.shared::cluster.v2.u64 {%0, %1}, [%2];" : "=l"(pm[b][0]), "=l"(pm[b][1]) : "r"(remote));
+    }
+  }
+  c[0] = c[1] = m[0] = m[1] = 0ull;
+#pragma unroll
+  for (int b = 0; b < FS_MAX_BLOCKS; ++b) {
+    c[0] += pc[b][0]; c[1] += pc[b][1];
+    m[0] += pm[b][0]; m[1] += pm[b][1];
+  }
 }
 
 // sum over the block; every thread gets it
@@ -238,37 +278,40 @@ __device__ __forceinline__ u64 fs_block_sum(u64 v, u64* scratch /* 33 */) {
   return scratch[32];
 }
 
-// One item per lane (or none) into a histogram.  Called by whole warps.  Lanes that fall into the same
-// bin as the first lane still waiting add once, through that lane (up to three such groups: a flat row
-// puts a whole warp into one or two bins, and thirty-two additions to one address would queue up);
-// the lanes left after that add for themselves (a peaked row spreads a warp over many bins).
+// A bin's mass as two 32-bit words: shared memory adds those in one step, while an addition of 64 bits is a loop of compare and
+// swap that starts over whenever another warp was quicker.  (A row's first histogram, most of whose items share a
+// dozen bins, took 80 us that way, whatever the number of blocks.)
+__device__ __forceinline__ void fs_add_mass(u64* bin, u64 w) {
+  unsigned* word = reinterpret_cast<unsigned*>(bin);
+  const unsigned low = (unsigned)w;
+  const unsigned carry = atomicAdd(word, low) + low < low ? 1u : 0u;
+  const unsigned high = (unsigned)(w >> 32) + carry;
+  if (high) atomicAdd(word + 1, high);
+}
+
+// One item per lane (or none) into a histogram.  Called by whole warps.  Lanes that fall into the same bin as the first lane add
+// once, through that lane, if there are many of them (a flat row puts a whole warp into one bin, and thirty-two additions to one
+// address queue up); the others add for themselves.
 __device__ __forceinline__ void fs_add(unsigned* count, u64* mass, bool mine, unsigned bin, u64 w) {
-  unsigned waiting = __ballot_sync(0xffffffffu, mine);
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int round = 0; round < 3; ++round) {
-    if (waiting == 0) return;
-    const int leader = __ffs(waiting) - 1;
-    const unsigned lead_bin = __shfl_sync(0xffffffffu, bin, leader);
-    const bool in_group = ((waiting >> lane) & 1u) && bin == lead_bin;
-    const unsigned group = __ballot_sync(0xffffffffu, in_group);
-    if (__popc(group) >= 4) {
-      const unsigned lo = __reduce_add_sync(0xffffffffu, in_group ? (unsigned)(w & 0xFFFFFu) : 0u);
-      const unsigned mid = __reduce_add_sync(0xffffffffu, in_group ? (unsigned)((w >> 20) & 0xFFFFFu) : 0u);
-      const unsigned hi = __reduce_add_sync(0xffffffffu, in_group ? (unsigned)(w >> 40) : 0u);
-      if (lane == leader) {
-        atomicAdd(&count[lead_bin], (unsigned)__popc(group));
-        atomicAdd(&mass[lead_bin], (u64)lo + ((u64)mid << 20) + ((u64)hi << 40));
-      }
-    } else if (in_group) {
-      atomicAdd(&count[bin], 1u);
-      atomicAdd(&mass[bin], w);
+  const unsigned waiting = __ballot_sync(0xffffffffu, mine);
+  if (waiting == 0) return;
+  const int lane = threadIdx.x & 31, leader = __ffs(waiting) - 1;
+  const unsigned lead_bin = __shfl_sync(0xffffffffu, bin, leader);
+  const bool in_group = mine && bin == lead_bin;
+  const unsigned group = __ballot_sync(0xffffffffu, in_group);
+  if (__popc(group) >= 8) {
+    const unsigned lo = __reduce_add_sync(0xffffffffu, in_group ? (unsigned)(w & 0xFFFFFu) : 0u);
+    const unsigned mid = __reduce_add_sync(0xffffffffu, in_group ? (unsigned)((w >> 20) & 0xFFFFFu) : 0u);
+    const unsigned hi = __reduce_add_sync(0xffffffffu, in_group ? (unsigned)(w >> 40) : 0u);
+    if (lane == leader) {
+      atomicAdd(&count[lead_bin], (unsigned)__popc(group));
+      fs_add_mass(&mass[lead_bin], (u64)lo + ((u64)mid << 20) + ((u64)hi << 40));
     }
-    waiting &= ~group;
+    mine = mine && !in_group;
   }
-  if ((waiting >> lane) & 1u) {
+  if (mine) {
     atomicAdd(&count[bin], 1u);
-    atomicAdd(&mass[bin], w);
+    fs_add_mass(&mass[bin], w);
   }
 }
 
@@ -276,23 +319,32 @@ __device__ __forceinline__ void fs_add(unsigned* count, u64* mass, bool mine, un
 #define FS_BY_MASS 1
 #define FS_BY_KEY 2
 
-// Walks a histogram from its top bin down.  BY_COUNT / BY_MASS: the bin in which the running count or
-// mass (starting at `base`, what lies above the histogram's range) first exceeds `want`.  BY_KEY: the
-// bin `want`.  Leaves the bin in found[0], the count of the bins above it in found[1] and their mass
-// in the mailbox; every thread reads them after the call.
+// Walks a histogram (that of a row: `blocks` > 1 adds up the blocks' own) from its top bin down.  BY_COUNT / BY_MASS: the bin in
+// which the running count or mass (starting at `base`, what lies above the histogram's range) first exceeds `want`.
+// BY_KEY: the bin `want`.  Leaves the bin in found[0], the count of the bins above it in found[1], its own count in found[2] and
+// the mass of the bins above it in the mailbox; every thread reads them after the call.
 template <int MODE>
-__device__ void fs_scan(const unsigned* count, const u64* mass, int nbins, u64 want, u64 base, FsShared& sh) {
+__device__ void fs_scan(const unsigned* count, const u64* mass, int blocks, int nbins, u64 want, u64 base, FsShared& sh) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) {                        // what holds if no bin is found (a row of NaN)
+  // thread t owns bins nbins - 1 - 2t and nbins - 2 - 2t; an inclusive scan over the threads, in the order
+  // of falling bins, tells each what lies above its bins
+  const int b0 = nbins - 1 - 2 * (int)threadIdx.x, b1 = b0 - 1;
+  u64 c0 = 0, c1 = 0, m0 = 0, m1 = 0;
+  if (b1 >= 0) {                                 // nbins is even: both or none
+    if (blocks == 1) {
+      c0 = count[b0]; c1 = count[b1]; m0 = mass[b0]; m1 = mass[b1];
+    } else {
+      u64 c[2], m[2];
+      fs_peer_bins(&count[b1], &mass[b1], blocks, c, m);     // b1 is even: both on a border of two
+      c0 = c[1]; c1 = c[0]; m0 = m[1]; m1 = m[0];
+    }
+  }
+  if (threadIdx.x == 0) {                        // what holds if no bin is found (a row of NaN): bin 0
     sh.found[0] = 0;
     sh.found[1] = 0;
     sh.mass[FS_BINS] = 0;
   }
-  // thread t owns bins nbins - 1 - 2t and nbins - 2 - 2t; an inclusive scan over the threads, in the order
-  // of falling bins, tells each what lies above its bins
-  const int b0 = nbins - 1 - 2 * (int)threadIdx.x, b1 = b0 - 1;
-  const u64 c0 = b0 >= 0 ? (u64)count[b0] : 0ull, c1 = b1 >= 0 ? (u64)count[b1] : 0ull;
-  const u64 m0 = b0 >= 0 ? mass[b0] : 0ull, m1 = b1 >= 0 ? mass[b1] : 0ull;
+  if (b1 == 0) sh.found[2] = (unsigned)c1;
   u64 run_c = c0 + c1, run_m = m0 + m1;
 #pragma unroll
   for (int offset = 1; offset < 32; offset <<= 1) {
@@ -326,10 +378,12 @@ __device__ void fs_scan(const unsigned* count, const u64* mass, int nbins, u64 w
   if (first) {
     sh.found[0] = (unsigned)b0;
     sh.found[1] = (unsigned)start_c;
+    sh.found[2] = (unsigned)c0;
     sh.mass[FS_BINS] = start_m;
   } else if (second) {
     sh.found[0] = (unsigned)b1;
     sh.found[1] = (unsigned)(start_c + c0);
+    sh.found[2] = (unsigned)c1;
     sh.mass[FS_BINS] = start_m + m0;
   }
   __syncthreads();
@@ -344,9 +398,9 @@ struct FsCrossing {
 
 // BY_COUNT / BY_MASS: the item, in descending order of p, at which the running count or the running
 // mass first exceeds `want` (before <= want < before + own); the caller guarantees that it exists.
-// BY_KEY: the probability with the bits `want`.  `p` is the row of stored probabilities.
+// BY_KEY: the probability with the bits `want`.  `p` is this block's slice, `n` its length.
 template <int MODE>
-__device__ FsCrossing fs_search(const float* __restrict__ p, int vocab, u64 want, FsShared& sh) {
+__device__ FsCrossing fs_search(const float* __restrict__ p, int n, int blocks, u64 want, FsShared& sh) {
   FsCrossing c;
   c.above = 0;
   c.mass_above = 0;
@@ -359,43 +413,37 @@ __device__ FsCrossing fs_search(const float* __restrict__ p, int vocab, u64 want
     const u64 target = MODE == FS_BY_KEY ? (u64)(((unsigned)want >> shift) & ((1u << bits) - 1)) : want;
     const u64 base = MODE == FS_BY_COUNT ? c.above : c.mass_above;
     if (level == 0) {
-      fs_scan<MODE>(sh.first_count, sh.first_mass, 1 << bits, target, base, sh);
+      // every block holds the whole row's first histogram
+      fs_scan<MODE>(sh.first_count, sh.first_mass, 1, 1 << bits, target, base, sh);
     } else {
+      if (blocks > 1) srb_cluster_sync();        // the others have read the histogram before
       for (int b = threadIdx.x; b < FS_BINS; b += FS_THREADS) {
         sh.count[b] = 0;
         sh.mass[b] = 0;
       }
       __syncthreads();
-      // the stored row is padded to a multiple of four with values that match no prefix
-      const float4* p4 = reinterpret_cast<const float4*>(p);
-      const int quads = (vocab + 3) >> 2;
-      for (int start = 0; start < quads; start += FS_THREADS * FS_QUADS) {
-        float4 value[FS_QUADS];
+      // whole warps stay together: entries behind the slice match no prefix (the sign bit)
+      for (int start = 0; start < n; start += FS_THREADS * 4) {
+        const int i = start + 4 * (int)threadIdx.x;
+        const float4 value = i < n ? *reinterpret_cast<const float4*>(p + i) : make_float4(-1.f, -1.f, -1.f, -1.f);
+        const unsigned key[4] = {__float_as_uint(value.x), __float_as_uint(value.y), __float_as_uint(value.z), __float_as_uint(value.w)};
+        bool mine[4];
 #pragma unroll
-        for (int j = 0; j < FS_QUADS; ++j) {
-          const int i = start + j * FS_THREADS + (int)threadIdx.x;
-          value[j] = i < quads ? p4[i] : make_float4(-1.f, -1.f, -1.f, -1.f);     // the sign bit never matches a prefix
-        }
+        for (int e = 0; e < 4; ++e) mine[e] = (key[e] >> (32 - fixed_bits)) == prefix;
+        if (!__any_sync(0xffffffffu, mine[0] | mine[1] | mine[2] | mine[3])) continue;
 #pragma unroll
-        for (int j = 0; j < FS_QUADS; ++j) {
-          const float four[4] = {value[j].x, value[j].y, value[j].z, value[j].w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const unsigned key = __float_as_uint(four[e]);
-            const bool mine = (key >> (32 - fixed_bits)) == prefix;
-            fs_add(sh.count, sh.mass, mine, (key >> shift) & ((1u << bits) - 1), fs_mass(four[e]));
-          }
-        }
+        for (int e = 0; e < 4; ++e)
+          fs_add(sh.count, sh.mass, mine[e], (key[e] >> shift) & ((1u << bits) - 1), fs_mass(__uint_as_float(key[e])));
       }
-      __syncthreads();
-      fs_scan<MODE>(sh.count, sh.mass, 1 << bits, target, base, sh);
+      if (blocks > 1) srb_cluster_sync(); else __syncthreads();
+      fs_scan<MODE>(sh.count, sh.mass, blocks, 1 << bits, target, base, sh);
     }
     const unsigned bin = sh.found[0];
     c.above += sh.found[1];
     c.mass_above += sh.mass[FS_BINS];
     prefix = (prefix << bits) | bin;
     fixed_bits += bits;
-    if (level == 2) c.equal = sh.count[bin];
+    if (level == 2) c.equal = sh.found[2];
     __syncthreads();
   }
   c.key = prefix;
@@ -404,30 +452,33 @@ __device__ FsCrossing fs_search(const float* __restrict__ p, int vocab, u64 want
 
 // rows_index (or null: row b is block b) picks the rows of `logits` that are sampled here; the
 // per-row options are indexed by the row.  top_k <= 0 or >= vocab, top_p >= 1 and min_p <= 0
-// switch the cut off.  `stored` holds one row of `vocab` floats per block.
+// switch the cut off.  Grid (blocks per row, rows), the blocks of a row a cluster; a block owns `slice` entries, a multiple of four.
+// SHARED: they stay in its shared memory; otherwise in `stored`, rows of `vocab` floats rounded up to a multiple of four.
+template <bool SHARED>
 __global__ void __launch_bounds__(FS_THREADS)
 sample_filtered_kernel(const float* __restrict__ logits, int vocab, long long stride, const int* __restrict__ rows_index,
                        const float* __restrict__ temperature, const int* __restrict__ top_k,
                        const float* __restrict__ top_p, const float* __restrict__ min_p,
-                       const float* __restrict__ uniform, float* __restrict__ stored, int* __restrict__ out) {
+                       const float* __restrict__ uniform, int slice, float* __restrict__ stored, int* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char fs_raw[];
   FsShared& sh = *reinterpret_cast<FsShared*>(fs_raw);
-  // grid (blocks per row, rows): the blocks of a row form a thread-block cluster.  Each takes a slice of
-  // the vocabulary through the two heavy passes (the maximum; the probabilities and the histogram of
-  // their first bits), block 0 adds the histograms up through the cluster's shared memory and goes on alone.
   const int r = rows_index ? rows_index[blockIdx.y] : blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int blocks = gridDim.x, rank = blockIdx.x;
-  const float* l = logits + (size_t)r * stride;
-  const int pitch = (vocab + 3) & ~3;                 // rows of `stored` start on 16-byte boundaries
-  float* p = stored + (size_t)blockIdx.y * pitch;
+  const float* l = logits + (size_t)r * stride + (size_t)rank * slice;
+  float* p = SHARED ? reinterpret_cast<float*>(fs_raw + sizeof(FsShared))
+                    : stored + (size_t)blockIdx.y * ((vocab + 3) & ~3) + (size_t)rank * slice;
   const float t = temperature[r];
-  const int slice = (pitch + blocks - 1) / blocks;
-  const int slice_begin = min(pitch, rank * slice), slice_end = min(pitch, slice_begin + slice);
-  // the largest scaled logit
+  const int live = max(0, min(slice, vocab - rank * slice));         // entries of the row in this slice
+  const int padded = (live + 3) & ~3;
+  // the largest scaled logit; the raw logits stay where the probabilities will be
   float best = -INFINITY;
 #pragma unroll 8
-  for (int i = slice_begin + threadIdx.x; i < min(slice_end, vocab); i += FS_THREADS) best = fmaxf(best, __fdiv_rn(l[i], t));
+  for (int i = threadIdx.x; i < live; i += FS_THREADS) {
+    const float raw = l[i];
+    if (SHARED) p[i] = raw;
+    best = fmaxf(best, __fdiv_rn(raw, t));
+  }
 #pragma unroll
   for (int offset = 16; offset > 0; offset >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, offset));
   if (lane == 0) sh.warp_max[warp] = best;
@@ -444,41 +495,39 @@ sample_filtered_kernel(const float* __restrict__ logits, int vocab, long long st
     srb_cluster_sync();
     for (int b = 0; b < blocks; ++b) best = fmaxf(best, srb_load_peer_shared(&sh.slice_max, b));
   }
-  // the probabilities, stored for the passes to come, and the histogram of their first 11 bits
-  for (int start = slice_begin; start < slice_end; start += FS_THREADS * FS_BATCH) {
+  // the probabilities, kept for the passes to come, and the histogram of their first 11 bits
+  for (int start = 0; start < padded; start += FS_THREADS * FS_BATCH) {
     float raw[FS_BATCH];
 #pragma unroll
     for (int j = 0; j < FS_BATCH; ++j) {
       const int i = start + j * FS_THREADS + (int)threadIdx.x;
-      raw[j] = i < slice_end && i < vocab ? l[i] : 0.f;
+      raw[j] = i < live ? (SHARED ? p[i] : l[i]) : 0.f;
     }
 #pragma unroll
     for (int j = 0; j < FS_BATCH; ++j) {
+      if (start + j * FS_THREADS >= padded) break;         // the same for the whole block
       const int i = start + j * FS_THREADS + (int)threadIdx.x;
-      const bool live = i < slice_end && i < vocab;
       const float value = expf(__fdiv_rn(raw[j], t) - best);
-      if (i < slice_end) p[i] = live ? value : -1.f;
-      fs_add(sh.first_count, sh.first_mass, live, __float_as_uint(value) >> 21, fs_mass(value));
+      if (i < padded) p[i] = i < live ? value : -1.f;
+      fs_add(sh.first_count, sh.first_mass, i < live, __float_as_uint(value) >> 21, fs_mass(value));
     }
   }
+  __syncthreads();
   if (blocks > 1) {
-    srb_cluster_sync();                              // every block's histogram and slice of `stored` are complete
-    if (rank == 0) {
-      for (int b = threadIdx.x; b < FS_BINS; b += FS_THREADS) {
-        unsigned c = sh.first_count[b];
-        u64 m = sh.first_mass[b];
-        for (int other = 1; other < blocks; ++other) {
-          c += fs_peer_u32(&sh.first_count[b], other);
-          m += fs_peer_u64(&sh.first_mass[b], other);
-        }
-        sh.first_count[b] = c;
-        sh.first_mass[b] = m;
-      }
+    // every block adds up all blocks' first histograms, two bins a thread
+    static_assert(FS_BINS == 2 * FS_THREADS, "two bins a thread");
+    srb_cluster_sync();
+    u64 c[2], m[2];
+    const int bin = 2 * (int)threadIdx.x;
+    fs_peer_bins(&sh.first_count[bin], &sh.first_mass[bin], blocks, c, m);
+    srb_cluster_sync();                                    // everybody has read them
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      sh.first_count[bin + h] = (unsigned)c[h];
+      sh.first_mass[bin + h] = m[h];
     }
-    srb_cluster_sync();                              // nobody leaves while its histogram may still be read
-    if (rank != 0) return;
+    __syncthreads();
   }
-  __syncthreads();                                   // the block reads what was written to `stored`
 
   // a prefix of the sorted order: everything above `key`, and the first `n` of those equal to it
   FsCrossing cut;
@@ -496,7 +545,7 @@ sample_filtered_kernel(const float* __restrict__ logits, int vocab, long long st
   const int k = top_k[r];
   u64 total;
   if (k > 0 && k < vocab) {
-    const FsCrossing c = fs_search<FS_BY_COUNT>(p, vocab, (u64)(k - 1), sh);
+    const FsCrossing c = fs_search<FS_BY_COUNT>(p, live, blocks, (u64)(k - 1), sh);
     const u64 ties = (u64)k - c.above;               // of the items equal to the k-th, those that make k full
     tighten(c, ties);
     total = c.mass_above + ties * fs_mass(__uint_as_float(c.key));
@@ -512,13 +561,13 @@ sample_filtered_kernel(const float* __restrict__ logits, int vocab, long long st
     u64 limit = (u64)ceil((double)tp * (double)total);
     if (limit < 1) limit = 1;
     if (limit > total) limit = total;
-    const FsCrossing c = fs_search<FS_BY_MASS>(p, vocab, limit - 1, sh);
+    const FsCrossing c = fs_search<FS_BY_MASS>(p, live, blocks, limit - 1, sh);
     const u64 w = fs_mass(__uint_as_float(c.key));
     if (w > 0) tighten(c, (limit - c.mass_above + w - 1) / w);
   }
   // min-p: p_i >= p_0 * min_p, and p_0 = 1
   const float mp = min_p[r];
-  if (mp > 0.f) tighten(fs_search<FS_BY_KEY>(p, vocab, (u64)__float_as_uint(1.0f * mp), sh), ~0ull);
+  if (mp > 0.f) tighten(fs_search<FS_BY_KEY>(p, live, blocks, (u64)__float_as_uint(1.0f * mp), sh), ~0ull);
 
   // mass of what is kept, and the pick: the first kept item whose running mass exceeds u * kept
   u64 kept = total;
@@ -526,19 +575,19 @@ sample_filtered_kernel(const float* __restrict__ logits, int vocab, long long st
     if (n > cut.equal) n = cut.equal;
     kept = cut.mass_above + n * fs_mass(__uint_as_float(cut.key));
   }
-  int answer = 0;
-  if (kept > 0) {
+  if (kept == 0) {                                         // the same in every block
+    if (rank == 0 && threadIdx.x == 0) out[r] = 0;
+  } else {
     u64 target = (u64)((double)uniform[r] * (double)kept);
     if (target >= kept) target = kept - 1;
-    const FsCrossing c = fs_search<FS_BY_MASS>(p, vocab, target, sh);
+    const FsCrossing c = fs_search<FS_BY_MASS>(p, live, blocks, target, sh);
     const u64 w = fs_mass(__uint_as_float(c.key));
     u64 which = w > 0 ? (target - c.mass_above) / w : 0;       // among the items equal to it, in index order
     if (c.equal > 0 && which >= c.equal) which = c.equal - 1;
-    // Its index: thread t owns the items t * per .. (t + 1) * per - 1, a scan over the threads' counts of
-    // matches finds the thread that holds the wanted one, and it walks its items again.
-    if (threadIdx.x == 0) sh.index = 0;
-    const int per = ((pitch / 4 + FS_THREADS - 1) / FS_THREADS) * 4;      // a multiple of four: 16-byte loads
-    const int begin = min(pitch, (int)threadIdx.x * per), end = min(pitch, begin + per);
+    // Its index: thread t owns the items t * per .. (t + 1) * per - 1 of the slice, a scan over the threads' counts of
+    // matches (and the blocks' before this one) finds the thread that holds the wanted one, and it walks its items again.
+    const int per = ((padded / 4 + FS_THREADS - 1) / FS_THREADS) * 4;     // a multiple of four: 16-byte loads
+    const int begin = min(padded, (int)threadIdx.x * per), end = min(padded, begin + per);
     unsigned mine = 0;
 #pragma unroll 4
     for (int i = begin; i < end; i += 4) {
@@ -552,24 +601,38 @@ sample_filtered_kernel(const float* __restrict__ logits, int vocab, long long st
       const unsigned other = __shfl_up_sync(0xffffffffu, run, offset);
       if (lane >= offset) run += other;
     }
+    if (lane == 31) sh.totals[warp] = run;                 // (the last scan's readers have passed a barrier)
     __syncthreads();
-    if (lane == 31) sh.count[warp] = run;
-    __syncthreads();
-    unsigned before = run - mine;
-    for (int w2 = 0; w2 < warp; ++w2) before += sh.count[w2];
-    if (mine > 0 && before <= (unsigned)which && (unsigned)which < before + mine) {
-      unsigned rank = before;
+    unsigned before = run - mine, total_here = 0;
+    for (int w2 = 0; w2 < FS_THREADS / 32; ++w2) {
+      const unsigned v = (unsigned)sh.totals[w2];
+      if (w2 < warp) before += v;
+      total_here += v;
+    }
+    unsigned total_row = total_here;
+    if (blocks > 1) {
+      if (threadIdx.x == 0) sh.found[3] = total_here;
+      srb_cluster_sync();
+      total_row = 0;
+      for (int other = 0; other < blocks; ++other) {
+        const unsigned v = fs_peer_u32(&sh.found[3], other);
+        if (other < rank) before += v;
+        total_row += v;
+      }
+    }
+    if ((u64)total_row <= which) {
+      if (rank == 0 && threadIdx.x == 0) out[r] = 0;       // a row of NaN
+    } else if (mine > 0 && before <= (unsigned)which && (unsigned)which < before + mine) {
+      unsigned at = before;
       for (int i = begin; i < end; ++i) {
         if (__float_as_uint(p[i]) == c.key) {
-          if (rank == (unsigned)which) sh.index = i;
-          ++rank;
+          if (at == (unsigned)which) out[r] = rank * slice + i;
+          ++at;
         }
       }
     }
-    __syncthreads();
-    answer = sh.index;
   }
-  if (threadIdx.x == 0) out[r] = answer;
+  if (blocks > 1) srb_cluster_sync();                      // nobody leaves while its shared memory may still be read
 }
 
 // One token for each of the `count` rows named in rows_index (null: rows 0 .. count - 1), into out[row].
@@ -583,19 +646,28 @@ extern "C" int srb_sample_filtered(const float* logits, int vocab, long long str
   if (vocab <= 0 || stride < vocab) SRB_FAIL("sample_filtered: vocabulary %d and stride %lld do not fit", vocab, stride);
   if (!temperature || !top_k || !top_p || !min_p || !uniform || !out || !scratch)
     SRB_FAIL("sample_filtered: an option array, the scratch memory or the output is missing");
-  static bool configured = false;
-  if (!configured) {
-    SRB_CUDA_CALL(cudaFuncSetAttribute(sample_filtered_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sizeof(FsShared)));
-    configured = true;
-  }
-  // blocks per row: as many (a power of two, 8 at most) as keep all of them resident at once
-  int blocks = 1;
-  while (blocks < 8 && count * blocks * 2 <= srb_sm_count()) blocks *= 2;
   if (count > 65535) SRB_FAIL("sample_filtered: %d rows exceed one launch", count);
-  SRB_CUDA_CALL(srb_launch_clustered(sample_filtered_kernel, dim3(blocks, count), dim3(FS_THREADS), sizeof(FsShared),
-                                     (cudaStream_t)stream, dim3(blocks, 1, 1), logits, vocab, stride, rows_index,
-                                     temperature, top_k, top_p, min_p, uniform, scratch, out));
+  // Blocks per row (a power of two): as many as keep a slice in a block's shared memory, and up to four where the
+  // slices are long and all rows' blocks are resident at once (more do not pay: a search is six barriers of the cluster, 14 us by
+  // four blocks and 18 by eight at 151,936 entries).  Where a row takes eight blocks, 200 KB each, some fifteen rows run
+  // at once, and many rows go through scratch memory with fewer blocks each; so does a vocabulary of more than eight
+  // slices (360 thousand entries).
+  constexpr int SHARED_SLICE = (227 * 1024 - 1024 - (int)sizeof(FsShared)) / 16 * 4;
+  int blocks = 1;
+  while (blocks < FS_MAX_BLOCKS && (long long)SHARED_SLICE * blocks < vocab) blocks *= 2;
+  while (blocks < 4 && vocab / blocks > 16384 && (long long)count * blocks * 2 <= srb_sm_count()) blocks *= 2;
+  if (blocks == FS_MAX_BLOCKS && count >= 16) {
+    blocks = 1;
+    while (blocks < 4 && (long long)count * blocks * 2 <= srb_sm_count()) blocks *= 2;
+  }
+  const int quads = (vocab + 3) / 4, slice = (quads + blocks - 1) / blocks * 4;
+  const bool shared = slice <= SHARED_SLICE;
+  const size_t smem = sizeof(FsShared) + (shared ? (size_t)slice * 4 : 0);
+  auto kernel = shared ? sample_filtered_kernel<true> : sample_filtered_kernel<false>;
+  SRB_CUDA_CALL(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  SRB_CUDA_CALL(srb_launch_clustered(kernel, dim3(blocks, count), dim3(FS_THREADS), smem, (cudaStream_t)stream,
+                                     dim3(blocks, 1, 1), logits, vocab, stride, rows_index, temperature, top_k, top_p, min_p,
+                                     uniform, slice, scratch, out));
   SRB_LAUNCH_CHECK("sample_filtered");
   return SRB_OK;
 }

@@ -769,6 +769,38 @@ def test_sampling_with_top_k_top_p_and_min_p(vocab):
     assert got[2] == 2                                                     # five equal items, u = 0.5: the third by index
 
 
+@pytest.mark.parametrize("vocab,rows", [(3, 2), (45003, 2), (45003, 80), (151936, 40), (360007, 3), (200001, 20), (420001, 2)])
+def test_sampling_with_cuts_over_slices_of_the_vocabulary(vocab, rows):
+    """Vocabularies of one slice of shared memory, of several, and of more than a cluster holds; few rows and more than the
+    device has room for at once.  Equal logits in different slices are told apart by their index."""
+    g = torch.Generator().manual_seed(vocab)
+    logits = torch.randn(rows, vocab, generator=g) * 2.5
+    logits[1] = torch.round(logits[1])                                     # ties in every slice
+    k = torch.tensor([(0, 50, 0)[r % 3] for r in range(rows)], dtype=torch.int32)
+    top_p = torch.tensor([(0.9, 0.95, 1.0)[r % 3] for r in range(rows)])
+    min_p = torch.tensor([(0.0, 0.0, 0.05)[r % 3] for r in range(rows)])
+    temperature, u = torch.rand(rows, generator=g) + 0.5, torch.rand(rows, generator=g)
+    out = torch.full((rows,), -1, dtype=torch.int32, device=DEV)
+    args = [t.to(DEV) for t in (temperature, k, top_p, min_p, u)]
+    ops.sample_filtered(logits.to(DEV), None, *args, out)
+    got = out.cpu().tolist()
+    for r in range(rows):
+        scaled = logits[r].double() / float(temperature[r])
+        p, order = torch.sort(torch.exp(scaled - scaled.max()), descending=True, stable=True)
+        if 0 < int(k[r]) < vocab:
+            p = p[:int(k[r])]
+        before = torch.cumsum(p, 0) - p
+        p = p[(before < float(top_p[r]) * p.sum()) & (p >= float(min_p[r]) * p[0])]
+        running, target = torch.cumsum(p, 0), float(u[r]) * float(p.sum())
+        # the item that holds the target, up to the rounding of 32-bit exponentials (1e-7 each, summed) at its edges
+        at = (order[:len(p) + 1] == got[r]).nonzero()
+        assert len(at) == 1, (r, got[r])
+        at, room = int(at), 1e-6 * float(p.sum())
+        above = float(running[min(at, len(p) - 1)]) if at < len(p) else float(running[-1]) + room
+        below = float(running[at - 1]) if at > 0 else 0.0
+        assert below - room <= target <= above + room, (r, got[r], at, below, target, above)
+
+
 def test_penalties_from_counts_on_the_device():
     """Counts of seen tokens per request (prompt counted once, sampled tokens as they are chosen) and the
     reference's penalties applied from them, against the plain implementation."""
