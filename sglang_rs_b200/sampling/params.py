@@ -42,6 +42,12 @@ class SamplingParams:
                 bad(f"{name} must be in [-2, 2]")
         if self.repetition_penalty is not None and not 0.0 < self.repetition_penalty <= 2.0:
             bad("repetition_penalty must be in (0, 2]")
+        # what a step asks of every row, worked out once per request: (a row's kind, temperature, top_k, top_p, min_p)
+        kind = "greedy" if self.is_greedy else "cut" if self.filters else "plain"
+        object.__setattr__(self, "choice", (kind, self.effective_temperature, int(self.top_k) if self.top_k is not None else 0,
+                                            float(self.top_p) if self.top_p is not None else 1.0,
+                                            float(self.min_p) if self.min_p is not None else 0.0))
+        object.__setattr__(self, "penalised", self.has_penalties)
 
     @classmethod
     def from_dict(cls, options: Optional[Mapping[str, Any]]) -> "SamplingParams":

@@ -18,6 +18,7 @@ import random
 import zlib
 from typing import List, Sequence
 
+import numpy as np
 import torch
 
 from .. import ops
@@ -84,52 +85,73 @@ class Sampler:
         GPU.  ``request_ids`` name the rows' requests, for those with penalties (``logits`` is then
         changed in place, and the chosen tokens are counted as seen)."""
         rows = logits.shape[0]
-        penalised = [r for r in range(rows) if params[r].has_penalties]
-        # what the kernels need per row, in one tensor of floats and one of ints: two copies per step at most
         temperature, uniform = [0.0] * rows, [0.0] * rows          # of the rows sampled without cuts
-        cut_temperature, top_p, min_p = [1.0] * rows, [1.0] * rows, [0.0] * rows
-        presence, frequency, repetition = [0.0] * rows, [0.0] * rows, [1.0] * rows
-        top_k, seen_row = [0] * rows, [-1] * rows
-        cut = []                                                   # rows with top-k / top-p / min-p
-        for r, p in enumerate(params):
-            if p.has_penalties:
-                seen_row[r] = self.seen.row_of(request_ids[r]) if r < len(request_ids) else -1
-                if seen_row[r] < 0:
+        cut, cut_options = [], []                                  # rows with top-k / top-p / min-p, and what they ask for
+        penalised, penalties = [], []
+        plain = False
+        for r in range(rows):
+            p = params[r]
+            if p.penalised:
+                seen_row = self.seen.row_of(request_ids[r]) if r < len(request_ids) else -1
+                if seen_row < 0:
                     raise RuntimeError("a request with penalties has no row of counts; SeenCounts.open was not called")
-                presence[r], frequency[r] = p.presence_penalty or 0.0, p.frequency_penalty or 0.0
-                repetition[r] = p.repetition_penalty if p.repetition_penalty is not None else 1.0
-            if p.is_greedy:
+                penalised.append(r)
+                penalties.append((seen_row, p.presence_penalty or 0.0, p.frequency_penalty or 0.0,
+                                  p.repetition_penalty if p.repetition_penalty is not None else 1.0))
+            choice = p.choice
+            if choice[0] == "greedy":
                 continue
             uniform[r] = randoms[r].next_unit()
-            if p.filters:
+            if choice[0] == "cut":
                 cut.append(r)
-                cut_temperature[r] = p.effective_temperature
-                top_k[r] = int(p.top_k) if p.top_k is not None else 0
-                top_p[r] = float(p.top_p) if p.top_p is not None else 1.0
-                min_p[r] = float(p.min_p) if p.min_p is not None else 0.0
+                cut_options.append(choice)
             else:
-                temperature[r] = p.effective_temperature
-        plain = any(t > 0 for t in temperature)
-        floats = ints = None
-        if plain or cut or penalised:
-            floats = torch.tensor([temperature, uniform, cut_temperature, top_p, min_p, presence, frequency, repetition],
-                                  dtype=torch.float32).pin_memory().to(self.device, non_blocking=True)
-        if cut or penalised:
-            ints = torch.tensor([top_k, seen_row, cut + [0] * (rows - len(cut))],
-                                dtype=torch.int32).pin_memory().to(self.device, non_blocking=True)
+                temperature[r] = choice[1]
+                plain = True
+        device = self._upload(rows, temperature, uniform, cut, cut_options, penalised, penalties) \
+            if plain or cut or penalised else None
         if penalised:
-            ops.apply_penalties(logits, self.seen.table, ints[1], floats[5], floats[6], floats[7])
+            seen_row, presence, frequency, repetition = device[-4:]
+            ops.apply_penalties(logits, self.seen.table, seen_row.view(torch.int32), presence, frequency, repetition)
         if len(cut) == rows:
             picked = torch.empty(rows, dtype=torch.int32, device=logits.device)      # every row is written below
         elif plain:
-            picked = ops.sample(logits, floats[0], floats[1])
+            picked = ops.sample(logits, device[0], device[1])
         else:
             picked = ops.sample(logits, None, None)
         if cut:
-            ops.sample_filtered(logits, ints[2, :len(cut)], floats[2], ints[0], floats[3], floats[4], floats[1], picked)
+            cut_temperature, top_p, min_p, top_k, index = device[2:7]
+            ops.sample_filtered(logits, index[:len(cut)].view(torch.int32), cut_temperature, top_k.view(torch.int32), top_p,
+                                min_p, device[1], picked)
         if penalised:
-            ops.count_picked(self.seen.table, ints[1], picked)
+            ops.count_picked(self.seen.table, seen_row.view(torch.int32), picked)
         return picked
+
+    def _upload(self, rows: int, temperature, uniform, cut, cut_options, penalised, penalties):
+        """What the step's kernels need per row, in one pinned buffer and one copy: float rows on the device (rows of ints
+        among them, by their bits): temperature, uniform; with cuts temperature, top_p, min_p, top_k and the rows that have
+        them; with penalties the rows of counts, presence, frequency and repetition."""
+        count = 2 + (5 if cut else 0) + (4 if penalised else 0)
+        staging = torch.empty((count, rows), dtype=torch.float32, pin_memory=True)
+        floats = staging.numpy()
+        ints = floats.view(np.int32)
+        floats[0], floats[1] = temperature, uniform
+        if cut:
+            floats[2:5] = ((1.0,), (1.0,), (0.0,))                 # of the rows without cuts, which no block takes up
+            ints[5:7] = 0
+            at = np.asarray(cut)
+            _, heat, top_k, top_p, min_p = zip(*cut_options)
+            floats[2, at], floats[3, at], floats[4, at] = heat, top_p, min_p
+            ints[5, at] = np.array(top_k, np.int32)                # (refuses what 32 bits do not hold)
+            ints[6, :len(cut)] = at
+        if penalised:
+            floats[-3:] = ((0.0,), (0.0,), (1.0,))
+            ints[-4] = -1
+            at = np.asarray(penalised)
+            seen_row, presence, frequency, repetition = zip(*penalties)
+            ints[-4, at] = seen_row
+            floats[-3, at], floats[-2, at], floats[-1, at] = presence, frequency, repetition
+        return staging.to(self.device, non_blocking=True).unbind(0)
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams], randoms: Sequence[RequestRandom],
                request_ids: Sequence = ()) -> List[int]:
