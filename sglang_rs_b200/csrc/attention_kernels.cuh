@@ -169,21 +169,47 @@ __device__ __forceinline__ void load_rows(float* tile, int pitch, const T* pool,
   }
 }
 
-// WIDE: rows of keys and values are multiples of four elements and start on four elements' borders: they move four
-// elements at a time, and a score is four chains of additions (entries 0, 4, .. / 1, 5, .. / 2, 6, .. / 3, 7, ..).  Moved one
-// element at a time with two divisions each, a tile of 32 keys of 128 took 85 us in a block of 64 threads.
+// Floats: a block's tile as asynchronous copies of 16 bytes, one group: 32 key rows `k_pitch` floats apart, behind them the value rows
+// (`v_pool` null: none).  `offset`: lane l has the row of the pool that holds key l, -1: zeros.  A warp takes whole rows.
+__device__ __forceinline__ void copy_tile_async(float* tile, int k_pitch, const float* k_pool, const float* v_pool, int d, int vd,
+                                                long long offset) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  auto copy = [](float* to, const float* from, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from), "r"(bytes) : "memory");
+  };
+  for (int key = warp; key < KEY_BLOCK; key += warps) {
+    const long long at = __shfl_sync(0xffffffffu, offset, key);
+    const int bytes = at < 0 ? 0 : 16;
+    for (int e = lane * 4; e < d; e += 128) copy(tile + key * k_pitch + e, k_pool + (at < 0 ? 0 : at * d + e), bytes);
+    if (v_pool)
+      for (int e = lane * 4; e < vd; e += 128) copy(tile + KEY_BLOCK * k_pitch + key * vd + e, v_pool + (at < 0 ? 0 : at * vd + e), bytes);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// FORM: how a tile of 32 keys and values comes.  ATTN_NARROW: one element at a time, whatever the sizes.  ATTN_WIDE: rows of
+// keys and values are multiples of four elements and start on four elements' borders; they move four elements at a time
+// through registers, and a score is four chains of additions (entries 0, 4, .. / 1, 5, .. / 2, 6, .. / 3, 7, ..).  ATTN_ASYNC (floats,
+// which need no conversion): the same rows as asynchronous copies, all of a tile in flight at once, into two tiles that
+// take turns, so that the copies of a tile run under the arithmetic of the one before.  Decoded rows of the 0.6B shape in
+// float32 (two rows of some 230 keys in splits of 128) take 17 us, through registers with four loads in flight 31.
 // A warp per query head that shares the kv head: up to 32 of them, 15 where values are wider than 512 entries (registers).
-template <typename T, int DIM_PER_LANE, bool WIDE>
+#define ATTN_NARROW 0
+#define ATTN_WIDE 1
+#define ATTN_ASYNC 2
+template <typename T, int DIM_PER_LANE, int FORM>
 __global__ void __launch_bounds__(DIM_PER_LANE <= 16 ? 1024 : 480)
 paged_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const T* __restrict__ v_pool, T* __restrict__ out,
                        float* __restrict__ part_acc, float* __restrict__ part_ml, AttnParams p) {
   extern __shared__ __align__(16) float smem[];
   const int d = p.head_dim, vd = p.value_dim;
   const int groups = p.n_q / p.n_kv;
+  constexpr bool WIDE = FORM != ATTN_NARROW, ASYNC = FORM == ATTN_ASYNC;
   const int k_pitch = d + (WIDE ? 4 : 1);                // a lane per key: neighbouring keys on different banks
   float* k_tile = smem;                                  // [32][k_pitch]
   float* v_tile = k_tile + KEY_BLOCK * k_pitch;          // [32][vd], or the key tile itself
-  float* q_tile = v_tile + (p.shared_values ? 0 : KEY_BLOCK * vd);   // [heads_per_block][d]
+  const int tile_floats = KEY_BLOCK * (k_pitch + (p.shared_values ? 0 : vd));
+  float* q_tile = smem + (ASYNC ? 2 : 1) * tile_floats;  // [heads_per_block][d]
   const int v_stride = p.shared_values ? k_pitch : vd;
   if (p.shared_values) v_tile = k_tile;
   __shared__ long long key_offset[KEY_BLOCK];            // which row of the pool each key's is, -1 = masked
@@ -221,32 +247,59 @@ paged_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, co
 #pragma unroll
   for (int j = 0; j < DIM_PER_LANE; ++j) acc[j] = 0.f;
 
-  int base = lo & ~(KEY_BLOCK - 1);
-  for (int next; base < hi; base = next) {
-    next = base + KEY_BLOCK;
-    if (next >= p.keep_first && next < (begin & ~(KEY_BLOCK - 1))) next = begin & ~(KEY_BLOCK - 1);   // blocks without a visible key
-    __syncthreads();                                     // previous tile fully consumed
-    if (threadIdx.x < KEY_BLOCK) {
-      const int key = base + threadIdx.x;
-      long long offset = -1;
-      if (key >= lo && key < hi && (key >= begin || key < p.keep_first)) {
-        const int page = p.block_table[(size_t)request * p.table_stride + key / p.page_size];
-        if (page < 0 || page >= p.num_pages) {
-          atomicOr(p.error_word, SRB_FLAG_BAD_PAGE);
-        } else {
-          offset = ((long long)page * p.n_kv + kv_head) * p.page_size + key % p.page_size;
-        }
+  // the tile after `base`: blocks without a visible key are passed over
+  auto following = [&](int base) {
+    const int next = base + KEY_BLOCK;
+    return next >= p.keep_first && next < (begin & ~(KEY_BLOCK - 1)) ? begin & ~(KEY_BLOCK - 1) : next;
+  };
+  // the row of the pool that holds a key, -1 = masked
+  auto pool_row = [&](int key, bool report) {
+    long long offset = -1;
+    if (key >= lo && key < hi && (key >= begin || key < p.keep_first)) {
+      const int page = p.block_table[(size_t)request * p.table_stride + key / p.page_size];
+      if (page < 0 || page >= p.num_pages) {
+        if (report) atomicOr(p.error_word, SRB_FLAG_BAD_PAGE);
+      } else {
+        offset = ((long long)page * p.n_kv + kv_head) * p.page_size + key % p.page_size;
       }
-      key_offset[threadIdx.x] = offset;
     }
-    __syncthreads();
+    return offset;
+  };
+  int base = lo & ~(KEY_BLOCK - 1), turn = 0;
+  long long my_row = -1;                                 // ASYNC: of key `lane` of the tile at hand
+  if constexpr (ASYNC) {
+    my_row = pool_row(base + lane, warp == 0);
+    copy_tile_async(smem, k_pitch, k_pool, p.shared_values ? nullptr : v_pool, d, vd, my_row);
+  }
+  for (int next; base < hi; base = next, turn ^= 1) {
+    next = following(base);
+    long long next_row = -1;
+    if constexpr (ASYNC) {
+      if (next < hi) {
+        next_row = pool_row(next + lane, warp == 0);
+        // (read last a turn ago, behind the barrier at the end of the loop)
+        copy_tile_async(smem + (turn ^ 1) * tile_floats, k_pitch, k_pool, p.shared_values ? nullptr : v_pool, d, vd, next_row);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+      }
+      k_tile = smem + turn * tile_floats;
+      v_tile = p.shared_values ? k_tile : k_tile + KEY_BLOCK * k_pitch;
+      __syncthreads();                                   // everybody's copies of this tile have landed
+    } else {
+      __syncthreads();                                   // previous tile fully consumed
+      if (threadIdx.x < KEY_BLOCK) key_offset[threadIdx.x] = pool_row(base + threadIdx.x, true);
+      __syncthreads();
+    }
     float s = 0.f;
     const float* qv = q_tile + (live ? warp : 0) * d;
     const float* kv = k_tile + lane * k_pitch;
     if (WIDE) {
-      load_rows(k_tile, k_pitch, k_pool, d, key_offset);
-      if (!p.shared_values) load_rows(v_tile, vd, v_pool, vd, key_offset);
-      __syncthreads();
+      if (!ASYNC) {
+        load_rows(k_tile, k_pitch, k_pool, d, key_offset);
+        if (!p.shared_values) load_rows(v_tile, vd, v_pool, vd, key_offset);
+        __syncthreads();
+      }
       // one key per lane
       float s4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 8
@@ -274,7 +327,7 @@ paged_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, co
     }
     s *= p.scale;
     if (p.softcap > 0.f) s = srb_capped(s / p.softcap, p.softcap);
-    if (key_offset[lane] < 0) s = -INFINITY;
+    if ((ASYNC ? my_row : key_offset[lane]) < 0) s = -INFINITY;
 
     const float m_new = fmaxf(m, srb_warp_max(s));       // finite: the tile holds a visible key
     const float correction = expf(m - m_new);            // exp(-inf) = 0 on the first tile
@@ -291,6 +344,10 @@ paged_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, co
         const int e = lane + 32 * j;
         if (e < vd) acc[j] += pk * v_tile[key * v_stride + e];
       }
+    }
+    if (ASYNC) {
+      my_row = next_row;
+      __syncthreads();                                   // this tile may be written again
     }
   }
   if (!live) return;
@@ -328,6 +385,130 @@ paged_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, co
   }
 }
 
+// Rows of prompt portions in floats: as paged_attention_kernel in its ATTN_ASYNC form, tile by tile the same arithmetic, but a
+// block takes ROW_WARPS / (heads per kv head) neighbouring rows, a warp per (row, head), which read the same tiles while they
+// belong to the same request.  With one row per block and two query heads per kv head six warps an SM had work and every row's
+// keys were copied again: 227 us for two prompts of 225 tokens and 16
+// heads of 128, 95 us this way.
+#define ROW_WARPS 8
+template <int DIM_PER_LANE>
+__global__ void __launch_bounds__(ROW_WARPS * 32)
+paged_attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k_pool, const float* __restrict__ v_pool,
+                            float* __restrict__ out, int rows, AttnParams p) {
+  extern __shared__ __align__(16) float smem[];
+  const int d = p.head_dim, vd = p.value_dim, groups = p.n_q / p.n_kv, per_block = ROW_WARPS / groups;
+  const int k_pitch = d + 4, v_stride = p.shared_values ? k_pitch : vd;
+  const int tile_floats = KEY_BLOCK * (k_pitch + (p.shared_values ? 0 : vd));
+  float* q_tile = smem + 2 * tile_floats;                // [row][head][d]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kv_head = blockIdx.y;
+  const int row0 = blockIdx.x * per_block, row_end = min(rows, row0 + per_block);
+  const int row = row0 + warp / groups, q_head = kv_head * groups + warp % groups;
+  const bool mine = row < row_end;
+  const int pos = mine ? p.positions[row] : -1;          // a row before position 0 is padding
+  const int begin = srb_first_visible(pos, p.window, p.chunk), hi = pos + 1;
+  for (int i = threadIdx.x; i < (row_end - row0) * groups * d; i += blockDim.x)
+    q_tile[i] = q[((size_t)(row0 + i / (groups * d)) * p.n_q + (size_t)kv_head * groups) * d + i % (groups * d)];
+
+  float m = -INFINITY, l = 0.f;
+  float acc[DIM_PER_LANE];
+#pragma unroll
+  for (int j = 0; j < DIM_PER_LANE; ++j) acc[j] = 0.f;
+
+  // a run: the block's neighbouring rows of one request; its tiles span what any of them sees
+  for (int first = row0, last; first < row_end; first = last) {
+    const int request = p.row_request[first];
+    int low = 0x7fffffff, high = 0;
+    for (last = first; last < row_end && p.row_request[last] == request; ++last) {
+      const int at = p.positions[last];
+      if (at < 0) continue;
+      low = min(low, srb_first_visible(at, p.window, p.chunk));
+      high = max(high, at + 1);
+    }
+    const bool in_run = mine && row >= first && row < last && pos >= 0;
+    auto pool_row = [&](int key) {
+      long long offset = -1;
+      if (key >= low && key < high) {
+        const int page = p.block_table[(size_t)request * p.table_stride + key / p.page_size];
+        if (page < 0 || page >= p.num_pages) {
+          if (warp == 0) atomicOr(p.error_word, SRB_FLAG_BAD_PAGE);
+        } else {
+          offset = ((long long)page * p.n_kv + kv_head) * p.page_size + key % p.page_size;
+        }
+      }
+      return offset;
+    };
+    int base = high > 0 ? low & ~(KEY_BLOCK - 1) : 0, turn = 0;
+    __syncthreads();                                     // q is there, and the run before has read its last tile
+    long long my_row = -1;
+    if (base < high) {
+      my_row = pool_row(base + lane);
+      copy_tile_async(smem, k_pitch, k_pool, p.shared_values ? nullptr : v_pool, d, vd, my_row);
+    }
+    for (; base < high; base += KEY_BLOCK, turn ^= 1) {
+      long long next_row = -1;
+      if (base + KEY_BLOCK < high) {
+        next_row = pool_row(base + KEY_BLOCK + lane);
+        copy_tile_async(smem + (turn ^ 1) * tile_floats, k_pitch, k_pool, p.shared_values ? nullptr : v_pool, d, vd, next_row);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+      }
+      __syncthreads();                                   // everybody's copies of this tile have landed
+      if (in_run && base < hi && base + KEY_BLOCK > begin) {
+        const float* k_tile = smem + turn * tile_floats;
+        const float* v_tile = p.shared_values ? k_tile : k_tile + KEY_BLOCK * k_pitch;
+        const float* qv = q_tile + warp * d;
+        const float* kv = k_tile + lane * k_pitch;
+        float s4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+        for (int e = 0; e < d; e += 4) {
+          const float4 x = load_four(qv + e), y = load_four(kv + e);
+          s4[0] += x.x * y.x; s4[1] += x.y * y.y; s4[2] += x.z * y.z; s4[3] += x.w * y.w;
+        }
+        float s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+        s *= p.scale;
+        if (p.softcap > 0.f) s = srb_capped(s / p.softcap, p.softcap);
+        const int key = base + lane;
+        if (my_row < 0 || key < begin || key >= hi) s = -INFINITY;
+
+        const float m_new = fmaxf(m, srb_warp_max(s));   // finite: the tile holds a visible key
+        const float correction = expf(m - m_new);        // exp(-inf) = 0 on the first tile
+        const float prob = expf(s - m_new);              // 0 for masked keys
+        l = l * correction + srb_warp_sum(prob);
+        m = m_new;
+#pragma unroll
+        for (int j = 0; j < DIM_PER_LANE; ++j) acc[j] *= correction;
+#pragma unroll 8
+        for (int k = 0; k < KEY_BLOCK; ++k) {
+          const float pk = __shfl_sync(0xffffffffu, prob, k);
+#pragma unroll
+          for (int j = 0; j < DIM_PER_LANE; ++j) {
+            const int e = lane + 32 * j;
+            if (e < vd) acc[j] += pk * v_tile[k * v_stride + e];
+          }
+        }
+      }
+      my_row = next_row;
+      __syncthreads();                                   // this tile may be written again
+    }
+  }
+  if (!mine || pos < 0) return;
+  if (p.sinks) {
+    const float sink = p.sinks[q_head];
+    const float m_new = fmaxf(m, sink);
+    const float correction = expf(m - m_new);
+    l = l * correction + expf(sink - m_new);
+#pragma unroll
+    for (int j = 0; j < DIM_PER_LANE; ++j) acc[j] *= correction;
+  }
+  const float inv = (p.gates ? p.gates[(size_t)row * p.n_q + q_head] * p.out_scale : p.out_scale) / l;
+#pragma unroll
+  for (int j = 0; j < DIM_PER_LANE; ++j) {
+    const int e = lane + 32 * j;
+    if (e < vd) out[(size_t)row * p.out_pitch + (size_t)q_head * vd + e] = acc[j] * inv;
+  }
+}
+
 // Merges a row's partials in split order: M = max m_s, out = sum acc_s e^(m_s - M) / sum l_s e^(m_s - M).
 template <typename T>
 __global__ void attention_combine_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
@@ -360,17 +541,34 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_acc, con
 template <typename T, int DIM_PER_LANE>
 static int launch_attention(const void* q, const void* k_pool, const void* v_pool, void* out, float* part_acc,
                             float* part_ml, const AttnParams& p, int rows, cudaStream_t s) {
-  auto bytes = [&p](int extra) {
-    return ((size_t)KEY_BLOCK * (p.head_dim + extra) + (p.shared_values ? 0 : (size_t)KEY_BLOCK * p.value_dim) +
+  auto bytes = [&p](int extra, int tiles) {
+    return (tiles * ((size_t)KEY_BLOCK * (p.head_dim + extra) + (p.shared_values ? 0 : (size_t)KEY_BLOCK * p.value_dim)) +
             (size_t)p.heads_per_block * p.head_dim) * sizeof(float);
   };
   // rows of whole groups of four elements on four elements' borders (each half of a key row of two maps too)
   const size_t group = 4 * sizeof(T);
   const bool wide = p.head_dim % (p.maps == 2 ? 8 : 4) == 0 && p.value_dim % 4 == 0 &&
-                    ((uintptr_t)k_pool | (uintptr_t)v_pool) % group == 0 && bytes(4) <= 227 * 1024;
-  const size_t smem = bytes(wide ? 4 : 1);
+                    ((uintptr_t)k_pool | (uintptr_t)v_pool) % group == 0 && bytes(4, 1) <= 227 * 1024;
+  // two tiles in flight while a second block still fits beside this one (values up to some 200 entries wide)
+  const bool async = wide && sizeof(T) == 4 && bytes(4, 2) <= 113 * 1024;
+  if constexpr (sizeof(T) == 4) {
+    // rows of prompts, up to four query heads per kv head: two rows a block and more
+    const int groups = p.n_q / p.n_kv;
+    const size_t shared = bytes(4, 2) + (size_t)(ROW_WARPS - p.heads_per_block) * p.head_dim * sizeof(float);
+    if (async && p.split_size == 0 && p.maps == 1 && p.keep_first == 0 && groups <= ROW_WARPS / 2 && p.n_kv <= 65535 && shared <= 113 * 1024) {
+      auto rows_kernel = paged_attention_rows_kernel<DIM_PER_LANE>;
+      if (shared > 48 * 1024) SRB_CUDA_CALL(cudaFuncSetAttribute(rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared));
+      const int per_block = ROW_WARPS / groups;
+      rows_kernel<<<dim3((rows + per_block - 1) / per_block, p.n_kv), ROW_WARPS * 32, shared, s>>>(
+          (const float*)q, (const float*)k_pool, (const float*)v_pool, (float*)out, rows, p);
+      SRB_LAUNCH_CHECK("paged_attention rows");
+      return SRB_OK;
+    }
+  }
+  const size_t smem = bytes(wide ? 4 : 1, async ? 2 : 1);
   if (smem > 227 * 1024) SRB_FAIL("paged_attention: %zu bytes of shared memory exceed 232448", smem);
-  auto kernel = wide ? paged_attention_kernel<T, DIM_PER_LANE, true> : paged_attention_kernel<T, DIM_PER_LANE, false>;
+  auto kernel = async ? paged_attention_kernel<T, DIM_PER_LANE, sizeof(T) == 4 ? ATTN_ASYNC : ATTN_WIDE>
+                      : wide ? paged_attention_kernel<T, DIM_PER_LANE, ATTN_WIDE> : paged_attention_kernel<T, DIM_PER_LANE, ATTN_NARROW>;
   if (smem > 48 * 1024) SRB_CUDA_CALL(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid(p.split_size == 0 ? 1 : p.max_splits, p.n_kv * p.head_chunks, rows);
   if (grid.y > 65535) SRB_FAIL("paged_attention: %d blocks along the heads exceed 65535", (int)grid.y);
