@@ -41,6 +41,20 @@ extern "C" int sx_gemm_splits(int tokens, int features, int k, int sms, int own_
   return (k_blocks + per_split - 1) / per_split;
 }
 
+// Whether a bfloat16 gate/up product of this shape goes to the CTA-pair kernel (gemm_bf16_pair.cu) or to the library's
+// product and the activation kernel.  From `min_tokens` rows on always; from two fifths of them on where the pairs' rounds of
+// 256 tokens x 128 features are at least 78 % full.  Measured in a graph, weights out of HBM (sizes of Qwen3 0.6B, 1.7B, 8B):
+// 640 rows (rounds 81 % full) 11.2, 27.1, 95.9 us against 13.2, 31.3, 103.8 us; 1,024 rows of 8B (87 %) 138 against 147, 1,279
+// (93 %) 164 against 180; but 776 rows of 8B (66 %) 134 against 123, 1,040 (75 %) 158 against 145.
+extern "C" int sx_pair_takes(int tokens, int inner, int k, int min_tokens, int sms) {
+  if (inner <= 0 || inner % 8 != 0 || k % 8 != 0 || tokens <= 0) return 0;
+  if (tokens >= min_tokens) return 1;
+  if ((long long)tokens * 5 < (long long)min_tokens * 2) return 0;
+  const long long pairs = std::max(1, sms / 2), tiles = (long long)((tokens + 255) / 256) * ((inner + 127) / 128);
+  const long long rounds = (tiles + pairs - 1) / pairs;
+  return (double)tokens * inner >= 0.78 * (double)(rounds * pairs) * (256 * 128);
+}
+
 #define SX_DECODE_BLOCKS_PER_SM 3
 #define SX_DECODE_MAX_SPLITS 64
 #define SX_DECODE_MIN_UNITS 2            // a block walks at least this many 64-key units
@@ -396,7 +410,7 @@ struct Run {
     } else if (bf16 && rows <= step.own_gemm_max_tokens && k % 8 == 0) {
       SX_KERNEL(gemm_bf16, (x, f.gate_up.weight, act, rows, f.inner, k, k, k, f.inner, f.gate_up.out_features, f.inner,
                             SX_GEMM_GATED, 1, f.activation, step.error_word, stream));
-    } else if (bf16 && f.gate_up.out_features == 2 * f.inner && rows >= step.pair_gemm_min_tokens && f.inner % 8 == 0 && k % 8 == 0) {
+    } else if (bf16 && f.gate_up.out_features == 2 * f.inner && sx_pair_takes(rows, f.inner, k, step.pair_gemm_min_tokens, step.sms)) {
       SX_KERNEL(gemm_bf16_pair, (x, f.gate_up.weight, act, rows, f.inner, k, k, k, f.inner, f.gate_up.out_features, f.inner,
                                  SX_GEMM_GATED, f.activation, step.error_word, stream));
     } else {

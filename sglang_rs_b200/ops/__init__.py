@@ -1066,12 +1066,12 @@ def route(h: torch.Tensor, router: torch.Tensor, top: int, renormalize: bool = F
 #: (Qwen3-8B sizes on B200, chained in a graph: QKV 12 against 20 us, down 23 against 52 us; a 12-layer
 #: decode step at batch 128 takes 3.80 ms instead of 4.48 ms)
 OWN_GEMM_MAX_TOKENS = int(os.environ.get("SRB_OWN_GEMM_MAX_TOKENS", "64"))
-#: from this many rows on the gate/up product runs on the persistent CTA-pair kernel, which takes SiLU(gate) * up
-#: into its epilogue.  Measured at Qwen3-8B sizes on B200, chained in a graph, against the library's product
-#: followed by the SiLU kernel: 64.8 against 53.7 us at 256 rows (96 tiles of 256 tokens leave the second
-#: round of the 74 pairs mostly empty), 155 against 155 us at 1,024, 214 against 219 us at 1,536, 280 against
-#: 301 us at 2,048.  The plain products stay with the library at every size: the pair kernel reaches 0.92 to
-#: 1.0 of it alone, and whole prefill steps measured no gain from switching them.
+#: from this many rows on the gate/up product always runs on the persistent CTA-pair kernel, which takes SiLU(gate) * up
+#: into its epilogue; below it where its rounds of tiles are full enough (:func:`pair_gemm_takes`).  Measured against the
+#: library's product followed by the SiLU kernel (Qwen3-8B sizes, chained): 256 against 299 us at 2,048 rows, 194 against
+#: 215 us at 1,536, 72 against 59 us at 264 (a second row of tiles for eight rows).  The plain products stay with the
+#: library at every size: the pair kernel reaches 0.92 to 1.0 of it alone, and whole prefill steps measured no gain from
+#: switching them.
 PAIR_GEMM_MIN_TOKENS = int(os.environ.get("SRB_PAIR_GEMM_MIN_TOKENS", "1280"))
 
 
@@ -1154,7 +1154,7 @@ def gated_product(x: torch.Tensor, weight: torch.Tensor, inner: int, error_word:
         return gemm_bf16(x, weight, error_word, mode="gated", features=inner, up_row_offset=inner, activation=activation,
                          activation_param=activation_param)
     if (x.dtype == torch.bfloat16 and error_word is not None and weight.shape[0] == 2 * inner
-            and pair_gemm_takes(x.shape[0], inner, x.shape[1])):
+            and pair_gemm_takes(x.shape[0], inner, x.shape[1], gated=True)):
         return gemm_bf16_pair(x, weight, error_word, mode="gated", features=inner, up_row_offset=inner,
                               activation=activation, activation_param=activation_param)
     gate_up = linear(x, weight, error_word=error_word)
@@ -1237,8 +1237,12 @@ def gemm_bf16_pair(x: torch.Tensor, w: torch.Tensor, error_word: torch.Tensor, *
     return out if pitch == features else out[:, :features]
 
 
-def pair_gemm_takes(tokens: int, features: int, k: int) -> bool:
-    """True if a bfloat16 gate/up product of this shape goes to the CTA-pair kernel."""
+def pair_gemm_takes(tokens: int, features: int, k: int, gated: bool = False) -> bool:
+    """True if a bfloat16 product with an activation goes to the CTA-pair kernel.  ``gated``: a gate/up product of
+    ``features`` features; fewer rows than ``PAIR_GEMM_MIN_TOKENS`` then go there too where they fill the kernel's rounds of
+    tiles (csrc/step_exec.cu, where the step executor asks the same)."""
+    if gated:
+        return bool(records.library().sx_pair_takes(int(tokens), int(features), int(k), PAIR_GEMM_MIN_TOKENS, sm_count()))
     return tokens >= PAIR_GEMM_MIN_TOKENS and features % 8 == 0 and k % 8 == 0
 
 

@@ -204,3 +204,17 @@ def test_grouped_products_on_pairs_of_ctas(mode, features, k, tile_slots):
     # 32-bit sums of exact products; bfloat16 results round to 2^-9 of themselves
     assert relative_error(out[:slots, :features], want) < (1e-5 if mode == "f32" else 5e-3)
     assert torch.all(out[slots:] == 7.0) and torch.all(out[:, features:] == 7.0)
+
+
+@pytest.mark.parametrize("tokens,takes", [(511, False), (520, False), (640, True), (768, True), (776, False), (1024, True)])
+def test_gate_up_of_fewer_rows_goes_where_the_rounds_are_full(tokens, takes):
+    """Below the row count from which the CTA-pair kernel always runs it takes the sizes that fill its rounds of tiles (of 148
+    SMs): the same result from either side of the line."""
+    inner, k = 6144, 72
+    assert ops.sm_count() != 148 or ops.pair_gemm_takes(tokens, inner, k, gated=True) == takes
+    x, w = operands(tokens, 2 * inner, k, seed=tokens)
+    word = ops.new_error_word(DEV)
+    got = ops.gated_product(x.to(DEV), w.to(DEV), inner, word)
+    ops.raise_on_error_word(word)
+    both = (x.to(DEV).double() @ w.to(DEV).double().T).cpu()
+    assert got.shape == (tokens, inner) and relative_error(got, GATED["silu"](both[:, :inner], both[:, inner:])) < 1e-2
