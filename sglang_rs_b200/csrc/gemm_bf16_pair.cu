@@ -15,6 +15,8 @@
 // registers -> a swizzled 4 KB tile of 32 tokens x 128 bytes -> one TMA store, no barrier between warps.  With the weight
 // rows in the lanes (gate and up 64 lanes apart) they met through shared memory behind a barrier every 32 tokens and half
 // of the four warps computed: 19 us a tile, twice what its products take at K = 2,048.
+// Gate/up of 2,048 tokens: 117 -> 71 us at 2,048 x 12,288 (1,450 TFLOP/s; 384 tiles are 5.2 rounds of 74 pairs), 286 -> 244 to
+// 256 us at 4,096 x 24,576 (1,610 to 1,690).  The tensor pipe under the chip's power limit bounds it, and rounds that are not full.
 //
 // Warps of each CTA: 0 copies (TMA), 1 issues products (even CTA only) and owns the tensor memory,
 // 2-9 epilogue.  Barriers: full[s] lives in the even CTA and counts the bytes of both CTAs' copies;
