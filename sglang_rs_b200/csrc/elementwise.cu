@@ -90,6 +90,10 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = raw;
 }
 
+// x^2 + y^2 + z^2 + w^2 with its roundings written out: which of the multiplications the compiler would fuse differs from kernel to
+// kernel, and with it the last bit.
+__device__ __forceinline__ float sum_of_squares(float4 v) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, v.x * v.x))); }
+
 // The same for widths that are a multiple of 4 and fit 4 * ITER values per thread: the row
 // stays in registers, every load of a thread is issued before the first use (the row is
 // small and the kernel is bound by latency, not by bandwidth), and the additions keep the
@@ -143,7 +147,8 @@ add_rmsnorm_vec_kernel(float* __restrict__ residual, const T* __restrict__ delta
         }
       }
       if (write_residual) *reinterpret_cast<float4*>(residual + src + i) = x[it];
-      partial += x[it].x * x[it].x + x[it].y * x[it].y + x[it].z * x[it].z + x[it].w * x[it].w;
+      if (ITER == 1) partial += sum_of_squares(x[it]);
+      else partial += fmaf(x[it].w, x[it].w, fmaf(x[it].z, x[it].z, fmaf(x[it].x, x[it].x, x[it].y * x[it].y)));
     }
   }
   const float total = srb_block_sum(partial, scratch);
@@ -162,7 +167,8 @@ add_rmsnorm_vec_kernel(float* __restrict__ residual, const T* __restrict__ delta
 // and as many of `delta` in flight and a dozen rows share an SM.  (A thread per four entries has one load of each in flight and
 // its block of up to 1,024 threads then meets at two barriers: 32.5 us for 2,048 rows of 4,096, 101 MB, and 15.3 us for rows of
 // 2,048; 15.2 and 9.8 us now, the second mostly out of L2.)  Sums of squares are formed in the other kernel's
-// order: a warp's butterfly per 128 entries, those added from left to right.  Same bits.
+// order (sum_of_squares, a warp's butterfly per 128 entries, those added from left to right): a row's bits do not depend on which
+// of the two kernels its step takes.
 #define NORM_ROW_THREADS 128
 template <typename T, int ITER>
 __global__ void __launch_bounds__(NORM_ROW_THREADS)
@@ -192,7 +198,7 @@ add_rmsnorm_rows_kernel(float* __restrict__ residual, const T* __restrict__ delt
     const int i = (it * NORM_ROW_THREADS + threadIdx.x) * 4;
     if (delta) { x[it].x += d[it].x; x[it].y += d[it].y; x[it].z += d[it].z; x[it].w += d[it].w; }
     if (write_residual && i < width) *reinterpret_cast<float4*>(residual + src + i) = x[it];
-    const float sum = srb_warp_sum(x[it].x * x[it].x + x[it].y * x[it].y + x[it].z * x[it].z + x[it].w * x[it].w);
+    const float sum = srb_warp_sum(sum_of_squares(x[it]));
     if (lane == 0) sums[it * WARPS + warp] = sum;
   }
   __syncthreads();

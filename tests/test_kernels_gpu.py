@@ -127,6 +127,39 @@ def test_add_rmsnorm_of_few_and_of_many_rows(dtype, width, parts, rows):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width", [4, 516, 1024, 1028, 2048, 2052, 4096])
+@pytest.mark.parametrize("with_delta", [True, False])
+def test_add_rmsnorm_of_a_row_is_the_same_beside_many_and_beside_few(dtype, width, with_delta):
+    """From some hundreds of rows on a kernel of its own takes the step, whose order of additions and roundings is that of the
+    kernel for fewer rows: a row's bits are the same in both, and in steps that pick their rows.  Rows whose first four
+    entries hold all of the sum show which multiplications are fused."""
+    g = torch.Generator().manual_seed(width)
+    rows, eps = 2000, 1e-6
+    residual = torch.randn(rows, width, generator=g)
+    residual[::2, 4:] *= 1e-22
+    residual = residual.to(DEV)
+    delta = torch.randn(rows, width, generator=g)
+    delta[::2, 4:] = 0
+    delta = delta.to(DEV, dtype) if with_delta else None
+    weight = (1 + torch.rand(width, generator=g)).to(DEV)
+    many, few = torch.empty(rows, width, device=DEV, dtype=dtype), torch.empty(rows, width, device=DEV, dtype=dtype)
+    sum_many, sum_few = residual.clone(), residual.clone()
+    ops.add_rmsnorm(sum_many, delta, weight, eps, many)
+    for first in range(0, rows, 100):
+        part = slice(first, first + 100)
+        ops.add_rmsnorm(sum_few[part], delta[part] if with_delta else None, weight, eps, few[part])
+    assert torch.equal(sum_many, sum_few) and torch.equal(many, few)
+    # 1 / sqrt(mean + eps) of a sum of `width` squares in 32-bit, and two products: a dozen roundings; then the stored type's
+    want = pm.plain_rms_norm(sum_many.double().cpu(), weight.double().cpu(), eps)
+    close(many, want, dtype, "many rows")
+    pick = torch.randperm(rows, generator=g)[:1200].to(DEV, torch.int32)
+    picked = torch.empty(1200, width, device=DEV, dtype=dtype)
+    untouched = residual.clone()
+    ops.add_rmsnorm(untouched, delta, weight, eps, picked, row_index=pick, write_residual=False)
+    assert torch.equal(picked, many[pick.long()]) and torch.equal(untouched, residual)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_norm_and_rope_take_partial_sums(dtype):
     """A product cut along K hands its consumer float partial sums; they are added in order."""
     g = torch.Generator().manual_seed(2)
