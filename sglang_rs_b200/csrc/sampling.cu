@@ -81,7 +81,7 @@ sample_pick_kernel(const float* __restrict__ logits, int vocab, int stride, cons
                    const float* __restrict__ uniform, const float* __restrict__ chunk_max,
                    const int* __restrict__ chunk_arg, const float* __restrict__ chunk_sum, int* __restrict__ out) {
   __shared__ __align__(16) float part_sum[SAMPLE_THREADS];
-  __shared__ float part_max[SAMPLE_CHUNKS], chunk_mass[SAMPLE_CHUNKS];
+  __shared__ float part_max[SAMPLE_CHUNKS], part_mass[SAMPLE_CHUNKS], part_factor[SAMPLE_CHUNKS];
   __shared__ int part_arg[SAMPLE_CHUNKS];
   __shared__ float sh_max, sh_target, sh_prefix;
   __shared__ int sh_chunk;
@@ -89,9 +89,10 @@ sample_pick_kernel(const float* __restrict__ logits, int vocab, int stride, cons
   const float* l = logits + (size_t)row * stride;
   const float temp = temperature ? temperature[row] : 0.f;
   const size_t base = (size_t)row * SAMPLE_CHUNKS;
-  // One thread adds and compares in chunk order (the order decides the token); what it reads, the chunks' masses under the row's
-  // maximum among it, is brought and computed by a thread per chunk.  (By one thread, exponentials and all, the kernel
-  // took 25 us for 64 rows; 12 us now.)
+  // One thread adds and compares in chunk order (the order decides the token, and so do the roundings: a chunk's mass under its own
+  // maximum times the factor that brings it under the row's goes into the sum unrounded); what it reads, the factors among it, is
+  // brought and computed by a thread per chunk.  (By one thread, exponentials and all, the kernel took 25 us for 64
+  // rows; 12 us now.)
   if (threadIdx.x < SAMPLE_CHUNKS) {
     part_max[threadIdx.x] = chunk_max[base + threadIdx.x];
     part_arg[threadIdx.x] = chunk_arg[base + threadIdx.x];
@@ -105,8 +106,10 @@ sample_pick_kernel(const float* __restrict__ logits, int vocab, int stride, cons
       best = part_max[c];
       best_index = part_arg[c];
     }
-  if (temp > 0.f && threadIdx.x < SAMPLE_CHUNKS)
-    chunk_mass[threadIdx.x] = chunk_sum[base + threadIdx.x] * expf((part_max[threadIdx.x] - best) / temp);
+  if (temp > 0.f && threadIdx.x < SAMPLE_CHUNKS) {
+    part_mass[threadIdx.x] = chunk_sum[base + threadIdx.x];
+    part_factor[threadIdx.x] = expf((part_max[threadIdx.x] - best) / temp);
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     sh_max = best;
@@ -116,21 +119,21 @@ sample_pick_kernel(const float* __restrict__ logits, int vocab, int stride, cons
     } else {
       float total = 0.f;
 #pragma unroll 16
-      for (int c = 0; c < SAMPLE_CHUNKS; ++c) total += chunk_mass[c];
+      for (int c = 0; c < SAMPLE_CHUNKS; ++c) total = fmaf(part_mass[c], part_factor[c], total);
       const float target = uniform[row] * total;
       float running = 0.f;
       int owner = -1;
       for (int c = 0; c < SAMPLE_CHUNKS; ++c) {
-        const float mass = chunk_mass[c];
-        if (target < running + mass) {
+        const float next = fmaf(part_mass[c], part_factor[c], running);
+        if (target < next) {
           owner = c;
           break;
         }
-        running += mass;
+        running = next;
       }
       if (owner < 0) {                             // rounding left the target at the total: last chunk with mass
         owner = SAMPLE_CHUNKS - 1;
-        while (owner > 0 && !(chunk_sum[base + owner] > 0.f)) --owner;
+        while (owner > 0 && !(part_mass[owner] > 0.f)) --owner;
         running = target;                          // forces the last token with p > 0 below
       }
       sh_chunk = owner;

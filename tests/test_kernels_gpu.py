@@ -2,6 +2,7 @@
 sizes other than the engine's tests use, in 32-bit and in bfloat16."""
 import math
 
+import numpy as np
 import pytest
 import torch
 
@@ -744,6 +745,42 @@ def plain_filtered_pick(kept, u):
         if not found and running > target:
             pick, found = token, True
     return pick, tokens, gap
+
+
+def test_sampling_rounds_as_one_sum_over_chunks():
+    """The running sum over the vocabulary's 64 chunks takes each chunk's mass times its factor unrounded.  Chunks of three equal
+    logits have the mass 3 exactly, so the sum is followed here number by number, at uniform numbers a few last bits around every
+    chunk's border, where another rounding is another token."""
+    chunks, size = 64, 3
+    values = -3.0 * torch.rand(chunks, generator=torch.Generator().manual_seed(9))
+    values[0] = 0.0
+    factor = torch.exp(values.to(DEV)).cpu().numpy()
+    f32, f64 = np.float32, np.float64
+
+    def add(mass, other, running):                          # 32-bit fused multiply-add: exact in 64 bits, rounded once
+        return f32(f64(mass) * f64(other) + f64(running))
+    borders = [f32(0)]
+    for c in range(chunks):
+        borders.append(add(size, factor[c], borders[-1]))
+    uniform = []
+    for border in borders[1:-1]:
+        u = f32(border / borders[-1])
+        for _ in range(6):
+            u = np.nextafter(u, f32(0))
+        for _ in range(12):
+            uniform.append(u)
+            u = np.nextafter(u, f32(1))
+    want = []
+    for u in uniform:
+        target = f32(u * borders[-1])
+        chunk = next((c for c in range(chunks) if target < borders[c + 1]), None)
+        running, token = borders[chunk], 0
+        while token < size - 1 and not target < f32(running + factor[chunk]):
+            running, token = f32(running + factor[chunk]), token + 1
+        want.append(chunk * size + token)
+    logits = values.repeat_interleave(size).expand(len(want), -1).contiguous().to(DEV)
+    got = ops.sample(logits, torch.ones(len(want), device=DEV), torch.tensor(np.array(uniform)).to(DEV))
+    assert got.cpu().tolist() == want
 
 
 @pytest.mark.parametrize("vocab", [1531, 20011])
