@@ -478,14 +478,22 @@ paged_attention_rows_kernel(const float* __restrict__ q, const float* __restrict
         m = m_new;
 #pragma unroll
         for (int j = 0; j < DIM_PER_LANE; ++j) acc[j] *= correction;
-#pragma unroll 8
-        for (int k = 0; k < KEY_BLOCK; ++k) {
+        // Only the keys that this row sees: the tile holds those of the block's other rows too, and their values, times a
+        // probability of 0, would bring their infinities and NaN into this row.
+        const int from = max(begin - base, 0), to = min(hi - base, KEY_BLOCK);
+        auto add_value = [&](int k) {
           const float pk = __shfl_sync(0xffffffffu, prob, k);
 #pragma unroll
           for (int j = 0; j < DIM_PER_LANE; ++j) {
             const int e = lane + 32 * j;
             if (e < vd) acc[j] += pk * v_tile[k * v_stride + e];
           }
+        };
+        if (from == 0 && to == KEY_BLOCK) {
+#pragma unroll 8
+          for (int k = 0; k < KEY_BLOCK; ++k) add_value(k);
+        } else {
+          for (int k = from; k < to; ++k) add_value(k);
         }
       }
       my_row = next_row;

@@ -254,6 +254,25 @@ def test_generic_attention_by_fours_and_one_by_one(dtype, n_q, n_kv, d, page):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("bad", [math.inf, math.nan])
+@pytest.mark.parametrize("n_q,n_kv,window", [(4, 2, None), (2, 2, 20), (12, 2, 20)])
+def test_a_value_that_is_not_finite_stays_with_the_rows_that_see_its_key(dtype, bad, n_q, n_kv, window):
+    """Neighbouring rows of a prompt share tiles of keys; a row takes nothing of a value whose key lies behind its own
+    position or ahead of its window."""
+    case = paged_case(dtype, n_q, n_kv, 64, 16, (70,), (30,), window, seed=3)
+    clean = run_attention(case, 0.125, 0)
+    key = 50                                                # rows 40 .. 69: ten of them end before it
+    case["v_pool"] = case["v_pool"].clone()
+    case["v_pool"][case["table"][0, key // 16].long(), :, key % 16] = bad
+    got = run_attention(case, 0.125, 0)
+    for row, position in enumerate(range(40, 70)):
+        if position >= key and (window is None or position - window < key):
+            assert not bool(torch.isfinite(got[row]).any()), position
+        else:
+            assert torch.equal(got[row], clean[row]), position
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n_q,n_kv,d,rot,inter", [(4, 2, 16, 16, False), (5, 1, 48, 48, False), (3, 3, 128, 64, False),
                                                   (2, 1, 80, 80, True), (8, 2, 256, 256, False)])
 def test_qk_norm_rope_kv(dtype, n_q, n_kv, d, rot, inter):
