@@ -33,8 +33,8 @@
 //    (`float_out`) and srb_map_combine (attention.cu) joins them; the tensor-core kernels join them in their last step.
 //
 // Work split: one block per (row, kv head and chunk of its query heads, split); the block's warp w
-// owns query head kv_head * G + chunk * heads_per_block + w (at most 32 warps, so more than 32 query
-// heads per kv head go in several chunks).  Keys are visited in blocks of 32 aligned to absolute multiples of 32,
+// owns query head kv_head * G + chunk * heads_per_block + w (at most 32 warps, 15 for values wider than 512
+// entries, so more query heads per kv head go in several chunks).  Keys are visited in blocks of 32 aligned to absolute multiples of 32,
 // and a split covers `split_size` keys aligned to absolute multiples of split_size, so a
 // row's arithmetic depends on its own position only, never on how the step was cut or
 // what else is in the batch.  With split_size == 0 the block walks all keys and writes
@@ -193,12 +193,14 @@ __device__ __forceinline__ void copy_tile_async(float* tile, int k_pitch, const 
 // which need no conversion): the same rows as asynchronous copies, all of a tile in flight at once, into two tiles that
 // take turns, so that the copies of a tile run under the arithmetic of the one before.  Decoded rows of the 0.6B shape in
 // float32 (two rows of some 230 keys in splits of 128) take 17 us, through registers with four loads in flight 31.
-// A warp per query head that shares the kv head: up to 32 of them, 15 where values are wider than 512 entries (registers).
+// A warp per query head that shares the kv head: up to 32 of them, 15 where values are wider than 512 entries (registers;
+// the dispatch cuts the heads into chunks by the same numbers).
+#define ATTN_WIDE_VALUE_WARPS 15
 #define ATTN_NARROW 0
 #define ATTN_WIDE 1
 #define ATTN_ASYNC 2
 template <typename T, int DIM_PER_LANE, int FORM>
-__global__ void __launch_bounds__(DIM_PER_LANE <= 16 ? 1024 : 480)
+__global__ void __launch_bounds__(DIM_PER_LANE <= 16 ? 1024 : 32 * ATTN_WIDE_VALUE_WARPS)
 paged_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const T* __restrict__ v_pool, T* __restrict__ out,
                        float* __restrict__ part_acc, float* __restrict__ part_ml, AttnParams p) {
   extern __shared__ __align__(16) float smem[];
@@ -634,7 +636,8 @@ static int paged_attention_dispatch_masked(const void* q, const void* k_pool, co
   if (const char* fault = srb_apply_terms(p, terms)) SRB_FAIL("paged_attention: %s", fault);
   if (p.maps == 2 && !p.float_out) SRB_FAIL("paged_attention: the results of two maps are floats that srb_map_combine joins");
   const int groups = n_q / n_kv;
-  p.head_chunks = (groups + 31) / 32;
+  const int most = value_dim > 512 ? ATTN_WIDE_VALUE_WARPS : 32;       // heads, a warp each, that a block may have
+  p.head_chunks = (groups + most - 1) / most;
   p.heads_per_block = (groups + p.head_chunks - 1) / p.head_chunks;
   cudaStream_t s = (cudaStream_t)stream;
   const int per_lane = (value_dim + 31) / 32;

@@ -175,6 +175,28 @@ def test_attention_over_shared_rows_with_a_sink(dtype, heads, split):
         close(out[r], torch.softmax(scores, -1) @ seen(values, dtype)[:pos + 1], dtype, f"row {r}, own values")
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("value_dim,heads", [(512, 32), (513, 15), (513, 16), (576, 34), (1024, 32)])
+def test_attention_over_wide_shared_rows_with_many_heads(dtype, value_dim, heads):
+    """Values wider than 512 entries need so many registers that a block takes 15 heads; more go in several blocks."""
+    from sglang_rs_b200 import ops
+    torch.manual_seed(heads)
+    width, page, length = value_dim + (4 if value_dim % 4 == 0 else 3), 16, 40
+    keys, q = torch.randn(length, width), torch.randn(1, heads, width)
+    pool = torch.zeros((3, 1, page, width), dtype=dtype, device=DEV)
+    pool.view(-1, width)[:length] = keys.to(DEV, dtype)
+    table, zero = torch.arange(3, dtype=torch.int32, device=DEV).view(1, 3), torch.zeros(1, dtype=torch.int32, device=DEV)
+    word = ops.new_error_word(DEV)
+    want = torch.softmax(torch.einsum("hd,jd->hj", seen(q, dtype)[0], seen(keys, dtype)) * 0.05, -1) @ seen(keys, dtype)[:, :value_dim]
+    for split in (0, 32):
+        out = torch.empty((1, heads, value_dim), dtype=dtype, device=DEV)
+        acc, ml = torch.empty(2 * heads * value_dim, device=DEV), torch.empty(2 * heads * 2, device=DEV)
+        ops.paged_attention(q.to(DEV, dtype), pool, None, out, zero + length - 1, zero, table, scale=0.05, window=0, split_size=split,
+                            max_splits=2 if split else 1, scratch_acc=acc, scratch_ml=ml, error_word=word)
+        close(out[0], want, dtype, f"split {split}")
+    assert int(word.item()) == 0
+
+
 @pytest.mark.parametrize("heads,width,value_dim", [(3, 48, 32), (8, 80, 64), (16, 144, 96), (34, 32, 32), (5, 160, 128), (2, 528, 512)])
 def test_tensor_core_attention_over_shared_rows(heads, width, value_dim):
     """The bfloat16 kernel for rows that are key and value: prompt portions given as tiles (several requests, a portion
