@@ -42,11 +42,13 @@ class SamplingParams:
                 bad(f"{name} must be in [-2, 2]")
         if self.repetition_penalty is not None and not 0.0 < self.repetition_penalty <= 2.0:
             bad("repetition_penalty must be in (0, 2]")
-        # what a step asks of every row, worked out once per request: (a row's kind, temperature, top_k, top_p, min_p)
+        # what a step asks of every row, worked out once per request: (a row's kind, temperature, top_k, top_p, min_p); the cuts'
+        # options are read where there are cuts alone (a top_k of another row may be any number, infinity among them)
         kind = "greedy" if self.is_greedy else "cut" if self.filters else "plain"
-        object.__setattr__(self, "choice", (kind, self.effective_temperature, int(self.top_k) if self.top_k is not None else 0,
-                                            float(self.top_p) if self.top_p is not None else 1.0,
-                                            float(self.min_p) if self.min_p is not None else 0.0))
+        cuts = (0, 1.0, 0.0) if kind != "cut" else (int(self.top_k) if self.top_k is not None else 0,
+                                                    float(self.top_p) if self.top_p is not None else 1.0,
+                                                    float(self.min_p) if self.min_p is not None else 0.0)
+        object.__setattr__(self, "choice", (kind, self.effective_temperature, *cuts))
         object.__setattr__(self, "penalised", self.has_penalties)
 
     @classmethod

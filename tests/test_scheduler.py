@@ -1,4 +1,5 @@
 """The scheduler's decisions (no GPU): a fake step function stands in for the model."""
+import math
 import random
 
 import pytest
@@ -401,3 +402,12 @@ def test_decode_split_counts_follow_the_shape_only():
                 splits = ops.decode_splits(rows, n_kv, keys, sms=148)
                 assert 1 <= splits <= ops.decode_splits_bound(keys) <= ops.DECODE_MAX_SPLITS
                 assert splits == ops.decode_splits(rows, n_kv, keys, sms=148)
+
+
+def test_a_top_k_that_cuts_nothing_may_be_any_number():
+    """The largest logit alone is asked for, or no cut is on: the option is never read as a whole number."""
+    nan = float("nan")
+    assert SamplingParams(temperature=0.0, top_k=math.inf).choice[0] == "greedy"
+    assert SamplingParams(temperature=0.7, top_k=nan).choice == ("plain", 0.7, 0, 1.0, 0.0)
+    assert SamplingParams(temperature=0.7, top_k=-math.inf).choice == ("plain", 0.7, 0, 1.0, 0.0)
+    assert SamplingParams(temperature=0.7, top_k=-1, top_p=0.9).choice == ("cut", 0.7, -1, 0.9, 0.0)
