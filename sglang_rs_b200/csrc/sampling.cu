@@ -667,7 +667,10 @@ extern "C" int srb_sample_filtered(const float* logits, int vocab, long long str
   const bool shared = slice <= SHARED_SLICE;
   const size_t smem = sizeof(FsShared) + (shared ? (size_t)slice * 4 : 0);
   auto kernel = shared ? sample_filtered_kernel<true> : sample_filtered_kernel<false>;
-  SRB_CUDA_CALL(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the limit is the function's and not the launch's: the same number in every call, so that no other thread's call lowers it
+  // between this line and the launch
+  const int limit = (int)sizeof(FsShared) + (shared ? SHARED_SLICE * 4 : 0);
+  SRB_CUDA_CALL(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
   SRB_CUDA_CALL(srb_launch_clustered(kernel, dim3(blocks, count), dim3(FS_THREADS), smem, (cudaStream_t)stream,
                                      dim3(blocks, 1, 1), logits, vocab, stride, rows_index, temperature, top_k, top_p, min_p,
                                      uniform, slice, scratch, out));

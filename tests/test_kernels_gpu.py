@@ -1,6 +1,7 @@
 """Each kernel alone against the plain implementation's function for the same part, at
 sizes other than the engine's tests use, in 32-bit and in bfloat16."""
 import math
+import threading
 
 import numpy as np
 import pytest
@@ -29,6 +30,45 @@ def close(got, want, dtype, what=""):
 def rounded(t, dtype):
     """What the kernel sees: the value after storage in ``dtype``, widened to 64-bit."""
     return t.to(dtype).to(torch.float64)
+
+
+def recorded(monkeypatch, call):
+    """The C calls that ``call`` makes, as functions that make them again with nothing between: the tensors must be kept."""
+    calls, load = [], ops.load_library
+
+    class Recorder:
+        def __init__(self, library):
+            self.library = library
+
+        def __getattr__(self, name):
+            function = getattr(self.library, name)
+
+            def record(*args):
+                calls.append((function, args))
+                return function(*args)
+            return record
+    with monkeypatch.context() as patch:
+        patch.setattr(ops, "load_library", lambda name: Recorder(load(name)))
+        call()
+    return calls
+
+
+def from_threads(monkeypatch, launches, times):
+    """Every launch again and again from a thread of its own, all at the same time; the statuses that are not 0."""
+    def many(calls, failed):
+        for _ in range(times):
+            failed += [s for s in (function(*args) for function, args in calls) if s != 0]
+    failed, threads = [], []
+    for launch in launches:
+        calls = [c for c in recorded(monkeypatch, launch) if c[0].__name__ in ("srb_sample_filtered", "srb_paged_attention_terms")]
+        assert calls
+        threads.append(threading.Thread(target=many, args=(calls, failed)))
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    torch.cuda.synchronize()
+    return failed
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
@@ -888,6 +928,21 @@ def test_sampling_with_cuts_over_slices_of_the_vocabulary(vocab, rows):
         above = float(running[min(at, len(p) - 1)]) if at < len(p) else float(running[-1]) + room
         below = float(running[at - 1]) if at > 0 else 0.0
         assert below - room <= target <= above + room, (r, got[r], at, below, target, above)
+
+
+def test_sampling_with_cuts_from_several_threads(monkeypatch):
+    """Rows of short and of long slices at the same time: no thread's launch depends on another's sizes.  (Slices of these sizes
+    stay in shared memory: the scratch memory of the recorded calls, which is gone, is not touched.)"""
+    keep, launches = [], []
+    for vocab in (64, 45000, 128, 44000):
+        g = torch.Generator().manual_seed(vocab)
+        logits, u, ones = torch.randn(1, vocab, generator=g).to(DEV), torch.rand(1, generator=g).to(DEV), torch.ones(1, device=DEV)
+        k, out = torch.full((1,), 3, dtype=torch.int32, device=DEV), torch.full((1,), -1, dtype=torch.int32, device=DEV)
+        keep.append((logits, u, ones, k, out, torch.zeros(1, device=DEV)))
+        launches.append(lambda t=keep[-1]: ops.sample_filtered(t[0], None, t[2], t[3], t[2], t[5], t[1], t[4]))
+    assert not from_threads(monkeypatch, launches, 2000)
+    for logits, _, _, _, out, _ in keep:
+        assert int(out) in torch.topk(logits, 3).indices.tolist()[0]
 
 
 def test_penalties_from_counts_on_the_device():
