@@ -548,6 +548,11 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_acc, con
   }
 }
 
+// Shared memory that a block may ask for.  The limit set ahead of a launch is the kernel's and not the launch's, so it is the same number
+// in every call: another thread's call of another size does not lower it in between.
+#define ATTN_SHARED_MOST (227 * 1024 - KEY_BLOCK * 8)    // beside the keys' rows
+#define ATTN_SHARED_TWO_BLOCKS (113 * 1024)
+
 template <typename T, int DIM_PER_LANE>
 static int launch_attention(const void* q, const void* k_pool, const void* v_pool, void* out, float* part_acc,
                             float* part_ml, const AttnParams& p, int rows, cudaStream_t s) {
@@ -558,16 +563,17 @@ static int launch_attention(const void* q, const void* k_pool, const void* v_poo
   // rows of whole groups of four elements on four elements' borders (each half of a key row of two maps too)
   const size_t group = 4 * sizeof(T);
   const bool wide = p.head_dim % (p.maps == 2 ? 8 : 4) == 0 && p.value_dim % 4 == 0 &&
-                    ((uintptr_t)k_pool | (uintptr_t)v_pool) % group == 0 && bytes(4, 1) <= 227 * 1024;
+                    ((uintptr_t)k_pool | (uintptr_t)v_pool) % group == 0 && bytes(4, 1) <= ATTN_SHARED_MOST;
   // two tiles in flight while a second block still fits beside this one (values up to some 200 entries wide)
-  const bool async = wide && sizeof(T) == 4 && bytes(4, 2) <= 113 * 1024;
+  const bool async = wide && sizeof(T) == 4 && bytes(4, 2) <= ATTN_SHARED_TWO_BLOCKS;
   if constexpr (sizeof(T) == 4) {
     // rows of prompts, up to four query heads per kv head: two rows a block and more
     const int groups = p.n_q / p.n_kv;
     const size_t shared = bytes(4, 2) + (size_t)(ROW_WARPS - p.heads_per_block) * p.head_dim * sizeof(float);
-    if (async && p.split_size == 0 && p.maps == 1 && p.keep_first == 0 && groups <= ROW_WARPS / 2 && p.n_kv <= 65535 && shared <= 113 * 1024) {
+    if (async && p.split_size == 0 && p.maps == 1 && p.keep_first == 0 && groups <= ROW_WARPS / 2 && p.n_kv <= 65535 && shared <= ATTN_SHARED_TWO_BLOCKS) {
       auto rows_kernel = paged_attention_rows_kernel<DIM_PER_LANE>;
-      if (shared > 48 * 1024) SRB_CUDA_CALL(cudaFuncSetAttribute(rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared));
+      if (shared > 48 * 1024)
+        SRB_CUDA_CALL(cudaFuncSetAttribute(rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATTN_SHARED_TWO_BLOCKS));
       const int per_block = ROW_WARPS / groups;
       rows_kernel<<<dim3((rows + per_block - 1) / per_block, p.n_kv), ROW_WARPS * 32, shared, s>>>(
           (const float*)q, (const float*)k_pool, (const float*)v_pool, (float*)out, rows, p);
@@ -576,10 +582,11 @@ static int launch_attention(const void* q, const void* k_pool, const void* v_poo
     }
   }
   const size_t smem = bytes(wide ? 4 : 1, async ? 2 : 1);
-  if (smem > 227 * 1024) SRB_FAIL("paged_attention: %zu bytes of shared memory exceed 232448", smem);
+  if (smem > ATTN_SHARED_MOST) SRB_FAIL("paged_attention: %zu bytes of shared memory exceed %d", smem, ATTN_SHARED_MOST);
   auto kernel = async ? paged_attention_kernel<T, DIM_PER_LANE, sizeof(T) == 4 ? ATTN_ASYNC : ATTN_WIDE>
                       : wide ? paged_attention_kernel<T, DIM_PER_LANE, ATTN_WIDE> : paged_attention_kernel<T, DIM_PER_LANE, ATTN_NARROW>;
-  if (smem > 48 * 1024) SRB_CUDA_CALL(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024)
+    SRB_CUDA_CALL(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, async ? ATTN_SHARED_TWO_BLOCKS : ATTN_SHARED_MOST));
   dim3 grid(p.split_size == 0 ? 1 : p.max_splits, p.n_kv * p.head_chunks, rows);
   if (grid.y > 65535) SRB_FAIL("paged_attention: %d blocks along the heads exceed 65535", (int)grid.y);
   // at least four warps bring the rows, whatever the number of heads that share them

@@ -312,6 +312,24 @@ def test_a_value_that_is_not_finite_stays_with_the_rows_that_see_its_key(dtype, 
             assert torch.equal(got[row], clean[row]), position
 
 
+@pytest.mark.parametrize("split", [0, 64])
+@pytest.mark.parametrize("groups", [(1, 4), (6, 12)])
+def test_generic_attention_from_several_threads(monkeypatch, groups, split):
+    """Blocks with little and with much shared memory at the same time: no thread's launch depends on another's sizes."""
+    kept, launches = [], []
+    for n_q, d in ((groups[0], 100), (groups[1], 128), (groups[0], 104), (groups[1], 124)):
+        case, out = paged_case(torch.float32, n_q, 1, d, 16, (40,), (3,), None, seed=d), torch.empty(3, n_q, d, device=DEV)
+        scratch = (torch.empty(3 * n_q * d, device=DEV), torch.empty(3 * n_q * 2, device=DEV), ops.new_error_word(DEV))
+        kept.append((case, out, scratch))
+        launches.append(lambda c=case, o=out, t=scratch: ops.paged_attention(
+            c["q"], c["k_pool"], c["v_pool"], o, c["positions"], c["row_request"], c["table"], scale=0.1, window=0, split_size=split,
+            max_splits=1, scratch_acc=t[0], scratch_ml=t[1], error_word=t[2]))
+    assert not from_threads(monkeypatch, launches, 2000)
+    for case, out, scratch in kept:
+        close(out, expected_attention(case, 0.1), torch.float32)
+        ops.raise_on_error_word(scratch[2])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n_q,n_kv,d,rot,inter", [(4, 2, 16, 16, False), (5, 1, 48, 48, False), (3, 3, 128, 64, False),
                                                   (2, 1, 80, 80, True), (8, 2, 256, 256, False)])
