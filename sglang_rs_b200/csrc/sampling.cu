@@ -652,16 +652,30 @@ extern "C" int srb_sample_filtered(const float* logits, int vocab, long long str
   if (count > 65535) SRB_FAIL("sample_filtered: %d rows exceed one launch", count);
   // Blocks per row (a power of two): as many as keep a slice in a block's shared memory, and up to four where the
   // slices are long and all rows' blocks are resident at once (more do not pay: a search is six barriers of the cluster, 14 us by
-  // four blocks and 18 by eight at 151,936 entries).  Where a row takes eight blocks, 200 KB each, some fifteen rows run
-  // at once, and many rows go through scratch memory with fewer blocks each; so does a vocabulary of more than eight
-  // slices (360 thousand entries).
+  // four blocks and 18 by eight at 151,936 entries).
   constexpr int SHARED_SLICE = (227 * 1024 - 1024 - (int)sizeof(FsShared)) / 16 * 4;
+  const int sms = srb_sm_count();
   int blocks = 1;
   while (blocks < FS_MAX_BLOCKS && (long long)SHARED_SLICE * blocks < vocab) blocks *= 2;
-  while (blocks < 4 && vocab / blocks > 16384 && (long long)count * blocks * 2 <= srb_sm_count()) blocks *= 2;
-  if (blocks == FS_MAX_BLOCKS && count >= 16) {
+  while (blocks < 4 && vocab / blocks > 16384 && (long long)count * blocks * 2 <= sms) blocks *= 2;
+  // A block takes up to 200 KB, an SM of its own, so with more blocks than SMs rows run in rounds.  Then it is quicker to run as many
+  // rows as there are SMs at once, by fewer blocks each, with slices in scratch memory (peaked entries, three cuts; flat rows
+  // gain more):
+  //  * two blocks for four: 64 rows of 151,936 entries 144 us against 181;
+  //  * one for four: 128 rows of 100,000 entries 178 us against 311; but three rounds of four blocks hold their own over long rows
+  //    (96 rows of 128,256 entries 223 us against 258, of 180,000 entries 314 against 281);
+  //  * one for two: 96 rows of 50,000 entries 88 us against 130; beyond a row per SM the two are equal (192 rows: 177 and 195 us, of
+  //    64,000 entries 231 and 219);
+  //  * for eight, of which some fifteen rows run at a time, from 16 rows on.
+  // A vocabulary of more than eight slices (360 thousand entries) is always in scratch memory.
+  const long long rounds = ((long long)count * blocks + sms - 1) / sms;
+  bool fewer = false;
+  if (blocks == FS_MAX_BLOCKS) fewer = count >= 16;
+  else if (blocks == 4) fewer = rounds > 3 || (rounds > 1 && (rounds == 2 || vocab <= 131072));
+  else if (blocks == 2) fewer = rounds > 1 && count <= sms;
+  if (fewer) {
     blocks = 1;
-    while (blocks < 4 && (long long)count * blocks * 2 <= srb_sm_count()) blocks *= 2;
+    while (blocks < 4 && (long long)count * blocks * 2 <= sms) blocks *= 2;
   }
   const int quads = (vocab + 3) / 4, slice = (quads + blocks - 1) / blocks * 4;
   const bool shared = slice <= SHARED_SLICE;

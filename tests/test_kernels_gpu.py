@@ -948,6 +948,26 @@ def test_sampling_with_cuts_over_slices_of_the_vocabulary(vocab, rows):
         assert below - room <= target <= above + room, (r, got[r], at, below, target, above)
 
 
+@pytest.mark.parametrize("vocab,batches", [(60000, (75, 148, 149)), (100000, (38, 75, 112)), (151936, (38, 75, 112)), (200003, (16,))])
+def test_sampling_with_cuts_by_shared_and_by_scratch_memory(vocab, batches):
+    """How many rows a step has decides how many blocks take a row and where its slices lie, and never its token."""
+    g = torch.Generator().manual_seed(vocab)
+    rows = 3
+    logits = torch.randn(rows, vocab, generator=g) * 2.5
+    logits[1] = torch.round(logits[1])                                     # ties in every slice
+    options = [torch.rand(rows, generator=g) + 0.5, torch.tensor([0, 50, 0], dtype=torch.int32), torch.tensor([0.9, 0.95, 1.0]),
+               torch.tensor([0.0, 0.0, 0.05]), torch.rand(rows, generator=g)]
+
+    def tokens(count):
+        at = torch.arange(count) % rows
+        out = torch.full((count,), -1, dtype=torch.int32, device=DEV)
+        ops.sample_filtered(logits[at].to(DEV), None, *[t[at].to(DEV) for t in options], out)
+        return out.cpu()
+    few = tokens(rows)
+    for count in batches:
+        assert torch.equal(tokens(count), few[torch.arange(count) % rows]), count
+
+
 def test_sampling_with_cuts_from_several_threads(monkeypatch):
     """Rows of short and of long slices at the same time: no thread's launch depends on another's sizes.  (Slices of these sizes
     stay in shared memory: the scratch memory of the recorded calls, which is gone, is not touched.)"""
