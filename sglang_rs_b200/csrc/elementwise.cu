@@ -163,7 +163,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ residual, const T* __restrict__ delta
   srb_mark(SRB_MARK_NORM, 2);
 }
 
-// The same for many rows (prompt portions), which memory bounds: 128 threads a row, so that a thread has ITER loads of the residual
+// The same for many rows (prompt portions; the line is drawn at the launch), which memory bounds: 128 threads a row, so that a thread has ITER loads of the residual
 // and as many of `delta` in flight and a dozen rows share an SM.  (A thread per four entries has one load of each in flight and
 // its block of up to 1,024 threads then meets at two barriers: 32.5 us for 2,048 rows of 4,096, 101 MB, and 15.3 us for rows of
 // 2,048; 15.2 and 9.8 us now, the second mostly out of L2.)  Sums of squares are formed in the other kernel's
@@ -299,8 +299,15 @@ static int launch_add_rmsnorm(float* residual, const void* delta, const float* d
   // widths that are a multiple of 4 (so float4 accesses stay aligned) and fit the registers
   const bool aligned = width % 4 == 0 && (((uintptr_t)residual | (uintptr_t)delta_parts | (uintptr_t)weight) & 15) == 0 &&
                        (((uintptr_t)delta | (uintptr_t)out) & (4 * sizeof(T) - 1)) == 0 && part_stride % 4 == 0;
-  // more rows than SMs: narrow blocks, several to an SM; with fewer, a row's latency counts, and a wide block has less of it
-  if (aligned && num_parts == 0 && rows > srb_sm_count() && width <= 4096) {
+  // Narrow blocks, several to an SM, where the wide ones of the other kernel (a thread per four entries) would run in more than one
+  // round: as many rows on an SM as its threads and registers take.  In a single round a wide block has the shorter latency: 256
+  // rows of 2,048 bfloat16 entries 2.4 us against 2.9, 592 rows the same, 740 rows 5.3 against 3.4; 1,024 floats are quicker
+  // from some 1,200 rows on, rows of up to 512 entries hardly ever.  More than 2,048 entries gain from a row per SM on in bfloat16
+  // (149 to 296 rows: 0.74 to 1.05 of the time), from three on in floats (4,096 entries: 1.06 to 1.31 of the time at 296 to 400
+  // rows, 0.71 at 444).  Rows of 4,608 to 8,192 entries, with 16 loads a thread, would take 0.8 to 0.94 of the time in floats
+  // and 0.76 to 1.14 in bfloat16 from 512 rows on, and up to 1.8 below: they are left to the other kernel.
+  const int rows_per_sm = width > 2048 ? (sizeof(T) == 2 ? 1 : 3) : width > 1024 ? 4 : width > 512 ? 8 : 32;
+  if (aligned && num_parts == 0 && rows > rows_per_sm * srb_sm_count() && width <= 4096) {
     const auto kernel = width <= 1024 ? add_rmsnorm_rows_kernel<T, 2> : width <= 2048 ? add_rmsnorm_rows_kernel<T, 4> : add_rmsnorm_rows_kernel<T, 8>;
     SRB_CUDA_CALL(srb_launch(kernel, dim3(rows), dim3(NORM_ROW_THREADS), 0, s, residual, (const T*)delta, weight, (T*)out, row_index,
                              width, eps, write_residual));
