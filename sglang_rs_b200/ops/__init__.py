@@ -908,16 +908,31 @@ def head_linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, gate: 
 
 # --------------------------------------------------------------------------- routed experts
 
-#: bfloat16 steps with many choices per expert run the experts' two products on the grouped mode of the tcgen05
-#: kernel for many rows (csrc/gemm_bf16_pair.cu) over rows gathered into slot order; SRB_GROUPED_EXPERTS=0 keeps the mma.sync tiles
+#: bfloat16 steps with more than 8 choices per expert run the experts' two products on the grouped modes of the tcgen05
+#: kernels (csrc/gemm_bf16_pair.cu, csrc/gemm_bf16.cu) over rows gathered into slot order; SRB_GROUPED_EXPERTS=0 keeps the mma.sync
+#: tiles.  At the line the two ways are alike (8 to 12 choices on CTA pairs 0.84 to 1.10 of the time of mma.sync tiles of 32
+#: slots, at 64 experts of 2,048 x 1,408 1.00 to 0.91), far above it they are not (129 choices there: some 300 against 723 us).
 GROUPED_EXPERTS = os.environ.get("SRB_GROUPED_EXPERTS", "1") not in ("0", "off", "false")
 #: from this many rows on the router's logits come from the product kernels (every block of the fused router kernel reads
 #: the whole router matrix: 94 us at 2,048 rows and 64 experts of width 2,048 against the product's few)
 ROUTER_PRODUCT_MIN_ROWS = 128
-#: slots of a tile of the grouped products (128 or 256): 256 reads an expert's weight tile once for twice as many rows
+#: slots of a tile of the grouped products (128 or 256): 256 reads an expert's weight tile once for twice as many rows (64 experts of
+#: 2,048 x 1,408 on CTA pairs: 129 choices each 314 us against 405; up to 65 choices the two are within 6 %)
 GROUPED_TILE_SLOTS = int(os.environ.get("SRB_GROUPED_TILE_SLOTS", "256"))
 #: how a router's logits become scores, by the numbers of csrc/moe.cu
 ROUTER_SCORING = {"softmax": 0, "sigmoid": 1}
+
+
+def grouped_product_is_small(entries: int, experts: int, width: int, inner: int) -> bool:
+    """True if the experts' grouped products go to the one-CTA kernel (csrc/gemm_bf16.cu) and not to the CTA-pair kernel.
+
+    A tile of the pair kernel takes longer from its first copy to its last store (a lane has 64 features of one slot to activate, a
+    thread of the other kernel a feature of the few slots), which shows where a launch is a round of tiles or two.  The whole part,
+    one-CTA kernel against pairs: 8 experts of 512 x 512, 16 choices each 26 against 32 us, 32 choices 31 against 32; 8 of 1,024 x
+    2,048 (2^24 entries) at 9 choices 48 against 54, at 24 equal, at 32 57 against 55; 16 of 1,024 x 2,048 at 9 choices 73 against
+    71, at 32 87 against 75; 64 of 1,024 x 512 at 9 83 against 75."""
+    weights = experts * width * inner
+    return entries <= (32 if weights <= 1 << 22 else 24) * experts and weights <= 1 << 24
 
 
 @traced("routed_experts")
@@ -951,9 +966,9 @@ def routed_experts(h: torch.Tensor, router: torch.Tensor, w_gate_up: torch.Tenso
     products), nothing decided on the host.
 
     The two products: float32 and odd sizes on FFMA or 64 x 64 mma tiles; bfloat16 on mma.sync tiles with asynchronous
-    copies, or, where a step has many choices per expert (tiles of 128 slots), on tcgen05 tensor cores through the
-    grouped mode of :func:`gemm_bf16_pair`'s kernel: the rows are gathered into slot order first, so that a tile's operand is
-    consecutive rows that TMA can fetch."""
+    copies, or, where a step has many choices per expert, on tcgen05 tensor cores through the grouped mode of
+    :func:`gemm_bf16_pair`'s kernel, or of :func:`gemm_bf16`'s where they are small: the rows are gathered into slot order first, so
+    that a tile's operand is consecutive rows that TMA can fetch."""
     _need(h, "h"); _need(router, "router", h.dtype); _need(w_gate_up, "w_gate_up", h.dtype); _need(w_down, "w_down", h.dtype)
     rows, width = h.shape
     experts, inner = w_gate_up.shape[0], w_gate_up.shape[1] // (2 if gated else 1)
@@ -1009,17 +1024,22 @@ def routed_experts(h: torch.Tensor, router: torch.Tensor, w_gate_up: torch.Tenso
     _check(lib, lib.srb_moe_plan_of(_ptr(chosen), rows, top, experts, tile_slots, _ptr(plan), _ptr(slot_row),
                                     _ptr(entry_slot), _ptr(weights), _ptr(slot_weight), _ptr(error_word), stream))
     if grouped:
-        product = load_library("gemm_bf16_pair")
         gathered = torch.empty((entries, width), dtype=h.dtype, device=device)
         # the plan's last offset is the number of slots handed out (choices of experts without tensors get none)
         used = ctypes.c_void_p(plan.data_ptr() + 4 * (1 + experts))
         _check(lib, lib.srb_moe_gather_used(_ptr(h), _ptr(slot_row), entries, width, _ptr(gathered), used, code, stream))
-        _check(product, product.srb_gemm_bf16_pair_grouped(
-            _ptr(gathered), _ptr(w_gate_up), _ptr(act), _ptr(plan), tile_slots, entries, experts,
+        if grouped_product_is_small(entries, experts, width, inner):
+            product, tiles = load_library("gemm_bf16"), (lib.srb_moe_max_tiles_of(rows, top, experts, tile_slots), tile_slots)
+            grouped_product = product.srb_gemm_bf16_grouped
+        else:
+            product, tiles = load_library("gemm_bf16_pair"), (tile_slots,)
+            grouped_product = product.srb_gemm_bf16_pair_grouped
+        _check(product, grouped_product(
+            _ptr(gathered), _ptr(w_gate_up), _ptr(act), _ptr(plan), *tiles, entries, experts,
             (2 if gated else 1) * inner, inner, width, inner, inner if gated else 0, GEMM_MODES["gated" if gated else "act"],
             act_code, act_param, _ptr(slot_weight), _ptr(error_word), stream))
-        _check(product, product.srb_gemm_bf16_pair_grouped(
-            _ptr(act), _ptr(w_down), _ptr(y), _ptr(plan), tile_slots, entries, experts, width, width, inner, width, 0,
+        _check(product, grouped_product(
+            _ptr(act), _ptr(w_down), _ptr(y), _ptr(plan), *tiles, entries, experts, width, width, inner, width, 0,
             GEMM_MODES["f32"], 0, ctypes.c_float(0.0), None, _ptr(error_word), stream))
     else:
         element = h.element_size()

@@ -206,6 +206,31 @@ def test_grouped_products_on_pairs_of_ctas(mode, features, k, tile_slots):
     assert torch.all(out[slots:] == 7.0) and torch.all(out[:, features:] == 7.0)
 
 
+@pytest.mark.parametrize("rows,small", [(33, True), (128, True), (129, False)])
+def test_routed_experts_on_either_side_of_small_products(monkeypatch, rows, small):
+    """Few choices over few weights go to the one-CTA kernel, more to CTA pairs; each of the two kernels on both sides."""
+    experts, width, inner, top = 8, 72, 40, 2
+    assert ops.grouped_product_is_small(rows * top, experts, width, inner) == small
+    g = torch.Generator().manual_seed(rows)
+    h, router = torch.randn(rows, width, generator=g).to(torch.bfloat16), (torch.randn(experts, width, generator=g) * 0.3).to(torch.bfloat16)
+    up = (torch.randn(experts, 2 * inner, width, generator=g) * 0.3).to(torch.bfloat16)
+    down = (torch.randn(experts, width, inner, generator=g) * 0.3).to(torch.bfloat16)
+    chosen, weights = (t.cpu() for t in ops.route(h.to(DEV), router.to(DEV), top))
+    want = torch.zeros(rows, width, dtype=torch.float64)
+    for r in range(rows):
+        for expert, weight in zip(chosen[r].tolist(), weights[r].double()):
+            both = up[expert].double() @ h[r].double()
+            act = GATED["silu"](both[:inner], both[inner:]).to(torch.bfloat16)
+            want[r] += weight * (down[expert].double() @ act.double())
+    for way in (small, not small):
+        monkeypatch.setattr(ops, "grouped_product_is_small", lambda *_: way)
+        word = ops.new_error_word(DEV)
+        got = ops.routed_experts(h.to(DEV), router.to(DEV), up.to(DEV), down.to(DEV), top, "silu", False, word)
+        ops.raise_on_error_word(word)
+        # activations that fall on the other side of a bfloat16 rounding: 2^-8 of one of 40 terms
+        assert relative_error(got, want) < 2e-3
+
+
 @pytest.mark.parametrize("tokens,takes", [(511, False), (520, False), (640, True), (768, True), (776, False), (1024, True)])
 def test_gate_up_of_fewer_rows_goes_where_the_rounds_are_full(tokens, takes):
     """Below the row count from which the CTA-pair kernel always runs it takes the sizes that fill its rounds of tiles (of 148
