@@ -564,9 +564,11 @@ static int launch_attention(const void* q, const void* k_pool, const void* v_poo
   const size_t group = 4 * sizeof(T);
   const bool wide = p.head_dim % (p.maps == 2 ? 8 : 4) == 0 && p.value_dim % 4 == 0 &&
                     ((uintptr_t)k_pool | (uintptr_t)v_pool) % group == 0 && bytes(4, 1) <= ATTN_SHARED_MOST;
-  // two tiles in flight while a second block still fits beside this one (values up to some 200 entries wide)
-  const bool async = wide && sizeof(T) == 4 && bytes(4, 2) <= ATTN_SHARED_TWO_BLOCKS;
-  if constexpr (sizeof(T) == 4) {
+  // two tiles in flight while a second block still fits beside this one (values up to some 200 entries wide; those of
+  // more than 512, with which two tiles take at least 131 KB, never)
+  constexpr bool MAY_ASYNC = sizeof(T) == 4 && DIM_PER_LANE <= 16;
+  const bool async = MAY_ASYNC && wide && bytes(4, 2) <= ATTN_SHARED_TWO_BLOCKS;
+  if constexpr (MAY_ASYNC) {
     // rows of prompts, up to four query heads per kv head: two rows a block and more
     const int groups = p.n_q / p.n_kv;
     const size_t shared = bytes(4, 2) + (size_t)(ROW_WARPS - p.heads_per_block) * p.head_dim * sizeof(float);
@@ -583,7 +585,7 @@ static int launch_attention(const void* q, const void* k_pool, const void* v_poo
   }
   const size_t smem = bytes(wide ? 4 : 1, async ? 2 : 1);
   if (smem > ATTN_SHARED_MOST) SRB_FAIL("paged_attention: %zu bytes of shared memory exceed %d", smem, ATTN_SHARED_MOST);
-  auto kernel = async ? paged_attention_kernel<T, DIM_PER_LANE, sizeof(T) == 4 ? ATTN_ASYNC : ATTN_WIDE>
+  auto kernel = async ? paged_attention_kernel<T, DIM_PER_LANE, MAY_ASYNC ? ATTN_ASYNC : ATTN_WIDE>
                       : wide ? paged_attention_kernel<T, DIM_PER_LANE, ATTN_WIDE> : paged_attention_kernel<T, DIM_PER_LANE, ATTN_NARROW>;
   if (smem > 48 * 1024)
     SRB_CUDA_CALL(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, async ? ATTN_SHARED_TWO_BLOCKS : ATTN_SHARED_MOST));
