@@ -262,21 +262,27 @@ def test_gemm_f32_is_true_32_bit(m, n, k):
 
 @pytest.mark.parametrize("n,k", [(7, 63), (9, 65), (129, 1024), (128, 1025), (1024, 2052), (40, 6148)])
 def test_gemm_f32_edges_of_segments_rounds_tiles_and_parts(n, k):
-    """Both kernels (up to 16 rows, and tiles) at the edges of their cuts, with operands on and off 16-byte borders."""
+    """Both kernels (up to 16 rows, and tiles) at the edges of their cuts, with operands on 16-byte borders (where K is a
+    multiple of 4: two of the three places in a wider matrix) and off them: the same bits."""
     g = torch.Generator().manual_seed(n + k)
-    wide, w, b = torch.randn(130, k + 1, generator=g), torch.randn(n, k, generator=g), torch.randn(n, generator=g)
+    x, w, b = torch.randn(130, k, generator=g), torch.randn(n, k, generator=g), torch.randn(n, generator=g)
     w_d, b_d = w.to(DEV), b.to(DEV)
     # a result is chains of 64 fused multiply-adds, a sum over k / 64 chains, one over at most 8 parts, and the bias
     steps = 64 + (k + 63) // 64 + 8 + 1
-    for columns in (slice(0, k), slice(1, k + 1)):
-        x = wide[:, columns].double()
-        want = x @ w.double().T + b.double()
-        bound = steps * 2.0 ** -24 * (x.abs() @ w.double().abs().T + b.double().abs())
-        rows = wide.to(DEV)[:, columns]
+    want = x.double() @ w.double().T + b.double()
+    bound = steps * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T + b.double().abs())
+    first = None
+    for offset in (0, 4, 1):
+        held = torch.full((130, (k + 7) // 4 * 4), math.nan, device=DEV)
+        rows = held[:, offset:offset + k]
+        rows.copy_(x)
+        assert rows.stride(0) % 4 == 0 and (rows.data_ptr() % 16 == 0) == (offset != 1)
         whole = ops.linear(rows, w_d, b_d)
         assert bool(((whole.cpu().double() - want).abs() <= bound).all())
+        first = whole if first is None else first
+        assert torch.equal(whole, first), offset
         for m in (1, 2, 3, 8, 9, 16, 17, 64, 65):
-            assert torch.equal(ops.linear(rows[130 - m:], w_d, b_d), whole[130 - m:]), (m, columns)
+            assert torch.equal(ops.linear(rows[130 - m:], w_d, b_d), whole[130 - m:]), (m, offset)
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
