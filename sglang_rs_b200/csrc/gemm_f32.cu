@@ -9,7 +9,8 @@
 // Two kernels, because two things bound this product:
 //  * few rows (up to FEW_ROWS): the weights have to be read once and everything else hides behind that.  A block owns
 //    8 weight rows; all of its copies of a round of 16 segments are in flight at once (two rounds deep, 32 KB each).  A thread
-//    owns one chain: (weight row, segment), for all rows of A.
+//    owns one chain: (weight row, segment), for all rows of A.  More than 8 rows read the weights once per 8: 9 to 16 rows still take
+//    0.53 to 0.89 of the tiles' time (weights of 64 x 64 to 151,936 x 1,024; 1.06 at 12,288 x 4,096), 17 rows 0.56 to 1.6.
 //  * more rows: arithmetic.  64 x 128 tiles with 8 x 8 results a thread in packed pairs (fma.rn.f32x2: two IEEE fused
 //    multiply-adds an instruction, which leaves issue slots for the loads), the parts of K in the blocks of a cluster
 //    that add their tiles through shared memory, since tiles alone leave most SMs idle when N is small.

@@ -42,10 +42,14 @@ extern "C" int sx_gemm_splits(int tokens, int features, int k, int sms, int own_
 }
 
 // Whether a bfloat16 gate/up product of this shape goes to the CTA-pair kernel (gemm_bf16_pair.cu) or to the library's
-// product and the activation kernel.  From `min_tokens` rows on always; from two fifths of them on where the pairs' rounds of
-// 256 tokens x 128 features are at least 78 % full.  Measured in a graph, weights out of HBM (sizes of Qwen3 0.6B, 1.7B, 8B):
+// product and the activation kernel.  From two fifths of `min_tokens` on where the pairs' rounds of 256 tokens x 128 features are at
+// least 78 % full, from `min_tokens` rows on always.  Measured in a graph, weights out of HBM (sizes of Qwen3 0.6B, 1.7B, 8B):
 // 640 rows (rounds 81 % full) 11.2, 27.1, 95.9 us against 13.2, 31.3, 103.8 us; 1,024 rows of 8B (87 %) 138 against 147, 1,279
-// (93 %) 164 against 180; but 776 rows of 8B (66 %) 134 against 123, 1,040 (75 %) 158 against 145.
+// (93 %) 164 against 180; but 776 rows of 8B (66 %) 134 against 123, 1,040 (75 %) 158 against 145.  Below two fifths nothing is to be
+// had: 480 rows of 8B (81 %) take 0.98 of the library's time.  From `min_tokens` on the pairs' epilogue saves more than part-empty rounds
+// cost: 1,600 rows of 0.6B (68 %) 0.90 of the library's time, 2,400 (76 %) 0.77, 1,820 rows of 1.7B (77 %) 0.93, of 8B (84 %) 1.02;
+// only where a narrow product's rounds are half empty would the library be ahead (1,408 features at K = 2,048, 1,600 and 1,820
+// rows, 46 and 53 %: 1.23 and 1.17).
 extern "C" int sx_pair_takes(int tokens, int inner, int k, int min_tokens, int sms) {
   if (inner <= 0 || inner % 8 != 0 || k % 8 != 0 || tokens <= 0) return 0;
   if (tokens >= min_tokens) return 1;
