@@ -43,6 +43,7 @@
 #pragma once
 #include "common.cuh"
 #include <math.h>
+#include <type_traits>
 
 #define KEY_BLOCK 32
 
@@ -456,7 +457,10 @@ paged_attention_rows_kernel(const float* __restrict__ q, const float* __restrict
         asm volatile("cp.async.wait_group 0;" ::: "memory");
       }
       __syncthreads();                                   // everybody's copies of this tile have landed
-      if (in_run && base < hi && base + KEY_BLOCK > begin) {
+      // Only the keys that this row sees: the tile holds those of the block's other rows too, and their values, times a probability
+      // of 0, would bring their infinities and NaN into this row.
+      const int from = max(begin - base, 0), to = min(hi - base, KEY_BLOCK);
+      auto tile = [&](auto whole) {
         const float* k_tile = smem + turn * tile_floats;
         const float* v_tile = p.shared_values ? k_tile : k_tile + KEY_BLOCK * k_pitch;
         const float* qv = q_tile + warp * d;
@@ -470,8 +474,7 @@ paged_attention_rows_kernel(const float* __restrict__ q, const float* __restrict
         float s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
         s *= p.scale;
         if (p.softcap > 0.f) s = srb_capped(s / p.softcap, p.softcap);
-        const int key = base + lane;
-        if (my_row < 0 || key < begin || key >= hi) s = -INFINITY;
+        if (my_row < 0 || (!whole.value && (lane < from || lane >= to))) s = -INFINITY;
 
         const float m_new = fmaxf(m, srb_warp_max(s));   // finite: the tile holds a visible key
         const float correction = expf(m - m_new);        // exp(-inf) = 0 on the first tile
@@ -480,9 +483,6 @@ paged_attention_rows_kernel(const float* __restrict__ q, const float* __restrict
         m = m_new;
 #pragma unroll
         for (int j = 0; j < DIM_PER_LANE; ++j) acc[j] *= correction;
-        // Only the keys that this row sees: the tile holds those of the block's other rows too, and their values, times a
-        // probability of 0, would bring their infinities and NaN into this row.
-        const int from = max(begin - base, 0), to = min(hi - base, KEY_BLOCK);
         auto add_value = [&](int k) {
           const float pk = __shfl_sync(0xffffffffu, prob, k);
 #pragma unroll
@@ -491,12 +491,16 @@ paged_attention_rows_kernel(const float* __restrict__ q, const float* __restrict
             if (e < vd) acc[j] += pk * v_tile[k * v_stride + e];
           }
         };
-        if (from == 0 && to == KEY_BLOCK) {
+        if constexpr (whole.value) {
 #pragma unroll 8
           for (int k = 0; k < KEY_BLOCK; ++k) add_value(k);
         } else {
           for (int k = from; k < to; ++k) add_value(k);
         }
+      };
+      if (in_run && from < to) {
+        if (from == 0 && to == KEY_BLOCK) tile(std::true_type());
+        else tile(std::false_type());
       }
       my_row = next_row;
       __syncthreads();                                   // this tile may be written again
