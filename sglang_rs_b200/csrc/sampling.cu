@@ -81,7 +81,7 @@ sample_pick_kernel(const float* __restrict__ logits, int vocab, int stride, cons
                    const float* __restrict__ uniform, const float* __restrict__ chunk_max,
                    const int* __restrict__ chunk_arg, const float* __restrict__ chunk_sum, int* __restrict__ out) {
   __shared__ __align__(16) float part_sum[SAMPLE_THREADS];
-  __shared__ float part_max[SAMPLE_CHUNKS], part_mass[SAMPLE_CHUNKS], part_factor[SAMPLE_CHUNKS];
+  __shared__ __align__(16) float part_max[SAMPLE_CHUNKS], part_mass[SAMPLE_CHUNKS], part_factor[SAMPLE_CHUNKS];
   __shared__ int part_arg[SAMPLE_CHUNKS];
   __shared__ float sh_max, sh_target, sh_prefix;
   __shared__ int sh_chunk;
@@ -123,13 +123,16 @@ sample_pick_kernel(const float* __restrict__ logits, int vocab, int stride, cons
       const float target = uniform[row] * total;
       float running = 0.f;
       int owner = -1;
-      for (int c = 0; c < SAMPLE_CHUNKS; ++c) {
-        const float next = fmaf(part_mass[c], part_factor[c], running);
-        if (target < next) {
-          owner = c;
-          break;
+      for (int c = 0; c < SAMPLE_CHUNKS && owner < 0; c += 4) {
+        const float4 m4 = *reinterpret_cast<const float4*>(part_mass + c), f4 = *reinterpret_cast<const float4*>(part_factor + c);
+        const float mass[4] = {m4.x, m4.y, m4.z, m4.w}, factor[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (owner >= 0) continue;
+          const float next = fmaf(mass[e], factor[e], running);
+          if (target < next) owner = c + e;
+          else running = next;
         }
-        running = next;
       }
       if (owner < 0) {                             // rounding left the target at the total: last chunk with mass
         owner = SAMPLE_CHUNKS - 1;
