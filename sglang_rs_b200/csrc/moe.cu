@@ -232,22 +232,43 @@ extern "C" int srb_moe_select(const float* logits, long long pitch, int rows, in
                            weights, nullptr, stream);
 }
 
-// One block.  plan: [0] number of tiles, then offsets[experts + 1], then per tile (expert, first slot).
+// plan: [0] number of tiles, then offsets[experts + 1], then per tile (expert, first slot).
 // slot_row[slot]: the row whose entry sits in the slot; entry_slot[row * top + k]: the slot of that entry.
-__global__ void moe_plan_kernel(const int* __restrict__ chosen, int entries, int top, int experts, int max_tiles,
-                                int tile_rows, int* __restrict__ plan, int* __restrict__ slot_row, int* __restrict__ entry_slot,
-                                const float* __restrict__ weights, float* __restrict__ slot_weight, int* error_word) {
-  __shared__ int count[MOE_MAX_EXPERTS];
+//
+// A chain of latencies: count the entries of every expert, add up, hand out the slots.  One block, or the blocks of a cluster, each
+// with an equal run of the entries: an expert's slots go to the blocks in turn.  The count that an entry finds is its place among
+// those of its block, so the second pass adds two numbers.
+__global__ void __launch_bounds__(1024)
+moe_plan_kernel(const int* __restrict__ chosen, int entries, int top, int experts, int max_tiles,
+                int tile_rows, int* __restrict__ plan, int* __restrict__ slot_row, int* __restrict__ entry_slot,
+                const float* __restrict__ weights, float* __restrict__ slot_weight, int* error_word) {
+  __shared__ int count[MOE_MAX_EXPERTS];           // of this block's entries; the others read it
+  __shared__ int total[MOE_MAX_EXPERTS];
+  __shared__ int before[MOE_MAX_EXPERTS];          // of the blocks ahead of this one
   __shared__ int first[MOE_MAX_EXPERTS + 1];
   __shared__ int tile_first[MOE_MAX_EXPERTS + 1];
   srb_launch_dependents();
   srb_grid_dependency_wait();
+  const int blocks = gridDim.x, rank = blockIdx.x, per_block = (entries + blocks - 1) / blocks;
+  const int begin = min(entries, rank * per_block), end = min(entries, begin + per_block);
   for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
   __syncthreads();
 #pragma unroll 4
-  for (int i = threadIdx.x; i < entries; i += blockDim.x) {
+  for (int i = begin + threadIdx.x; i < end; i += blockDim.x) {
     const int e = chosen[i];
-    if (e >= 0 && e < experts) atomicAdd(&count[e], 1);
+    entry_slot[i] = e >= 0 && e < experts ? atomicAdd(&count[e], 1) : -1;
+  }
+  __syncthreads();
+  if (blocks > 1) srb_cluster_sync();
+  for (int e = threadIdx.x; e < experts; e += blockDim.x) {
+    int ahead = 0, all = 0;
+    for (int b = 0; b < blocks; ++b) {
+      const int n = blocks > 1 ? __float_as_int(srb_load_peer_shared(reinterpret_cast<const float*>(&count[e]), b)) : count[e];
+      if (b < rank) ahead += n;
+      all += n;
+    }
+    before[e] = ahead;
+    total[e] = all;
   }
   __syncthreads();
   // running sums of the experts' slots and tiles by one warp, 32 experts at a time
@@ -255,7 +276,7 @@ __global__ void moe_plan_kernel(const int* __restrict__ chosen, int entries, int
     const int lane = threadIdx.x;
     int slots = 0, tiles = 0;
     for (int e0 = 0; e0 < experts; e0 += 32) {
-      const int mine = e0 + lane < experts ? count[e0 + lane] : 0;
+      const int mine = e0 + lane < experts ? total[e0 + lane] : 0;
       const int mine_tiles = (mine + tile_rows - 1) / tile_rows;
       int run = mine, run_tiles = mine_tiles;
 #pragma unroll
@@ -273,36 +294,42 @@ __global__ void moe_plan_kernel(const int* __restrict__ chosen, int entries, int
     if (lane == 0) {
       first[experts] = slots;
       tile_first[experts] = tiles;
-      plan[0] = tiles <= max_tiles ? tiles : max_tiles;
-      if (tiles > max_tiles) atomicOr(error_word, SRB_FLAG_BAD_SLOT);
-    }
-  }
-  __syncthreads();
-  int* offsets = plan + 1;
-  int* tiles = plan + 1 + experts + 1;
-  for (int e = threadIdx.x; e <= experts; e += blockDim.x) offsets[e] = first[e];
-  for (int e = threadIdx.x; e < experts; e += blockDim.x) {
-    const int n = tile_first[e + 1] - tile_first[e];
-    for (int t = 0; t < n; ++t) {
-      const int at = tile_first[e] + t;
-      if (at < max_tiles) {
-        tiles[2 * at] = e;
-        tiles[2 * at + 1] = first[e] + t * tile_rows;
+      if (rank == 0) {
+        plan[0] = tiles <= max_tiles ? tiles : max_tiles;
+        if (tiles > max_tiles) atomicOr(error_word, SRB_FLAG_BAD_SLOT);
       }
     }
-    count[e] = 0;                       // becomes the number of the expert's slots handed out so far
   }
   __syncthreads();
+  if (rank == 0) {
+    int* offsets = plan + 1;
+    int* tiles = plan + 1 + experts + 1;
+    for (int e = threadIdx.x; e <= experts; e += blockDim.x) offsets[e] = first[e];
+    for (int e = threadIdx.x; e < experts; e += blockDim.x) {
+      const int n = tile_first[e + 1] - tile_first[e];
+      for (int t = 0; t < n; ++t) {
+        const int at = tile_first[e] + t;
+        if (at < max_tiles) {
+          tiles[2 * at] = e;
+          tiles[2 * at + 1] = first[e] + t * tile_rows;
+        }
+      }
+    }
+  }
 #pragma unroll 4
-  for (int i = threadIdx.x; i < entries; i += blockDim.x) {
-    const int e = chosen[i];
-    if (e < 0 || e >= experts) { entry_slot[i] = -1; continue; }
-    const int slot = first[e] + atomicAdd(&count[e], 1);
+  for (int i = begin + threadIdx.x; i < end; i += blockDim.x) {
+    const int place = entry_slot[i];                 // this thread's own number from above
+    if (place < 0) continue;
+    const int e = chosen[i], slot = first[e] + before[e] + place;
     slot_row[slot] = i / top;
     if (slot_weight) slot_weight[slot] = weights[i];
     entry_slot[i] = slot;
   }
+  if (blocks > 1) srb_cluster_sync();                // nobody leaves while its counts may still be read
 }
+
+#define MOE_PLAN_ENTRIES 2048      // more entries than this are counted by
+#define MOE_PLAN_BLOCKS 8          // blocks
 
 extern "C" int srb_moe_plan_ints(int rows, int top, int experts) {
   const int max_tiles = (rows * top) / moe_tile_rows(rows, top, experts) + experts;
@@ -326,8 +353,9 @@ extern "C" int srb_moe_plan_of(const int* chosen, int rows, int top, int experts
   if (rows <= 0) return SRB_OK;
   if (experts <= 0 || experts > MOE_MAX_EXPERTS || top <= 0 || tile_rows <= 0)
     SRB_FAIL("moe_plan: %d experts, %d chosen, tiles of %d", experts, top, tile_rows);
-  SRB_CUDA_CALL(srb_launch(moe_plan_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, chosen, rows * top, top, experts,
-                           (rows * top) / tile_rows + experts, tile_rows, plan, slot_row, entry_slot, weights, slot_weight, error_word));
+  const int blocks = rows * top > MOE_PLAN_ENTRIES ? MOE_PLAN_BLOCKS : 1;
+  SRB_CUDA_CALL(srb_launch_clustered(moe_plan_kernel, dim3(blocks), dim3(1024), 0, (cudaStream_t)stream, dim3(blocks), chosen,
+                           rows * top, top, experts, (rows * top) / tile_rows + experts, tile_rows, plan, slot_row, entry_slot, weights, slot_weight, error_word));
   SRB_LAUNCH_CHECK("moe_plan");
   return SRB_OK;
 }
@@ -764,22 +792,32 @@ extern "C" int srb_moe_combine(const float* y, const int* entry_slot, const floa
 // rows of h in slot order: out[slot, :] = h[slot_row[slot], :] (16 bytes a thread where the rows allow it), for
 // products that take their operands as whole tiles of consecutive rows.  `used` (or null) points at the number of slots
 // that the plan handed out (its last offset): choices without a slot leave the slots behind it without a row.
+// A warp per slot: a row of 4 KB is eight loads a lane, all in flight.
+#define MOE_GATHER_WARPS 8
 template <typename T>
-__global__ void moe_gather_kernel(const T* __restrict__ h, const int* __restrict__ slot_row, int width, T* __restrict__ out,
-                                  const int* __restrict__ used) {
+__global__ void __launch_bounds__(32 * MOE_GATHER_WARPS)
+moe_gather_kernel(const T* __restrict__ h, const int* __restrict__ slot_row, int slots, int width, T* __restrict__ out,
+                  const int* __restrict__ used) {
   srb_launch_dependents();
   srb_grid_dependency_wait();
-  const int slot = blockIdx.x;
-  if (used && slot >= *used) return;
+  const int slot = blockIdx.x * MOE_GATHER_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (slot >= slots || (used && slot >= *used)) return;
   const T* src = h + (size_t)slot_row[slot] * width;
   T* dst = out + (size_t)slot * width;
   if ((width * sizeof(T)) % 16 == 0 && (((uintptr_t)h | (uintptr_t)out) & 15) == 0) {
     const int pieces = width * sizeof(T) / 16;
-    for (int i = threadIdx.x; i < pieces; i += blockDim.x)
-      reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
+    for (int first = lane; first < pieces; first += 32 * 8) {
+      uint4 v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (first + 32 * j < pieces) v[j] = reinterpret_cast<const uint4*>(src)[first + 32 * j];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (first + 32 * j < pieces) reinterpret_cast<uint4*>(dst)[first + 32 * j] = v[j];
+    }
     return;
   }
-  for (int i = threadIdx.x; i < width; i += blockDim.x) dst[i] = src[i];
+  for (int i = lane; i < width; i += 32) dst[i] = src[i];
 }
 
 extern "C" int srb_moe_gather_used(const void* h, const int* slot_row, int slots, int width, void* out, const int* used,
@@ -792,10 +830,11 @@ extern "C" int srb_moe_gather_used(const void* h, const int* slot_row, int slots
                                    int dtype, void* stream) {
   if (slots <= 0 || width <= 0) return SRB_OK;
   cudaStream_t s = (cudaStream_t)stream;
+  const dim3 grid((slots + MOE_GATHER_WARPS - 1) / MOE_GATHER_WARPS), block(32 * MOE_GATHER_WARPS);
   if (dtype == SRB_DTYPE_F32)
-    SRB_CUDA_CALL(srb_launch(moe_gather_kernel<float>, dim3(slots), dim3(128), 0, s, (const float*)h, slot_row, width, (float*)out, used));
+    SRB_CUDA_CALL(srb_launch(moe_gather_kernel<float>, grid, block, 0, s, (const float*)h, slot_row, slots, width, (float*)out, used));
   else if (dtype == SRB_DTYPE_BF16)
-    SRB_CUDA_CALL(srb_launch(moe_gather_kernel<__nv_bfloat16>, dim3(slots), dim3(128), 0, s, (const __nv_bfloat16*)h, slot_row,
+    SRB_CUDA_CALL(srb_launch(moe_gather_kernel<__nv_bfloat16>, grid, block, 0, s, (const __nv_bfloat16*)h, slot_row, slots,
                              width, (__nv_bfloat16*)out, used));
   else
     SRB_FAIL("moe_gather: unknown dtype %d", dtype);

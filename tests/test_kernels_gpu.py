@@ -1021,3 +1021,35 @@ def test_penalties_from_counts_on_the_device():
         else:
             want = logits[r]
         assert torch.allclose(got[r].cpu().double(), want.double(), atol=1e-6), r
+
+
+@pytest.mark.parametrize("rows,top,experts,tile", [(1, 1, 1, 32), (2048, 1, 7, 128), (2049, 1, 7, 128), (683, 3, 40, 256), (2048, 6, 64, 256),
+                                                   (300, 8, 1024, 128)])
+def test_plan_of_routed_experts_by_one_block_and_by_a_cluster(rows, top, experts, tile):
+    """Up to 2,048 choices one block makes the plan, more a cluster: every choice of an expert with matrices has a slot of its own
+    among its expert's, choices beyond the experts have none, and the tiles cover the slots."""
+    lib = ops.load_library("moe")
+    g = torch.Generator().manual_seed(rows + top)
+    chosen = torch.randint(0, experts + (experts > 7), (rows * top,), generator=g, dtype=torch.int32)
+    weights = torch.rand(rows * top, generator=g)
+    plan = torch.zeros(lib.srb_moe_plan_ints_of(rows, top, experts, tile), dtype=torch.int32, device=DEV)
+    slot_row, entry_slot = (torch.full((rows * top,), -7, dtype=torch.int32, device=DEV) for _ in range(2))
+    slot_weight, word = torch.zeros(rows * top, device=DEV), ops.new_error_word(DEV)
+    on, w_on = chosen.to(DEV), weights.to(DEV)
+    ops._check(lib, lib.srb_moe_plan_of(ops._ptr(on), rows, top, experts, tile, ops._ptr(plan), ops._ptr(slot_row),
+                                        ops._ptr(entry_slot), ops._ptr(w_on), ops._ptr(slot_weight), ops._ptr(word), ops._stream()))
+    ops.raise_on_error_word(word)
+    plan, slot_row, entry_slot, slot_weight = (t.cpu() for t in (plan, slot_row, entry_slot, slot_weight))
+    counts = torch.bincount(chosen[chosen < experts].long(), minlength=experts)
+    first = torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)])
+    assert torch.equal(plan[1:experts + 2].long(), first)
+    tiles = [(e, int(first[e]) + t * tile) for e in range(experts) for t in range((int(counts[e]) + tile - 1) // tile)]
+    assert int(plan[0]) == len(tiles)
+    assert plan[experts + 2:experts + 2 + 2 * len(tiles)].view(-1, 2).tolist() == [list(t) for t in tiles]
+    live = chosen < experts
+    assert bool((entry_slot[~live] == -1).all())
+    slots = entry_slot[live].long()
+    assert torch.equal(slots.sort().values, torch.arange(int(first[-1])))
+    assert bool(((slots >= first[chosen[live].long()]) & (slots < first[chosen[live].long() + 1])).all())
+    assert torch.equal(slot_row[slots].long(), torch.arange(rows * top)[live] // top)
+    assert torch.equal(slot_weight[slots], weights[live])
