@@ -2,6 +2,7 @@
 #include "attention_kernels.cuh"
 
 SRB_DEFINE_LAST_ERROR()
+SRB_DEFINE_PDL_SWITCH()
 
 // Scratch (only when split_size > 0): part_acc holds rows * n_q * max_splits * head_dim
 // floats and part_ml rows * n_q * max_splits * 2 floats.

@@ -523,11 +523,144 @@ paged_attention_rows_kernel(const float* __restrict__ q, const float* __restrict
   }
 }
 
+// Decoded rows in floats, a split of SPLIT_TILES * 32 keys a block: its tiles side by side, a warp per (tile, head), and the warps' results
+// joined at the end in the order of the tiles.  All keys and values of the split are on their way at once; one tile after the other by a
+// warp per head, the latencies of four tiles add up.
+#define SPLIT_TILES 4
+#define SPLIT_MAX_HEADS 4                                // that share a kv head
+template <int DIM_PER_LANE>
+__global__ void __launch_bounds__(32 * SPLIT_TILES * SPLIT_MAX_HEADS)
+paged_attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_pool, const float* __restrict__ v_pool,
+                             float* __restrict__ part_acc, float* __restrict__ part_ml, AttnParams p) {
+  extern __shared__ __align__(16) float smem[];
+  __shared__ float tile_m[SPLIT_TILES * SPLIT_MAX_HEADS], tile_l[SPLIT_TILES * SPLIT_MAX_HEADS];
+  const int d = p.head_dim, vd = p.value_dim, groups = p.n_q / p.n_kv;
+  const int k_pitch = d + 4, v_stride = p.shared_values ? k_pitch : vd;
+  float* k_rows = smem;                                  // [128][k_pitch], behind them the values' rows
+  float* v_rows = p.shared_values ? k_rows : k_rows + SPLIT_TILES * KEY_BLOCK * k_pitch;
+  float* q_rows = p.shared_values ? k_rows + SPLIT_TILES * KEY_BLOCK * k_pitch : v_rows + SPLIT_TILES * KEY_BLOCK * vd;
+  const int split = blockIdx.x, kv_head = blockIdx.y, row = blockIdx.z;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tile = warp / groups, head = warp % groups;
+  srb_launch_dependents();
+  srb_grid_dependency_wait();
+  const int pos = p.positions[row];
+  int lo, hi;
+  row_key_range(p, pos, split, lo, hi);
+  if (lo >= hi) return;
+  const int request = p.row_request[row];
+  // the key of this lane, and the row of the pool that holds it: -1 = masked
+  const int key0 = lo / p.split_size * p.split_size + tile * KEY_BLOCK, key = key0 + lane;
+  const bool some = key0 < hi && key0 + KEY_BLOCK > lo;  // a key of this tile is visible
+  long long at = -1;
+  if (key >= lo && key < hi) {
+    const int page = p.block_table[(size_t)request * p.table_stride + key / p.page_size];
+    if (page < 0 || page >= p.num_pages) {
+      if (head == 0) atomicOr(p.error_word, SRB_FLAG_BAD_PAGE);
+    } else {
+      at = ((long long)page * p.n_kv + kv_head) * p.page_size + key % p.page_size;
+    }
+  }
+  auto copy_rows = [&](float* to, int pitch, const float* pool, int width) {
+    if (some) {
+      for (int k = head; k < KEY_BLOCK; k += groups) {
+        const long long from = __shfl_sync(0xffffffffu, at, k);
+        const int bytes = from < 0 ? 0 : 16;             // 0: zeros
+        for (int e = lane * 4; e < width; e += 128)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(
+                           to + (size_t)(tile * KEY_BLOCK + k) * pitch + e)), "l"(pool + (from < 0 ? 0 : from * width + e)), "r"(bytes) : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  copy_rows(k_rows, k_pitch, k_pool, d);
+  if (p.shared_values) asm volatile("cp.async.commit_group;" ::: "memory");
+  else copy_rows(v_rows, vd, v_pool, vd);
+  for (int i = threadIdx.x; i < groups * d; i += blockDim.x)
+    q_rows[i] = q[((size_t)row * p.n_q + (size_t)kv_head * groups) * d + i];
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+  __syncthreads();
+
+  float m = -INFINITY, l = 0.f, prob = 0.f;
+  if (some) {
+    // one key per lane, four chains
+    const float* qv = q_rows + head * d;
+    const float* kv = k_rows + (size_t)(tile * KEY_BLOCK + lane) * k_pitch;
+    float s4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+    for (int e = 0; e < d; e += 4) {
+      const float4 x = load_four(qv + e), y = load_four(kv + e);
+      s4[0] += x.x * y.x; s4[1] += x.y * y.y; s4[2] += x.z * y.z; s4[3] += x.w * y.w;
+    }
+    float s = ((s4[0] + s4[1]) + (s4[2] + s4[3])) * p.scale;
+    if (p.softcap > 0.f) s = srb_capped(s / p.softcap, p.softcap);
+    if (at < 0) s = -INFINITY;
+    m = srb_warp_max(s);
+    prob = s == -INFINITY && m == -INFINITY ? 0.f : expf(s - m);         // 0 for masked keys
+    l = srb_warp_sum(prob);
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  float acc[DIM_PER_LANE];
+#pragma unroll
+  for (int j = 0; j < DIM_PER_LANE; ++j) acc[j] = 0.f;
+  if (some) {
+#pragma unroll 8
+    for (int k = 0; k < KEY_BLOCK; ++k) {
+      const float pk = __shfl_sync(0xffffffffu, prob, k);
+#pragma unroll
+      for (int j = 0; j < DIM_PER_LANE; ++j) {
+        const int e = lane + 32 * j;
+        if (e < vd) acc[j] += pk * v_rows[(size_t)(tile * KEY_BLOCK + k) * v_stride + e];
+      }
+    }
+  }
+  __syncthreads();                                       // the tiles are read: the results of the warps lie over them
+  float* results = smem;                                 // [tile][head][vd]
+#pragma unroll
+  for (int j = 0; j < DIM_PER_LANE; ++j) {
+    const int e = lane + 32 * j;
+    if (e < vd) results[warp * vd + e] = acc[j];
+  }
+  if (lane == 0) {
+    tile_m[warp] = m;
+    tile_l[warp] = l;
+  }
+  __syncthreads();
+  // a warp joins the tiles of one head
+  if (warp >= groups) return;
+  float most = -INFINITY;
+#pragma unroll
+  for (int t = 0; t < SPLIT_TILES; ++t) most = fmaxf(most, tile_m[t * groups + warp]);
+  float factor[SPLIT_TILES], sum = 0.f;
+#pragma unroll
+  for (int t = 0; t < SPLIT_TILES; ++t) {
+    const float mine = tile_m[t * groups + warp], mass = tile_l[t * groups + warp];
+    factor[t] = mine == -INFINITY ? (mass == 0.f ? 0.f : 1.f) : expf(mine - most);        // (a mass that is not a number stays)
+    sum += mass * factor[t];
+  }
+  const size_t slot = ((size_t)row * p.n_q + (size_t)kv_head * groups + warp) * p.max_splits + split;
+#pragma unroll
+  for (int j = 0; j < DIM_PER_LANE; ++j) {
+    const int e = lane + 32 * j;
+    if (e >= vd) continue;
+    float v = 0.f;
+#pragma unroll
+    for (int t = 0; t < SPLIT_TILES; ++t) v += results[(t * groups + warp) * vd + e] * factor[t];
+    part_acc[slot * vd + e] = v;
+  }
+  if (lane == 0) {
+    part_ml[slot * 2] = most;
+    part_ml[slot * 2 + 1] = sum;
+  }
+}
+
 // Merges a row's partials in split order: M = max m_s, out = sum acc_s e^(m_s - M) / sum l_s e^(m_s - M).
 template <typename T>
 __global__ void attention_combine_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
                                          T* __restrict__ out, AttnParams p) {
   const int row = blockIdx.x, q_head = blockIdx.y;
+  srb_launch_dependents();
+  srb_grid_dependency_wait();
   const int pos = p.positions[row];
   if (pos < 0) return;                                   // a padding row: no block wrote partials for it
   const int wanted = row_split_count(p, pos);
@@ -587,6 +720,20 @@ static int launch_attention(const void* q, const void* k_pool, const void* v_poo
       return SRB_OK;
     }
   }
+  bool side_by_side = false;
+  if constexpr (MAY_ASYNC) {
+    // splits of four tiles whose keys and values fit a block together
+    const int groups = p.n_q / p.n_kv;
+    const size_t shared = bytes(4, SPLIT_TILES);
+    side_by_side = wide && p.split_size == SPLIT_TILES * KEY_BLOCK && p.maps == 1 && p.keep_first == 0 && groups <= SPLIT_MAX_HEADS &&
+                   p.n_kv <= 65535 && shared <= ATTN_SHARED_MOST - 1024;
+    if (side_by_side) {
+      auto split_kernel = paged_attention_split_kernel<DIM_PER_LANE>;
+      SRB_CUDA_CALL(cudaFuncSetAttribute(split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATTN_SHARED_MOST - 1024));
+      SRB_CUDA_CALL(srb_launch(split_kernel, dim3(p.max_splits, p.n_kv, rows), dim3(32 * SPLIT_TILES * groups), shared, s, (const float*)q,
+                               (const float*)k_pool, (const float*)v_pool, part_acc, part_ml, p));
+    }
+  }
   const size_t smem = bytes(wide ? 4 : 1, async ? 2 : 1);
   if (smem > ATTN_SHARED_MOST) SRB_FAIL("paged_attention: %zu bytes of shared memory exceed %d", smem, ATTN_SHARED_MOST);
   auto kernel = async ? paged_attention_kernel<T, DIM_PER_LANE, MAY_ASYNC ? ATTN_ASYNC : ATTN_WIDE>
@@ -596,12 +743,14 @@ static int launch_attention(const void* q, const void* k_pool, const void* v_poo
   dim3 grid(p.split_size == 0 ? 1 : p.max_splits, p.n_kv * p.head_chunks, rows);
   if (grid.y > 65535) SRB_FAIL("paged_attention: %d blocks along the heads exceed 65535", (int)grid.y);
   // at least four warps bring the rows, whatever the number of heads that share them
-  kernel<<<grid, (p.heads_per_block < 4 ? 4 : p.heads_per_block) * 32, smem, s>>>(
-      (const T*)q, (const T*)k_pool, (const T*)v_pool, (T*)out, part_acc, part_ml, p);
-  SRB_LAUNCH_CHECK("paged_attention");
+  if (!side_by_side) {
+    kernel<<<grid, (p.heads_per_block < 4 ? 4 : p.heads_per_block) * 32, smem, s>>>(
+        (const T*)q, (const T*)k_pool, (const T*)v_pool, (T*)out, part_acc, part_ml, p);
+    SRB_LAUNCH_CHECK("paged_attention");
+  }
   if (p.split_size != 0) {
     dim3 cgrid(rows, p.n_q);
-    attention_combine_kernel<T><<<cgrid, 64, 0, s>>>(part_acc, part_ml, (T*)out, p);
+    SRB_CUDA_CALL(srb_launch(attention_combine_kernel<T>, cgrid, dim3(64), 0, s, (const float*)part_acc, (const float*)part_ml, (T*)out, p));
     SRB_LAUNCH_CHECK("attention_combine");
   }
   return SRB_OK;

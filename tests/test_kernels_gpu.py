@@ -1081,3 +1081,13 @@ def test_scores_that_are_not_finite_in_the_tensor_core_prefill_attention(bad):
             assert bool(torch.isfinite(got).all()), key
         else:
             assert not bool(torch.isfinite(got[key:]).any()), key
+
+
+@pytest.mark.parametrize("n_q,n_kv,d,page", [(2, 2, 20, 8), (4, 2, 128, 16), (3, 1, 64, 4), (8, 2, 256, 16), (5, 1, 128, 16)])
+@pytest.mark.parametrize("window", [None, 20, 150])
+def test_float_splits_of_four_tiles(n_q, n_kv, d, page, window):
+    """Splits of 128 keys in floats: up to four query heads per kv head as tiles side by side (where they fit a block), more one after
+    the other; rows at the first and last key of a tile and of a split, windows that begin inside a tile."""
+    lengths = (1, 32, 33, 128, 129, 260, 287)
+    case = paged_case(torch.float32, n_q, n_kv, d, page, lengths, (1,) * len(lengths), window, seed=d)
+    close(run_attention(case, 1.0 / math.sqrt(d), 128), expected_attention(case, 1.0 / math.sqrt(d)), torch.float32, "split 128")
