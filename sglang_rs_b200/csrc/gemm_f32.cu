@@ -1,343 +1,474 @@
-// C[M, N] = A[M, K] * W[N, K]^T (+ bias[N]) in true 32-bit: FFMA on the CUDA cores, no
-// tensor cores and therefore no reduced-precision matrix mode.
+// C[M, N] = A[M, K] * W[N, K]^T (+ bias[N]) to 32-bit precision on the 5th-generation tensor cores.
 //
-// The order of additions is a function of N and K only, so a row's result depends neither on M nor on the row's
-// place in the batch, whichever of the two kernels below computes it: K is cut into segments of SEG entries, each
-// summed in index order by one chain of fused multiply-adds; the segments of a part are added in order, and the
-// parts (gemm_parts, at most 8) are added in order.  (Short chains also round less than one chain over all of K.)
+// A float is the sum of three bfloat16 numbers exactly: its upper 8 bits of precision (cut off, so that the largest floats stay
+// finite), the upper 8 of what is left (rounded), and the rest.  A product of two floats is then nine products of bfloat16
+// numbers, which are exact in 32 bits; the three smallest (2^-24 of the product and less, of either sign) are left out, the six
+// others go to tcgen05.mma.  The unit adds with truncation, so nothing is left in it for long: of every 32 entries of K (two steps of
+// the instruction) the products of the upper parts have a sum of their own and the five others another; both start from zero and are
+// added to the result in registers, rounded to nearest.
 //
-// Two kernels, because two things bound this product:
-//  * few rows (up to FEW_ROWS): the weights have to be read once and everything else hides behind that.  A block owns
-//    8 weight rows; all of its copies of a round of 16 segments are in flight at once (two rounds deep, 32 KB each).  A thread
-//    owns one chain: (weight row, segment), for all rows of A.  More than 8 rows read the weights once per 8: 9 to 16 rows still take
-//    0.53 to 0.89 of the tiles' time (weights of 64 x 64 to 151,936 x 1,024; 1.06 at 12,288 x 4,096), 17 rows 0.56 to 1.6.
-//  * more rows: arithmetic.  64 x 128 tiles with 8 x 8 results a thread in packed pairs (fma.rn.f32x2: two IEEE fused
-//    multiply-adds an instruction, which leaves issue slots for the loads), the parts of K in the blocks of a cluster
-//    that add their tiles through shared memory, since tiles alone leave most SMs idle when N is small.
+// The order of additions is a function of N and K only, so a row's result depends neither on M nor on the row's place in the
+// batch: sums of 32 entries are added in order to a part, and the parts (gemm_parts, at most 8) in order to the result.
+//
+// The weights are the M side of the instruction.  Up to 16 rows of A: a block owns 128 rows of W and a part of K.  More rows: a pair
+// of blocks on neighbouring SMs (cta_group::2) owns 256 rows of W and TOKENS (32, 64 or 128) rows of A, of which each block brings 128
+// and TOKENS / 2, and one, two or all parts of K.  The blocks of a tile are a cluster and add their sums through shared memory.
+// Warps of a block: eight bring both operands (plain loads: rows may start on any float; a thread asks for its pieces of the next chunk
+// while it splits those of the one before) and leave the parts in the swizzled layout that the unit reads; one issues the products (of the
+// pair, in its even block); the others read finished sums out of tensor memory and add them up.  No barrier spans the block in between.
+//
+// An element that comes out infinite or not a number is computed again by one chain of fused multiply-adds: the parts of an infinity are
+// not its sum.
 //
 // Weight layout and meaning as the reference's `linear`: row-major [out, in],
 // y[o] = sum_i x[i] * W[o, i] (crates/sglang-kernel/src/cpu.rs:73-108).
+//
+// Every wait is bounded; if one runs out the block's warps leave their loops and its results are computed by the plain chains too.
 #include "common.cuh"
+#include "tcgen05_helpers.cuh"
+#include <algorithm>
 
 SRB_DEFINE_LAST_ERROR()
 SRB_DEFINE_PDL_SWITCH()
 
-#define SEG 64                // entries of K that one chain of additions covers
-#define FEW_ROWS 16
-#define FEW_FEATURES 8        // weight rows of a block
-#define FEW_SEGS 16           // segments of a round: 128 threads
-#define FEW_THREADS (FEW_FEATURES * FEW_SEGS)
-#define ROUND_K (SEG * FEW_SEGS)
-#define W_PITCH (ROUND_K + 4)                // floats; 8 neighbouring rows fall on different banks
-#define X_PITCH (FEW_SEGS * (SEG + 4))       // a row's segments too
+#define F32_FEATURES 128      // weight rows of a block
+#define F32_CHUNK 64          // entries of K in a buffer of shared memory: a swizzled row of 128 bytes
+#define F32_PLANES 3          // bfloat16 parts of a float
+#define F32_MAX_PARTS 8
+#define F32_MAX_BLOCKS 8      // blocks of a cluster
 
-#define TILE_M 64
-#define TILE_N 128
-#define TILE_K 16
-#define TILE_THREADS 128
-#define A_PITCH (TILE_M + 4)
-#define B_PITCH (TILE_N + 4)
-
-// Parts of K: as many as make about three blocks per SM at 256 rows, each with at least one segment, equal in segments but for the last.
-__host__ __device__ static inline int gemm_part_segments(int n, int k) {
-  const int segments = (k + SEG - 1) / SEG;
-  const int tiles = 4 * ((n + TILE_N - 1) / TILE_N);
+// Parts of K: as many (a power of two) as keep the blocks of up to 16 rows resident at once, two to an SM, each of at least two chunks.
+struct F32Parts { int count, chunks; };      // parts, and the chunks of each but the last
+static inline F32Parts gemm_parts(int n, int k) {
+  const int chunks = (k + F32_CHUNK - 1) / F32_CHUNK, tiles = (n + F32_FEATURES - 1) / F32_FEATURES;
   int parts = 1;
-  while (parts < 8 && parts * 2 <= segments && tiles * parts < 444) parts *= 2;
-  return (segments + parts - 1) / parts;
+  while (parts < F32_MAX_PARTS && parts * 4 <= chunks && tiles * parts * 2 <= 296) parts *= 2;
+  while (parts > 1 && (parts - 1) * ((chunks + parts - 1) / parts) >= chunks) parts /= 2;        // no part is empty
+  return {parts, (chunks + parts - 1) / parts};
 }
 
-template <int BYTES>
-__device__ __forceinline__ void copy_async(float* dst, const float* src, bool inside) {
-  const unsigned to = (unsigned)__cvta_generic_to_shared(dst);
-  const int size = inside ? BYTES : 0;                       // 0: the destination is filled with zeros, the source is not read
-  if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src), "r"(size) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(src), "r"(size) : "memory");
-}
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int PENDING> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
+struct F32Args {
+  const float *a, *w, *bias;
+  float* c;
+  int m, n, k, lda, ldw, ldc;
+  int parts, part_chunks;     // of K; chunks of a part
+  int block_parts;            // parts that a block adds up: all, two or one
+};
 
-// ---------------------------------------------------------------------------------------------- few rows
-// blockIdx.x: 8 weight rows; blockIdx.y: ROWS rows of A.  WIDE: rows of both operands start on 16 bytes.
-template <int ROWS, bool WIDE>
-__global__ void __launch_bounds__(FEW_THREADS)
-gemm_f32_few_kernel(const float* __restrict__ a, const float* __restrict__ w, const float* __restrict__ bias,
-                    float* __restrict__ c, int m, int n, int k, int lda, int ldw, int ldc, int part_segments, int stages) {
-  extern __shared__ __align__(16) float few_smem[];
-  constexpr int STAGE = FEW_FEATURES * W_PITCH + ROWS * X_PITCH;
-  constexpr int UNIT = WIDE ? 4 : 1;
-  float* sums = few_smem + stages * STAGE;                   // [feature][segment][row] of a round
-  const int col0 = blockIdx.x * FEW_FEATURES, row0 = blockIdx.y * ROWS;
-  const int rounds = (k + ROUND_K - 1) / ROUND_K;
-  const int feature = threadIdx.x & (FEW_FEATURES - 1), segment = threadIdx.x / FEW_FEATURES;
+// TOKENS rows of A of a block, or of a pair of blocks
+template <int TOKENS, bool PAIR>
+struct F32Shape {
+  static constexpr int X_ROWS = PAIR ? TOKENS / 2 : TOKENS;              // rows of A that a block brings
+  static constexpr int LOADERS = 256;                                    // threads that bring the operands: warps 0 to 7
+  static constexpr int ADDERS = PAIR ? 256 : 128;                        // threads that add up: warps 8 and up
+  static constexpr int THREADS = LOADERS + ADDERS + 32;                  // the last warp issues the products
+  static constexpr unsigned W_PLANE = F32_FEATURES * 128, X_PLANE = X_ROWS * 128;
+  static constexpr unsigned BUFFER = F32_PLANES * (W_PLANE + X_PLANE);
+  static constexpr unsigned LEVEL = PAIR ? TOKENS * F32_FEATURES * 4 : 0;      // sums of earlier parts
+  static constexpr unsigned SMEM = 2 * BUFFER + LEVEL + 1024;
+  static constexpr unsigned TMEM = 4 * TOKENS;                           // two sums, two buffers of them
+  static constexpr int BLOCKS = PAIR ? 1 : 2;                            // an SM
+};
 
-  auto load_w = [&](int round) {
-    float* to = few_smem + (round % stages) * STAGE;
-    const int k0 = round * ROUND_K;
-    const int units = (min(k - k0, ROUND_K) + SEG - 1) / SEG * (SEG / UNIT);     // whole segments, zeros behind K
-    for (int f = 0; f < FEW_FEATURES; ++f) {
-      const bool live = col0 + f < n;
-      const float* from = w + (size_t)(live ? col0 + f : 0) * ldw;
-      for (int u = threadIdx.x; u < units; u += FEW_THREADS) {
-        const int at = k0 + u * UNIT;
-        const bool inside = live && at < k;
-        copy_async<UNIT * 4>(to + f * W_PITCH + u * UNIT, inside ? from + at : w, inside);
-      }
-    }
-  };
-  auto load_x = [&](int round) {
-    float* to = few_smem + (round % stages) * STAGE + FEW_FEATURES * W_PITCH;
-    const int k0 = round * ROUND_K;
-    const int units = (min(k - k0, ROUND_K) + SEG - 1) / SEG * (SEG / UNIT);
-    for (int r = 0; r < ROWS; ++r) {
-      const bool live = row0 + r < m;
-      const float* from = a + (size_t)(live ? row0 + r : 0) * lda;
-      for (int u = threadIdx.x; u < units; u += FEW_THREADS) {
-        const int at = k0 + u * UNIT;
-        const bool inside = live && at < k;
-        const int seg = u * UNIT / SEG;
-        copy_async<UNIT * 4>(to + r * X_PITCH + seg * (SEG + 4) + (u * UNIT - seg * SEG), inside ? from + at : a, inside);
-      }
-    }
-  };
-
-  // The weights of the first rounds are asked into L2 ahead of the wait for the kernels ahead (nothing is read yet, so it
-  // does not matter who writes them); the copies follow it.
-  const int early = min(stages, rounds);
-  if (WIDE && threadIdx.x < FEW_FEATURES && col0 + threadIdx.x < n) {
-    const int entries = min(k, early * ROUND_K);
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(w + (size_t)(col0 + threadIdx.x) * ldw), "r"(entries * 4) : "memory");
-  }
-  srb_launch_dependents();
-  srb_grid_dependency_wait();
-  for (int r = 0; r < early; ++r) {
-    load_w(r);
-    load_x(r);
-    copy_commit();                                           // group r
-  }
-
-  float total = 0.f, part = 0.f;                             // of (feature, row) = thread, for the first 8 * ROWS threads
-  constexpr int OWNED = (FEW_FEATURES * ROWS + FEW_THREADS - 1) / FEW_THREADS;
-  static_assert(OWNED == 1, "a thread adds the segments of one result");
-  const int own_feature = threadIdx.x / ROWS, own_row = threadIdx.x % ROWS;
-  const bool owner = threadIdx.x < FEW_FEATURES * ROWS;
-  for (int round = 0; round < rounds; ++round) {
-    // the groups behind this round's: stages - 1 of them, or as many rounds as are left
-    const int later = min(stages - 1, rounds - 1 - round);
-    if (later > 0) copy_wait<1>();
-    else copy_wait<0>();
-    __syncthreads();
-    const float* stage = few_smem + (round % stages) * STAGE;
-    const int segments = (min(k - round * ROUND_K, ROUND_K) + SEG - 1) / SEG;
-    if (segment < segments) {
-      const float* wv = stage + feature * W_PITCH + segment * SEG;
-      const float* xv = stage + FEW_FEATURES * W_PITCH + segment * (SEG + 4);
-      float acc[ROWS];
-#pragma unroll
-      for (int r = 0; r < ROWS; ++r) acc[r] = 0.f;
-#pragma unroll 8
-      for (int e = 0; e < SEG; e += 4) {
-        const float4 wq = *reinterpret_cast<const float4*>(wv + e);
-#pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-          const float4 xq = *reinterpret_cast<const float4*>(xv + r * X_PITCH + e);
-          acc[r] = fmaf(xq.x, wq.x, acc[r]);
-          acc[r] = fmaf(xq.y, wq.y, acc[r]);
-          acc[r] = fmaf(xq.z, wq.z, acc[r]);
-          acc[r] = fmaf(xq.w, wq.w, acc[r]);
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < ROWS; ++r) sums[(feature * FEW_SEGS + segment) * ROWS + r] = acc[r];
-    }
-    __syncthreads();
-    if (round + stages < rounds) {
-      load_w(round + stages);
-      load_x(round + stages);
-      copy_commit();
-    }
-    if (owner) {
-      for (int s = 0; s < segments; ++s) {
-        part += sums[(own_feature * FEW_SEGS + s) * ROWS + own_row];
-        const int done = round * FEW_SEGS + s + 1;
-        if (done % part_segments == 0) {
-          total += part;
-          part = 0.f;
-        }
-      }
-    }
-  }
-  // a last part that is shorter than the others (0 if there is none: x + 0 is x)
-  total += part;
-  if (owner && col0 + own_feature < n && row0 + own_row < m)
-    c[(size_t)(row0 + own_row) * ldc + col0 + own_feature] = total + (bias ? bias[col0 + own_feature] : 0.f);
+__host__ __device__ constexpr unsigned f32_idesc(int m, int n) {         // D float, A and B bfloat16, both K-major
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((unsigned)(m >> 4) << 24);
 }
 
-// ---------------------------------------------------------------------------------------------- more rows
+// ---- the forms of the instructions for one block and for a pair
+template <bool PAIR>
+__device__ __forceinline__ void f32_tmem_alloc(unsigned holder, unsigned columns) {
+  if (!PAIR) { tmem_alloc(holder, columns); return; }
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(holder), "r"(columns) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+template <bool PAIR>
+__device__ __forceinline__ void f32_tmem_dealloc(unsigned address, unsigned columns) {
+  if (!PAIR) { tmem_dealloc(address, columns); return; }
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(address), "r"(columns) : "memory");
+}
+template <bool PAIR>
+__device__ __forceinline__ void f32_umma(unsigned tmem_d, unsigned long long w, unsigned long long x, unsigned idesc, unsigned accumulate) {
+  if (!PAIR) { umma_bf16(tmem_d, w, x, idesc, accumulate); return; }
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+               ::"r"(tmem_d), "l"(w), "l"(x), "r"(idesc), "r"(accumulate) : "memory");
+}
+// arrives on the barrier (in both blocks of the pair) once the products issued so far are done
+template <bool PAIR>
+__device__ __forceinline__ void f32_commit(unsigned bar, unsigned short pair_mask) {
+  if (!PAIR) { umma_commit(bar); return; }
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"(pair_mask) : "memory");
+}
+// arrives on the barrier of the block that issues the products
+template <bool PAIR>
+__device__ __forceinline__ void f32_arrive(unsigned bar, unsigned rank) {
+  if (!PAIR) { mbar_arrive(bar); return; }
+  asm volatile("{\n.reg .b32 remote;\nmapa.shared::cluster.u32 remote, %0, %1;\n"
+               "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [remote];\n}\n" ::"r"(bar), "r"(rank) : "memory");
+}
+// twice 8 columns of this thread's lane of tensor memory, in pairs
 typedef unsigned long long pair_t;          // two floats in a 64-bit register, for the packed instructions
-__device__ __forceinline__ pair_t pack(float lo, float hi) {
+__device__ __forceinline__ void tmem_load_2x8(unsigned first, unsigned second, pair_t (&v)[4], pair_t (&u)[4]) {
+  unsigned r[16];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n"
+               "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n"
+               "tcgen05.wait::ld.sync.aligned;"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                 "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(first), "r"(second) : "memory");
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[i] = ((pair_t)r[2 * i + 1] << 32) | r[2 * i];
+    u[i] = ((pair_t)r[9 + 2 * i] << 32) | r[8 + 2 * i];
+  }
+}
+__device__ __forceinline__ void add2(pair_t& acc, pair_t x) { asm volatile("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(x)); }
+__device__ __forceinline__ pair_t pack2(float low, float high) {
   pair_t v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(low), "f"(high));
   return v;
 }
-__device__ __forceinline__ void unpack(pair_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ void fma2(pair_t& acc, pair_t x, pair_t y) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y)); }
-__device__ __forceinline__ void add2(pair_t& acc, pair_t x) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(x)); }
+__device__ __forceinline__ float low_of(pair_t v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float high_of(pair_t v) { return __uint_as_float((unsigned)(v >> 32)); }
 
-// blockIdx.x: 128 weight rows, blockIdx.y: 64 rows of A, blockIdx.z (the rank in the cluster): part of K
+// Four neighbouring entries of a row, zeros outside of it.  WIDE: rows start on 16 bytes and K is a multiple of 4.
 template <bool WIDE>
-__global__ void __launch_bounds__(TILE_THREADS, 2)
-gemm_f32_tile_kernel(const float* __restrict__ a, const float* __restrict__ w, const float* __restrict__ bias,
-                     float* __restrict__ c, int m, int n, int k, int lda, int ldw, int ldc, int part_segments) {
-  // two buffers of operands, [k][row]; the finished tile of a part lies over them
-  __shared__ __align__(16) float smem[TILE_M * B_PITCH > 2 * TILE_K * (A_PITCH + B_PITCH) ? TILE_M * B_PITCH
-                                                                                       : 2 * TILE_K * (A_PITCH + B_PITCH)];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;             // 16 x 8 threads
-  const int row0 = blockIdx.y * TILE_M, col0 = blockIdx.x * TILE_N;
-  const int k_begin = blockIdx.z * part_segments * SEG, k_end = min(k, k_begin + part_segments * SEG);
-  const int steps = max(0, (k_end - k_begin + TILE_K - 1) / TILE_K);
+__device__ __forceinline__ float4 load_four(const float* row, int at, int k, bool live) {
+  float4 v;
+  if (WIDE) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %5, 0;\nmov.b32 %0, 0;\nmov.b32 %1, 0;\nmov.b32 %2, 0;\nmov.b32 %3, 0;\n"
+        "@p ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];\n}\n"
+        : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w) : "l"(row + at), "r"((int)(live && at < k)) : "memory");
+  } else {
+    v.x = live && at < k ? row[at] : 0.f;
+    v.y = live && at + 1 < k ? row[at + 1] : 0.f;
+    v.z = live && at + 2 < k ? row[at + 2] : 0.f;
+    v.w = live && at + 3 < k ? row[at + 3] : 0.f;
+  }
+  return v;
+}
+
+__device__ __forceinline__ unsigned pack_rn(float low, float high) {
+  unsigned r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(high), "f"(low));
+  return r;
+}
+__device__ __forceinline__ float upper_of(float v) { return __uint_as_float(__float_as_uint(v) & 0xffff0000u); }
+
+// the three parts of two floats, packed
+__device__ __forceinline__ void split_two(float x, float y, unsigned (&part)[F32_PLANES]) {
+  part[0] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+  const float rx = x - upper_of(x), ry = y - upper_of(y);                // exact
+  part[1] = pack_rn(rx, ry);
+  part[2] = pack_rn(rx - __uint_as_float(part[1] << 16), ry - upper_of(__uint_as_float(part[1])));
+}
+// The parts of four neighbouring entries of row `row` into the planes of a swizzled tile (rows of 64 entries, 128 bytes; the
+// 16-byte pieces of a row change places with its number), planes `plane_bytes` apart.
+__device__ __forceinline__ void put_four(unsigned tile, unsigned plane_bytes, int row, int quad, float4 v) {
+  unsigned p[F32_PLANES], q[F32_PLANES];
+  split_two(v.x, v.y, p);
+  split_two(v.z, v.w, q);
+  const unsigned at = tile + row * 128 + ((((unsigned)quad >> 1) ^ ((unsigned)row & 7u)) << 4) + ((unsigned)quad & 1u) * 8;
+#pragma unroll
+  for (int i = 0; i < F32_PLANES; ++i)
+    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + i * plane_bytes), "r"(p[i]), "r"(q[i]) : "memory");
+}
+
+// one element by fused multiply-adds in index order
+__device__ __noinline__ float plain_element(const float* a, const float* w, int k) {
+  float v = 0.f;
+  for (int i = 0; i < k; ++i) v = fmaf(a[i], w[i], v);
+  return v;
+}
+
+// blockIdx.x: 128 weight rows (neighbours are a pair), blockIdx.y: TOKENS rows of A, blockIdx.z: a range of K
+template <int TOKENS, bool PAIR, bool WIDE>
+__global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKENS, PAIR>::BLOCKS) gemm_f32_kernel(F32Args args) {
+  using S = F32Shape<TOKENS, PAIR>;
+  constexpr int LOADER_WARPS = S::LOADERS / 32, ADDER_WARPS = S::ADDERS / 32, ISSUE_WARP = LOADER_WARPS + ADDER_WARPS;
+  constexpr int OWN = TOKENS / (S::ADDERS / 128);                        // an adder warp has a quarter of the lanes and OWN tokens
+  constexpr int W_LOADS = F32_FEATURES * 16 / S::LOADERS, X_LOADS = S::X_ROWS * 16 / S::LOADERS, LINES = S::LOADERS / 16;
+  constexpr unsigned PAIRED = PAIR ? 2 : 1;
+  static_assert(X_LOADS >= 1 && OWN % 8 == 0 && S::TMEM >= 32 && S::TMEM <= 512, "shapes");
+  extern __shared__ unsigned char smem_unaligned[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_unaligned + 1023) & ~(uintptr_t)1023);
+  // of the buffers of shared memory: filled (in the issuing block), read; of the sums: finished, taken out (in the issuing block)
+  __shared__ __align__(8) unsigned long long full_bar[2], empty_bar[2], sum_full[2], sum_empty[2];
+  __shared__ unsigned tmem_holder;
+  __shared__ int abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const unsigned rank = srb_cluster_rank(), leader = PAIR ? rank & ~1u : rank;
+  const int feature0 = blockIdx.x * F32_FEATURES, token0 = blockIdx.y * TOKENS;
+  const int all_chunks = (args.k + F32_CHUNK - 1) / F32_CHUNK;
+  const int chunk0 = blockIdx.z * args.block_parts * args.part_chunks;
+  const int chunks = min(all_chunks, chunk0 + args.block_parts * args.part_chunks) - chunk0;
+
+  if (tid == 0) {
+    abort_flag = 0;
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&full_bar[b]), PAIRED * LOADER_WARPS);          // one lane of each warp, of both blocks
+      mbar_init(smem_u32(&empty_bar[b]), 1);
+      mbar_init(smem_u32(&sum_full[b]), 1);
+      mbar_init(smem_u32(&sum_empty[b]), PAIRED * ADDER_WARPS);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == ISSUE_WARP) f32_tmem_alloc<PAIR>(smem_u32(&tmem_holder), S::TMEM);
+  tc_fence_before();
+  if (PAIR) srb_cluster_sync();                                          // both blocks' barriers exist before anyone signals them
+  else __syncthreads();
+  tc_fence_after();
+  const unsigned tmem_base = tmem_holder;
+  const unsigned smem_base = smem_u32(smem);
+  float* level = reinterpret_cast<float*>(smem + 2 * S::BUFFER);
+  // sums of an adder's feature (its lane of tensor memory)
+  const int quarter = warp & 3, group = (warp - LOADER_WARPS) >> 2;
+  pair_t part[OWN / 2];
   srb_launch_dependents();
-  srb_grid_dependency_wait();
 
-  // a thread brings 4 neighbouring entries of K of 2 rows of A and of 4 rows of W
-  const int quad = (tid & 3) * 4, line = tid >> 2;                       // 32 lines
-  float4 held[6];
-  auto fetch = [&](int step) {
-    const int at = k_begin + step * TILE_K + quad;
+  if (warp < LOADER_WARPS) {
+    const int row = tid >> 4, quad = tid & 15;                           // of the first load; the next ones are LINES rows on
+    float4 held_w[W_LOADS], held_x[X_LOADS];
+    auto load_w = [&](int i, int chunk) {
+      const int r = feature0 + row + i * LINES;
+      held_w[i] = load_four<WIDE>(args.w + (size_t)r * args.ldw, (chunk0 + chunk) * F32_CHUNK + quad * 4, args.k, r < args.n && chunk < chunks);
+    };
+    auto load_x = [&](int i, int chunk) {
+      const int r = token0 + (int)(rank - leader) * S::X_ROWS + row + i * LINES;
+      held_x[i] = load_four<WIDE>(args.a + (size_t)r * args.lda, (chunk0 + chunk) * F32_CHUNK + quad * 4, args.k, r < args.m && chunk < chunks);
+    };
+    // A chunk's operands are split and put in place while the next one's travel.  The second half of those is asked for only
+    // behind the fence, which would wait for loads that have just been issued.
+    constexpr int EARLY = W_LOADS / 2;
+    auto put_w = [&](int chunk) {
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      const int row = i < 2 ? row0 + line + 32 * i : col0 + line + 32 * (i - 2);
-      const bool live = row < (i < 2 ? m : n);
-      const float* from = i < 2 ? a + (size_t)row * lda + at : w + (size_t)row * ldw + at;
-      if (WIDE) {
-        held[i] = live && at < k_end ? *reinterpret_cast<const float4*>(from) : make_float4(0.f, 0.f, 0.f, 0.f);
-      } else {
-        held[i].x = live && at + 0 < k_end ? from[0] : 0.f;
-        held[i].y = live && at + 1 < k_end ? from[1] : 0.f;
-        held[i].z = live && at + 2 < k_end ? from[2] : 0.f;
-        held[i].w = live && at + 3 < k_end ? from[3] : 0.f;
+      for (int i = 0; i < W_LOADS; ++i) {
+        put_four(smem_base + (chunk & 1) * S::BUFFER, S::W_PLANE, row + i * LINES, quad, held_w[i]);
+        if (i < EARLY) load_w(i, chunk + 1);
       }
+    };
+    auto load_late_w = [&](int chunk) {
+#pragma unroll
+      for (int i = EARLY; i < W_LOADS; ++i) load_w(i, chunk);
+    };
+    auto put_x = [&](int chunk) {
+#pragma unroll
+      for (int i = 0; i < X_LOADS; ++i)
+        put_four(smem_base + (chunk & 1) * S::BUFFER + F32_PLANES * S::W_PLANE, S::X_PLANE, row + i * LINES, quad, held_x[i]);
+      fence_proxy_async_shared();
+      __syncwarp();
+      if (lane == 0) f32_arrive<PAIR>(smem_u32(&full_bar[chunk & 1]), leader);
+#pragma unroll
+      for (int i = 0; i < X_LOADS; ++i) load_x(i, chunk + 1);
+    };
+    // The weights are written by no kernel of a step, so both buffers' share of them is brought ahead of the wait for the kernels ahead.
+#pragma unroll
+    for (int i = 0; i < W_LOADS; ++i) load_w(i, 0);
+    put_w(0);
+    load_late_w(1);
+    if (chunks > 1) {
+      put_w(1);
+      load_late_w(2);
     }
-  };
-  auto put = [&](int buffer) {
-    float* at_a = smem + buffer * TILE_K * (A_PITCH + B_PITCH);
-    float* at_b = at_a + TILE_K * A_PITCH;
+    srb_grid_dependency_wait();
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      float* to = i < 2 ? at_a + quad * A_PITCH + line + 32 * i : at_b + quad * B_PITCH + line + 32 * (i - 2);
-      const int pitch = i < 2 ? A_PITCH : B_PITCH;
-      to[0] = held[i].x; to[pitch] = held[i].y; to[2 * pitch] = held[i].z; to[3 * pitch] = held[i].w;
+    for (int i = 0; i < X_LOADS; ++i) load_x(i, 0);
+    put_x(0);
+    if (chunks > 1) put_x(1);
+    for (int chunk = 2; chunk < chunks; ++chunk) {
+      // the products of the chunk before the last have read this buffer
+      if (!mbar_wait_warp(smem_u32(&empty_bar[chunk & 1]), ((unsigned)(chunk >> 1) & 1u) ^ 1u, &abort_flag)) break;
+      put_w(chunk);
+      put_x(chunk);
+      load_late_w(chunk + 1);
     }
-  };
-
-  pair_t acc[8][4], sum[8][4];
+  } else if (warp == ISSUE_WARP) {
+    if (rank == leader) {
+      constexpr unsigned idesc = f32_idesc(PAIR ? 2 * F32_FEATURES : F32_FEATURES, TOKENS);
+      const unsigned short pair_mask = (unsigned short)(3u << leader);
+      const unsigned long long w_desc = smem_descriptor(smem_base), x_desc = smem_descriptor(smem_base + F32_PLANES * S::W_PLANE);
+      constexpr unsigned long long W2 = S::W_PLANE >> 4, X2 = S::X_PLANE >> 4, W3 = 2 * W2, X3 = 2 * X2;
+      for (int chunk = 0; chunk < chunks; ++chunk) {
+        const int b = chunk & 1;
+        bool ok = mbar_wait_warp(smem_u32(&full_bar[b]), (unsigned)(chunk >> 1) & 1u, &abort_flag);
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+        for (int h = 0; h < 2; ++h) {
+          ok = ok && mbar_wait_warp(smem_u32(&sum_empty[h]), ((unsigned)chunk & 1u) ^ 1u, &abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          if (elect_one()) {
+            const unsigned upper = tmem_base + h * 2 * TOKENS, others = upper + TOKENS;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = sum[i][j] = 0ull;
-
-  if (steps > 0) {
-    fetch(0);
-    put(0);
-  }
-  __syncthreads();
-  for (int step = 0; step < steps; ++step) {
-    const float* at_a = smem + (step & 1) * TILE_K * (A_PITCH + B_PITCH);
-    const float* at_b = at_a + TILE_K * A_PITCH;
-    if (step + 1 < steps) fetch(step + 1);
-#pragma unroll
-    for (int e = 0; e < TILE_K; ++e) {
-      const float4 a0 = *reinterpret_cast<const float4*>(at_a + e * A_PITCH + ty * 4);
-      const float4 a1 = *reinterpret_cast<const float4*>(at_a + e * A_PITCH + 32 + ty * 4);
-      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(at_b + e * B_PITCH + tx * 4);
-      const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(at_b + e * B_PITCH + 64 + tx * 4);
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const pair_t x = pack(av[i], av[i]);
-        fma2(acc[i][0], x, b0.x);
-        fma2(acc[i][1], x, b0.y);
-        fma2(acc[i][2], x, b1.x);
-        fma2(acc[i][3], x, b1.y);
-      }
-    }
-    if ((step + 1) % (SEG / TILE_K) == 0 || step + 1 == steps) {         // a segment is complete
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          add2(sum[i][j], acc[i][j]);
-          acc[i][j] = 0ull;
+            for (int s = 0; s < 2; ++s) {
+              const unsigned long long at = (unsigned long long)((b * S::BUFFER) >> 4) + (h * 2 + s) * 2, w = w_desc + at, x = x_desc + at;
+              f32_umma<PAIR>(upper, w, x, idesc, s > 0 ? 1u : 0u);
+              f32_umma<PAIR>(others, w + W3, x, idesc, s > 0 ? 1u : 0u);
+              f32_umma<PAIR>(others, w, x + X3, idesc, 1u);
+              f32_umma<PAIR>(others, w + W2, x + X2, idesc, 1u);
+              f32_umma<PAIR>(others, w + W2, x, idesc, 1u);
+              f32_umma<PAIR>(others, w, x + X2, idesc, 1u);
+            }
+            f32_commit<PAIR>(smem_u32(&sum_full[h]), pair_mask);
+            if (h == 1) f32_commit<PAIR>(smem_u32(&empty_bar[b]), pair_mask);
+          }
+          __syncwarp();
         }
+        if (!ok) break;
+      }
     }
-    if (step + 1 < steps) put((step + 1) & 1);
-    __syncthreads();
+  } else {
+    srb_grid_dependency_wait();                                          // the output may still be read by a kernel ahead
+    const unsigned column = tmem_base + ((unsigned)(quarter * 32) << 16) + group * OWN;
+#pragma unroll
+    for (int j = 0; j < OWN / 2; ++j) part[j] = 0ull;
+    bool ok = true;
+    float* own_level = level + group * OWN * F32_FEATURES + quarter * 32 + lane;
+    int parts_done = 0;
+    for (int chunk = 0; chunk < chunks && ok; ++chunk) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        ok = ok && mbar_wait_warp(smem_u32(&sum_full[h]), (unsigned)chunk & 1u, &abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int j0 = 0; j0 < OWN; j0 += 8) {
+          pair_t upper[4], others[4];
+          tmem_load_2x8(column + h * 2 * TOKENS + j0, column + h * 2 * TOKENS + TOKENS + j0, upper, others);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            add2(upper[j], others[j]);
+            add2(part[j0 / 2 + j], upper[j]);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) f32_arrive<PAIR>(smem_u32(&sum_empty[h]), leader);
+      }
+      if (PAIR && args.block_parts > 1 && ((chunk0 + chunk + 1) % args.part_chunks == 0 || chunk + 1 == chunks)) {
+        // A part is complete.  A block with all of them keeps their running sum; one with two leaves the first beside the second.
+        const bool last = chunk + 1 == chunks;
+        if (!last || args.block_parts == args.parts) {
+#pragma unroll
+          for (int j = 0; j < OWN / 2; ++j) {
+            float* at = own_level + 2 * j * F32_FEATURES;
+            if (parts_done > 0) part[j] = pack2(at[0] + low_of(part[j]), at[F32_FEATURES] + high_of(part[j]));
+            if (!last) {
+              at[0] = low_of(part[j]);
+              at[F32_FEATURES] = high_of(part[j]);
+              part[j] = 0ull;
+            }
+          }
+        }
+        ++parts_done;
+      }
+    }
+    if (!ok) {
+#pragma unroll
+      for (int j = 0; j < OWN / 2; ++j) part[j] = 0x7fffffff7fffffffull;
+    }
   }
 
-  const int parts = gridDim.z;
-  if (parts > 1) {
+  auto finish = [&](int row, int col, float v) {
+    if (row >= args.m || col >= args.n) return;
+    if (!isfinite(v)) v = plain_element(args.a + (size_t)row * args.lda, args.w + (size_t)col * args.ldw, args.k);
+    args.c[(size_t)row * args.ldc + col] = v + (args.bias ? args.bias[col] : 0.f);
+  };
+  const bool adder = warp >= LOADER_WARPS && warp < ISSUE_WARP;
+  const int blocks = gridDim.z;
+  if (blocks == 1) {
+    if (adder) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float* to = smem + ((i >> 2) * 32 + ty * 4 + (i & 3)) * B_PITCH + tx * 4;
-      *reinterpret_cast<ulonglong2*>(to) = make_ulonglong2(sum[i][0], sum[i][1]);
-      *reinterpret_cast<ulonglong2*>(to + 64) = make_ulonglong2(sum[i][2], sum[i][3]);
+      for (int j = 0; j < OWN; ++j)
+        finish(token0 + group * OWN + j, feature0 + quarter * 32 + lane, j & 1 ? high_of(part[j / 2]) : low_of(part[j / 2]));
     }
+    __syncwarp();
+    if (PAIR) srb_cluster_sync();                                        // nobody leaves while the other block may still signal
+  } else {
+    // This block's sums as [token][128 features] over the idle buffers (all products have read them).  The block of the cluster with
+    // range z of K adds rows z, z + blocks, ... over all ranges.
+    float* tile = reinterpret_cast<float*>(smem);
+    if (adder) {
+#pragma unroll
+      for (int j = 0; j < OWN; ++j)
+        tile[(group * OWN + j) * F32_FEATURES + quarter * 32 + lane] = j & 1 ? high_of(part[j / 2]) : low_of(part[j / 2]);
+    }
+    __syncwarp();
     srb_cluster_sync();
-    // block r of the cluster adds rows r, r + parts, ... of the tile over all parts, in part order
-    for (int r = blockIdx.z; r < TILE_M; r += parts) {
-      const int row = row0 + r, col = col0 + tid;
-      if (row >= m) break;
-      if (col >= n) continue;
-      float v = 0.f;
-      for (int b = 0; b < parts; ++b) v += srb_load_peer_shared(smem + r * B_PITCH + tid, b);
-      c[(size_t)row * ldc + col] = v + (bias ? bias[col] : 0.f);
+    constexpr int ROWS_AT_ONCE = S::THREADS / F32_FEATURES;
+    const int col = tid & (F32_FEATURES - 1), line = tid / F32_FEATURES;
+    const bool two = PAIR && args.block_parts == 2;
+    for (int r = (int)blockIdx.z + line * blocks; line < ROWS_AT_ONCE && r < TOKENS; r += ROWS_AT_ONCE * blocks) {
+      if (token0 + r >= args.m) break;
+      float first[F32_MAX_BLOCKS], second[F32_MAX_BLOCKS];
+#pragma unroll
+      for (int b = 0; b < F32_MAX_BLOCKS; ++b) {
+        const unsigned peer = (rank - blockIdx.z * PAIRED) + b * PAIRED;
+        first[b] = second[b] = 0.f;
+        if (b < blocks) {
+          if (two) first[b] = srb_load_peer_shared(level + r * F32_FEATURES + col, peer);
+          second[b] = srb_load_peer_shared(tile + r * F32_FEATURES + col, peer);
+        }
+      }
+      float v = two ? first[0] + second[0] : second[0];
+#pragma unroll
+      for (int b = 1; b < F32_MAX_BLOCKS; ++b) {
+        if (b < blocks) {
+          if (two) v += first[b];
+          v += second[b];
+        }
+      }
+      finish(token0 + r, feature0 + col, v);
     }
+    __syncwarp();
     srb_cluster_sync();                                                  // nobody leaves while its tile may still be read
-    return;
   }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int row = row0 + (i >> 2) * 32 + ty * 4 + (i & 3);
-    if (row >= m) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int col = col0 + (j >> 1) * 64 + tx * 4 + (j & 1) * 2;
-      float lo, hi;
-      unpack(sum[i][j], lo, hi);
-      if (col < n) c[(size_t)row * ldc + col] = 0.f + lo + (bias ? bias[col] : 0.f);
-      if (col + 1 < n) c[(size_t)row * ldc + col + 1] = 0.f + hi + (bias ? bias[col + 1] : 0.f);
-    }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == ISSUE_WARP) {
+    tc_fence_after();
+    f32_tmem_dealloc<PAIR>(tmem_base, S::TMEM);
   }
 }
 
-template <int ROWS, bool WIDE>
-static int launch_few(const float* a, const float* w, const float* bias, float* c, int m, int n, int k, int lda, int ldw, int ldc,
-                      int part_segments, cudaStream_t s) {
-  constexpr size_t STAGE = (size_t)(FEW_FEATURES * W_PITCH + ROWS * X_PITCH) * sizeof(float);
-  const int rounds = (k + ROUND_K - 1) / ROUND_K, stages = rounds < 2 ? rounds : 2;
-  const size_t smem = stages * STAGE + (size_t)FEW_FEATURES * FEW_SEGS * ROWS * sizeof(float);
-  SRB_CUDA_CALL(cudaFuncSetAttribute(gemm_f32_few_kernel<ROWS, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(2 * STAGE + FEW_FEATURES * FEW_SEGS * ROWS * sizeof(float))));
-  dim3 grid((n + FEW_FEATURES - 1) / FEW_FEATURES, (m + ROWS - 1) / ROWS);
-  SRB_CUDA_CALL(srb_launch(gemm_f32_few_kernel<ROWS, WIDE>, grid, dim3(FEW_THREADS), smem, s, a, w, bias, c, m, n, k, lda, ldw, ldc,
-                           part_segments, stages));
+template <int TOKENS, bool PAIR, bool WIDE>
+static int launch(F32Args args, int blocks, cudaStream_t s) {
+  using S = F32Shape<TOKENS, PAIR>;
+  auto kernel = gemm_f32_kernel<TOKENS, PAIR, WIDE>;
+  SRB_CUDA_CALL(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
+  args.block_parts = args.parts / blocks;
+  const unsigned features = (args.n + F32_FEATURES - 1) / F32_FEATURES;
+  dim3 grid(PAIR ? (features + 1) / 2 * 2 : features, (args.m + TOKENS - 1) / TOKENS, blocks);
+  if (grid.y > 65535) SRB_FAIL("gemm_f32: %d rows exceed one launch", args.m);
+  SRB_CUDA_CALL(srb_launch_clustered(kernel, grid, dim3(S::THREADS), S::SMEM, s, dim3(PAIR ? 2 : 1, 1, blocks), args));
   return SRB_OK;
+}
+
+template <int TOKENS, bool WIDE>
+static int launch_pairs(const F32Args& args, cudaStream_t s) {
+  // Pairs that share a tile: one that takes all of K, or as many as there are parts or half of that (4 at most), whichever ends first if
+  // a pair takes its chunks and some six more for its start and end.
+  const long long pairs = std::max(1, srb_sm_count() / 2);
+  const long long tiles = (long long)((args.n + 2 * F32_FEATURES - 1) / (2 * F32_FEATURES)) * ((args.m + TOKENS - 1) / TOKENS);
+  int blocks = 1;
+  long long best = -1;
+  for (int b : {1, args.parts / 2, args.parts}) {
+    if (b < 1 || b > F32_MAX_BLOCKS / 2) continue;
+    const long long cost = (tiles * b + pairs - 1) / pairs * ((long long)args.parts / b * args.part_chunks + 6);
+    if (best < 0 || cost < best) {
+      best = cost;
+      blocks = b;
+    }
+  }
+  return launch<TOKENS, true, WIDE>(args, blocks, s);
 }
 
 template <bool WIDE>
-static int dispatch(const float* a, const float* w, const float* bias, float* c, int m, int n, int k, int lda, int ldw, int ldc,
-                    cudaStream_t s) {
-  const int part_segments = gemm_part_segments(n, k);
-  if (m == 1) return launch_few<1, WIDE>(a, w, bias, c, m, n, k, lda, ldw, ldc, part_segments, s);
-  if (m == 2) return launch_few<2, WIDE>(a, w, bias, c, m, n, k, lda, ldw, ldc, part_segments, s);
-  if (m <= 4) return launch_few<4, WIDE>(a, w, bias, c, m, n, k, lda, ldw, ldc, part_segments, s);
-  if (m <= FEW_ROWS) return launch_few<8, WIDE>(a, w, bias, c, m, n, k, lda, ldw, ldc, part_segments, s);
-  const int segments = (k + SEG - 1) / SEG;
-  dim3 grid((n + TILE_N - 1) / TILE_N, (m + TILE_M - 1) / TILE_M, (segments + part_segments - 1) / part_segments);
-  if (grid.y > 65535) SRB_FAIL("gemm_f32: %d rows exceed one launch", m);
-  SRB_CUDA_CALL(srb_launch_clustered(gemm_f32_tile_kernel<WIDE>, grid, dim3(TILE_THREADS), 0, s, dim3(1, 1, grid.z), a, w, bias, c,
-                                     m, n, k, lda, ldw, ldc, part_segments));
-  return SRB_OK;
+static int dispatch(const F32Args& args, cudaStream_t s) {
+  if (args.m <= 16) return launch<16, false, WIDE>(args, args.parts, s);
+  if (args.m <= 32) return launch_pairs<32, WIDE>(args, s);
+  if (args.m <= 64) return launch_pairs<64, WIDE>(args, s);
+  return launch_pairs<128, WIDE>(args, s);
 }
 
 extern "C" int srb_gemm_f32(const float* a, const float* w, const float* bias, float* c, int m, int n, int k,
@@ -346,7 +477,11 @@ extern "C" int srb_gemm_f32(const float* a, const float* w, const float* bias, f
   if (k <= 0) SRB_FAIL("gemm_f32: inner size %d must be positive", k);
   if (lda < k || ldw < k || ldc < n) SRB_FAIL("gemm_f32: a leading dimension is smaller than its row");
   if ((m + 63) / 64 > 65535) SRB_FAIL("gemm_f32: %d rows exceed one launch", m);
+  const F32Parts parts = gemm_parts(n, k);
+  F32Args args = {};
+  args.a = a; args.w = w; args.bias = bias; args.c = c;
+  args.m = m; args.n = n; args.k = k; args.lda = lda; args.ldw = ldw; args.ldc = ldc;
+  args.parts = parts.count; args.part_chunks = parts.chunks;
   const bool wide = k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
-  return wide ? dispatch<true>(a, w, bias, c, m, n, k, lda, ldw, ldc, (cudaStream_t)stream)
-              : dispatch<false>(a, w, bias, c, m, n, k, lda, ldw, ldc, (cudaStream_t)stream);
+  return wide ? dispatch<true>(args, (cudaStream_t)stream) : dispatch<false>(args, (cudaStream_t)stream);
 }
