@@ -8,8 +8,6 @@ from __future__ import annotations
 from dataclasses import dataclass
 from typing import Any, Mapping, Optional, Tuple
 
-import numpy as np
-
 GREEDY_EPSILON = 1.1920929e-07       # f32::EPSILON: a temperature at or below it is greedy
 
 
@@ -52,20 +50,6 @@ class SamplingParams:
                                                     float(self.min_p) if self.min_p is not None else 0.0)
         object.__setattr__(self, "choice", (kind, self.effective_temperature, *cuts))
         object.__setattr__(self, "penalised", self.has_penalties)
-        object.__setattr__(self, "packed", self._packed())
-
-    def _packed(self) -> Optional[bytes]:
-        """``choice`` as a step's kernels read it, five words: the temperature of a row without cuts (0: greedy); of a row
-        with cuts its temperature, top_p, min_p and, as an integer, top_k (1, 1, 0 and 0 without).  None if 32 bits do not hold
-        top_k, which is refused when the row is sampled."""
-        kind, temperature, top_k, top_p, min_p = self.choice
-        if not -2 ** 31 <= top_k < 2 ** 31:
-            return None
-        words = np.empty(5, np.float32)
-        with np.errstate(over="ignore"):
-            words[:4] = (temperature if kind == "plain" else 0.0, temperature if kind == "cut" else 1.0, top_p, min_p)
-        words.view(np.int32)[4] = top_k
-        return words.tobytes()
 
     @classmethod
     def from_dict(cls, options: Optional[Mapping[str, Any]]) -> "SamplingParams":

@@ -35,8 +35,7 @@ class RequestRandom:
         self._generator = random.Random(int(key))
 
     def next_unit(self) -> float:
-        unit = self._generator.random()                       # in [0, 1)
-        return unit if unit < ONE_BELOW else ONE_BELOW
+        return min(max(self._generator.random(), 0.0), ONE_BELOW)
 
 
 class SeenCounts:
@@ -86,8 +85,8 @@ class Sampler:
         GPU.  ``request_ids`` name the rows' requests, for those with penalties (``logits`` is then
         changed in place, and the chosen tokens are counted as seen)."""
         rows = logits.shape[0]
-        packed, uniform = [], [0.0] * rows                         # what every row asks for, and its number
-        cut = []                                                   # rows with top-k / top-p / min-p
+        temperature, uniform = [0.0] * rows, [0.0] * rows          # of the rows sampled without cuts
+        cut, cut_options = [], []                                  # rows with top-k / top-p / min-p, and what they ask for
         penalised, penalties = [], []
         plain = False
         for r in range(rows):
@@ -99,18 +98,18 @@ class Sampler:
                 penalised.append(r)
                 penalties.append((seen_row, p.presence_penalty or 0.0, p.frequency_penalty or 0.0,
                                   p.repetition_penalty if p.repetition_penalty is not None else 1.0))
-            packed.append(p.packed)
-            kind = p.choice[0]
-            if kind == "greedy":
+            choice = p.choice
+            if choice[0] == "greedy":
                 continue
             uniform[r] = randoms[r].next_unit()
-            if kind == "cut":
+            if choice[0] == "cut":
                 cut.append(r)
-                if p.packed is None:
-                    raise OverflowError(f"top_k {p.choice[2]} is outside what 32 bits hold")
+                cut_options.append(choice)
             else:
+                temperature[r] = choice[1]
                 plain = True
-        device = self._upload(rows, packed, uniform, cut, penalised, penalties) if plain or cut or penalised else None
+        device = self._upload(rows, temperature, uniform, cut, cut_options, penalised, penalties) \
+            if plain or cut or penalised else None
         if penalised:
             seen_row, presence, frequency, repetition = device[-4:]
             ops.apply_penalties(logits, self.seen.table, seen_row.view(torch.int32), presence, frequency, repetition)
@@ -128,7 +127,7 @@ class Sampler:
             ops.count_picked(self.seen.table, seen_row.view(torch.int32), picked)
         return picked
 
-    def _upload(self, rows: int, packed, uniform, cut, penalised, penalties):
+    def _upload(self, rows: int, temperature, uniform, cut, cut_options, penalised, penalties):
         """What the step's kernels need per row, in one pinned buffer and one copy: float rows on the device (rows of ints
         among them, by their bits): temperature, uniform; with cuts temperature, top_p, min_p, top_k and the rows that have
         them; with penalties the rows of counts, presence, frequency and repetition."""
@@ -136,12 +135,15 @@ class Sampler:
         staging = torch.empty((count, rows), dtype=torch.float32, pin_memory=True)
         floats = staging.numpy()
         ints = floats.view(np.int32)
-        words = np.frombuffer(b"".join(packed), np.int32).reshape(rows, 5)       # SamplingParams.packed
-        ints[0], floats[1] = words[:, 0], uniform
+        floats[0], floats[1] = temperature, uniform
         if cut:
-            ints[2:6] = words[:, 1:].T
-            ints[6, :len(cut)] = cut
-            ints[6, len(cut):] = 0
+            floats[2:5] = ((1.0,), (1.0,), (0.0,))                 # of the rows without cuts, which no block takes up
+            ints[5:7] = 0
+            at = np.asarray(cut)
+            _, heat, top_k, top_p, min_p = zip(*cut_options)
+            floats[2, at], floats[3, at], floats[4, at] = heat, top_p, min_p
+            ints[5, at] = np.array(top_k, np.int32)                # (refuses what 32 bits do not hold)
+            ints[6, :len(cut)] = at
         if penalised:
             floats[-3:] = ((0.0,), (0.0,), (1.0,))
             ints[-4] = -1
