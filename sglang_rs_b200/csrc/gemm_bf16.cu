@@ -211,8 +211,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       ok = mbar_wait(smem_u32(&acc_bar), 0, &abort_flag);
       tc_fence_after();
     }
-    // The pipeline's stages are idle once the accumulator is complete: in SiLU mode the up half
-    // passes through them to the warps that hold the gate half ([64 features][16 tokens] floats).
+    // The pipeline's stages are idle once the accumulator is complete: in SiLU mode half of the gate and half of the up sums
+    // pass through them ([16 tokens][64 features] floats).
     float* exchange = reinterpret_cast<float*>(smem);
     const unsigned lane_address = tmem_base + ((unsigned)(quarter * 32) << 16);
 #pragma unroll 1
@@ -233,17 +233,23 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         for (int j = 0; j < 16; ++j) acc[j] *= __shfl_sync(0xffffffffu, factor, j);
       }
       if (EPI == EPI_SILU) {
-        if (quarter >= 2) {
+        // Gate lanes compute the first eight of the tokens and up lanes the others: each hands over the half that it does not use,
+        // as [token][64 features], so that a warp's 32 neighbours fall on 32 banks.  (With the up half as [feature][16 tokens], sixteen
+        // lanes on a bank, and the gate lanes computing alone, gate/up of 64 rows took 44.4 us at 4,096 x 24,576 against 41.4 now, 14.7
+        // against 11.1 at 1,024 x 6,144.)
+        const int column = (quarter & 1) * 32 + lane;
+        const bool up_lane = quarter >= 2;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) exchange[((quarter & 1) * 32 + lane) * 16 + j] = acc[j];
-        }
+        for (int j = 0; j < 8; ++j) exchange[((up_lane ? 0 : 8) + j) * 64 + column] = up_lane ? acc[j] : acc[8 + j];
         asm volatile("bar.sync 1, 128;" ::: "memory");       // the four epilogue warps only
-        if (quarter < 2 && ok && feature < args.features) {
+        if (ok && feature < args.features) {
+          const int first = up_lane ? 8 : 0;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int token = token0 + c + j;
+          for (int j = 0; j < 8; ++j) {
+            const int token = token0 + c + first + j;
             if (token >= token_limit) break;
-            const float g = acc[j], u = exchange[((quarter & 1) * 32 + lane) * 16 + j];
+            const float other = exchange[(first + j) * 64 + column];
+            const float g = up_lane ? other : acc[j], u = up_lane ? acc[8 + j] : other;
             reinterpret_cast<__nv_bfloat16*>(args.out)[(size_t)token * args.ldo + feature] =
                 __float2bfloat16_rn(srb_gated<true>(args.activation, g, u, args.act_param));
           }
