@@ -70,16 +70,20 @@ struct GemmArgs {
   const float* slot_weight;  // a factor on the input of every slot (its sums are multiplied by it), or null
 };
 
-template <int BLOCK_T, int EPI, int STAGES>
+// HALF: a block owns 64 weight rows (32 gate rows over 32 up rows) and its tile of W has only those; the instruction still reads 128, and the
+// sums of what lies behind them (lanes 64 and up) are nobody's.
+template <int BLOCK_T, int EPI, int STAGES, bool HALF>
 __global__ void __launch_bounds__(GEMM_THREADS, BLOCK_T <= 64 ? 2 : 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                  GemmArgs args) {
   // SiLU mode: the 128 rows of the A tile are 64 gate rows over the 64 up rows of the same features
-  constexpr int A_BYTES = GEMM_BLOCK_F * GEMM_BLOCK_K * 2;
+  static_assert(!HALF || EPI != EPI_ADD, "whole tiles are added");
+  constexpr int W_ROWS = HALF ? GEMM_BLOCK_F / 2 : GEMM_BLOCK_F;
+  constexpr int A_BYTES = W_ROWS * GEMM_BLOCK_K * 2;
   constexpr int B_BYTES = BLOCK_T * GEMM_BLOCK_K * 2;
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr int ACC_COLUMNS = BLOCK_T;
-  constexpr int FEATURES_PER_BLOCK = EPI == EPI_SILU ? GEMM_BLOCK_F / 2 : GEMM_BLOCK_F;
+  constexpr int FEATURES_PER_BLOCK = EPI == EPI_SILU ? W_ROWS / 2 : W_ROWS;
   constexpr unsigned TMEM_COLUMNS = ACC_COLUMNS <= 32 ? 32 : ACC_COLUMNS <= 64 ? 64 : ACC_COLUMNS <= 128 ? 128
                                                                                : ACC_COLUMNS <= 256 ? 256 : 512;
   extern __shared__ unsigned char smem_unaligned[];
@@ -204,8 +208,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     // epilogue: warp w may read TMEM lanes 32 * (w % 4) .. + 32
     srb_grid_dependency_wait();             // the output buffer may still be read by a kernel ahead
     const int quarter = warp & 3;
-    // SiLU mode: lanes 0..63 hold gate, lanes 64..127 up of the same 64 features
-    const int feature = EPI == EPI_SILU ? feature0 + (quarter & 1) * 32 + lane : feature0 + quarter * 32 + lane;
+    // SiLU mode: lanes 0..63 hold gate, lanes 64..127 up of the same 64 features (HALF: 0..31 and 32..63, 32 features)
+    const bool used = !HALF || quarter < 2, up_lane = HALF ? quarter == 1 : quarter >= 2;
+    const int column = (HALF ? 0 : (quarter & 1) * 32) + lane;
+    const int feature = EPI == EPI_SILU ? feature0 + column : feature0 + quarter * 32 + lane;
     bool ok = true;
     if (num_kb > 0) {
       ok = mbar_wait(smem_u32(&acc_bar), 0, &abort_flag);
@@ -222,7 +228,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       // the factors of these 16 slots, a lane each, fetched ahead of the accumulators
       const float factor = (EPI == EPI_SILU || EPI == EPI_ACT) && args.slot_weight
                                ? args.slot_weight[min(token0 + c + (lane & 15), token_limit - 1)] : 1.0f;
-      if (ok && num_kb > 0) {
+      if (ok && used && num_kb > 0) {
         tmem_load_16(lane_address + c, acc);
       } else {
 #pragma unroll
@@ -237,12 +243,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         // as [token][64 features], so that a warp's 32 neighbours fall on 32 banks.  (With the up half as [feature][16 tokens], sixteen
         // lanes on a bank, and the gate lanes computing alone, gate/up of 64 rows took 44.4 us at 4,096 x 24,576 against 41.4 now, 14.7
         // against 11.1 at 1,024 x 6,144.)
-        const int column = (quarter & 1) * 32 + lane;
-        const bool up_lane = quarter >= 2;
+        if (used) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) exchange[((up_lane ? 0 : 8) + j) * 64 + column] = up_lane ? acc[j] : acc[8 + j];
+          for (int j = 0; j < 8; ++j) exchange[((up_lane ? 0 : 8) + j) * 64 + column] = up_lane ? acc[j] : acc[8 + j];
+        }
         asm volatile("bar.sync 1, 128;" ::: "memory");       // the four epilogue warps only
-        if (ok && feature < args.features) {
+        if (ok && used && feature < args.features) {
           const int first = up_lane ? 8 : 0;
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
@@ -259,7 +265,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         // this block's partial tile as [token][128 features] floats over the idle pipeline stages
 #pragma unroll
         for (int j = 0; j < 16; ++j) exchange[(c + j) * GEMM_BLOCK_F + quarter * 32 + lane] = acc[j];
-      } else if (ok && feature < args.features) {
+      } else if (ok && used && feature < args.features) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const int token = token0 + c + j;
@@ -343,18 +349,20 @@ static int make_map(CUtensorMap* map, const void* base, long long rows, long lon
   return SRB_OK;
 }
 
-template <int BLOCK_T, int EPI>
+template <int BLOCK_T, int EPI, bool HALF>
 static int launch_gemm(const CUtensorMap& map_w, const CUtensorMap& map_x, const GemmArgs& args, int splits,
                        cudaStream_t s) {
-  constexpr int STAGE_BYTES = GEMM_BLOCK_F * GEMM_BLOCK_K * 2 + BLOCK_T * GEMM_BLOCK_K * 2;
+  constexpr int W_ROWS = HALF ? GEMM_BLOCK_F / 2 : GEMM_BLOCK_F;
+  constexpr int STAGE_BYTES = W_ROWS * GEMM_BLOCK_K * 2 + BLOCK_T * GEMM_BLOCK_K * 2;
   // Few tokens (decode): about 100 KB of stages, so that two blocks share an SM and one block's
   // set-up and epilogue hide behind the other's stream of weights.  Many tokens: one block per SM.
   constexpr int BUDGET = BLOCK_T <= 64 ? 108 * 1024 : 200 * 1024;
   constexpr int STAGES = BUDGET / STAGE_BYTES >= 8 ? 8 : BUDGET / STAGE_BYTES;
   static_assert(STAGES >= 3, "a pipeline needs at least three stages");
-  constexpr int FEATURES_PER_BLOCK = EPI == EPI_SILU ? GEMM_BLOCK_F / 2 : GEMM_BLOCK_F;
-  const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024;
-  auto kernel = gemm_bf16_kernel<BLOCK_T, EPI, STAGES>;
+  constexpr int FEATURES_PER_BLOCK = EPI == EPI_SILU ? W_ROWS / 2 : W_ROWS;
+  // (behind the last stage of 64 rows the instruction reads as far as 128 rows would go)
+  const size_t smem = (size_t)STAGES * STAGE_BYTES + (GEMM_BLOCK_F - W_ROWS) * GEMM_BLOCK_K * 2 + 1024;
+  auto kernel = gemm_bf16_kernel<BLOCK_T, EPI, STAGES, HALF>;
   SRB_CUDA_CALL(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((args.tokens + BLOCK_T - 1) / BLOCK_T, (args.features + FEATURES_PER_BLOCK - 1) / FEATURES_PER_BLOCK, splits);
   if (grid.y > 65535) SRB_FAIL("gemm_bf16: %d features exceed one launch", args.features);
@@ -364,15 +372,29 @@ static int launch_gemm(const CUtensorMap& map_w, const CUtensorMap& map_x, const
 }
 
 template <int EPI>
-static int dispatch_tokens(int block_t, const CUtensorMap& map_w, const CUtensorMap& map_x, const GemmArgs& args,
+static int dispatch_tokens(int block_t, bool half, const CUtensorMap& map_w, const CUtensorMap& map_x, const GemmArgs& args,
                            int splits, cudaStream_t s) {
-  switch (block_t) {
-    case 16: return launch_gemm<16, EPI>(map_w, map_x, args, splits, s);
-    case 32: return launch_gemm<32, EPI>(map_w, map_x, args, splits, s);
-    case 64: return launch_gemm<64, EPI>(map_w, map_x, args, splits, s);
-    case 128: return launch_gemm<128, EPI>(map_w, map_x, args, splits, s);
-    default: return launch_gemm<256, EPI>(map_w, map_x, args, splits, s);
+  if constexpr (EPI != EPI_ADD) {
+    if (half && block_t == 32) return launch_gemm<32, EPI, true>(map_w, map_x, args, splits, s);
+    if (half) return launch_gemm<64, EPI, true>(map_w, map_x, args, splits, s);
   }
+  switch (block_t) {
+    case 16: return launch_gemm<16, EPI, false>(map_w, map_x, args, splits, s);
+    case 32: return launch_gemm<32, EPI, false>(map_w, map_x, args, splits, s);
+    case 64: return launch_gemm<64, EPI, false>(map_w, map_x, args, splits, s);
+    case 128: return launch_gemm<128, EPI, false>(map_w, map_x, args, splits, s);
+    default: return launch_gemm<256, EPI, false>(map_w, map_x, args, splits, s);
+  }
+}
+
+// Whether the blocks of a product of few rows own 64 weight rows instead of 128 (the K splits, and with them the bits, are the same): from 17
+// tokens on, where whole tiles leave SMs without a block.  Measured behind a norm kernel, 64 tokens: q/k/v of 2,048 x 4,096 9.04 to
+// 7.82 us, gate/up of 2,048 x 12,288 19.5 to 17.8, of 1,024 x 6,144 13.1 to 12.4; 20 tokens 15.2 to 14.5 and 9.30 to 9.28.  With
+// up to 16 tokens a launch is bound by its chain of latencies and twice the blocks bring nothing (1 token 5.07 and 5.03 us, 12.8 both).
+static bool gemm_halves(int block_t, int features, int splits, int mode) {
+  if (block_t < 32 || block_t > 64 || mode == EPI_ADD) return false;
+  const int per_block = mode == EPI_SILU ? GEMM_BLOCK_F / 2 : GEMM_BLOCK_F;
+  return (long long)((features + per_block - 1) / per_block) * splits <= srb_sm_count();
 }
 
 // Tokens per block for a step of `tokens` rows: the smallest tile that holds them, 256 at most.
@@ -417,7 +439,8 @@ extern "C" int srb_gemm_bf16_param(const void* x, const void* w, void* out, int 
 
   CUtensorMap map_w, map_x;
   // rows beyond `features` (or beyond the matrix) are never stored; the map covers all rows of w
-  if (make_map(&map_w, w, rows_of_w, k, ldw, mode == EPI_SILU ? GEMM_BLOCK_F / 2 : GEMM_BLOCK_F) != SRB_OK)
+  const bool half = gemm_halves(block_t, features, splits, mode);
+  if (make_map(&map_w, w, rows_of_w, k, ldw, (mode == EPI_SILU ? GEMM_BLOCK_F / 2 : GEMM_BLOCK_F) / (half ? 2 : 1)) != SRB_OK)
     return SRB_ERR_INVALID;
   if (make_map(&map_x, x, tokens, k, ldx, block_t) != SRB_OK) return SRB_ERR_INVALID;
 
@@ -431,12 +454,12 @@ extern "C" int srb_gemm_bf16_param(const void* x, const void* w, void* out, int 
   if (used_splits != splits) SRB_FAIL("gemm_bf16: %d splits leave one without work for %d blocks of K", splits, total_k_blocks);
   cudaStream_t s = (cudaStream_t)stream;
   switch (mode) {
-    case EPI_BF16: return dispatch_tokens<EPI_BF16>(block_t, map_w, map_x, args, splits, s);
-    case EPI_F32: return dispatch_tokens<EPI_F32>(block_t, map_w, map_x, args, splits, s);
-    case EPI_SILU: return dispatch_tokens<EPI_SILU>(block_t, map_w, map_x, args, 1, s);
-    case EPI_ADD: return dispatch_tokens<EPI_ADD>(block_t, map_w, map_x, args, splits, s);
-    case EPI_ACT: return dispatch_tokens<EPI_ACT>(block_t, map_w, map_x, args, 1, s);
-    default: return dispatch_tokens<EPI_PARTIAL>(block_t, map_w, map_x, args, splits, s);
+    case EPI_BF16: return dispatch_tokens<EPI_BF16>(block_t, half, map_w, map_x, args, splits, s);
+    case EPI_F32: return dispatch_tokens<EPI_F32>(block_t, half, map_w, map_x, args, splits, s);
+    case EPI_SILU: return dispatch_tokens<EPI_SILU>(block_t, half, map_w, map_x, args, 1, s);
+    case EPI_ADD: return dispatch_tokens<EPI_ADD>(block_t, half, map_w, map_x, args, splits, s);
+    case EPI_ACT: return dispatch_tokens<EPI_ACT>(block_t, half, map_w, map_x, args, 1, s);
+    default: return dispatch_tokens<EPI_PARTIAL>(block_t, half, map_w, map_x, args, splits, s);
   }
 }
 
@@ -464,7 +487,7 @@ static int launch_grouped(const CUtensorMap& map_w, const CUtensorMap& map_x, co
   constexpr int STAGES = 200 * 1024 / STAGE_BYTES;
   constexpr int FEATURES_PER_BLOCK = EPI == EPI_SILU ? GEMM_BLOCK_F / 2 : GEMM_BLOCK_F;
   const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024;
-  auto kernel = gemm_bf16_kernel<BLOCK_T, EPI, STAGES>;
+  auto kernel = gemm_bf16_kernel<BLOCK_T, EPI, STAGES, false>;
   SRB_CUDA_CALL(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // tiles are the fastest grid dimension: the blocks of one feature block of one expert's neighbours run together
   dim3 grid(max_tiles, (args.features + FEATURES_PER_BLOCK - 1) / FEATURES_PER_BLOCK, 1);

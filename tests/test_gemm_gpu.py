@@ -243,3 +243,21 @@ def test_gate_up_of_fewer_rows_goes_where_the_rounds_are_full(tokens, takes):
     ops.raise_on_error_word(word)
     both = (x.to(DEV).double() @ w.to(DEV).double().T).cpu()
     assert got.shape == (tokens, inner) and relative_error(got, GATED["silu"](both[:, :inner], both[:, inner:])) < 1e-2
+
+
+@pytest.mark.parametrize("tokens", [17, 32, 33, 64])
+@pytest.mark.parametrize("features,k", [(32, 64), (65, 72), (200, 328), (4096, 1032)])
+def test_blocks_of_64_weight_rows_give_the_bits_of_whole_tiles(tokens, features, k):
+    """From 17 tokens on products that leave SMs idle run in blocks of 64 weight rows; up to 16 tokens the tiles are whole."""
+    g = torch.Generator().manual_seed(tokens + features)
+    x = torch.randn(tokens, k, generator=g).to(DEV, torch.bfloat16)
+    w = (torch.randn(2 * features, k, generator=g) * 0.1).to(DEV, torch.bfloat16)
+    word = ops.new_error_word(DEV)
+    calls = [dict(mode="bf16"), dict(mode="f32"), dict(mode="gated", features=features, up_row_offset=features, activation="silu")]
+    if k > 64:
+        calls.append(dict(mode="partial", splits=2))
+    for options in calls:
+        product = lambda rows: ops.gemm_bf16(rows, w if options["mode"] == "gated" else w[:features], word, **options)
+        whole = torch.cat([product(x[r:r + 16]) for r in range(0, tokens, 16)], dim=1 if options["mode"] == "partial" else 0)
+        assert torch.equal(product(x), whole), options
+    ops.raise_on_error_word(word)
