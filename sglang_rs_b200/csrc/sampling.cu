@@ -7,11 +7,13 @@
 // uniform u in [0, 1) picks the first index, in vocabulary order, whose running sum of
 // p exceeds u * sum(p).  A row with temperature <= 0 falls back to argmax.
 // Two kernels: 64 blocks per row reduce their chunk of the vocabulary, one block per row
-// finishes (a vocabulary of 150 thousand entries is too long for one block per row).
+// finishes (a vocabulary of 150 thousand entries is too long for one block per row).  Rows that the kernel with cuts will
+// take need not be read here: `rows_index` names the others (null: all).
 #include "common.cuh"
 #include <math.h>
 
 SRB_DEFINE_LAST_ERROR()
+SRB_DEFINE_PDL_SWITCH()
 
 #define SAMPLE_CHUNKS 64        // blocks that share one row's vocabulary in the first pass
 #define SAMPLE_THREADS 256
@@ -19,12 +21,14 @@ SRB_DEFINE_LAST_ERROR()
 // Pass 1, grid (SAMPLE_CHUNKS, rows): maximum, its lowest index, and sum of exp((l - max) / T)
 // over the block's contiguous chunk of the vocabulary.
 __global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_chunk_kernel(const float* __restrict__ logits, int vocab, int stride, const float* __restrict__ temperature,
-                    float* __restrict__ chunk_max, int* __restrict__ chunk_arg, float* __restrict__ chunk_sum) {
+sample_chunk_kernel(const float* __restrict__ logits, const int* __restrict__ rows_index, int vocab, int stride,
+                    const float* __restrict__ temperature, float* __restrict__ chunk_max, int* __restrict__ chunk_arg, float* __restrict__ chunk_sum) {
   __shared__ float sh_value[SAMPLE_THREADS / 32];
   __shared__ int sh_index[SAMPLE_THREADS / 32];
   __shared__ float scratch[33];
-  const int row = blockIdx.y, chunk = blockIdx.x;
+  srb_launch_dependents();
+  srb_grid_dependency_wait();
+  const int row = rows_index ? rows_index[blockIdx.y] : blockIdx.y, chunk = blockIdx.x;
   const float* l = logits + (size_t)row * stride;
   const int per_chunk = (vocab + SAMPLE_CHUNKS - 1) / SAMPLE_CHUNKS;
   const int begin = min(vocab, chunk * per_chunk), end = min(vocab, begin + per_chunk);
@@ -77,7 +81,8 @@ sample_chunk_kernel(const float* __restrict__ logits, int vocab, int stride, con
 // Pass 2, one block per row: the row's maximum; for a sampled row the chunk in which the
 // running sum (in vocabulary order) passes u * total, then the token inside that chunk.
 __global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_pick_kernel(const float* __restrict__ logits, int vocab, int stride, const float* __restrict__ temperature,
+sample_pick_kernel(const float* __restrict__ logits, const int* __restrict__ rows_index, int vocab, int stride,
+                   const float* __restrict__ temperature,
                    const float* __restrict__ uniform, const float* __restrict__ chunk_max,
                    const int* __restrict__ chunk_arg, const float* __restrict__ chunk_sum, int* __restrict__ out) {
   __shared__ __align__(16) float part_sum[SAMPLE_THREADS];
@@ -85,7 +90,9 @@ sample_pick_kernel(const float* __restrict__ logits, int vocab, int stride, cons
   __shared__ int part_arg[SAMPLE_CHUNKS];
   __shared__ float sh_max, sh_target, sh_prefix;
   __shared__ int sh_chunk;
-  const int row = blockIdx.x;
+  srb_launch_dependents();
+  srb_grid_dependency_wait();
+  const int row = rows_index ? rows_index[blockIdx.x] : blockIdx.x;
   const float* l = logits + (size_t)row * stride;
   const float temp = temperature ? temperature[row] : 0.f;
   const size_t base = (size_t)row * SAMPLE_CHUNKS;
@@ -468,6 +475,8 @@ sample_filtered_kernel(const float* __restrict__ logits, int vocab, long long st
                        const float* __restrict__ uniform, int slice, float* __restrict__ stored, int* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char fs_raw[];
   FsShared& sh = *reinterpret_cast<FsShared*>(fs_raw);
+  srb_launch_dependents();
+  srb_grid_dependency_wait();
   const int r = rows_index ? rows_index[blockIdx.y] : blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int blocks = gridDim.x, rank = blockIdx.x;
@@ -771,23 +780,27 @@ extern "C" int srb_sample_scratch_floats(int rows) { return rows * SAMPLE_CHUNKS
 
 // logits [rows, stride] with `vocab` valid columns; temperature and uniform are [rows] or
 // null (null temperature = greedy for every row); out [rows] int32; scratch holds
-// srb_sample_scratch_floats(rows) 4-byte words.
-extern "C" int srb_sample(const float* logits, int rows, int vocab, int stride, const float* temperature,
-                          const float* uniform, int* out, float* scratch, void* stream) {
-  if (rows <= 0) return SRB_OK;
+// srb_sample_scratch_floats(rows) 4-byte words.  `rows_index` (int32 [count] on the device, or null: all rows): the rows
+// that get a token, each below `rows`.
+extern "C" int srb_sample_rows(const float* logits, const int* rows_index, int count, int rows, int vocab, int stride,
+                               const float* temperature, const float* uniform, int* out, float* scratch, void* stream) {
+  if (rows <= 0 || count <= 0) return SRB_OK;
   if (vocab <= 0 || stride < vocab) SRB_FAIL("sample: vocabulary %d and stride %d do not fit", vocab, stride);
   if (temperature && !uniform) SRB_FAIL("sample: temperature sampling needs uniform numbers");
   if (!scratch) SRB_FAIL("sample: scratch memory is needed");
-  if (rows > 65535) SRB_FAIL("sample: %d rows exceed one launch", rows);
+  if (rows > 65535 || count > rows) SRB_FAIL("sample: %d of %d rows exceed one launch", count, rows);
   float* chunk_max = scratch;
   int* chunk_arg = reinterpret_cast<int*>(scratch + (size_t)rows * SAMPLE_CHUNKS);
   float* chunk_sum = scratch + (size_t)rows * SAMPLE_CHUNKS * 2;
   cudaStream_t s = (cudaStream_t)stream;
-  sample_chunk_kernel<<<dim3(SAMPLE_CHUNKS, rows), SAMPLE_THREADS, 0, s>>>(logits, vocab, stride, temperature,
-                                                                          chunk_max, chunk_arg, chunk_sum);
-  SRB_LAUNCH_CHECK("sample_chunk");
-  sample_pick_kernel<<<rows, SAMPLE_THREADS, 0, s>>>(logits, vocab, stride, temperature, uniform, chunk_max,
-                                                     chunk_arg, chunk_sum, out);
-  SRB_LAUNCH_CHECK("sample_pick");
+  SRB_CUDA_CALL(srb_launch(sample_chunk_kernel, dim3(SAMPLE_CHUNKS, count), dim3(SAMPLE_THREADS), 0, s, logits, rows_index, vocab, stride,
+                           temperature, chunk_max, chunk_arg, chunk_sum));
+  SRB_CUDA_CALL(srb_launch(sample_pick_kernel, dim3(count), dim3(SAMPLE_THREADS), 0, s, logits, rows_index, vocab, stride, temperature,
+                           uniform, chunk_max, chunk_arg, chunk_sum, out));
   return SRB_OK;
+}
+
+extern "C" int srb_sample(const float* logits, int rows, int vocab, int stride, const float* temperature,
+                          const float* uniform, int* out, float* scratch, void* stream) {
+  return srb_sample_rows(logits, nullptr, rows, rows, vocab, stride, temperature, uniform, out, scratch, stream);
 }

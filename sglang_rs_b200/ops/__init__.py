@@ -1826,9 +1826,10 @@ def scale_values(values: torch.Tensor, factor: float) -> None:
 
 @traced("sampling")
 def sample(logits: torch.Tensor, temperature: Optional[torch.Tensor], uniform: Optional[torch.Tensor],
-           out: Optional[torch.Tensor] = None) -> torch.Tensor:
+           out: Optional[torch.Tensor] = None, rows_index: Optional[torch.Tensor] = None) -> torch.Tensor:
     """One token per row of 32-bit logits: argmax where temperature is None or <= 0, else
-    inverse-CDF sampling of softmax(logits / temperature) with the row's uniform number."""
+    inverse-CDF sampling of softmax(logits / temperature) with the row's uniform number.  ``rows_index`` (int32): only the
+    rows that it names get a token (``out`` keeps what it has elsewhere)."""
     _need(logits, "logits", torch.float32)
     rows, vocab = logits.shape
     if out is None:
@@ -1837,9 +1838,13 @@ def sample(logits: torch.Tensor, temperature: Optional[torch.Tensor], uniform: O
     if temperature is not None:
         _need(temperature, "temperature", torch.float32); _need(uniform, "uniform", torch.float32)
     lib = load_library("sampling")
+    count = rows
+    if rows_index is not None:
+        _need(rows_index, "rows_index", torch.int32)
+        count = rows_index.numel()
     scratch = torch.empty(lib.srb_sample_scratch_floats(rows), dtype=torch.float32, device=logits.device)
-    _check(lib, lib.srb_sample(_ptr(logits), rows, vocab, logits.stride(0), _ptr(temperature), _ptr(uniform),
-                               _ptr(out), _ptr(scratch), _stream()), launches=2)
+    _check(lib, lib.srb_sample_rows(_ptr(logits), _ptr(rows_index), count, rows, vocab, logits.stride(0), _ptr(temperature), _ptr(uniform),
+                                    _ptr(out), _ptr(scratch), _stream()), launches=2)
     return out
 
 

@@ -113,16 +113,18 @@ class Sampler:
         if penalised:
             seen_row, presence, frequency, repetition = device[-4:]
             ops.apply_penalties(logits, self.seen.table, seen_row.view(torch.int32), presence, frequency, repetition)
-        if len(cut) == rows:
-            picked = torch.empty(rows, dtype=torch.int32, device=logits.device)      # every row is written below
+        if cut:
+            # the rows with cuts first in `index`, the others behind them: every row is written by one of the two
+            cut_temperature, top_p, min_p, top_k, index = device[2:7]
+            index = index.view(torch.int32)
+            picked = torch.empty(rows, dtype=torch.int32, device=logits.device)
+            if len(cut) < rows:
+                ops.sample(logits, device[0] if plain else None, device[1] if plain else None, picked, index[len(cut):])
+            ops.sample_filtered(logits, index[:len(cut)], cut_temperature, top_k.view(torch.int32), top_p, min_p, device[1], picked)
         elif plain:
             picked = ops.sample(logits, device[0], device[1])
         else:
             picked = ops.sample(logits, None, None)
-        if cut:
-            cut_temperature, top_p, min_p, top_k, index = device[2:7]
-            ops.sample_filtered(logits, index[:len(cut)].view(torch.int32), cut_temperature, top_k.view(torch.int32), top_p,
-                                min_p, device[1], picked)
         if penalised:
             ops.count_picked(self.seen.table, seen_row.view(torch.int32), picked)
         return picked
@@ -144,6 +146,9 @@ class Sampler:
             floats[2, at], floats[3, at], floats[4, at] = heat, top_p, min_p
             ints[5, at] = np.array(top_k, np.int32)                # (refuses what 32 bits do not hold)
             ints[6, :len(cut)] = at
+            others = np.ones(rows, bool)
+            others[at] = False
+            ints[6, len(cut):] = np.flatnonzero(others)
         if penalised:
             floats[-3:] = ((0.0,), (0.0,), (1.0,))
             ints[-4] = -1
