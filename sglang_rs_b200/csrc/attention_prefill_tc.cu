@@ -142,10 +142,10 @@ __device__ __forceinline__ void ex2_by_polynomial(float a0, float a1, float& p0,
                                          __uint_as_float((__float_as_uint(s1) << 23) + 0x3f800000u));
   unpack2(mul2(p, power), p0, p1);
 }
-// Which of eight neighbouring pairs of scores take it: two (not beside the polynomial of capped scores, which has those units
-// already).  More of them cost the softmax warps more instructions than the exponential unit saves: 2,048 rows behind 6,143 keys, 16
-// heads of 128, none 134.3 us, two 125.0, three 136.8, four 146.0; 2,048 rows from position 0, 32 heads, 44.1, 43.2, 45.3 and 47.3.
-#define TC_POLYNOMIAL_PAIRS 0x88u
+// Which of eight neighbouring pairs of scores take it (not beside the polynomial of capped scores, which has those units already).
+#ifndef TC_POLYNOMIAL_PAIRS
+#define TC_POLYNOMIAL_PAIRS 0x92u
+#endif
 
 // HEADS query heads of one kv head share a block (1 or 2): they read the same K and V tiles from
 // shared memory, which halves the traffic from L2.  STAGES tiles of K and of V are in flight.
