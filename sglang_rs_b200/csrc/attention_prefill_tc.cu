@@ -115,38 +115,6 @@ __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigne
   return d;
 }
 
-// Two exponentials 2^a, a <= 8, on the multiply-add units, for the share of a row's scores that the exponential unit has no time for:
-// a = n + f with n the nearest integer, 2^f by a polynomial (minimax with p(0) = 1, |f| <= 1/2: 9.1e-8, with its roundings at most
-// 2^-22.5 of the value, which is what ex2.approx promises), times 2^n put together from its bits.  2^-127 and less is 0, so -inf gives
-// 0 exactly; what is not a number stays so.
-__device__ __forceinline__ float max_nan(float a, float b) {
-  float d;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
-  return d;
-}
-__device__ __forceinline__ void ex2_by_polynomial(float a0, float a1, float& p0, float& p1) {
-  constexpr float ROUND = 12582912.0f;                     // 1.5 * 2^23: a sum with it is an integer, n in its low bits
-  const unsigned long long a = pack2(max_nan(a0, -127.0f), max_nan(a1, -127.0f));
-  const unsigned long long shifted = add2(a, pack2(ROUND, ROUND));
-  const unsigned long long n = add2(shifted, pack2(-ROUND, -ROUND));
-  const unsigned long long f = fma2(n, pack2(-1.0f, -1.0f), a);
-  unsigned long long p = pack2(0x1.5bba14p-10f, 0x1.5bba14p-10f);
-  p = fma2(p, f, pack2(0x1.3cea88p-7f, 0x1.3cea88p-7f));
-  p = fma2(p, f, pack2(0x1.c6b752p-5f, 0x1.c6b752p-5f));
-  p = fma2(p, f, pack2(0x1.ebf9bcp-3f, 0x1.ebf9bcp-3f));
-  p = fma2(p, f, pack2(0x1.62e42ap-1f, 0x1.62e42ap-1f));
-  p = fma2(p, f, pack2(1.0f, 1.0f));
-  float s0, s1;
-  unpack2(shifted, s0, s1);
-  const unsigned long long power = pack2(__uint_as_float((__float_as_uint(s0) << 23) + 0x3f800000u),
-                                         __uint_as_float((__float_as_uint(s1) << 23) + 0x3f800000u));
-  unpack2(mul2(p, power), p0, p1);
-}
-// Which of eight neighbouring pairs of scores take it (not beside the polynomial of capped scores, which has those units already).
-#ifndef TC_POLYNOMIAL_PAIRS
-#define TC_POLYNOMIAL_PAIRS 0x92u
-#endif
-
 // HEADS query heads of one kv head share a block (1 or 2): they read the same K and V tiles from
 // shared memory, which halves the traffic from L2.  STAGES tiles of K and of V are in flight.
 
@@ -451,11 +419,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           float a0, a1, a2, a3;
           unpack2(fma2(pack2(sv[c + j], sv[c + j + 1]), scale2, neg_m2), a0, a1);
           unpack2(fma2(pack2(sv[c + j + 2], sv[c + j + 3]), scale2, neg_m2), a2, a3);
-          float p0, p1, p2, p3;                            // 2^(-inf) = 0 for masked keys
-          if (!CAP && (TC_POLYNOMIAL_PAIRS >> (j / 2 % 8) & 1)) ex2_by_polynomial(a0, a1, p0, p1);
-          else { p0 = ex2(a0); p1 = ex2(a1); }
-          if (!CAP && (TC_POLYNOMIAL_PAIRS >> (j / 2 % 8 + 1) & 1)) ex2_by_polynomial(a2, a3, p2, p3);
-          else { p2 = ex2(a2); p3 = ex2(a3); }
+          const float p0 = ex2(a0), p1 = ex2(a1), p2 = ex2(a2), p3 = ex2(a3);          // 2^(-inf) = 0 for masked keys
           sums2[0] = add2(sums2[0], pack2(p0, p1));
           sums2[1] = add2(sums2[1], pack2(p2, p3));
           __nv_bfloat162 lo = __floats2bfloat162_rn(p0, p1), hi = __floats2bfloat162_rn(p2, p3);

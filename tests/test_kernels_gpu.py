@@ -1055,34 +1055,6 @@ def test_plan_of_routed_experts_by_one_block_and_by_a_cluster(rows, top, experts
     assert torch.equal(slot_weight[slots], weights[live])
 
 
-@pytest.mark.parametrize("bad", [math.inf, -math.inf, math.nan])
-def test_scores_that_are_not_finite_in_the_tensor_core_prefill_attention(bad):
-    """Exponentials from the exponential unit and from the polynomial beside it agree on what is not finite: a row that sees a key
-    whose score is infinite upwards or not a number has no number either, one whose score is -inf passes it over."""
-    rows, n, d = 130, 130, 128
-    case = paged_case(torch.bfloat16, 2, 1, d, 16, (n,), (rows,), None, seed=9)
-    tiles = torch.tensor([[r, min(128, rows - r), 0, r] for r in range(0, rows, 128)], dtype=torch.int32, device=DEV)
-
-    def run():
-        out, word = torch.empty_like(case["q"]), ops.new_error_word(DEV)
-        ops.tiled_attention_tc(case["q"], case["k_pool"], case["v_pool"], out, tiles, case["table"], scale=0.125, window=0, error_word=word)
-        ops.raise_on_error_word(word)
-        return out
-    case["q"][:, :, 0] = 1.0
-    pages, kept = case["table"][0], case["k_pool"]
-    for key in range(64, 80):                                # every pair of eight neighbouring ones
-        case["k_pool"] = kept.clone()
-        row = case["k_pool"][int(pages[key // 16]), 0, key % 16]
-        row[0] = bad
-        got = run()
-        row.zero_()
-        assert torch.equal(got[:key], run()[:key]), key
-        if bad == -math.inf:
-            assert bool(torch.isfinite(got).all()), key
-        else:
-            assert not bool(torch.isfinite(got[key:]).any()), key
-
-
 @pytest.mark.parametrize("n_q,n_kv,d,page", [(2, 2, 20, 8), (4, 2, 128, 16), (3, 1, 64, 4), (8, 2, 256, 16), (5, 1, 128, 16)])
 @pytest.mark.parametrize("window", [None, 20, 150])
 def test_float_splits_of_four_tiles(n_q, n_kv, d, page, window):
