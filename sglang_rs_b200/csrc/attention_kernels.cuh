@@ -531,7 +531,7 @@ paged_attention_rows_kernel(const float* __restrict__ q, const float* __restrict
 template <int DIM_PER_LANE>
 __global__ void __launch_bounds__(32 * SPLIT_TILES * SPLIT_MAX_HEADS)
 paged_attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_pool, const float* __restrict__ v_pool,
-                             float* __restrict__ part_acc, float* __restrict__ part_ml, AttnParams p) {
+                             float* __restrict__ out, float* __restrict__ part_acc, float* __restrict__ part_ml, AttnParams p) {
   extern __shared__ __align__(16) float smem[];
   __shared__ float tile_m[SPLIT_TILES * SPLIT_MAX_HEADS], tile_l[SPLIT_TILES * SPLIT_MAX_HEADS];
   const int d = p.head_dim, vd = p.value_dim, groups = p.n_q / p.n_kv;
@@ -542,11 +542,14 @@ paged_attention_split_kernel(const float* __restrict__ q, const float* __restric
   const int split = blockIdx.x, kv_head = blockIdx.y, row = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tile = warp / groups, head = warp % groups;
   srb_launch_dependents();
-  srb_grid_dependency_wait();
+  // the step's index arrays were copied in before its first kernel: they are read ahead of the wait for the kernels ahead
   const int pos = p.positions[row];
   int lo, hi;
   row_key_range(p, pos, split, lo, hi);
-  if (lo >= hi) return;
+  if (lo >= hi) {
+    srb_grid_dependency_wait();
+    return;
+  }
   const int request = p.row_request[row];
   // the key of this lane, and the row of the pool that holds it: -1 = masked
   const int key0 = lo / p.split_size * p.split_size + tile * KEY_BLOCK, key = key0 + lane;
@@ -560,6 +563,7 @@ paged_attention_split_kernel(const float* __restrict__ q, const float* __restric
       at = ((long long)page * p.n_kv + kv_head) * p.page_size + key % p.page_size;
     }
   }
+  srb_grid_dependency_wait();
   auto copy_rows = [&](float* to, int pitch, const float* pool, int width) {
     if (some) {
       for (int k = head; k < KEY_BLOCK; k += groups) {
@@ -638,7 +642,25 @@ paged_attention_split_kernel(const float* __restrict__ q, const float* __restric
     factor[t] = mine == -INFINITY ? (mass == 0.f ? 0.f : 1.f) : expf(mine - most);        // (a mass that is not a number stays)
     sum += mass * factor[t];
   }
-  const size_t slot = ((size_t)row * p.n_q + (size_t)kv_head * groups + warp) * p.max_splits + split;
+  const int q_head = kv_head * groups + warp;
+  if (p.max_splits == 1) {
+    // the one split of a short context: what attention_combine_kernel makes of it, which is not launched then
+    if (row_split_count(p, pos) > 1 && q_head == 0 && lane == 0 && p.error_word) atomicOr(p.error_word, SRB_FLAG_TOO_FEW_SPLITS);
+    const float top = p.sinks ? fmaxf(p.sinks[q_head], most) : most;
+    const float scale = expf(most - top), mass = (p.sinks ? expf(p.sinks[q_head] - top) : 0.f) + sum * scale;
+    const float inv = (p.gates ? p.gates[(size_t)row * p.n_q + q_head] * p.out_scale : p.out_scale) / mass;
+#pragma unroll
+    for (int j = 0; j < DIM_PER_LANE; ++j) {
+      const int e = lane + 32 * j;
+      if (e >= vd) continue;
+      float v = 0.f;
+#pragma unroll
+      for (int t = 0; t < SPLIT_TILES; ++t) v += results[(t * groups + warp) * vd + e] * factor[t];
+      out[(size_t)row * p.out_pitch + (size_t)q_head * vd + e] = v * scale * inv;
+    }
+    return;
+  }
+  const size_t slot = ((size_t)row * p.n_q + q_head) * p.max_splits + split;
 #pragma unroll
   for (int j = 0; j < DIM_PER_LANE; ++j) {
     const int e = lane + 32 * j;
@@ -731,7 +753,8 @@ static int launch_attention(const void* q, const void* k_pool, const void* v_poo
       auto split_kernel = paged_attention_split_kernel<DIM_PER_LANE>;
       SRB_CUDA_CALL(cudaFuncSetAttribute(split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATTN_SHARED_MOST - 1024));
       SRB_CUDA_CALL(srb_launch(split_kernel, dim3(p.max_splits, p.n_kv, rows), dim3(32 * SPLIT_TILES * groups), shared, s, (const float*)q,
-                               (const float*)k_pool, (const float*)v_pool, part_acc, part_ml, p));
+                               (const float*)k_pool, (const float*)v_pool, (float*)out, part_acc, part_ml, p));
+      if (p.max_splits == 1) return SRB_OK;
     }
   }
   const size_t smem = bytes(wide ? 4 : 1, async ? 2 : 1);
