@@ -192,8 +192,8 @@ __device__ __forceinline__ void copy_tile_async(float* tile, int k_pitch, const 
 // keys and values are multiples of four elements and start on four elements' borders; they move four elements at a time
 // through registers, and a score is four chains of additions (entries 0, 4, .. / 1, 5, .. / 2, 6, .. / 3, 7, ..).  ATTN_ASYNC (floats,
 // which need no conversion): the same rows as asynchronous copies, all of a tile in flight at once, into two tiles that
-// take turns, so that the copies of a tile run under the arithmetic of the one before.  Decoded rows of the 0.6B shape in
-// float32 (two rows of some 230 keys in splits of 128) take 17 us, through registers with four loads in flight 31.
+// take turns, so that the copies of a tile run under the arithmetic of the one before (two rows of some 230 keys in splits of 128, 16 heads
+// on 8 of 128: 17 us, through registers with four loads in flight 31; such splits now go to paged_attention_split_kernel).
 // A warp per query head that shares the kv head: up to 32 of them, 15 where values are wider than 512 entries (registers;
 // the dispatch cuts the heads into chunks by the same numbers).
 #define ATTN_WIDE_VALUE_WARPS 15
@@ -525,7 +525,7 @@ paged_attention_rows_kernel(const float* __restrict__ q, const float* __restrict
 
 // Decoded rows in floats, a split of SPLIT_TILES * 32 keys a block: its tiles side by side, a warp per (tile, head), and the warps' results
 // joined at the end in the order of the tiles.  All keys and values of the split are on their way at once; one tile after the other by a
-// warp per head, the latencies of four tiles add up.
+// warp per head, the latencies of four tiles add up: two rows of some 230 keys, 16 heads on 8 of 128, 17.1 us a layer then, 9.1 now.
 #define SPLIT_TILES 4
 #define SPLIT_MAX_HEADS 4                                // that share a kv head
 template <int DIM_PER_LANE>

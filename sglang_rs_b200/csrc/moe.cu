@@ -237,7 +237,8 @@ extern "C" int srb_moe_select(const float* logits, long long pitch, int rows, in
 //
 // A chain of latencies: count the entries of every expert, add up, hand out the slots.  One block, or the blocks of a cluster, each
 // with an equal run of the entries: an expert's slots go to the blocks in turn.  The count that an entry finds is its place among
-// those of its block, so the second pass adds two numbers.
+// those of its block, so the second pass adds two numbers.  (2,048 rows of 6 choices among 64 experts: 18.4 us by one block that counted
+// twice, 12.0 by eight.)
 __global__ void __launch_bounds__(1024)
 moe_plan_kernel(const int* __restrict__ chosen, int entries, int top, int experts, int max_tiles,
                 int tile_rows, int* __restrict__ plan, int* __restrict__ slot_row, int* __restrict__ entry_slot,
@@ -792,7 +793,8 @@ extern "C" int srb_moe_combine(const float* y, const int* entry_slot, const floa
 // rows of h in slot order: out[slot, :] = h[slot_row[slot], :] (16 bytes a thread where the rows allow it), for
 // products that take their operands as whole tiles of consecutive rows.  `used` (or null) points at the number of slots
 // that the plan handed out (its last offset): choices without a slot leave the slots behind it without a row.
-// A warp per slot: a row of 4 KB is eight loads a lane, all in flight.
+// A warp per slot: a row of 4 KB is eight loads a lane, all in flight.  (A block per slot with two loads a thread behind the one of the
+// slot's row: 28 us for 12,288 rows of 4 KB, 20 us now.)
 #define MOE_GATHER_WARPS 8
 template <typename T>
 __global__ void __launch_bounds__(32 * MOE_GATHER_WARPS)
