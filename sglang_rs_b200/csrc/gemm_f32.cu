@@ -21,8 +21,9 @@
 // What bounds it: the chain of roles over two buffers (450 rows, 4,096 x 1,024: 49.6 us; 36 with the splitting left out, 42 without later
 // loads, 43 with an eighth of the sums read, 45 without products), at 76 to 120 TFLOP/s of float products.  Fused multiply-adds over
 // tiles in shared memory took 124 us, 450 x 6,144 x 1,024 173 (now 79), 450 x 1,024 x 3,072 94 (59), 64 x 4,096 x 1,024 38 (25).
-// One and two rows are bound by latencies: 2 x 4,096 x 1,024 8.8 us behind another product, 7.5 by fused multiply-adds, 2 x 151,936 x
-// 1,024 144 and 151; inside a decode step, where the weights are split ahead of the wait, a step takes what it took.  Four stages of
+// One and two rows are bound by latencies and slower than fused multiply-adds, which could not give the same bits for all row counts:
+// 2 x 4,096 x 1,024 8.5 us behind another product (7.9 by fused multiply-adds), 2 x 1,024 x 3,072 9.7 with constant weights (the step
+// executor's), 12.0 where they are read behind the wait for the kernels ahead (7.8), 2 x 151,936 x 1,024 139 and 137 (160).  Four stages of
 // 32 entries in place of two buffers of 64, and the five small products summed over 128 entries, were 5 to 10 % slower.
 //
 // An element that comes out infinite or not a number is computed again by one chain of fused multiply-adds: the parts of an infinity are
@@ -42,6 +43,7 @@ SRB_DEFINE_PDL_SWITCH()
 #define F32_FEATURES 128      // weight rows of a block
 #define F32_CHUNK 64          // entries of K in a buffer of shared memory: a swizzled row of 128 bytes
 #define F32_PLANES 3          // bfloat16 parts of a float
+#define F32_EARLY_CHUNKS 4    // of the weights, that are asked into L2 ahead of the wait for the kernels ahead
 #define F32_MAX_PARTS 8
 #define F32_MAX_BLOCKS 8      // blocks of a cluster
 
@@ -61,6 +63,7 @@ struct F32Args {
   int m, n, k, lda, ldw, ldc;
   int parts, part_chunks;     // of K; chunks of a part
   int block_parts;            // parts that a block adds up: all, two or one
+  int constant;               // no kernel ahead writes w
 };
 
 // TOKENS rows of A of a block, or of a pair of blocks
@@ -270,23 +273,33 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
 #pragma unroll
       for (int i = 0; i < X_LOADS; ++i) load_x(i, chunk + 1);
     };
-    // The weights are written by no kernel of a step, so both buffers' share of them is brought ahead of the wait for the kernels ahead.
+    int chunk = 0;
+    if (args.constant) {
+      // Weights that no kernel ahead writes: both buffers' share of them is brought ahead of the wait for the kernels ahead.
 #pragma unroll
-    for (int i = 0; i < W_LOADS; ++i) load_w(i, 0);
-    put_w(0);
-    load_late_w(1);
-    if (chunks > 1) {
-      put_w(1);
-      load_late_w(2);
+      for (int i = 0; i < W_LOADS; ++i) load_w(i, 0);
+      put_w(0);
+      load_late_w(1);
+      if (chunks > 1) {
+        put_w(1);
+        load_late_w(2);
+      }
+      srb_grid_dependency_wait();
+#pragma unroll
+      for (int i = 0; i < X_LOADS; ++i) load_x(i, 0);
+      put_x(0);
+      if (chunks > 1) put_x(1);
+      chunk = min(2, chunks);
+    } else {
+      srb_grid_dependency_wait();
+#pragma unroll
+      for (int i = 0; i < X_LOADS; ++i) load_x(i, 0);
+#pragma unroll
+      for (int i = 0; i < W_LOADS; ++i) load_w(i, 0);
     }
-    srb_grid_dependency_wait();
-#pragma unroll
-    for (int i = 0; i < X_LOADS; ++i) load_x(i, 0);
-    put_x(0);
-    if (chunks > 1) put_x(1);
-    for (int chunk = 2; chunk < chunks; ++chunk) {
+    for (; chunk < chunks; ++chunk) {
       // the products of the chunk before the last have read this buffer
-      if (!mbar_wait_warp(smem_u32(&empty_bar[chunk & 1]), ((unsigned)(chunk >> 1) & 1u) ^ 1u, &abort_flag)) break;
+      if (chunk >= 2 && !mbar_wait_warp(smem_u32(&empty_bar[chunk & 1]), ((unsigned)(chunk >> 1) & 1u) ^ 1u, &abort_flag)) break;
       put_w(chunk);
       put_x(chunk);
       load_late_w(chunk + 1);
@@ -326,6 +339,11 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
       }
     }
   } else {
+    if (WIDE && tid - S::LOADERS < F32_FEATURES && feature0 + tid - S::LOADERS < args.n) {
+      // The weights of the first chunks are asked into L2 (nothing is read yet, so it does not matter who writes them).
+      const int first = chunk0 * F32_CHUNK, entries = min(args.k - first, min(chunks, F32_EARLY_CHUNKS) * F32_CHUNK);
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(args.w + (size_t)(feature0 + tid - S::LOADERS) * args.ldw + first), "r"(entries * 4) : "memory");
+    }
     srb_grid_dependency_wait();                                          // the output may still be read by a kernel ahead
     const unsigned column = tmem_base + ((unsigned)(quarter * 32) << 16) + group * OWN;
 #pragma unroll
@@ -479,8 +497,9 @@ static int dispatch(const F32Args& args, cudaStream_t s) {
   return launch_pairs<128, WIDE>(args, s);
 }
 
+// `constant_weights`: no kernel that the stream may still run writes w (the weights of a model), so it may be read before those are done.
 extern "C" int srb_gemm_f32(const float* a, const float* w, const float* bias, float* c, int m, int n, int k,
-                            int lda, int ldw, int ldc, void* stream) {
+                            int lda, int ldw, int ldc, int constant_weights, void* stream) {
   if (m <= 0 || n <= 0) return SRB_OK;
   if (k <= 0) SRB_FAIL("gemm_f32: inner size %d must be positive", k);
   if (lda < k || ldw < k || ldc < n) SRB_FAIL("gemm_f32: a leading dimension is smaller than its row");
@@ -490,6 +509,7 @@ extern "C" int srb_gemm_f32(const float* a, const float* w, const float* bias, f
   args.a = a; args.w = w; args.bias = bias; args.c = c;
   args.m = m; args.n = n; args.k = k; args.lda = lda; args.ldw = ldw; args.ldc = ldc;
   args.parts = parts.count; args.part_chunks = parts.chunks;
+  args.constant = constant_weights;
   const bool wide = k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
   return wide ? dispatch<true>(args, (cudaStream_t)stream) : dispatch<false>(args, (cudaStream_t)stream);
 }

@@ -285,6 +285,24 @@ def test_gemm_f32_edges_of_segments_rounds_tiles_and_parts(n, k):
             assert torch.equal(ops.linear(rows[130 - m:], w_d, b_d), whole[130 - m:]), (m, offset)
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 64, 64), (2, 1024, 1024), (16, 331, 1000), (40, 1024, 1024), (130, 257, 2052)])
+def test_float_products_whose_weights_the_kernel_ahead_writes(m, n, k):
+    """The second operand may come from a product just ahead, whose blocks let the next kernel in as they start."""
+    g = torch.Generator().manual_seed(n + k)
+    x = torch.randn(m, k, generator=g).to(DEV)
+    pairs = [(torch.randn(n, 512, generator=g).to(DEV), torch.randn(k, 512, generator=g).to(DEV)) for _ in range(6)]
+    want = []
+    for a, b in pairs:
+        weight = ops.linear(a, b)
+        torch.cuda.synchronize()
+        want.append(ops.linear(x, weight))
+        torch.cuda.synchronize()
+    weight = None
+    got = [ops.linear(x, ops.linear(a, b)) for a, b in pairs]
+    for one, other in zip(got, want):
+        assert torch.equal(one, other)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n_q,n_kv,d,page", [(4, 2, 128, 16), (1, 1, 20, 8), (3, 1, 18, 8), (12, 2, 64, 4)])
 def test_generic_attention_by_fours_and_one_by_one(dtype, n_q, n_kv, d, page):
