@@ -32,7 +32,8 @@
 // Weight layout and meaning as the reference's `linear`: row-major [out, in],
 // y[o] = sum_i x[i] * W[o, i] (crates/sglang-kernel/src/cpu.rs:73-108).
 //
-// Every wait is bounded; if one runs out the block's warps leave their loops and its results are computed by the plain chains too.
+// Every wait is bounded; if one runs out the block's warps leave their loops once the products in flight are done, its results are not
+// numbers, and the error word says so.
 #include "common.cuh"
 #include "tcgen05_helpers.cuh"
 #include <algorithm>
@@ -64,6 +65,7 @@ struct F32Args {
   int parts, part_chunks;     // of K; chunks of a part
   int block_parts;            // parts that a block adds up: all, two or one
   int constant;               // no kernel ahead writes w
+  int* error_word;            // or null
 };
 
 // TOKENS rows of A of a block, or of a pair of blocks
@@ -205,7 +207,7 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_unaligned + 1023) & ~(uintptr_t)1023);
   // of the buffers of shared memory: filled (in the issuing block), read; of the sums: finished, taken out (in the issuing block)
-  __shared__ __align__(8) unsigned long long full_bar[2], empty_bar[2], sum_full[2], sum_empty[2];
+  __shared__ __align__(8) unsigned long long full_bar[2], empty_bar[2], sum_full[2], sum_empty[2], drain_bar;
   __shared__ unsigned tmem_holder;
   __shared__ int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -223,6 +225,7 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
       mbar_init(smem_u32(&sum_full[b]), 1);
       mbar_init(smem_u32(&sum_empty[b]), PAIRED * ADDER_WARPS);
     }
+    mbar_init(smem_u32(&drain_bar), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == ISSUE_WARP) f32_tmem_alloc<PAIR>(smem_u32(&tmem_holder), S::TMEM);
@@ -310,9 +313,11 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
       const unsigned short pair_mask = (unsigned short)(3u << leader);
       const unsigned long long w_desc = smem_descriptor(smem_base), x_desc = smem_descriptor(smem_base + F32_PLANES * S::W_PLANE);
       constexpr unsigned long long W2 = S::W_PLANE >> 4, X2 = S::X_PLANE >> 4, W3 = 2 * W2, X3 = 2 * X2;
-      for (int chunk = 0; chunk < chunks; ++chunk) {
+      srb_grid_dependency_wait();                                        // the limit of the waits counts from here, as for the loaders
+      bool ok = true;
+      for (int chunk = 0; chunk < chunks && ok; ++chunk) {
         const int b = chunk & 1;
-        bool ok = mbar_wait_warp(smem_u32(&full_bar[b]), (unsigned)(chunk >> 1) & 1u, &abort_flag);
+        ok = mbar_wait_warp(smem_u32(&full_bar[b]), (unsigned)(chunk >> 1) & 1u, &abort_flag);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           ok = ok && mbar_wait_warp(smem_u32(&sum_empty[h]), ((unsigned)chunk & 1u) ^ 1u, &abort_flag);
@@ -335,9 +340,14 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
           }
           __syncwarp();
         }
-        if (!ok) break;
+      }
+      if (!ok) {                                                         // products that were issued may still read and write
+        if (elect_one()) f32_commit<PAIR>(smem_u32(&drain_bar), (unsigned short)(1u << leader));
+        __syncwarp();
+        mbar_wait_timed(smem_u32(&drain_bar), 0u);
       }
     }
+    srb_grid_dependency_wait();
   } else {
     if (WIDE && tid - S::LOADERS < F32_FEATURES && feature0 + tid - S::LOADERS < args.n) {
       // The weights of the first chunks are asked into L2 (nothing is read yet, so it does not matter who writes them).
@@ -389,15 +399,16 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
         ++parts_done;
       }
     }
-    if (!ok) {
-#pragma unroll
-      for (int j = 0; j < OWN / 2; ++j) part[j] = 0x7fffffff7fffffffull;
-    }
   }
+  __syncwarp();
+  __syncthreads();                                                       // every role has left its loop: nobody writes the buffers any more
+  const bool lost = abort_flag != 0;
+  if (tid == 0 && lost && args.error_word) atomicOr(args.error_word, SRB_FLAG_WAIT_TIMEOUT);
 
   auto finish = [&](int row, int col, float v) {
     if (row >= args.m || col >= args.n) return;
-    if (!isfinite(v)) v = plain_element(args.a + (size_t)row * args.lda, args.w + (size_t)col * args.ldw, args.k);
+    if (lost) v = __int_as_float(0x7fffffff);
+    else if (!isfinite(v)) v = plain_element(args.a + (size_t)row * args.lda, args.w + (size_t)col * args.ldw, args.k);
     args.c[(size_t)row * args.ldc + col] = v + (args.bias ? args.bias[col] : 0.f);
   };
   const bool adder = warp >= LOADER_WARPS && warp < ISSUE_WARP;
@@ -417,7 +428,8 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
     if (adder) {
 #pragma unroll
       for (int j = 0; j < OWN; ++j)
-        tile[(group * OWN + j) * F32_FEATURES + quarter * 32 + lane] = j & 1 ? high_of(part[j / 2]) : low_of(part[j / 2]);
+        tile[(group * OWN + j) * F32_FEATURES + quarter * 32 + lane] =
+            lost ? __int_as_float(0x7fffffff) : j & 1 ? high_of(part[j / 2]) : low_of(part[j / 2]);
     }
     __syncwarp();
     srb_cluster_sync();
@@ -497,9 +509,10 @@ static int dispatch(const F32Args& args, cudaStream_t s) {
   return launch_pairs<128, WIDE>(args, s);
 }
 
-// `constant_weights`: no kernel that the stream may still run writes w (the weights of a model), so it may be read before those are done.
+// `constant_weights`: no kernel that the stream may still run writes w (the weights of a model), so it may be read before those are done.  `error_word`
+// (or null) receives SRB_FLAG_WAIT_TIMEOUT.
 extern "C" int srb_gemm_f32(const float* a, const float* w, const float* bias, float* c, int m, int n, int k,
-                            int lda, int ldw, int ldc, int constant_weights, void* stream) {
+                            int lda, int ldw, int ldc, int constant_weights, int* error_word, void* stream) {
   if (m <= 0 || n <= 0) return SRB_OK;
   if (k <= 0) SRB_FAIL("gemm_f32: inner size %d must be positive", k);
   if (lda < k || ldw < k || ldc < n) SRB_FAIL("gemm_f32: a leading dimension is smaller than its row");
@@ -509,7 +522,7 @@ extern "C" int srb_gemm_f32(const float* a, const float* w, const float* bias, f
   args.a = a; args.w = w; args.bias = bias; args.c = c;
   args.m = m; args.n = n; args.k = k; args.lda = lda; args.ldw = ldw; args.ldc = ldc;
   args.parts = parts.count; args.part_chunks = parts.chunks;
-  args.constant = constant_weights;
+  args.constant = constant_weights; args.error_word = error_word;
   const bool wide = k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
   return wide ? dispatch<true>(args, (cudaStream_t)stream) : dispatch<false>(args, (cudaStream_t)stream);
 }

@@ -294,7 +294,7 @@ struct Run {
     produced->whole = out;
     if (skipped(skip_bit)) return SRB_OK;                      // a measurement leaves this product out
     if (model.dtype == SRB_DTYPE_F32) {
-      SX_KERNEL(gemm_f32, ((const float*)x, (const float*)l.weight, l.bias, (float*)out, m, n, k, k, k, n, 1, stream));
+      SX_KERNEL(gemm_f32, ((const float*)x, (const float*)l.weight, l.bias, (float*)out, m, n, k, k, k, n, 1, step.error_word, stream));
       return SRB_OK;
     }
     if (m <= step.own_gemm_max_tokens && k % 8 == 0) {

@@ -127,7 +127,7 @@ typedef struct SxKernels {
   SxLastError gated_mul_error;
   int (*add_bias)(void*, const float*, int, int, int, void*);
   SxLastError add_bias_error;
-  int (*gemm_f32)(const float*, const float*, const float*, float*, int, int, int, int, int, int, int, void*);
+  int (*gemm_f32)(const float*, const float*, const float*, float*, int, int, int, int, int, int, int, int*, void*);
   SxLastError gemm_f32_error;
   int (*gemm_bf16)(const void*, const void*, void*, int, int, int, int, int, int, int, int, int, int, int, int*, void*);
   SxLastError gemm_bf16_error;

@@ -1129,7 +1129,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         lib = load_library("gemm_f32")
         # (any call may have written the weights just ahead of this one: they are read behind it)
         _check(lib, lib.srb_gemm_f32(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), m, n, k, x.stride(0),
-                                     weight.stride(0), out.stride(0), 0, _stream()))
+                                     weight.stride(0), out.stride(0), 0, _ptr(error_word), _stream()))
         return out
     if m <= OWN_GEMM_MAX_TOKENS and error_word is not None and gemm_bf16_takes(k) and _rows_on_16_bytes(x):
         splits = gemm_splits(m, n, k) if partial_ok else 1

@@ -297,10 +297,26 @@ def test_float_products_whose_weights_the_kernel_ahead_writes(m, n, k):
         torch.cuda.synchronize()
         want.append(ops.linear(x, weight))
         torch.cuda.synchronize()
-    weight = None
-    got = [ops.linear(x, ops.linear(a, b)) for a, b in pairs]
+    weight, word = None, ops.new_error_word(DEV)
+    got = [ops.linear(x, ops.linear(a, b, error_word=word), error_word=word) for a, b in pairs]
+    ops.raise_on_error_word(word)
     for one, other in zip(got, want):
         assert torch.equal(one, other)
+
+
+def test_a_float_product_is_given_the_error_word(monkeypatch):
+    """Where a wait that runs out is noted: the kernel leaves no other sign of it than results that are not numbers."""
+    calls, library = [], ops.load_library("gemm_f32")
+
+    class Recorder:
+        def __getattr__(self, name):
+            return (lambda *a: calls.append(a) or 0) if name == "srb_gemm_f32" else getattr(library, name)
+
+    monkeypatch.setattr(ops, "load_library", lambda name: Recorder())
+    word = ops.new_error_word(DEV)
+    ops.linear(torch.ones(2, 8, device=DEV), torch.ones(4, 8, device=DEV), error_word=word)
+    ops.linear(torch.ones(2, 8, device=DEV), torch.ones(4, 8, device=DEV))
+    assert [getattr(c[-2], "value", c[-2]) or None for c in calls] == [word.data_ptr(), None]
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
