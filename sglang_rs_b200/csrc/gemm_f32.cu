@@ -1,30 +1,33 @@
 // C[M, N] = A[M, K] * W[N, K]^T (+ bias[N]) to 32-bit precision on the 5th-generation tensor cores.
 //
-// A float is the sum of three bfloat16 numbers exactly: its upper 8 bits of precision (cut off, so that the largest floats stay
-// finite), the upper 8 of what is left (rounded), and the rest.  A product of two floats is then nine products of bfloat16
-// numbers, which are exact in 32 bits; the three smallest (2^-24 of the product and less, of either sign) are left out, the six
-// others go to tcgen05.mma.  The unit adds with truncation, so nothing is left in it for long: of every 32 entries of K (two steps of
-// the instruction) the products of the upper parts have a sum of their own and the five others another; both start from zero and are
-// added to the result in registers, rounded to nearest.  Against 64 bits (2-norm, 450 rows, normal operands) the error is 0.5e-7 to
-// 1.2e-7 at K = 63 to 6,148; chains of 64 fused multiply-adds, what this kernel replaced, 1.4e-7 to 1.7e-7.  Where all operands are
-// positive the truncations add up: 6.1e-8 against 5.2e-8 at K = 3,072.
+// A float is the sum of three bfloat16 numbers: its upper six bits of precision to nearest, the upper eight of what is left to nearest, and
+// the rest.  A product of two floats is then nine products of bfloat16 numbers, which are exact in 32 bits; the smallest (2^-30 of the
+// product) is left out, the eight others go to tcgen05.mma.  The unit truncates what it adds, so nothing is left in it for long: of every
+// 64 entries of K the products of the upper parts have a sum of their own and the seven others another; both start from zero and are
+// added to the result in registers, rounded to nearest.  Products of six bits by six leave twelve bits of a sum to grow into: with eight
+// bits in the upper parts, the truncations of positive operands came to 3.3e-8 of the result even in sums of 32 entries; now 1.6e-8.
+// Against 64 bits (2-norm, 450 rows) the error of normal operands is 3.5e-8 to 1.2e-7 at K = 63 to 12,288 (chains of 64 fused
+// multiply-adds, what this kernel replaced, 1.4e-7 to 2.1e-7), of positive operands 4.1e-8 to 5.8e-8 (5.2e-8 to 1.1e-7), of normal operands
+// whose rows span 2^40 1.1e-7 to 1.6e-7 (1.1e-7 to 1.9e-7).
 //
 // The order of additions is a function of N and K only, so a row's result depends neither on M nor on the row's place in the
-// batch: sums of 32 entries are added in order to a part, and the parts (gemm_parts, at most 8) in order to the result.
+// batch: sums of 64 entries are added in order to a part, and the parts (gemm_parts, at most 8) in order or in pairs to the result.
 //
-// The weights are the M side of the instruction.  Up to 16 rows of A: a block owns 128 rows of W and a part of K.  More rows: a pair
-// of blocks on neighbouring SMs (cta_group::2) owns 256 rows of W and TOKENS (32, 64 or 128) rows of A, of which each block brings 128
-// and TOKENS / 2, and one, two or all parts of K.  The blocks of a tile are a cluster and add their sums through shared memory.
+// The weights are the M side of the instruction.  Up to 16 rows of A: a block owns 128 rows of W and one, two or all parts of K.  More
+// rows: a pair of blocks on neighbouring SMs (cta_group::2) owns 256 rows of W and TOKENS (32, 64 or 128) rows of A, of which each block
+// brings 128 and TOKENS / 2, and one, two or all parts of K.  The blocks of a tile are a cluster and add their sums through shared memory.
 // Warps of a block: eight bring both operands (plain loads: rows may start on any float; a thread asks for its pieces of the next chunk
 // while it splits those of the one before) and leave the parts in the swizzled layout that the unit reads; one issues the products (of the
 // pair, in its even block); the others read finished sums out of tensor memory and add them up.  No barrier spans the block in between.
-// What bounds it: the chain of roles over two buffers (450 rows, 4,096 x 1,024: 49.6 us; 36 with the splitting left out, 42 without later
-// loads, 43 with an eighth of the sums read, 45 without products), at 76 to 120 TFLOP/s of float products.  Fused multiply-adds over
-// tiles in shared memory took 124 us, 450 x 6,144 x 1,024 173 (now 79), 450 x 1,024 x 3,072 94 (59), 64 x 4,096 x 1,024 38 (25).
-// One and two rows are bound by latencies and slower than fused multiply-adds, which could not give the same bits for all row counts:
-// 2 x 4,096 x 1,024 8.5 us behind another product (7.9 by fused multiply-adds), 2 x 1,024 x 3,072 9.7 with constant weights (the step
-// executor's), 12.0 where they are read behind the wait for the kernels ahead (7.8), 2 x 151,936 x 1,024 139 and 137 (160).  Four stages of
-// 32 entries in place of two buffers of 64, and the five small products summed over 128 entries, were 5 to 10 % slower.
+// What bounds it: of some 3,500 cycles a chunk (450 rows) the products take 2,100 and the loaders 2,500, which split floats and wait for
+// L2; and a start and end of some 10,000.  Times in us, behind another product; in brackets six products in sums of 32 entries, then fused
+// multiply-adds over tiles in shared memory: 450 x 4,096 x 1,024 40 (50, 124), 450 x 6,144 x 1,024 72 (79, 173), 450 x 1,024 x 3,072 55 (60,
+// 94), 64 x 4,096 x 1,024 23 (25, 38), 2,048 x 4,096 x 1,024 151 (199, 456), 2,048 x 1,024 x 3,072, where pairs of blocks have two parts
+// each whatever the number of tiles, 144 (110, 350).
+// One and two rows are bound by latencies and by the unit's reads of W (eight per piece of it), and slower than fused multiply-adds, which
+// could not give the same bits for all row counts: 2 x 4,096 x 1,024 9.1 us (8.9, 7.9), 2 x 1,024 x 3,072 10.6 (9.8, 7.8), 2 x 151,936 x
+// 1,024 147 (141, 160) with constant weights, as the step executor's are; 11.4, 12.2 and 145 where they are read behind the wait for the
+// kernels ahead.
 //
 // An element that comes out infinite or not a number is computed again by one chain of fused multiply-adds: the parts of an infinity are
 // not its sum.
@@ -37,6 +40,7 @@
 #include "common.cuh"
 #include "tcgen05_helpers.cuh"
 #include <algorithm>
+#include <type_traits>
 
 SRB_DEFINE_LAST_ERROR()
 SRB_DEFINE_PDL_SWITCH()
@@ -48,14 +52,23 @@ SRB_DEFINE_PDL_SWITCH()
 #define F32_MAX_PARTS 8
 #define F32_MAX_BLOCKS 8      // blocks of a cluster
 
-// Parts of K: as many (a power of two) as keep the blocks of up to 16 rows resident at once, two to an SM, each of at least two chunks.
-struct F32Parts { int count, chunks; };      // parts, and the chunks of each but the last
+// Blocks along K for up to 16 rows, and parts of K, whose sums are rounded apart and then added.  Blocks: as many (a power of two) as are
+// resident at once, two to an SM, each of at least two chunks; eight only where an SM has one of them at most, since eight parts are
+// added in neighbouring pairs (a sequence of eight roundings was 5 % less exact on positive operands than multiply-adds) and a pair of
+// blocks that walks all of K has no room for that (two rows, 4,096 x 1,024: 9.7 us with four blocks, 10.1 with eight).  Parts: as many as
+// blocks, or, where that makes them long, twice as many or up to eight of at least eight chunks (of positive operands, 20,000 x 4,096, the
+// error is 5.2e-8 in eight parts and was 1.5e-7 in one).
+struct F32Parts { int count, chunks, blocks; };      // parts, the chunks of each but the last, blocks
 static inline F32Parts gemm_parts(int n, int k) {
   const int chunks = (k + F32_CHUNK - 1) / F32_CHUNK, tiles = (n + F32_FEATURES - 1) / F32_FEATURES;
-  int parts = 1;
-  while (parts < F32_MAX_PARTS && parts * 4 <= chunks && tiles * parts * 2 <= 296) parts *= 2;
+  int blocks = 1;
+  while (blocks < 4 && blocks * 4 <= chunks && tiles * blocks * 2 <= 296) blocks *= 2;
+  if (blocks == 4 && chunks >= 16 && tiles * 8 <= 148) blocks = 8;
+  int parts = blocks;
+  if (blocks == 4 && chunks > 64) parts = 8;
+  while (blocks < 4 && parts < (blocks == 1 ? F32_MAX_PARTS : 2 * blocks) && parts * 16 <= chunks) parts *= 2;
   while (parts > 1 && (parts - 1) * ((chunks + parts - 1) / parts) >= chunks) parts /= 2;        // no part is empty
-  return {parts, (chunks + parts - 1) / parts};
+  return {parts, (chunks + parts - 1) / parts, std::min(blocks, parts)};
 }
 
 struct F32Args {
@@ -64,6 +77,7 @@ struct F32Args {
   int m, n, k, lda, ldw, ldc;
   int parts, part_chunks;     // of K; chunks of a part
   int block_parts;            // parts that a block adds up: all, two or one
+  int in_pairs;               // neighbouring parts are added first
   int constant;               // no kernel ahead writes w
   int* error_word;            // or null
 };
@@ -79,7 +93,7 @@ struct F32Shape {
   static constexpr unsigned BUFFER = F32_PLANES * (W_PLANE + X_PLANE);
   static constexpr unsigned LEVEL = PAIR ? TOKENS * F32_FEATURES * 4 : 0;      // sums of earlier parts
   static constexpr unsigned SMEM = 2 * BUFFER + LEVEL + 1024;
-  static constexpr unsigned TMEM = 4 * TOKENS;                           // two sums, two buffers of them
+  static constexpr unsigned TMEM = 4 * TOKENS;                           // two sums of a chunk, two buffers of them
   static constexpr int BLOCKS = PAIR ? 1 : 2;                            // an SM
 };
 
@@ -169,10 +183,11 @@ __device__ __forceinline__ unsigned pack_rn(float low, float high) {
 }
 __device__ __forceinline__ float upper_of(float v) { return __uint_as_float(__float_as_uint(v) & 0xffff0000u); }
 
-// the three parts of two floats, packed
+// the three parts of two floats, packed: six bits to nearest, eight of what is left to nearest, the rest
 __device__ __forceinline__ void split_two(float x, float y, unsigned (&part)[F32_PLANES]) {
-  part[0] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
-  const float rx = x - upper_of(x), ry = y - upper_of(y);                // exact
+  const unsigned ux = (__float_as_uint(x) + 0x20000u) & 0xfffc0000u, uy = (__float_as_uint(y) + 0x20000u) & 0xfffc0000u;
+  part[0] = __byte_perm(ux, uy, 0x7632);
+  const float rx = x - __uint_as_float(ux), ry = y - __uint_as_float(uy);        // exact
   part[1] = pack_rn(rx, ry);
   part[2] = pack_rn(rx - __uint_as_float(part[1] << 16), ry - upper_of(__uint_as_float(part[1])));
 }
@@ -206,8 +221,8 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
   static_assert(X_LOADS >= 1 && OWN % 8 == 0 && S::TMEM >= 32 && S::TMEM <= 512, "shapes");
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_unaligned + 1023) & ~(uintptr_t)1023);
-  // of the buffers of shared memory: filled (in the issuing block), read; of the sums: finished, taken out (in the issuing block)
-  __shared__ __align__(8) unsigned long long full_bar[2], empty_bar[2], sum_full[2], sum_empty[2], drain_bar;
+  // of the buffers of shared memory: filled (in the issuing block), their products done; of the sums: taken out (in the issuing block)
+  __shared__ __align__(8) unsigned long long full_bar[2], done_bar[2], sum_empty[2], drain_bar;
   __shared__ unsigned tmem_holder;
   __shared__ int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -217,12 +232,21 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
   const int chunk0 = blockIdx.z * args.block_parts * args.part_chunks;
   const int chunks = min(all_chunks, chunk0 + args.block_parts * args.part_chunks) - chunk0;
 
+  float4 held_w[W_LOADS];
+  const int row = tid >> 4, quad = tid & 15;                             // of a loader's first load; the next ones are LINES rows on
+  auto load_w = [&](int i, int chunk) {
+    const int r = feature0 + row + i * LINES;
+    held_w[i] = load_four<WIDE>(args.w + (size_t)r * args.ldw, (chunk0 + chunk) * F32_CHUNK + quad * 4, args.k, r < args.n && chunk < chunks);
+  };
+  if (warp < LOADER_WARPS && args.constant) {                            // (beside the set-up)
+#pragma unroll
+    for (int i = 0; i < W_LOADS; ++i) load_w(i, 0);
+  }
   if (tid == 0) {
     abort_flag = 0;
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&full_bar[b]), PAIRED * LOADER_WARPS);          // one lane of each warp, of both blocks
-      mbar_init(smem_u32(&empty_bar[b]), 1);
-      mbar_init(smem_u32(&sum_full[b]), 1);
+      mbar_init(smem_u32(&done_bar[b]), 1);
       mbar_init(smem_u32(&sum_empty[b]), PAIRED * ADDER_WARPS);
     }
     mbar_init(smem_u32(&drain_bar), 1);
@@ -235,19 +259,15 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
   tc_fence_after();
   const unsigned tmem_base = tmem_holder;
   const unsigned smem_base = smem_u32(smem);
-  float* level = reinterpret_cast<float*>(smem + 2 * S::BUFFER);
+  float* level = reinterpret_cast<float*>(smem + (PAIR ? 2 * S::BUFFER : TOKENS * F32_FEATURES * 4));
   // sums of an adder's feature (its lane of tensor memory)
   const int quarter = warp & 3, group = (warp - LOADER_WARPS) >> 2;
   pair_t part[OWN / 2];
+  pair_t held[PAIR ? 1 : OWN / 2];                                       // few rows: the sums of earlier parts
   srb_launch_dependents();
 
   if (warp < LOADER_WARPS) {
-    const int row = tid >> 4, quad = tid & 15;                           // of the first load; the next ones are LINES rows on
-    float4 held_w[W_LOADS], held_x[X_LOADS];
-    auto load_w = [&](int i, int chunk) {
-      const int r = feature0 + row + i * LINES;
-      held_w[i] = load_four<WIDE>(args.w + (size_t)r * args.ldw, (chunk0 + chunk) * F32_CHUNK + quad * 4, args.k, r < args.n && chunk < chunks);
-    };
+    float4 held_x[X_LOADS];
     auto load_x = [&](int i, int chunk) {
       const int r = token0 + (int)(rank - leader) * S::X_ROWS + row + i * LINES;
       held_x[i] = load_four<WIDE>(args.a + (size_t)r * args.lda, (chunk0 + chunk) * F32_CHUNK + quad * 4, args.k, r < args.m && chunk < chunks);
@@ -268,8 +288,9 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
     };
     auto put_x = [&](int chunk) {
 #pragma unroll
-      for (int i = 0; i < X_LOADS; ++i)
+      for (int i = 0; i < X_LOADS; ++i) {
         put_four(smem_base + (chunk & 1) * S::BUFFER + F32_PLANES * S::W_PLANE, S::X_PLANE, row + i * LINES, quad, held_x[i]);
+      }
       fence_proxy_async_shared();
       __syncwarp();
       if (lane == 0) f32_arrive<PAIR>(smem_u32(&full_bar[chunk & 1]), leader);
@@ -278,9 +299,7 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
     };
     int chunk = 0;
     if (args.constant) {
-      // Weights that no kernel ahead writes: both buffers' share of them is brought ahead of the wait for the kernels ahead.
-#pragma unroll
-      for (int i = 0; i < W_LOADS; ++i) load_w(i, 0);
+      // Weights that no kernel ahead writes: both buffers' share of them is split ahead of the wait.
       put_w(0);
       load_late_w(1);
       if (chunks > 1) {
@@ -302,7 +321,7 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
     }
     for (; chunk < chunks; ++chunk) {
       // the products of the chunk before the last have read this buffer
-      if (chunk >= 2 && !mbar_wait_warp(smem_u32(&empty_bar[chunk & 1]), ((unsigned)(chunk >> 1) & 1u) ^ 1u, &abort_flag)) break;
+      if (chunk >= 2 && !mbar_wait_warp(smem_u32(&done_bar[chunk & 1]), ((unsigned)(chunk >> 1) & 1u) ^ 1u, &abort_flag)) break;
       put_w(chunk);
       put_x(chunk);
       load_late_w(chunk + 1);
@@ -315,31 +334,34 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
       constexpr unsigned long long W2 = S::W_PLANE >> 4, X2 = S::X_PLANE >> 4, W3 = 2 * W2, X3 = 2 * X2;
       srb_grid_dependency_wait();                                        // the limit of the waits counts from here, as for the loaders
       bool ok = true;
-      for (int chunk = 0; chunk < chunks && ok; ++chunk) {
-        const int b = chunk & 1;
-        ok = mbar_wait_warp(smem_u32(&full_bar[b]), (unsigned)(chunk >> 1) & 1u, &abort_flag);
+      auto issue = [&](auto buffer, int chunk) {
+        constexpr int b = decltype(buffer)::value;
+        if (!mbar_wait_warp(smem_u32(&full_bar[b]), (unsigned)(chunk >> 1) & 1u, &abort_flag) ||
+            !mbar_wait_warp(smem_u32(&sum_empty[b]), ((unsigned)(chunk >> 1) & 1u) ^ 1u, &abort_flag))
+          return false;
+        tc_fence_after();
+        if (elect_one()) {
+          const unsigned upper = tmem_base + b * 2 * TOKENS, others = upper + TOKENS;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          ok = ok && mbar_wait_warp(smem_u32(&sum_empty[h]), ((unsigned)chunk & 1u) ^ 1u, &abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-          if (elect_one()) {
-            const unsigned upper = tmem_base + h * 2 * TOKENS, others = upper + TOKENS;
-#pragma unroll
-            for (int s = 0; s < 2; ++s) {
-              const unsigned long long at = (unsigned long long)((b * S::BUFFER) >> 4) + (h * 2 + s) * 2, w = w_desc + at, x = x_desc + at;
-              f32_umma<PAIR>(upper, w, x, idesc, s > 0 ? 1u : 0u);
-              f32_umma<PAIR>(others, w + W3, x, idesc, s > 0 ? 1u : 0u);
-              f32_umma<PAIR>(others, w, x + X3, idesc, 1u);
-              f32_umma<PAIR>(others, w + W2, x + X2, idesc, 1u);
-              f32_umma<PAIR>(others, w + W2, x, idesc, 1u);
-              f32_umma<PAIR>(others, w, x + X2, idesc, 1u);
-            }
-            f32_commit<PAIR>(smem_u32(&sum_full[h]), pair_mask);
-            if (h == 1) f32_commit<PAIR>(smem_u32(&empty_bar[b]), pair_mask);
+          for (int s = 0; s < F32_CHUNK / 16; ++s) {
+            const unsigned long long w = w_desc + ((b * S::BUFFER) >> 4) + s * 2, x = x_desc + ((b * S::BUFFER) >> 4) + s * 2;
+            f32_umma<PAIR>(upper, w, x, idesc, s > 0 ? 1u : 0u);
+            f32_umma<PAIR>(others, w + W3, x + X2, idesc, s > 0 ? 1u : 0u);
+            f32_umma<PAIR>(others, w + W2, x + X3, idesc, 1u);
+            f32_umma<PAIR>(others, w + W3, x, idesc, 1u);
+            f32_umma<PAIR>(others, w, x + X3, idesc, 1u);
+            f32_umma<PAIR>(others, w + W2, x + X2, idesc, 1u);
+            f32_umma<PAIR>(others, w + W2, x, idesc, 1u);
+            f32_umma<PAIR>(others, w, x + X2, idesc, 1u);
           }
-          __syncwarp();
+          f32_commit<PAIR>(smem_u32(&done_bar[b]), pair_mask);
         }
+        __syncwarp();
+        return true;
+      };
+      for (int chunk = 0; chunk < chunks && ok; chunk += 2) {
+        ok = issue(std::integral_constant<int, 0>(), chunk);
+        if (ok && chunk + 1 < chunks) ok = issue(std::integral_constant<int, 1>(), chunk + 1);
       }
       if (!ok) {                                                         // products that were issued may still read and write
         if (elect_one()) f32_commit<PAIR>(smem_u32(&drain_bar), (unsigned short)(1u << leader));
@@ -349,7 +371,7 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
     }
     srb_grid_dependency_wait();
   } else {
-    if (WIDE && tid - S::LOADERS < F32_FEATURES && feature0 + tid - S::LOADERS < args.n) {
+    if (WIDE && !(PAIR && args.constant) && tid - S::LOADERS < F32_FEATURES && feature0 + tid - S::LOADERS < args.n) {
       // The weights of the first chunks are asked into L2 (nothing is read yet, so it does not matter who writes them).
       const int first = chunk0 * F32_CHUNK, entries = min(args.k - first, min(chunks, F32_EARLY_CHUNKS) * F32_CHUNK);
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(args.w + (size_t)(feature0 + tid - S::LOADERS) * args.ldw + first), "r"(entries * 4) : "memory");
@@ -362,31 +384,30 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
     float* own_level = level + group * OWN * F32_FEATURES + quarter * 32 + lane;
     int parts_done = 0;
     for (int chunk = 0; chunk < chunks && ok; ++chunk) {
+      const int b = chunk & 1;
+      ok = mbar_wait_warp(smem_u32(&done_bar[b]), (unsigned)(chunk >> 1) & 1u, &abort_flag);
+      if (!ok) break;
+      tc_fence_after();
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        ok = ok && mbar_wait_warp(smem_u32(&sum_full[h]), (unsigned)chunk & 1u, &abort_flag);
-        if (!ok) break;
-        tc_fence_after();
+      for (int j0 = 0; j0 < OWN; j0 += 8) {
+        pair_t upper[4], others[4];
+        tmem_load_2x8(column + b * 2 * TOKENS + j0, column + b * 2 * TOKENS + TOKENS + j0, upper, others);
 #pragma unroll
-        for (int j0 = 0; j0 < OWN; j0 += 8) {
-          pair_t upper[4], others[4];
-          tmem_load_2x8(column + h * 2 * TOKENS + j0, column + h * 2 * TOKENS + TOKENS + j0, upper, others);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            add2(upper[j], others[j]);
-            add2(part[j0 / 2 + j], upper[j]);
-          }
+        for (int j = 0; j < 4; ++j) {
+          add2(upper[j], others[j]);
+          add2(part[j0 / 2 + j], upper[j]);
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) f32_arrive<PAIR>(smem_u32(&sum_empty[h]), leader);
       }
-      if (PAIR && args.block_parts > 1 && ((chunk0 + chunk + 1) % args.part_chunks == 0 || chunk + 1 == chunks)) {
-        // A part is complete.  A block with all of them keeps their running sum; one with two leaves the first beside the second.
-        const bool last = chunk + 1 == chunks;
-        if (!last || args.block_parts == args.parts) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) f32_arrive<PAIR>(smem_u32(&sum_empty[b]), leader);
+      if (args.block_parts == 1 || ((chunk0 + chunk + 1) % args.part_chunks != 0 && chunk + 1 != chunks)) continue;
+      // A block with all parts keeps their running sum; one with two leaves the first beside the second.
+      const bool last = chunk + 1 == chunks;
+      if (!last || args.block_parts == args.parts) {
 #pragma unroll
-          for (int j = 0; j < OWN / 2; ++j) {
+        for (int j = 0; j < OWN / 2; ++j) {
+          if (PAIR) {
             float* at = own_level + 2 * j * F32_FEATURES;
             if (parts_done > 0) part[j] = pack2(at[0] + low_of(part[j]), at[F32_FEATURES] + high_of(part[j]));
             if (!last) {
@@ -394,72 +415,102 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
               at[F32_FEATURES] = high_of(part[j]);
               part[j] = 0ull;
             }
+          } else {
+            if (parts_done > 0) add2(part[j], held[PAIR ? 0 : j]);
+            if (!last) {
+              held[PAIR ? 0 : j] = part[j];
+              part[j] = 0ull;
+            }
           }
         }
-        ++parts_done;
+      }
+      ++parts_done;
+    }
+  }
+  __syncwarp();
+  __syncthreads();                                                       // every role has left its loop: the buffers take sums
+  const bool lost = abort_flag != 0;
+  if (tid == 0 && lost && args.error_word) atomicOr(args.error_word, SRB_FLAG_WAIT_TIMEOUT);
+
+  // This block's sums as [token][128 features], of two parts one behind the other.  The block of the cluster with range z of K adds rows
+  // z, z + blocks, ... over all ranges.
+  const int blocks = gridDim.z;
+  const bool two = blocks > 1 && args.block_parts == 2;
+  float* tile = reinterpret_cast<float*>(smem);
+  if (warp >= LOADER_WARPS && warp < ISSUE_WARP) {
+#pragma unroll
+    for (int j = 0; j < OWN; ++j) {
+      const int at = (group * OWN + j) * F32_FEATURES + quarter * 32 + lane;
+      tile[at] = lost ? __int_as_float(0x7fffffff) : j & 1 ? high_of(part[j / 2]) : low_of(part[j / 2]);
+      if (!PAIR && two) level[at] = j & 1 ? high_of(held[PAIR ? 0 : j / 2]) : low_of(held[PAIR ? 0 : j / 2]);
+    }
+  }
+  __syncwarp();
+  if (PAIR || blocks > 1) srb_cluster_sync();
+  else __syncthreads();
+  const unsigned first_rank = rank - blockIdx.z * PAIRED - (rank - leader);                  // of the blocks that share the tile
+  auto store = [&](int r, int f, float v) {
+    const int row = token0 + r, col = feature0 + f;
+    if (row >= args.m || col >= args.n) return;
+    if (!lost && !isfinite(v)) v = plain_element(args.a + (size_t)row * args.lda, args.w + (size_t)col * args.ldw, args.k);
+    args.c[(size_t)row * args.ldc + col] = v + (args.bias ? args.bias[col] : 0.f);
+  };
+  constexpr int LINES_AT_ONCE = S::THREADS / F32_FEATURES;
+  const int col = tid & (F32_FEATURES - 1), line = tid / F32_FEATURES, first_row = (int)blockIdx.z + line * blocks;
+  const int limit = min(TOKENS, args.m - token0);
+  if (line < LINES_AT_ONCE && first_row < limit) {
+    if (blocks == 1) {
+      constexpr int AT_ONCE = 4;
+      for (int r0 = first_row; r0 < limit; r0 += LINES_AT_ONCE * AT_ONCE) {
+        float v[AT_ONCE];
+#pragma unroll
+        for (int i = 0; i < AT_ONCE; ++i) v[i] = r0 + i * LINES_AT_ONCE < limit ? tile[(r0 + i * LINES_AT_ONCE) * F32_FEATURES + col] : 0.f;
+#pragma unroll
+        for (int i = 0; i < AT_ONCE; ++i)
+          if (r0 + i * LINES_AT_ONCE < limit) store(r0 + i * LINES_AT_ONCE, col, v[i]);
+      }
+    } else {
+      constexpr int MOST = PAIR ? F32_MAX_BLOCKS / 2 : F32_MAX_BLOCKS;
+      for (int r = first_row; r < limit; r += LINES_AT_ONCE * blocks) {
+        float first[MOST], second[MOST];
+#pragma unroll
+        for (int b = 0; b < MOST; ++b) {
+          const unsigned peer = first_rank + b * PAIRED + (rank - leader);
+          first[b] = second[b] = 0.f;
+          if (b < blocks) {
+            if (two) first[b] = srb_load_peer_shared(level + r * F32_FEATURES + col, peer);
+            second[b] = srb_load_peer_shared(tile + r * F32_FEATURES + col, peer);
+          }
+        }
+        float v = 0.f;
+        if (args.in_pairs) {
+          if (two) {
+#pragma unroll
+            for (int b = 0; b < MOST; ++b) v = b == 0 ? first[0] + second[0] : b < blocks ? v + (first[b] + second[b]) : v;
+          } else {
+#pragma unroll
+            for (int b = 0; b < MOST; b += 2) v = b == 0 ? second[0] + second[1] : b < blocks ? v + (second[b] + second[b + 1]) : v;
+          }
+        } else {
+          v = two ? first[0] + second[0] : second[0];
+#pragma unroll
+          for (int b = 1; b < MOST; ++b) {
+            if (b < blocks) {
+              if (two) v += first[b];
+              v += second[b];
+            }
+          }
+        }
+        store(r, col, v);
       }
     }
   }
   __syncwarp();
-  __syncthreads();                                                       // every role has left its loop: nobody writes the buffers any more
-  const bool lost = abort_flag != 0;
-  if (tid == 0 && lost && args.error_word) atomicOr(args.error_word, SRB_FLAG_WAIT_TIMEOUT);
-
-  auto finish = [&](int row, int col, float v) {
-    if (row >= args.m || col >= args.n) return;
-    if (lost) v = __int_as_float(0x7fffffff);
-    else if (!isfinite(v)) v = plain_element(args.a + (size_t)row * args.lda, args.w + (size_t)col * args.ldw, args.k);
-    args.c[(size_t)row * args.ldc + col] = v + (args.bias ? args.bias[col] : 0.f);
-  };
-  const bool adder = warp >= LOADER_WARPS && warp < ISSUE_WARP;
-  const int blocks = gridDim.z;
-  if (blocks == 1) {
-    if (adder) {
-#pragma unroll
-      for (int j = 0; j < OWN; ++j)
-        finish(token0 + group * OWN + j, feature0 + quarter * 32 + lane, j & 1 ? high_of(part[j / 2]) : low_of(part[j / 2]));
-    }
-    __syncwarp();
-    if (PAIR) srb_cluster_sync();                                        // nobody leaves while the other block may still signal
-  } else {
-    // This block's sums as [token][128 features] over the idle buffers (all products have read them).  The block of the cluster with
-    // range z of K adds rows z, z + blocks, ... over all ranges.
-    float* tile = reinterpret_cast<float*>(smem);
-    if (adder) {
-#pragma unroll
-      for (int j = 0; j < OWN; ++j)
-        tile[(group * OWN + j) * F32_FEATURES + quarter * 32 + lane] =
-            lost ? __int_as_float(0x7fffffff) : j & 1 ? high_of(part[j / 2]) : low_of(part[j / 2]);
-    }
-    __syncwarp();
-    srb_cluster_sync();
-    constexpr int ROWS_AT_ONCE = S::THREADS / F32_FEATURES;
-    const int col = tid & (F32_FEATURES - 1), line = tid / F32_FEATURES;
-    const bool two = PAIR && args.block_parts == 2;
-    for (int r = (int)blockIdx.z + line * blocks; line < ROWS_AT_ONCE && r < TOKENS; r += ROWS_AT_ONCE * blocks) {
-      if (token0 + r >= args.m) break;
-      float first[F32_MAX_BLOCKS], second[F32_MAX_BLOCKS];
-#pragma unroll
-      for (int b = 0; b < F32_MAX_BLOCKS; ++b) {
-        const unsigned peer = (rank - blockIdx.z * PAIRED) + b * PAIRED;
-        first[b] = second[b] = 0.f;
-        if (b < blocks) {
-          if (two) first[b] = srb_load_peer_shared(level + r * F32_FEATURES + col, peer);
-          second[b] = srb_load_peer_shared(tile + r * F32_FEATURES + col, peer);
-        }
-      }
-      float v = two ? first[0] + second[0] : second[0];
-#pragma unroll
-      for (int b = 1; b < F32_MAX_BLOCKS; ++b) {
-        if (b < blocks) {
-          if (two) v += first[b];
-          v += second[b];
-        }
-      }
-      finish(token0 + r, feature0 + col, v);
-    }
-    __syncwarp();
-    srb_cluster_sync();                                                  // nobody leaves while its tile may still be read
+  if (PAIR || blocks > 1) {
+    // Nobody leaves while its sums may still be read.  (What was read has arrived, as it was stored: no fence, which would wait for the
+    // stores.)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
@@ -491,7 +542,7 @@ static int launch_pairs(const F32Args& args, cudaStream_t s) {
   int blocks = 1;
   long long best = -1;
   for (int b : {1, args.parts / 2, args.parts}) {
-    if (b < 1 || b > F32_MAX_BLOCKS / 2) continue;
+    if (b < 1 || b > F32_MAX_BLOCKS / 2 || (args.in_pairs && b != args.parts / 2)) continue;      // (two parts that are added first)
     const long long cost = (tiles * b + pairs - 1) / pairs * ((long long)args.parts / b * args.part_chunks + 6);
     if (best < 0 || cost < best) {
       best = cost;
@@ -502,27 +553,26 @@ static int launch_pairs(const F32Args& args, cudaStream_t s) {
 }
 
 template <bool WIDE>
-static int dispatch(const F32Args& args, cudaStream_t s) {
-  if (args.m <= 16) return launch<16, false, WIDE>(args, args.parts, s);
+static int dispatch(const F32Args& args, int few_blocks, cudaStream_t s) {
+  if (args.m <= 16) return launch<16, false, WIDE>(args, few_blocks, s);
   if (args.m <= 32) return launch_pairs<32, WIDE>(args, s);
   if (args.m <= 64) return launch_pairs<64, WIDE>(args, s);
   return launch_pairs<128, WIDE>(args, s);
 }
 
-// `constant_weights`: no kernel that the stream may still run writes w (the weights of a model), so it may be read before those are done.  `error_word`
-// (or null) receives SRB_FLAG_WAIT_TIMEOUT.
+// `constant_weights`: no kernel that the stream may still run writes w (the weights of a model), so it may be read before those are done.
+// `error_word` (or null) receives SRB_FLAG_WAIT_TIMEOUT.
 extern "C" int srb_gemm_f32(const float* a, const float* w, const float* bias, float* c, int m, int n, int k,
                             int lda, int ldw, int ldc, int constant_weights, int* error_word, void* stream) {
   if (m <= 0 || n <= 0) return SRB_OK;
   if (k <= 0) SRB_FAIL("gemm_f32: inner size %d must be positive", k);
   if (lda < k || ldw < k || ldc < n) SRB_FAIL("gemm_f32: a leading dimension is smaller than its row");
-  if ((m + 63) / 64 > 65535) SRB_FAIL("gemm_f32: %d rows exceed one launch", m);
   const F32Parts parts = gemm_parts(n, k);
   F32Args args = {};
   args.a = a; args.w = w; args.bias = bias; args.c = c;
   args.m = m; args.n = n; args.k = k; args.lda = lda; args.ldw = ldw; args.ldc = ldc;
   args.parts = parts.count; args.part_chunks = parts.chunks;
-  args.constant = constant_weights; args.error_word = error_word;
+  args.in_pairs = parts.blocks == 8; args.constant = constant_weights; args.error_word = error_word;
   const bool wide = k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
-  return wide ? dispatch<true>(args, (cudaStream_t)stream) : dispatch<false>(args, (cudaStream_t)stream);
+  return wide ? dispatch<true>(args, parts.blocks, (cudaStream_t)stream) : dispatch<false>(args, parts.blocks, (cudaStream_t)stream);
 }
