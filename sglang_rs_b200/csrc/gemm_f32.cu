@@ -19,18 +19,24 @@
 // Warps of a block: eight bring both operands (plain loads: rows may start on any float; a thread asks for its pieces of the next chunk
 // while it splits those of the one before) and leave the parts in the swizzled layout that the unit reads; one issues the products (of the
 // pair, in its even block); the others read finished sums out of tensor memory and add them up.  No barrier spans the block in between.
-// What bounds it: of some 3,500 cycles a chunk (450 rows) the products take 2,100 and the loaders 2,500, which split floats and wait for
-// L2; and a start and end of some 10,000.  Times in us, behind another product; in brackets six products in sums of 32 entries, then fused
-// multiply-adds over tiles in shared memory: 450 x 4,096 x 1,024 40 (50, 124), 450 x 6,144 x 1,024 72 (79, 173), 450 x 1,024 x 3,072 55 (60,
-// 94), 64 x 4,096 x 1,024 23 (25, 38), 2,048 x 4,096 x 1,024 151 (199, 456), 2,048 x 1,024 x 3,072, where pairs of blocks have two parts
-// each whatever the number of tiles, 144 (110, 350).
-// One and two rows are bound by latencies and by the unit's reads of W (eight per piece of it), and slower than fused multiply-adds, which
-// could not give the same bits for all row counts: 2 x 4,096 x 1,024 9.1 us (8.9, 7.9), 2 x 1,024 x 3,072 10.6 (9.8, 7.8), 2 x 151,936 x
-// 1,024 147 (141, 160) with constant weights, as the step executor's are; 11.4, 12.2 and 145 where they are read behind the wait for the
-// kernels ahead.
 //
-// An element that comes out infinite or not a number is computed again by one chain of fused multiply-adds: the parts of an infinity are
-// not its sum.
+// The parts of an entry below 2^-126 lose bits, or all; products below that may be lost; infinities have no parts.  The loaders keep the
+// largest magnitude of each row of A and of a block's rows of W (two instructions to four entries; 2 us of 43 at 450 x 4,096 x 1,024).  A
+// result that is not large enough to hide what may be lost (K 2^-97 times the sum of both magnitudes leaves 2^-27 of it; rows of zeros are
+// exact), or whose operands have entries of 2^40 and more, is computed again in fused multiply-adds by a warp; one whose operands have an
+// entry that is not a number is not a number.  450 x 4,096 x 1,024 on one set of weights: 39 us; with a row that is not a number 39, all rows
+// 44; with a row of infinities or of entries above 2^40 93; a tenth of the entries below 2^-40 39; 250 rows of zeros 44.  (A thread a
+// result that is not finite: 105 for a row that is not a number, 15,700 for all.)
+//
+// What bounds it: of some 3,800 cycles a chunk (450 rows) the products take 2,100 and the loaders 2,800, which split floats and wait for
+// L2; and a start and end of some 12,000.  Times in us, behind another product; in brackets six products in sums of 32 entries without
+// regard for ranges, then fused multiply-adds over tiles in shared memory: 450 x 4,096 x 1,024 43 (50, 124), 450 x 6,144 x 1,024 81 (79,
+// 173), 450 x 1,024 x 3,072 60 (60, 94), 64 x 4,096 x 1,024 25 (25, 38), 2,048 x 4,096 x 1,024 163 (199, 456), 2,048 x 1,024 x 3,072, where
+// pairs of blocks have two parts each whatever the number of tiles, 158 (110, 350).
+// One and two rows are bound by latencies and by the unit's reads of W (eight per piece of it), and slower than fused multiply-adds, which
+// could not give the same bits for all row counts: 2 x 4,096 x 1,024 9.5 us (8.9, 7.9), 2 x 1,024 x 3,072 10.7 (9.8, 7.8), 2 x 151,936 x
+// 1,024 149 (141, 160) with constant weights, as the step executor's are; 11.6, 12.5 and 147 where they are read behind the wait for the
+// kernels ahead.
 //
 // Weight layout and meaning as the reference's `linear`: row-major [out, in],
 // y[o] = sum_i x[i] * W[o, i] (crates/sglang-kernel/src/cpu.rs:73-108).
@@ -78,6 +84,7 @@ struct F32Args {
   int parts, part_chunks;     // of K; chunks of a part
   int block_parts;            // parts that a block adds up: all, two or one
   int in_pairs;               // neighbouring parts are added first
+  float unit;                 // K * 2^-97
   int constant;               // no kernel ahead writes w
   int* error_word;            // or null
 };
@@ -191,23 +198,40 @@ __device__ __forceinline__ void split_two(float x, float y, unsigned (&part)[F32
   part[1] = pack_rn(rx, ry);
   part[2] = pack_rn(rx - __uint_as_float(part[1] << 16), ry - upper_of(__uint_as_float(part[1])));
 }
+// Notes on a row of W: it has an entry
+#define F32_LARGE 1u          // of 2^40 or more, or infinite
+#define F32_NAN 2u            // that is not a number
+#define F32_LIMIT 0x53800000u // the bits of 2^40
+// the largest magnitude so far, or not a number
+__device__ __forceinline__ void take_largest(float& high, float4 v) {
+  asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(high) : "f"(v.x), "f"(v.y));
+  asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(high) : "f"(v.z), "f"(v.w));
+}
+__device__ __noinline__ void note_row(float4 v, unsigned* row_notes) {
+  float high = 0.f;
+  take_largest(high, v);
+  if (!(high < 0x1p40f)) atomicOr(row_notes, high != high ? F32_NAN : F32_LARGE);
+}
+
 // The parts of four neighbouring entries of row `row` into the planes of a swizzled tile (rows of 64 entries, 128 bytes; the
 // 16-byte pieces of a row change places with its number), planes `plane_bytes` apart.
-__device__ __forceinline__ void put_four(unsigned tile, unsigned plane_bytes, int row, int quad, float4 v) {
+__device__ __forceinline__ void put_four(unsigned tile, unsigned plane_bytes, int row, int quad, float4 v, float& high) {
   unsigned p[F32_PLANES], q[F32_PLANES];
   split_two(v.x, v.y, p);
   split_two(v.z, v.w, q);
+  take_largest(high, v);
   const unsigned at = tile + row * 128 + ((((unsigned)quad >> 1) ^ ((unsigned)row & 7u)) << 4) + ((unsigned)quad & 1u) * 8;
 #pragma unroll
   for (int i = 0; i < F32_PLANES; ++i)
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + i * plane_bytes), "r"(p[i]), "r"(q[i]) : "memory");
 }
 
-// one element by fused multiply-adds in index order
-__device__ __noinline__ float plain_element(const float* a, const float* w, int k) {
+// one element by a warp: a chain of fused multiply-adds a lane, their sums in a tree
+__device__ __noinline__ float plain_element(const float* a, const float* w, int k, int lane) {
   float v = 0.f;
-  for (int i = 0; i < k; ++i) v = fmaf(a[i], w[i], v);
-  return v;
+#pragma unroll 4
+  for (int i = lane; i < k; i += 32) v = fmaf(a[i], w[i], v);
+  return srb_warp_sum(v);
 }
 
 // blockIdx.x: 128 weight rows (neighbours are a pair), blockIdx.y: TOKENS rows of A, blockIdx.z: a range of K
@@ -223,6 +247,9 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_unaligned + 1023) & ~(uintptr_t)1023);
   // of the buffers of shared memory: filled (in the issuing block), their products done; of the sums: taken out (in the issuing block)
   __shared__ __align__(8) unsigned long long full_bar[2], done_bar[2], sum_empty[2], drain_bar;
+  // the largest magnitude (as bits) of each row of A and of W, there 2^40 at most with the upper bit for rows that have notes
+  __shared__ unsigned x_most[S::X_ROWS], w_most, w_notes[F32_FEATURES];
+  __shared__ unsigned tile_x_most[PAIR ? TOKENS : 1], tile_w_most;                   // of all blocks that share the tile
   __shared__ unsigned tmem_holder;
   __shared__ int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -242,8 +269,10 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
 #pragma unroll
     for (int i = 0; i < W_LOADS; ++i) load_w(i, 0);
   }
+  for (int i = tid; i < F32_FEATURES; i += S::THREADS) w_notes[i] = 0;
   if (tid == 0) {
     abort_flag = 0;
+    w_most = 0;
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&full_bar[b]), PAIRED * LOADER_WARPS);          // one lane of each warp, of both blocks
       mbar_init(smem_u32(&done_bar[b]), 1);
@@ -268,6 +297,7 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
 
   if (warp < LOADER_WARPS) {
     float4 held_x[X_LOADS];
+    float w_high = 0.f, x_high[X_LOADS] = {};
     auto load_x = [&](int i, int chunk) {
       const int r = token0 + (int)(rank - leader) * S::X_ROWS + row + i * LINES;
       held_x[i] = load_four<WIDE>(args.a + (size_t)r * args.lda, (chunk0 + chunk) * F32_CHUNK + quad * 4, args.k, r < args.m && chunk < chunks);
@@ -278,7 +308,7 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
     auto put_w = [&](int chunk) {
 #pragma unroll
       for (int i = 0; i < W_LOADS; ++i) {
-        put_four(smem_base + (chunk & 1) * S::BUFFER, S::W_PLANE, row + i * LINES, quad, held_w[i]);
+        put_four(smem_base + (chunk & 1) * S::BUFFER, S::W_PLANE, row + i * LINES, quad, held_w[i], w_high);
         if (i < EARLY) load_w(i, chunk + 1);
       }
     };
@@ -289,7 +319,7 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
     auto put_x = [&](int chunk) {
 #pragma unroll
       for (int i = 0; i < X_LOADS; ++i) {
-        put_four(smem_base + (chunk & 1) * S::BUFFER + F32_PLANES * S::W_PLANE, S::X_PLANE, row + i * LINES, quad, held_x[i]);
+        put_four(smem_base + (chunk & 1) * S::BUFFER + F32_PLANES * S::W_PLANE, S::X_PLANE, row + i * LINES, quad, held_x[i], x_high[i]);
       }
       fence_proxy_async_shared();
       __syncwarp();
@@ -325,6 +355,23 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
       put_w(chunk);
       put_x(chunk);
       load_late_w(chunk + 1);
+    }
+#pragma unroll
+    for (int i = 0; i < X_LOADS; ++i) {                                  // (the sixteen lanes of a row are its only readers)
+      const unsigned most = __reduce_max_sync(lane < 16 ? 0xffffu : 0xffff0000u, __float_as_uint(x_high[i]));
+      if (quad == 0) x_most[row + i * LINES] = most;
+    }
+    const unsigned most = __reduce_max_sync(0xffffffffu, min(__float_as_uint(w_high), F32_LIMIT));
+    if (lane == 0) atomicMax(&w_most, most);
+    if (!(w_high < 0x1p40f)) {                                           // which rows: in a second look
+      atomicMax(&w_most, 0x80000000u | F32_LIMIT);
+#pragma unroll 1
+      for (int i = 0; i < W_LOADS; ++i) {
+        const int r = feature0 + row + i * LINES;
+#pragma unroll 1
+        for (chunk = 0; chunk < chunks; ++chunk)
+          note_row(load_four<WIDE>(args.w + (size_t)r * args.ldw, (chunk0 + chunk) * F32_CHUNK + quad * 4, args.k, r < args.n), &w_notes[row + i * LINES]);
+      }
     }
   } else if (warp == ISSUE_WARP) {
     if (rank == leader) {
@@ -449,22 +496,71 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
   if (PAIR || blocks > 1) srb_cluster_sync();
   else __syncthreads();
   const unsigned first_rank = rank - blockIdx.z * PAIRED - (rank - leader);                  // of the blocks that share the tile
+  auto noted = [&](const unsigned* word, unsigned peer) {
+    return __float_as_uint(srb_load_peer_shared(reinterpret_cast<const float*>(word), peer));
+  };
   auto store = [&](int r, int f, float v) {
     const int row = token0 + r, col = feature0 + f;
-    if (row >= args.m || col >= args.n) return;
-    if (!lost && !isfinite(v)) v = plain_element(args.a + (size_t)row * args.lda, args.w + (size_t)col * args.ldw, args.k);
-    args.c[(size_t)row * args.ldc + col] = v + (args.bias ? args.bias[col] : 0.f);
+    if (row < args.m && col < args.n) args.c[(size_t)row * args.ldc + col] = v + (args.bias ? args.bias[col] : 0.f);
   };
+  // Results below this may lack what the parts lose of small entries: 3 * 2^-126 an entry and 2^-126 a product.
+  auto least = [&](unsigned x, unsigned w) { return args.unit * (__uint_as_float(x) + __uint_as_float(w & 0x7fffffffu) + 2.f); };
+  auto unsure = [&](unsigned x, unsigned w, float smallest) { return (w >> 31) || x >= F32_LIMIT || __any_sync(0xffffffffu, smallest < least(x, w)); };
+  // A result that may not be sure, by a whole warp with one row, whose largest magnitude is x, and 32 neighbouring columns.
+  auto reconsidered = [&](int r, int f, unsigned x, unsigned w, float v) {
+    const int row = token0 + r, col = feature0 + f;
+    unsigned notes = 0;
+    for (int b = 0; (w >> 31) && b < blocks; ++b) notes |= noted(&w_notes[f], first_rank + b * PAIRED + (rank - leader));
+    const bool none = x > 0x7f800000u || (notes & F32_NAN);
+    const bool again = row < args.m && col < args.n && !none && (x >= F32_LIMIT || notes || (x != 0 && fabsf(v) < least(x, w)));
+    if (none) v = __int_as_float(0x7fffffff);
+    for (unsigned left = __ballot_sync(0xffffffffu, again); left; left &= left - 1) {
+      const int owner = __ffs(left) - 1;
+      const float sum = plain_element(args.a + (size_t)row * args.lda, args.w + (size_t)(col - lane + owner) * args.ldw, args.k, lane);
+      if (lane == owner) v = sum;
+    }
+    return v;
+  };
+  if (PAIR) {
+    static_assert(!PAIR || TOKENS < S::THREADS, "a thread each");
+    if (tid <= TOKENS) {
+      unsigned most = 0;
+#pragma unroll
+      for (int b = 0; b < F32_MAX_BLOCKS / 2; ++b)
+        if (b < blocks) most = max(most, tid < TOKENS ? noted(&x_most[tid % S::X_ROWS], first_rank + b * PAIRED + tid / S::X_ROWS)
+                                                      : noted(&w_most, first_rank + b * PAIRED + (rank - leader)));
+      *(tid < TOKENS ? &tile_x_most[tid] : &tile_w_most) = most;
+    }
+    __syncthreads();
+  }
   constexpr int LINES_AT_ONCE = S::THREADS / F32_FEATURES;
   const int col = tid & (F32_FEATURES - 1), line = tid / F32_FEATURES, first_row = (int)blockIdx.z + line * blocks;
   const int limit = min(TOKENS, args.m - token0);
+  const bool live = feature0 + col < args.n;
   if (line < LINES_AT_ONCE && first_row < limit) {
     if (blocks == 1) {
       constexpr int AT_ONCE = 4;
+      const unsigned w = PAIR ? tile_w_most : w_most;
       for (int r0 = first_row; r0 < limit; r0 += LINES_AT_ONCE * AT_ONCE) {
         float v[AT_ONCE];
 #pragma unroll
         for (int i = 0; i < AT_ONCE; ++i) v[i] = r0 + i * LINES_AT_ONCE < limit ? tile[(r0 + i * LINES_AT_ONCE) * F32_FEATURES + col] : 0.f;
+        float smallest = INFINITY;
+#pragma unroll
+        for (int i = 0; i < AT_ONCE; ++i)
+          if (live && r0 + i * LINES_AT_ONCE < limit) smallest = fminf(smallest, fabsf(v[i]));
+        const unsigned* row_most = PAIR ? tile_x_most : x_most;
+        unsigned x = 0;
+#pragma unroll
+        for (int i = 0; i < AT_ONCE; ++i) x = max(x, row_most[min(r0 + i * LINES_AT_ONCE, limit - 1)]);
+        if (unsure(x, w, smallest)) {
+#pragma unroll 1
+          for (int i = 0; i < AT_ONCE; ++i) {
+            const int r = r0 + i * LINES_AT_ONCE;
+            if (r < limit) store(r, col, reconsidered(r, col, row_most[r], w, tile[r * F32_FEATURES + col]));
+          }
+          continue;
+        }
 #pragma unroll
         for (int i = 0; i < AT_ONCE; ++i)
           if (r0 + i * LINES_AT_ONCE < limit) store(r0 + i * LINES_AT_ONCE, col, v[i]);
@@ -472,6 +568,11 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
     } else {
       constexpr int MOST = PAIR ? F32_MAX_BLOCKS / 2 : F32_MAX_BLOCKS;
       for (int r = first_row; r < limit; r += LINES_AT_ONCE * blocks) {
+        unsigned most = 0;
+        if (!PAIR) {                                                     // lanes b and 16 + b: the largest entry of the row and of W in range b of K
+          const unsigned range = first_rank + (lane & 15);
+          if ((lane & 15) < blocks) most = lane < 16 ? noted(&x_most[r % S::X_ROWS], range) : noted(&w_most, range);
+        }
         float first[MOST], second[MOST];
 #pragma unroll
         for (int b = 0; b < MOST; ++b) {
@@ -501,6 +602,9 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
             }
           }
         }
+        const unsigned x = PAIR ? tile_x_most[PAIR ? r : 0] : __reduce_max_sync(0xffffffffu, lane < 16 ? most : 0u);
+        const unsigned w = PAIR ? tile_w_most : __reduce_max_sync(0xffffffffu, lane < 16 ? 0u : most);
+        if (unsure(x, w, live ? fabsf(v) : INFINITY)) v = reconsidered(r, col, x, w, v);
         store(r, col, v);
       }
     }
@@ -573,6 +677,7 @@ extern "C" int srb_gemm_f32(const float* a, const float* w, const float* bias, f
   args.m = m; args.n = n; args.k = k; args.lda = lda; args.ldw = ldw; args.ldc = ldc;
   args.parts = parts.count; args.part_chunks = parts.chunks;
   args.in_pairs = parts.blocks == 8; args.constant = constant_weights; args.error_word = error_word;
+  args.unit = ldexpf((float)k, -97);
   const bool wide = k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
   return wide ? dispatch<true>(args, parts.blocks, (cudaStream_t)stream) : dispatch<false>(args, parts.blocks, (cudaStream_t)stream);
 }

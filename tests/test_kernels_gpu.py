@@ -318,6 +318,57 @@ def test_float_products_are_as_exact_as_multiply_adds(n, k):
     assert torch.equal(ops.linear(whole, whole).double(), whole.double() @ whole.double().T)
 
 
+@pytest.mark.parametrize("n,k", [(130, 72), (1024, 1024), (4096, 1024), (700, 1001)])
+def test_float_products_of_entries_that_bfloat16_parts_do_not_hold(n, k):
+    """Infinities, what is not a number, the largest and the smallest floats: kinds of results as in 64 bits, errors as of usual operands,
+    the same bits for few rows and many, and rows beside them untouched."""
+    g = torch.Generator(DEV).manual_seed(n + k)
+    x, w = torch.randn(140, k, generator=g, device=DEV), torch.randn(n, k, generator=g, device=DEV)
+    clean = ops.linear(x, w)
+    bound = 2 * ((k + 63) // 64 + 20) * 2.0 ** -24
+
+    def check(left, right, odd_rows):
+        got, want = ops.linear(left, right), left.double() @ right.double().T
+        size = left.double().abs() @ right.double().abs().T
+        most = torch.finfo(torch.float32).max
+        assert torch.equal(torch.isnan(got), torch.isnan(want))
+        endless = torch.isinf(want) | (want.abs() > most)
+        assert torch.equal(got[endless].double(), want[endless].sign() * math.inf)
+        sure = torch.isfinite(want) & (size < most)          # (sums may leave the range on the way otherwise)
+        assert bool(((got.double() - want).abs() <= bound * size + k * 2.0 ** -149)[sure].all())
+        for m in (2, 20, 70):
+            assert torch.equal(ops.linear(left[140 - m:], right).nan_to_num(nan=7.0), got[140 - m:].nan_to_num(nan=7.0)), m
+        if right is w:
+            same = [r for r in range(140) if r not in odd_rows]
+            assert torch.equal(got[same], clean[same])
+
+    def with_rows(rows, change):
+        left = x.clone()
+        for r in rows:
+            left[r] = change(left[r].clone(), r)
+        return left
+
+    def put(at, value):
+        def change(row, _):
+            row[at] = value
+            return row
+        return change
+
+    last = [0, 77, 137, 139]
+    for value in (math.nan, math.inf, -math.inf, 3.4e38, 2.0 ** 41):
+        check(with_rows(last, put(k - 1, value)), w, last)
+    check(with_rows(last, lambda row, r: torch.full_like(row, math.nan)), w, last)
+    check(with_rows(last, lambda row, r: row * 1e36), w * 0.01, last)
+    check(with_rows(last, lambda row, r: row * 1e-36), w * 1e30, last)
+    check(with_rows(last, lambda row, r: row * 1e-43), w * 1e12, last)
+    check(with_rows(last, lambda row, r: row * 1e-20), w * 1e-18, last)
+    check(with_rows(last, lambda row, r: torch.where(torch.arange(k, device=DEV) % 3 == 0, row * 1e-38, row)), w, last)
+    check(with_rows(last, lambda row, r: row * 0), w, last)
+    strange = w.clone()
+    strange[0, 1], strange[n - 1, 0], strange[n // 2] = math.nan, -math.inf, 1e-40
+    check(x, strange, ())
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 64, 64), (2, 1024, 1024), (16, 331, 1000), (40, 1024, 1024), (130, 257, 2052)])
 def test_float_products_whose_weights_the_kernel_ahead_writes(m, n, k):
     """The second operand may come from a product just ahead, whose blocks let the next kernel in as they start."""
