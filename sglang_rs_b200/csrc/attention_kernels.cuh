@@ -72,6 +72,7 @@ struct AttnParams {
   int maps = 1;                   // 2: two maps per head, n_q counts maps
   float map_lambda = 0.f, map_scale = 1.f, map_eps = 0.f;
   int float_out = 0;              // the generic kernel's results are floats
+  int steady_arrays = 0;          // no kernel that the stream may still run writes the index arrays
 };
 
 // What a caller may ask for beyond the arguments that every attention has (null pointer: nothing of it).
@@ -542,7 +543,7 @@ paged_attention_split_kernel(const float* __restrict__ q, const float* __restric
   const int split = blockIdx.x, kv_head = blockIdx.y, row = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tile = warp / groups, head = warp % groups;
   srb_launch_dependents();
-  // the step's index arrays were copied in before its first kernel: they are read ahead of the wait for the kernels ahead
+  if (!p.steady_arrays) srb_grid_dependency_wait();
   const int pos = p.positions[row];
   int lo, hi;
   row_key_range(p, pos, split, lo, hi);
@@ -791,7 +792,7 @@ static int paged_attention_dispatch_masked(const void* q, const void* k_pool, co
                                            int chunk, int split_size, int max_splits, float scale, int* error_word,
                                            int dtype, const float* sinks, int value_dim, void* stream,
                                            const float* gates = nullptr, long long out_pitch = 0, float out_scale = 1.0f,
-                                           const AttnTerms* terms = nullptr) {
+                                           const AttnTerms* terms = nullptr, bool steady_arrays = false) {
   if (rows <= 0) return SRB_OK;
   if (chunk < 0) SRB_FAIL("paged_attention: the chunk size must be non-negative");
   if (n_q <= 0 || n_kv <= 0 || n_q % n_kv != 0)
@@ -817,6 +818,7 @@ static int paged_attention_dispatch_masked(const void* q, const void* k_pool, co
   p.max_splits = split_size == 0 ? 1 : max_splits; p.scale = scale; p.error_word = error_word;
   p.sinks = sinks; p.value_dim = value_dim; p.shared_values = v_pool == nullptr; p.gates = gates;
   p.out_pitch = out_pitch ? out_pitch : (long long)n_q * value_dim; p.out_scale = out_scale;
+  p.steady_arrays = steady_arrays;
   if (p.out_pitch < (long long)n_q * value_dim) SRB_FAIL("paged_attention: rows of the output overlap");
   if (const char* fault = srb_apply_terms(p, terms)) SRB_FAIL("paged_attention: %s", fault);
   if (p.maps == 2 && !p.float_out) SRB_FAIL("paged_attention: the results of two maps are floats that srb_map_combine joins");

@@ -1182,3 +1182,24 @@ def test_float_splits_of_four_tiles(n_q, n_kv, d, page, window, lengths):
     results leave without the kernel that joins splits."""
     case = paged_case(torch.float32, n_q, n_kv, d, page, lengths, (1,) * len(lengths), window, seed=d)
     close(run_attention(case, 1.0 / math.sqrt(d), 128), expected_attention(case, 1.0 / math.sqrt(d)), torch.float32, "split 128")
+
+
+def test_float_splits_of_positions_that_the_kernel_ahead_writes():
+    """The index arrays may come from a kernel just ahead whose blocks let the next one in as they start: here positions that the
+    sampler picks."""
+    lengths = tuple(range(3, 128, 5))
+    case = paged_case(torch.float32, 4, 2, 128, 16, lengths, (1,) * len(lengths), None, seed=5)
+    rows = len(lengths)
+    want = run_attention(case, 0.1, 128)
+    logits = torch.zeros(rows, 151936, device=DEV)
+    logits[torch.arange(rows), case["positions"].long()] = 5.0
+    word, out = ops.new_error_word(DEV), torch.full_like(case["q"], math.nan)
+    a, m = ops.attention_scratch_sizes(rows, 4, 128, 1)
+    acc, ml = torch.empty(a, device=DEV), torch.empty(m, device=DEV)
+    for _ in range(20):
+        positions = torch.zeros(rows, dtype=torch.int32, device=DEV)
+        ops.sample(logits, None, None, positions)
+        ops.paged_attention(case["q"], case["k_pool"], case["v_pool"], out, positions, case["row_request"], case["table"], scale=0.1,
+                            window=0, split_size=128, max_splits=1, scratch_acc=acc, scratch_ml=ml, error_word=word)
+        assert torch.equal(out, want)
+    ops.raise_on_error_word(word)
