@@ -42,6 +42,7 @@
 // and srb_attention_combine merges the partials in split order.
 #pragma once
 #include "common.cuh"
+#include <algorithm>
 #include <math.h>
 #include <type_traits>
 
@@ -525,11 +526,16 @@ paged_attention_rows_kernel(const float* __restrict__ q, const float* __restrict
 }
 
 // Decoded rows in floats, a split of SPLIT_TILES * 32 keys a block: its tiles side by side, a warp per (tile, head), and the warps' results
-// joined at the end in the order of the tiles.  All keys and values of the split are on their way at once; one tile after the other by a
-// warp per head, the latencies of four tiles add up: two rows of some 230 keys, 16 heads on 8 of 128, 17.1 us a layer then, 9.1 now.
+// joined at the end in the order of the tiles.  All keys of the split are on their way at once, and its values beside them: one tile after
+// the other by a warp per head, the latencies of four tiles add up (two rows of some 230 keys, 16 heads on 8 of 128, 17.1 us a layer then,
+// 9.1 now).  IN_TURNS, the values follow into the memory of the keys once the scores are there, so that two to three times as many blocks
+// share an SM and cover each other's loads: for launches that do not fit the SMs at once.  The arithmetic is the same, so a row's bits do
+// not depend on the rows beside it.  16 heads on 8 of 128, rows x keys, us side by side / in turns / one tile after the other: 1 x 2,048 15.4
+// / 18.3 / 23.1 (128 blocks), 16 x 230 21.4 / 17.4 / 23.6 (256), 8 x 2,048 67 / 47 / 69, 64 x 2,048 475 / 244 / 385 (4.4 TB/s of keys); 8
+// heads of 64, three blocks an SM side by side: 8 x 512 16.9 / 19.3 / 19.8 (256), 16 x 512 29.7 / 21.1 / 23.3 (512), 64 x 2,048 252 / 160 / 214.
 #define SPLIT_TILES 4
 #define SPLIT_MAX_HEADS 4                                // that share a kv head
-template <int DIM_PER_LANE>
+template <int DIM_PER_LANE, bool IN_TURNS>
 __global__ void __launch_bounds__(32 * SPLIT_TILES * SPLIT_MAX_HEADS)
 paged_attention_split_kernel(const float* __restrict__ q, const float* __restrict__ k_pool, const float* __restrict__ v_pool,
                              float* __restrict__ out, float* __restrict__ part_acc, float* __restrict__ part_ml, AttnParams p) {
@@ -538,8 +544,8 @@ paged_attention_split_kernel(const float* __restrict__ q, const float* __restric
   const int d = p.head_dim, vd = p.value_dim, groups = p.n_q / p.n_kv;
   const int k_pitch = d + 4, v_stride = p.shared_values ? k_pitch : vd;
   float* k_rows = smem;                                  // [128][k_pitch], behind them the values' rows
-  float* v_rows = p.shared_values ? k_rows : k_rows + SPLIT_TILES * KEY_BLOCK * k_pitch;
-  float* q_rows = p.shared_values ? k_rows + SPLIT_TILES * KEY_BLOCK * k_pitch : v_rows + SPLIT_TILES * KEY_BLOCK * vd;
+  float* v_rows = IN_TURNS || p.shared_values ? k_rows : k_rows + SPLIT_TILES * KEY_BLOCK * k_pitch;
+  float* q_rows = k_rows + SPLIT_TILES * KEY_BLOCK * (IN_TURNS || p.shared_values ? max(k_pitch, v_stride) : k_pitch + vd);
   const int split = blockIdx.x, kv_head = blockIdx.y, row = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tile = warp / groups, head = warp % groups;
   srb_launch_dependents();
@@ -578,7 +584,7 @@ paged_attention_split_kernel(const float* __restrict__ q, const float* __restric
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   copy_rows(k_rows, k_pitch, k_pool, d);
-  if (p.shared_values) asm volatile("cp.async.commit_group;" ::: "memory");
+  if (IN_TURNS || p.shared_values) asm volatile("cp.async.commit_group;" ::: "memory");
   else copy_rows(v_rows, vd, v_pool, vd);
   for (int i = threadIdx.x; i < groups * d; i += blockDim.x)
     q_rows[i] = q[((size_t)row * p.n_q + (size_t)kv_head * groups) * d + i];
@@ -602,6 +608,10 @@ paged_attention_split_kernel(const float* __restrict__ q, const float* __restric
     m = srb_warp_max(s);
     prob = s == -INFINITY && m == -INFINITY ? 0.f : expf(s - m);         // 0 for masked keys
     l = srb_warp_sum(prob);
+  }
+  if (IN_TURNS) {
+    __syncthreads();                                     // the keys are read
+    copy_rows(v_rows, vd, v_pool, vd);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
@@ -751,9 +761,14 @@ static int launch_attention(const void* q, const void* k_pool, const void* v_poo
     side_by_side = wide && p.split_size == SPLIT_TILES * KEY_BLOCK && p.maps == 1 && p.keep_first == 0 && groups <= SPLIT_MAX_HEADS &&
                    p.n_kv <= 65535 && shared <= ATTN_SHARED_MOST - 1024;
     if (side_by_side) {
-      auto split_kernel = paged_attention_split_kernel<DIM_PER_LANE>;
+      // more blocks than are resident at once
+      const long long resident = (long long)srb_sm_count() * (228 * 1024 / (shared + 1024));
+      const bool in_turns = !p.shared_values && (long long)p.max_splits * p.n_kv * rows > resident;
+      const size_t most = !in_turns ? shared
+                                    : (SPLIT_TILES * KEY_BLOCK * (size_t)std::max(p.head_dim + 4, p.value_dim) + (size_t)groups * p.head_dim) * sizeof(float);
+      auto split_kernel = in_turns ? paged_attention_split_kernel<DIM_PER_LANE, true> : paged_attention_split_kernel<DIM_PER_LANE, false>;
       SRB_CUDA_CALL(cudaFuncSetAttribute(split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATTN_SHARED_MOST - 1024));
-      SRB_CUDA_CALL(srb_launch(split_kernel, dim3(p.max_splits, p.n_kv, rows), dim3(32 * SPLIT_TILES * groups), shared, s, (const float*)q,
+      SRB_CUDA_CALL(srb_launch(split_kernel, dim3(p.max_splits, p.n_kv, rows), dim3(32 * SPLIT_TILES * groups), most, s, (const float*)q,
                                (const float*)k_pool, (const float*)v_pool, (float*)out, part_acc, part_ml, p));
       if (p.max_splits == 1) return SRB_OK;
     }

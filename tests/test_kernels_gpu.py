@@ -1203,3 +1203,45 @@ def test_float_splits_of_positions_that_the_kernel_ahead_writes():
                             window=0, split_size=128, max_splits=1, scratch_acc=acc, scratch_ml=ml, error_word=word)
         assert torch.equal(out, want)
     ops.raise_on_error_word(word)
+
+
+@pytest.mark.parametrize("rows", [7, 200])
+@pytest.mark.parametrize("terms", ["sinks", "gates", "softcap", "chunk", "shared", "pitch", "window", "narrow"])
+def test_float_splits_of_few_and_many_blocks_with_terms(rows, terms):
+    """Splits of 128 keys with what a caller may ask for beyond the usual, against splits of 64 (other kernels); few blocks have keys and
+    values side by side, more than the SMs hold at once in turns: a row alone has the same bits."""
+    g = torch.Generator().manual_seed(rows + len(terms))
+    n_q, n_kv, d = (6, 2, 64) if terms == "narrow" else (4, 2, 128)
+    lengths = torch.randint(1, 290, (rows,), generator=g).tolist()
+    lengths[:4] = [1, 128, 129, 289]
+    case = paged_case(torch.float32, n_q, n_kv, d, 16, lengths, (1,) * rows, 140 if terms == "window" else None, seed=9)
+    options = {"sinks": dict(sinks=torch.randn(n_q, generator=g).to(DEV)), "softcap": dict(softcap=3.0), "chunk": dict(chunk=100)}.get(terms, {})
+    gates = torch.rand(rows, n_q, generator=g).to(DEV) if terms == "gates" else None
+    width = 96 if terms == "shared" else d
+
+    def run(split, first, last):
+        count, splits = last - first, 290 // split + 1
+        a, m = ops.attention_scratch_sizes(count, n_q, width, splits)
+        held = torch.full((count, n_q * width + (32 if terms == "pitch" else 0)), 7.0, device=DEV)
+        word = ops.new_error_word(DEV)
+        ops.paged_attention(case["q"][first:last], case["k_pool"], None if terms == "shared" else case["v_pool"],
+                            held[:, :n_q * width].view(count, n_q, width) if terms != "pitch" else held[:, :n_q * width].unflatten(1, (n_q, width)),
+                            case["positions"][first:last], case["row_request"][first:last], case["table"], scale=0.1,
+                            window=case["window"] or 0, split_size=split, max_splits=splits, scratch_acc=torch.empty(a, device=DEV),
+                            scratch_ml=torch.empty(m, device=DEV), error_word=word,
+                            gates=None if gates is None else gates[first:last], **options)
+        ops.raise_on_error_word(word)
+        assert bool((held[:, n_q * width:] == 7.0).all())
+        return held[:, :n_q * width].view(count, n_q, width) if terms != "pitch" else held[:, :n_q * width].unflatten(1, (n_q, width))
+
+    whole = run(128, 0, rows)
+    close(whole, run(64, 0, rows).double().cpu(), torch.float32, terms)
+    for r in (0, 1, 2, 3, rows - 1):
+        assert torch.equal(run(128, r, r + 1)[0], whole[r]), r
+
+
+def test_float_splits_note_a_page_out_of_range():
+    case = paged_case(torch.float32, 4, 2, 128, 16, (200, 40), (1, 1), None, seed=2)
+    case["table"][0, 9] = 1000                               # the second split of the first row
+    with pytest.raises(Exception):
+        run_attention(case, 0.1, 128)
