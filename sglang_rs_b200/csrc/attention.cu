@@ -20,6 +20,10 @@ extern "C" int srb_paged_attention(const void* q, const void* k_pool, const void
                                          dtype, nullptr, 0, stream, nullptr, 0, 1.0f, nullptr, true);
 }
 
+// How many kernels this thread's last call of these entries launched: splits that are joined take two, the one split of a short context
+// may leave with one.
+extern "C" int srb_paged_attention_launches() { return attention_launches; }
+
 // The same with the two optional terms: `sinks` (one float per query head, or null), values of `value_dim`
 // entries (0: as wide as the keys), and, with v_pool null, values that are the head of the key rows.
 extern "C" int srb_paged_attention_ex(const void* q, const void* k_pool, const void* v_pool, void* out,

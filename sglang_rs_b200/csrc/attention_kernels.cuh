@@ -723,6 +723,8 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_acc, con
 #define ATTN_SHARED_MOST (227 * 1024 - KEY_BLOCK * 8)    // beside the keys' rows
 #define ATTN_SHARED_TWO_BLOCKS (113 * 1024)
 
+static thread_local int attention_launches = 0;          // kernels that this thread's last call launched
+
 template <typename T, int DIM_PER_LANE>
 static int launch_attention(const void* q, const void* k_pool, const void* v_pool, void* out, float* part_acc,
                             float* part_ml, const AttnParams& p, int rows, cudaStream_t s) {
@@ -750,6 +752,7 @@ static int launch_attention(const void* q, const void* k_pool, const void* v_poo
       rows_kernel<<<dim3((rows + per_block - 1) / per_block, p.n_kv), ROW_WARPS * 32, shared, s>>>(
           (const float*)q, (const float*)k_pool, (const float*)v_pool, (float*)out, rows, p);
       SRB_LAUNCH_CHECK("paged_attention rows");
+      ++attention_launches;
       return SRB_OK;
     }
   }
@@ -770,6 +773,7 @@ static int launch_attention(const void* q, const void* k_pool, const void* v_poo
       SRB_CUDA_CALL(cudaFuncSetAttribute(split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATTN_SHARED_MOST - 1024));
       SRB_CUDA_CALL(srb_launch(split_kernel, dim3(p.max_splits, p.n_kv, rows), dim3(32 * SPLIT_TILES * groups), most, s, (const float*)q,
                                (const float*)k_pool, (const float*)v_pool, (float*)out, part_acc, part_ml, p));
+      ++attention_launches;
       if (p.max_splits == 1) return SRB_OK;
     }
   }
@@ -786,11 +790,13 @@ static int launch_attention(const void* q, const void* k_pool, const void* v_poo
     kernel<<<grid, (p.heads_per_block < 4 ? 4 : p.heads_per_block) * 32, smem, s>>>(
         (const T*)q, (const T*)k_pool, (const T*)v_pool, (T*)out, part_acc, part_ml, p);
     SRB_LAUNCH_CHECK("paged_attention");
+    ++attention_launches;
   }
   if (p.split_size != 0) {
     dim3 cgrid(rows, p.n_q);
     SRB_CUDA_CALL(srb_launch(attention_combine_kernel<T>, cgrid, dim3(64), 0, s, (const float*)part_acc, (const float*)part_ml, (T*)out, p));
     SRB_LAUNCH_CHECK("attention_combine");
+    ++attention_launches;
   }
   return SRB_OK;
 }
@@ -808,6 +814,7 @@ static int paged_attention_dispatch_masked(const void* q, const void* k_pool, co
                                            int dtype, const float* sinks, int value_dim, void* stream,
                                            const float* gates = nullptr, long long out_pitch = 0, float out_scale = 1.0f,
                                            const AttnTerms* terms = nullptr, bool steady_arrays = false) {
+  attention_launches = 0;
   if (rows <= 0) return SRB_OK;
   if (chunk < 0) SRB_FAIL("paged_attention: the chunk size must be non-negative");
   if (n_q <= 0 || n_kv <= 0 || n_q % n_kv != 0)

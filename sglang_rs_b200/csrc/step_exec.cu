@@ -401,7 +401,7 @@ struct Run {
                                   step.positions + launch.begin, step.row_request + launch.begin, group.block_table,
                                   group.table_stride, count, a.n_q, a.n_kv, a.head_dim, call.page_size, call.num_pages, a.window,
                                   launch.split_size, launch.max_splits, a.scale, step.error_word, model.dtype, stream));
-      if (launch.split_size) ++launches;                       // the merge of the splits is a launch of its own
+      if (kernels.paged_attention_launches) launches += kernels.paged_attention_launches() - 1;
     }
     return linear(out, rows, a.o, base + l.delta, false, true, produced, SX_SKIP_O);
   }

@@ -142,6 +142,8 @@ typedef struct SxKernels {
   int (*paged_attention)(const void*, const void*, const void*, void*, float*, float*, const int*, const int*, const int*, int,
                          int, int, int, int, int, int, int, int, int, float, int*, int, void*);
   SxLastError paged_attention_error;
+  int (*paged_attention_launches)(void);       // of the call before
+  SxLastError paged_attention_launches_error;
   int (*decode_attention)(const void*, const void*, const void*, void*, float*, float*, int*, const int*, const int*,
                           const int*, int, int, int, int, int, int, int, int, int, float, int*, void*);
   SxLastError decode_attention_error;

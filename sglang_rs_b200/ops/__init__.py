@@ -589,7 +589,8 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
         _ptr(row_request), _ptr(block_table), block_table.stride(0), rows, n_q, n_kv, head_dim, page_size,
         num_pages, int(window), int(chunk), int(split_size), int(max_splits), ctypes.c_float(scale), _ptr(error_word),
         dtype_code(q.dtype), _ptr(sinks), value_dim, _ptr(gates), ctypes.c_longlong(pitch), ctypes.c_float(out_scale),
-        _attention_terms(keep_first, softcap, join, join is not None), _stream()), launches=2 if split_size else 1)
+        _attention_terms(keep_first, softcap, join, join is not None), _stream()),
+           launches=lib.srb_paged_attention_launches())
     if join is not None:
         _check(lib, lib.srb_map_combine(_ptr(result), _ptr(out), rows, heads, value_dim, ctypes.c_longlong(out.stride(0)),
                                         ctypes.c_float(join.subtract), ctypes.c_float(join.scale), ctypes.c_float(join.eps),

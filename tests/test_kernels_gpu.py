@@ -1245,3 +1245,13 @@ def test_float_splits_note_a_page_out_of_range():
     case["table"][0, 9] = 1000                               # the second split of the first row
     with pytest.raises(Exception):
         run_attention(case, 0.1, 128)
+
+
+@pytest.mark.parametrize("dtype,split,length,launches", [(torch.float32, 128, 100, 1), (torch.float32, 128, 200, 2), (torch.float32, 64, 40, 2),
+                                                         (torch.bfloat16, 128, 100, 2), (torch.float32, 0, 100, 1), (torch.bfloat16, 0, 100, 1)])
+def test_launches_of_the_generic_attention_are_counted(dtype, split, length, launches):
+    """One split of 128 keys in floats leaves without the kernel that joins splits."""
+    case = paged_case(dtype, 4, 2, 128, 16, (length,), (1,), None, seed=1)
+    before = ops.launch_count
+    run_attention(case, 0.1, split)
+    assert ops.launch_count - before == launches
