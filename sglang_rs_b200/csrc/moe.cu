@@ -326,6 +326,7 @@ moe_plan_kernel(const int* __restrict__ chosen, int entries, int top, int expert
     if (slot_weight) slot_weight[slot] = weights[i];
     entry_slot[i] = slot;
   }
+  __syncwarp();                                      // (lanes left the loop apart)
   if (blocks > 1) srb_cluster_sync();                // nobody leaves while its counts may still be read
 }
 
