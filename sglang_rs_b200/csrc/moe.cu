@@ -235,10 +235,10 @@ extern "C" int srb_moe_select(const float* logits, long long pitch, int rows, in
 // plan: [0] number of tiles, then offsets[experts + 1], then per tile (expert, first slot).
 // slot_row[slot]: the row whose entry sits in the slot; entry_slot[row * top + k]: the slot of that entry.
 //
-// A chain of latencies: count the entries of every expert, add up, hand out the slots.  One block, or the blocks of a cluster, each
-// with an equal run of the entries: an expert's slots go to the blocks in turn.  The count that an entry finds is its place among
-// those of its block, so the second pass adds two numbers.  (2,048 rows of 6 choices among 64 experts: 18.4 us by one block that counted
-// twice, 12.0 by eight.)
+// A chain of latencies: count the entries of every expert, add up, hand out the slots by a second round of counting.  Or, for many
+// entries, the blocks of a CLUSTER, each with an equal run of them: an expert's slots go to the blocks in turn, and the count that an
+// entry finds is its place among those of its block, so the second pass adds two numbers.
+template <bool CLUSTER>
 __global__ void __launch_bounds__(1024)
 moe_plan_kernel(const int* __restrict__ chosen, int entries, int top, int experts, int max_tiles,
                 int tile_rows, int* __restrict__ plan, int* __restrict__ slot_row, int* __restrict__ entry_slot,
@@ -257,27 +257,30 @@ moe_plan_kernel(const int* __restrict__ chosen, int entries, int top, int expert
 #pragma unroll 4
   for (int i = begin + threadIdx.x; i < end; i += blockDim.x) {
     const int e = chosen[i];
-    entry_slot[i] = e >= 0 && e < experts ? atomicAdd(&count[e], 1) : -1;
+    if (CLUSTER) entry_slot[i] = e >= 0 && e < experts ? atomicAdd(&count[e], 1) : -1;
+    else if (e >= 0 && e < experts) atomicAdd(&count[e], 1);
   }
   __syncthreads();
-  if (blocks > 1) srb_cluster_sync();
-  for (int e = threadIdx.x; e < experts; e += blockDim.x) {
-    int ahead = 0, all = 0;
-    for (int b = 0; b < blocks; ++b) {
-      const int n = blocks > 1 ? __float_as_int(srb_load_peer_shared(reinterpret_cast<const float*>(&count[e]), b)) : count[e];
-      if (b < rank) ahead += n;
-      all += n;
+  if (CLUSTER) {
+    srb_cluster_sync();
+    for (int e = threadIdx.x; e < experts; e += blockDim.x) {
+      int ahead = 0, all = 0;
+      for (int b = 0; b < blocks; ++b) {
+        const int n = __float_as_int(srb_load_peer_shared(reinterpret_cast<const float*>(&count[e]), b));
+        if (b < rank) ahead += n;
+        all += n;
+      }
+      before[e] = ahead;
+      total[e] = all;
     }
-    before[e] = ahead;
-    total[e] = all;
+    __syncthreads();
   }
-  __syncthreads();
   // running sums of the experts' slots and tiles by one warp, 32 experts at a time
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     int slots = 0, tiles = 0;
     for (int e0 = 0; e0 < experts; e0 += 32) {
-      const int mine = e0 + lane < experts ? total[e0 + lane] : 0;
+      const int mine = e0 + lane < experts ? (CLUSTER ? total : count)[e0 + lane] : 0;
       const int mine_tiles = (mine + tile_rows - 1) / tile_rows;
       int run = mine, run_tiles = mine_tiles;
 #pragma unroll
@@ -315,23 +318,36 @@ moe_plan_kernel(const int* __restrict__ chosen, int entries, int top, int expert
           tiles[2 * at + 1] = first[e] + t * tile_rows;
         }
       }
+      if (!CLUSTER) count[e] = 0;                    // becomes the number of the expert's slots handed out so far
     }
   }
+  if (!CLUSTER) __syncthreads();
 #pragma unroll 4
   for (int i = begin + threadIdx.x; i < end; i += blockDim.x) {
-    const int place = entry_slot[i];                 // this thread's own number from above
-    if (place < 0) continue;
-    const int e = chosen[i], slot = first[e] + before[e] + place;
+    const int e = chosen[i];
+    int place;
+    if (CLUSTER) {
+      place = entry_slot[i];                         // this thread's own number from above
+      if (place < 0) continue;
+      place += before[e];
+    } else {
+      if (e < 0 || e >= experts) { entry_slot[i] = -1; continue; }
+      place = atomicAdd(&count[e], 1);
+    }
+    const int slot = first[e] + place;
     slot_row[slot] = i / top;
     if (slot_weight) slot_weight[slot] = weights[i];
     entry_slot[i] = slot;
   }
   __syncwarp();                                      // (lanes left the loop apart)
-  if (blocks > 1) srb_cluster_sync();                // nobody leaves while its counts may still be read
+  if (CLUSTER) srb_cluster_sync();                   // nobody leaves while its counts may still be read
 }
 
-#define MOE_PLAN_ENTRIES 2048      // more entries than this are counted by
-#define MOE_PLAN_BLOCKS 8          // blocks
+// More entries than this are counted by eight blocks.  us by one and by eight, 64 experts: 192 entries 2.6 and 4.0, 1,536 4.3 and 4.1, 2,046
+// 4.8 and 4.2, 3,072 5.9 and 4.3, 12,288 16.8 and 6.3; 8 experts: 1,536 3.4 and 3.9, 3,072 4.0 and 3.9; 1,024 experts: 1,536 11.7 and 12.3, 3,072
+// 13.7 and 12.4.
+#define MOE_PLAN_ENTRIES 2048
+#define MOE_PLAN_BLOCKS 8
 
 extern "C" int srb_moe_plan_ints(int rows, int top, int experts) {
   const int max_tiles = (rows * top) / moe_tile_rows(rows, top, experts) + experts;
@@ -356,7 +372,7 @@ extern "C" int srb_moe_plan_of(const int* chosen, int rows, int top, int experts
   if (experts <= 0 || experts > MOE_MAX_EXPERTS || top <= 0 || tile_rows <= 0)
     SRB_FAIL("moe_plan: %d experts, %d chosen, tiles of %d", experts, top, tile_rows);
   const int blocks = rows * top > MOE_PLAN_ENTRIES ? MOE_PLAN_BLOCKS : 1;
-  SRB_CUDA_CALL(srb_launch_clustered(moe_plan_kernel, dim3(blocks), dim3(1024), 0, (cudaStream_t)stream, dim3(blocks), chosen,
+  SRB_CUDA_CALL(srb_launch_clustered(blocks > 1 ? moe_plan_kernel<true> : moe_plan_kernel<false>, dim3(blocks), dim3(1024), 0, (cudaStream_t)stream, dim3(blocks), chosen,
                            rows * top, top, experts, (rows * top) / tile_rows + experts, tile_rows, plan, slot_row, entry_slot, weights, slot_weight, error_word));
   SRB_LAUNCH_CHECK("moe_plan");
   return SRB_OK;
@@ -794,33 +810,37 @@ extern "C" int srb_moe_combine(const float* y, const int* entry_slot, const floa
 // rows of h in slot order: out[slot, :] = h[slot_row[slot], :] (16 bytes a thread where the rows allow it), for
 // products that take their operands as whole tiles of consecutive rows.  `used` (or null) points at the number of slots
 // that the plan handed out (its last offset): choices without a slot leave the slots behind it without a row.
-// A warp per slot: a row of 4 KB is eight loads a lane, all in flight.  (A block per slot with two loads a thread behind the one of the
-// slot's row: 28 us for 12,288 rows of 4 KB, 20 us now.)
+// A warp per slot, eight loads a lane in flight, or a block of four warps: those bring a wide row sooner while the slots are few, and are
+// bound by their number where the slots are many (one a ns).  us by a block and by a warp a slot, again and again: 64 slots of 512 bytes 1.28
+// and 1.18, 12,288 13.1 and 3.2; 64 of 4 KB 1.54 and 1.70, 1,200 2.6 and 3.4, 2,400 3.8 and 4.3, 12,288 13.2 and 8.7; 1,200 of 8 KB 4.1 and 5.8, 12,288
+// 20.1 and 19.8; 12,288 of 16 KB 43.5 and 46.3.
 #define MOE_GATHER_WARPS 8
-template <typename T>
+static inline bool moe_gather_by_warps(int slots, size_t row_bytes) { return row_bytes <= 1024 || (slots > 4096 && row_bytes <= 8192); }
+template <typename T, bool WARPS>
 __global__ void __launch_bounds__(32 * MOE_GATHER_WARPS)
 moe_gather_kernel(const T* __restrict__ h, const int* __restrict__ slot_row, int slots, int width, T* __restrict__ out,
                   const int* __restrict__ used) {
   srb_launch_dependents();
   srb_grid_dependency_wait();
-  const int slot = blockIdx.x * MOE_GATHER_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  constexpr int LANES = WARPS ? 32 : 128, AT_ONCE = WARPS ? 8 : 2;
+  const int slot = WARPS ? blockIdx.x * MOE_GATHER_WARPS + (threadIdx.x >> 5) : blockIdx.x, lane = WARPS ? threadIdx.x & 31 : threadIdx.x;
   if (slot >= slots || (used && slot >= *used)) return;
   const T* src = h + (size_t)slot_row[slot] * width;
   T* dst = out + (size_t)slot * width;
   if ((width * sizeof(T)) % 16 == 0 && (((uintptr_t)h | (uintptr_t)out) & 15) == 0) {
     const int pieces = width * sizeof(T) / 16;
-    for (int first = lane; first < pieces; first += 32 * 8) {
-      uint4 v[8];
+    for (int first = lane; first < pieces; first += LANES * AT_ONCE) {
+      uint4 v[AT_ONCE];
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (first + 32 * j < pieces) v[j] = reinterpret_cast<const uint4*>(src)[first + 32 * j];
+      for (int j = 0; j < AT_ONCE; ++j)
+        if (first + LANES * j < pieces) v[j] = reinterpret_cast<const uint4*>(src)[first + LANES * j];
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (first + 32 * j < pieces) reinterpret_cast<uint4*>(dst)[first + 32 * j] = v[j];
+      for (int j = 0; j < AT_ONCE; ++j)
+        if (first + LANES * j < pieces) reinterpret_cast<uint4*>(dst)[first + LANES * j] = v[j];
     }
     return;
   }
-  for (int i = lane; i < width; i += 32) dst[i] = src[i];
+  for (int i = lane; i < width; i += LANES) dst[i] = src[i];
 }
 
 extern "C" int srb_moe_gather_used(const void* h, const int* slot_row, int slots, int width, void* out, const int* used,
@@ -833,12 +853,14 @@ extern "C" int srb_moe_gather_used(const void* h, const int* slot_row, int slots
                                    int dtype, void* stream) {
   if (slots <= 0 || width <= 0) return SRB_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  const dim3 grid((slots + MOE_GATHER_WARPS - 1) / MOE_GATHER_WARPS), block(32 * MOE_GATHER_WARPS);
+  const bool warps = moe_gather_by_warps(slots, (size_t)width * (dtype == SRB_DTYPE_F32 ? 4 : 2));
+  const dim3 grid(warps ? (slots + MOE_GATHER_WARPS - 1) / MOE_GATHER_WARPS : slots), block(warps ? 32 * MOE_GATHER_WARPS : 128);
   if (dtype == SRB_DTYPE_F32)
-    SRB_CUDA_CALL(srb_launch(moe_gather_kernel<float>, grid, block, 0, s, (const float*)h, slot_row, slots, width, (float*)out, used));
+    SRB_CUDA_CALL(srb_launch(warps ? moe_gather_kernel<float, true> : moe_gather_kernel<float, false>, grid, block, 0, s, (const float*)h, slot_row,
+                             slots, width, (float*)out, used));
   else if (dtype == SRB_DTYPE_BF16)
-    SRB_CUDA_CALL(srb_launch(moe_gather_kernel<__nv_bfloat16>, grid, block, 0, s, (const __nv_bfloat16*)h, slot_row, slots,
-                             width, (__nv_bfloat16*)out, used));
+    SRB_CUDA_CALL(srb_launch(warps ? moe_gather_kernel<__nv_bfloat16, true> : moe_gather_kernel<__nv_bfloat16, false>, grid, block, 0, s,
+                             (const __nv_bfloat16*)h, slot_row, slots, width, (__nv_bfloat16*)out, used));
   else
     SRB_FAIL("moe_gather: unknown dtype %d", dtype);
   SRB_LAUNCH_CHECK("moe_gather");
