@@ -800,8 +800,3 @@ extern "C" int srb_sample_rows(const float* logits, const int* rows_index, int c
                            uniform, chunk_max, chunk_arg, chunk_sum, out));
   return SRB_OK;
 }
-
-extern "C" int srb_sample(const float* logits, int rows, int vocab, int stride, const float* temperature,
-                          const float* uniform, int* out, float* scratch, void* stream) {
-  return srb_sample_rows(logits, nullptr, rows, rows, vocab, stride, temperature, uniform, out, scratch, stream);
-}

@@ -1111,7 +1111,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
            partial_ok: bool = False) -> torch.Tensor:
     """y = x @ weight^T (+ bias); weight is [out, in], row-major.
 
-    float32: the kernel of this package that splits a float into three bfloat16 parts, 32-bit to the end.  bfloat16: up to
+    float32: the kernel of this package that splits a float into three bfloat16 parts, 32-bit to the end; both operands may
+    come from the call just ahead.  bfloat16 (the weight is not one that a kernel just ahead still writes): up to
     ``OWN_GEMM_MAX_TOKENS`` rows the tcgen05 kernel of this package, above that cuBLAS
     (:func:`library_product`: what the reference's engine calls for every projection,
     crates/sglang-kernel/src/cublas.rs:383-410); both accumulate in 32-bit.  ``out_dtype``

@@ -44,7 +44,7 @@ def test_embedding_norm_and_gated_product(dtype):
 @pytest.mark.parametrize("m,n,k", [(1, 200, 136), (8, 333, 72), (64, 130, 512), (70, 257, 264), (300, 96, 200)])
 def test_products(dtype, m, n, k):
     """Few rows (this package's tcgen05 kernel in bfloat16, partial sums and all), more rows (the library), and
-    the 32-bit FFMA kernel, against the triple loop."""
+    the 32-bit kernel, against the triple loop."""
     g = torch.Generator().manual_seed(m + n)
     x, w, bias = torch.randn(m, k, generator=g), torch.randn(n, k, generator=g) * 0.1, torch.randn(n, generator=g)
     want = cpp.linear(seen(x, dtype), seen(w, dtype), bias)

@@ -1255,3 +1255,38 @@ def test_launches_of_the_generic_attention_are_counted(dtype, split, length, lau
     before = ops.launch_count
     run_attention(case, 0.1, split)
     assert ops.launch_count - before == launches
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("slots,width", [(1, 8), (5, 512), (9, 513), (300, 256), (300, 2048), (301, 2049), (4096, 1024), (4097, 1024), (4100, 4096)])
+def test_gather_of_rows_by_warps_and_by_blocks(dtype, slots, width):
+    """A warp or a block a slot, by the slots and the bytes of a row; slots behind the used ones keep what they hold."""
+    lib, g = ops.load_library("moe"), torch.Generator().manual_seed(slots + width)
+    h = torch.randn(40, width, generator=g).to(DEV, dtype)
+    slot_row = torch.randint(0, 40, (slots,), generator=g, dtype=torch.int32).to(DEV)
+    for used in (None, slots - slots // 3):
+        out = torch.full((slots, width), 7.0, device=DEV, dtype=dtype)
+        count = None if used is None else torch.tensor([used], dtype=torch.int32, device=DEV)
+        ops._check(lib, lib.srb_moe_gather_used(ops._ptr(h), ops._ptr(slot_row), slots, width, ops._ptr(out), ops._ptr(count),
+                                                ops.dtype_code(dtype), ops._stream()))
+        last = slots if used is None else used
+        assert torch.equal(out[:last], h[slot_row[:last].long()]) and bool((out[last:] == 7.0).all())
+
+
+@pytest.mark.parametrize("sampled", [False, True])
+def test_sampling_of_named_rows(sampled):
+    """Rows in any order, or none; the others keep what they hold."""
+    g = torch.Generator().manual_seed(3)
+    logits = (torch.randn(9, 5003, generator=g) * 3).to(DEV)
+    heat = torch.tensor([0.0, 0.5, 1.0, 2.0, 0.7, 0.0, 1.3, 0.9, 1.0], device=DEV) if sampled else None
+    uniform = torch.rand(9, generator=g).to(DEV) if sampled else None
+    whole = ops.sample(logits, heat, uniform)
+    for rows in ([8, 0, 3], [5], list(range(8, -1, -1)), []):
+        out = torch.full((9,), -7, dtype=torch.int32, device=DEV)
+        index = torch.tensor(rows, dtype=torch.int32, device=DEV)
+        ops.sample(logits, heat, uniform, out, index)
+        want = torch.full((9,), -7, dtype=torch.int32, device=DEV)
+        want[index.long()] = whole[index.long()]
+        assert torch.equal(out, want), rows
+    if not sampled:
+        assert torch.equal(whole.long(), logits.argmax(dim=1))
