@@ -56,7 +56,7 @@ SRB_DEFINE_PDL_SWITCH()
 #define F32_PLANES 3          // bfloat16 parts of a float
 #define F32_EARLY_CHUNKS 4    // of the weights, that are asked into L2 ahead of the wait for the kernels ahead
 #define F32_MAX_PARTS 8
-#define F32_MAX_BLOCKS 8      // blocks of a cluster
+#define F32_MAX_BLOCKS 8      // blocks of a cluster (16 where two share a part)
 
 // Blocks along K for up to 16 rows, and parts of K, whose sums are rounded apart and then added.  Blocks: as many (a power of two) as are
 // resident at once, two to an SM, each of at least two chunks; eight only where an SM has one of them at most, since eight parts are
@@ -64,7 +64,7 @@ SRB_DEFINE_PDL_SWITCH()
 // blocks that walks all of K has no room for that (two rows, 4,096 x 1,024: 9.7 us with four blocks, 10.1 with eight).  Parts: as many as
 // blocks, or, where that makes them long, twice as many or up to eight of at least eight chunks (of positive operands, 20,000 x 4,096, the
 // error is 5.2e-8 in eight parts and was 1.5e-7 in one).
-struct F32Parts { int count, chunks, blocks; };      // parts, the chunks of each but the last, blocks
+struct F32Parts { int count, chunks, blocks; };      // parts, the chunks of each but the last, blocks (twice the parts: each shares one)
 static inline F32Parts gemm_parts(int n, int k) {
   const int chunks = (k + F32_CHUNK - 1) / F32_CHUNK, tiles = (n + F32_FEATURES - 1) / F32_FEATURES;
   int blocks = 1;
@@ -74,7 +74,10 @@ static inline F32Parts gemm_parts(int n, int k) {
   if (blocks == 4 && chunks > 64) parts = 8;
   while (blocks < 4 && parts < (blocks == 1 ? F32_MAX_PARTS : 2 * blocks) && parts * 16 <= chunks) parts *= 2;
   while (parts > 1 && (parts - 1) * ((chunks + parts - 1) / parts) >= chunks) parts /= 2;        // no part is empty
-  return {parts, (chunks + parts - 1) / parts, std::min(blocks, parts)};
+  const int part_chunks = (chunks + parts - 1) / parts;
+  if (parts == blocks && parts >= 4 && (part_chunks == 4 || part_chunks == 6) && chunks == parts * part_chunks && tiles * parts * 2 <= 296)
+    return {parts, part_chunks, 2 * parts};
+  return {parts, part_chunks, std::min(blocks, parts)};
 }
 
 struct F32Args {
@@ -84,6 +87,7 @@ struct F32Args {
   int parts, part_chunks;     // of K; chunks of a part
   int block_parts;            // parts that a block adds up: all, two or one
   int in_pairs;               // neighbouring parts are added first
+  int halved;                 // two blocks share a part of four or six chunks; the second leaves the sums of its chunks apart
   float unit;                 // K * 2^-97
   int constant;               // no kernel ahead writes w
   int* error_word;            // or null
@@ -256,8 +260,9 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
   const unsigned rank = srb_cluster_rank(), leader = PAIR ? rank & ~1u : rank;
   const int feature0 = blockIdx.x * F32_FEATURES, token0 = blockIdx.y * TOKENS;
   const int all_chunks = (args.k + F32_CHUNK - 1) / F32_CHUNK;
-  const int chunk0 = blockIdx.z * args.block_parts * args.part_chunks;
-  const int chunks = min(all_chunks, chunk0 + args.block_parts * args.part_chunks) - chunk0;
+  const int half_chunks = args.part_chunks / 2;
+  const int chunk0 = !PAIR && args.halved ? blockIdx.z * half_chunks : blockIdx.z * args.block_parts * args.part_chunks;
+  const int chunks = !PAIR && args.halved ? half_chunks : min(all_chunks, chunk0 + args.block_parts * args.part_chunks) - chunk0;
 
   float4 held_w[W_LOADS];
   const int row = tid >> 4, quad = tid & 15;                             // of a loader's first load; the next ones are LINES rows on
@@ -292,7 +297,7 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
   // sums of an adder's feature (its lane of tensor memory)
   const int quarter = warp & 3, group = (warp - LOADER_WARPS) >> 2;
   pair_t part[OWN / 2];
-  pair_t held[PAIR ? 1 : OWN / 2];                                       // few rows: the sums of earlier parts
+  pair_t held[PAIR ? 1 : OWN / 2], middle[PAIR ? 1 : OWN / 2];           // few rows: the sums of earlier parts, or of chunks
   srb_launch_dependents();
 
   if (warp < LOADER_WARPS) {
@@ -448,6 +453,17 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
       tc_fence_before();
       __syncwarp();
       if (lane == 0) f32_arrive<PAIR>(smem_u32(&sum_empty[b]), leader);
+      if (!PAIR && args.halved) {
+        if (chunk + 1 < chunks && (blockIdx.z & 1)) {
+#pragma unroll
+          for (int j = 0; j < OWN / 2; ++j) {
+            if (chunk == 0) held[PAIR ? 0 : j] = part[j];
+            else middle[PAIR ? 0 : j] = part[j];
+            part[j] = 0ull;
+          }
+        }
+        continue;
+      }
       if (args.block_parts == 1 || ((chunk0 + chunk + 1) % args.part_chunks != 0 && chunk + 1 != chunks)) continue;
       // A block with all parts keeps their running sum; one with two leaves the first beside the second.
       const bool last = chunk + 1 == chunks;
@@ -482,7 +498,7 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
   // This block's sums as [token][128 features], of two parts one behind the other.  The block of the cluster with range z of K adds rows
   // z, z + blocks, ... over all ranges.
   const int blocks = gridDim.z;
-  const bool two = blocks > 1 && args.block_parts == 2;
+  const bool two = blocks > 1 && (args.block_parts == 2 || (!PAIR && args.halved));
   float* tile = reinterpret_cast<float*>(smem);
   if (warp >= LOADER_WARPS && warp < ISSUE_WARP) {
 #pragma unroll
@@ -490,6 +506,8 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
       const int at = (group * OWN + j) * F32_FEATURES + quarter * 32 + lane;
       tile[at] = lost ? __int_as_float(0x7fffffff) : j & 1 ? high_of(part[j / 2]) : low_of(part[j / 2]);
       if (!PAIR && two) level[at] = j & 1 ? high_of(held[PAIR ? 0 : j / 2]) : low_of(held[PAIR ? 0 : j / 2]);
+      if (!PAIR && args.halved && half_chunks == 3)
+        level[TOKENS * F32_FEATURES + at] = j & 1 ? high_of(middle[PAIR ? 0 : j / 2]) : low_of(middle[PAIR ? 0 : j / 2]);
     }
   }
   __syncwarp();
@@ -573,6 +591,30 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
           const unsigned range = first_rank + (lane & 15);
           if ((lane & 15) < blocks) most = lane < 16 ? noted(&x_most[r % S::X_ROWS], range) : noted(&w_most, range);
         }
+        float v = 0.f;
+        if (!PAIR && args.halved) {
+          float half[F32_MAX_PARTS], one[F32_MAX_PARTS], more[F32_MAX_PARTS], last[F32_MAX_PARTS];
+          const int at = r * F32_FEATURES + col;
+#pragma unroll
+          for (int b = 0; b < F32_MAX_PARTS; ++b) {
+            half[b] = one[b] = more[b] = last[b] = 0.f;
+            if (b < args.parts) {
+              half[b] = srb_load_peer_shared(tile + at, first_rank + 2 * b);
+              one[b] = srb_load_peer_shared(level + at, first_rank + 2 * b + 1);
+              if (half_chunks == 3) more[b] = srb_load_peer_shared(level + TOKENS * F32_FEATURES + at, first_rank + 2 * b + 1);
+              last[b] = srb_load_peer_shared(tile + at, first_rank + 2 * b + 1);
+            }
+          }
+#pragma unroll
+          for (int b = 0; b < F32_MAX_PARTS; ++b) half[b] = half_chunks == 3 ? half[b] + one[b] + more[b] + last[b] : half[b] + one[b] + last[b];
+          if (args.in_pairs) {
+#pragma unroll
+            for (int b = 0; b < F32_MAX_PARTS; b += 2) v = b == 0 ? half[0] + half[1] : v + (half[b] + half[b + 1]);
+          } else {
+#pragma unroll
+            for (int b = 0; b < F32_MAX_PARTS; ++b) v = b == 0 ? half[0] : b < args.parts ? v + half[b] : v;
+          }
+        } else {
         float first[MOST], second[MOST];
 #pragma unroll
         for (int b = 0; b < MOST; ++b) {
@@ -583,7 +625,6 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
             second[b] = srb_load_peer_shared(tile + r * F32_FEATURES + col, peer);
           }
         }
-        float v = 0.f;
         if (args.in_pairs) {
           if (two) {
 #pragma unroll
@@ -601,6 +642,7 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
               v += second[b];
             }
           }
+        }
         }
         const unsigned x = PAIR ? tile_x_most[PAIR ? r : 0] : __reduce_max_sync(0xffffffffu, lane < 16 ? most : 0u);
         const unsigned w = PAIR ? tile_w_most : __reduce_max_sync(0xffffffffu, lane < 16 ? 0u : most);
@@ -629,7 +671,9 @@ static int launch(F32Args args, int blocks, cudaStream_t s) {
   using S = F32Shape<TOKENS, PAIR>;
   auto kernel = gemm_f32_kernel<TOKENS, PAIR, WIDE>;
   SRB_CUDA_CALL(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
-  args.block_parts = args.parts / blocks;
+  if (blocks > F32_MAX_BLOCKS) SRB_CUDA_CALL(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  args.block_parts = std::max(1, args.parts / blocks);
+  args.halved = blocks > args.parts;
   const unsigned features = (args.n + F32_FEATURES - 1) / F32_FEATURES;
   dim3 grid(PAIR ? (features + 1) / 2 * 2 : features, (args.m + TOKENS - 1) / TOKENS, blocks);
   if (grid.y > 65535) SRB_FAIL("gemm_f32: %d rows exceed one launch", args.m);
@@ -676,7 +720,7 @@ extern "C" int srb_gemm_f32(const float* a, const float* w, const float* bias, f
   args.a = a; args.w = w; args.bias = bias; args.c = c;
   args.m = m; args.n = n; args.k = k; args.lda = lda; args.ldw = ldw; args.ldc = ldc;
   args.parts = parts.count; args.part_chunks = parts.chunks;
-  args.in_pairs = parts.blocks == 8; args.constant = constant_weights; args.error_word = error_word;
+  args.in_pairs = parts.count == 8 && parts.blocks >= 8; args.constant = constant_weights; args.error_word = error_word;
   args.unit = ldexpf((float)k, -97);
   const bool wide = k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
   return wide ? dispatch<true>(args, parts.blocks, (cudaStream_t)stream) : dispatch<false>(args, parts.blocks, (cudaStream_t)stream);
