@@ -24,19 +24,20 @@
 // largest magnitude of each row of A and of a block's rows of W (two instructions to four entries; 2 us of 43 at 450 x 4,096 x 1,024).  A
 // result that is not large enough to hide what may be lost (K 2^-97 times the sum of both magnitudes leaves 2^-27 of it; rows of zeros are
 // exact), or whose operands have entries of 2^40 and more, is computed again in fused multiply-adds by a warp; one whose operands have an
-// entry that is not a number is not a number.  450 x 4,096 x 1,024 on one set of weights: 39 us; with a row that is not a number 39, all rows
-// 44; with a row of infinities or of entries above 2^40 93; a tenth of the entries below 2^-40 39; 250 rows of zeros 44.  (A thread a
+// entry that is not a number is not a number.  450 x 4,096 x 1,024 on one set of weights: 38 us; with a row that is not a number 42, all rows
+// 45; with a row of infinities or of entries above 2^40 97; a tenth of the entries below 2^-40 39; 250 rows of zeros 46.  (A thread a
 // result that is not finite: 105 for a row that is not a number, 15,700 for all.)
 //
 // What bounds it: of some 3,800 cycles a chunk (450 rows) the products take 2,100 and the loaders 2,800, which split floats and wait for
-// L2; and a start and end of some 12,000.  Times in us, behind another product; in brackets six products in sums of 32 entries without
-// regard for ranges, then fused multiply-adds over tiles in shared memory: 450 x 4,096 x 1,024 43 (50, 124), 450 x 6,144 x 1,024 81 (79,
-// 173), 450 x 1,024 x 3,072 60 (60, 94), 64 x 4,096 x 1,024 25 (25, 38), 2,048 x 4,096 x 1,024 163 (199, 456), 2,048 x 1,024 x 3,072, where
-// pairs of blocks have two parts each whatever the number of tiles, 158 (110, 350).
-// One and two rows are bound by latencies and by the unit's reads of W (eight per piece of it), and slower than fused multiply-adds, which
-// could not give the same bits for all row counts: 2 x 4,096 x 1,024 9.5 us (8.9, 7.9), 2 x 1,024 x 3,072 10.7 (9.8, 7.8), 2 x 151,936 x
-// 1,024 149 (141, 160) with constant weights, as the step executor's are; 11.6, 12.5 and 147 where they are read behind the wait for the
-// kernels ahead.
+// L2; and a start and end of some 11,000.  Times in us, behind another product; in brackets six products in sums of 32 entries without
+// regard for ranges, then fused multiply-adds over tiles in shared memory: 450 x 4,096 x 1,024 43 (50, 124), 450 x 6,144 x 1,024 79 (79,
+// 173), 450 x 1,024 x 3,072 59 (60, 94), 64 x 4,096 x 1,024 23 (25, 38), 2,048 x 4,096 x 1,024 160 (198, 456), 2,048 x 1,024 x 3,072, where
+// pairs of blocks have two parts each whatever the number of tiles, 155 (110, 350).
+// One and two rows are bound by latencies and by the unit's reads of W (eight per piece of it: 1,400 cycles a chunk), and slower than fused
+// multiply-adds, which could not give the same bits for all row counts: 2 x 4,096 x 1,024 9.5 us (8.9, 7.9), 2 x 1,024 x 2,048 7.4 (7.2, 5.5),
+// 2 x 6,144 x 1,024 11.4 (10.4, 9.1), 2 x 1,024 x 3,072 9.3 (9.9, 7.8), 2 x 151,936 x 1,024 150 (141, 160) with constant weights, as the step
+// executor's are; 9.4, 8.6, 12.3, 10.3 and 148 where they are read behind the wait for the kernels ahead.  A life of one request at
+// the 0.6B shape (a prompt of 8 tokens, eight decoded) takes 14.7 ms (13.9, 13.4); with six products in this form it would take 13.9.
 //
 // Weight layout and meaning as the reference's `linear`: row-major [out, in],
 // y[o] = sum_i x[i] * W[o, i] (crates/sglang-kernel/src/cpu.rs:73-108).
@@ -59,11 +60,12 @@ SRB_DEFINE_PDL_SWITCH()
 #define F32_MAX_BLOCKS 8      // blocks of a cluster (16 where two share a part)
 
 // Blocks along K for up to 16 rows, and parts of K, whose sums are rounded apart and then added.  Blocks: as many (a power of two) as are
-// resident at once, two to an SM, each of at least two chunks; eight only where an SM has one of them at most, since eight parts are
-// added in neighbouring pairs (a sequence of eight roundings was 5 % less exact on positive operands than multiply-adds) and a pair of
-// blocks that walks all of K has no room for that (two rows, 4,096 x 1,024: 9.7 us with four blocks, 10.1 with eight).  Parts: as many as
-// blocks, or, where that makes them long, twice as many or up to eight of at least eight chunks (of positive operands, 20,000 x 4,096, the
-// error is 5.2e-8 in eight parts and was 1.5e-7 in one).
+// resident at once, two to an SM, each of at least two chunks.  Eight parts of eight blocks are added in neighbouring pairs (a sequence
+// of eight roundings was 5 % less exact on positive operands than multiply-adds), for which a pair of blocks that walks all of K has no room,
+// so there are four where an SM has more than one block.  Longer sums have more parts: twice as many as blocks, or up to eight of at least
+// eight chunks (of positive operands, 20,000 x 4,096, the error is 5.2e-8 in eight parts and was 1.5e-7 in one).  Parts of four or six
+// chunks are shared by two blocks where those are resident at once too: the second leaves the sums of its chunks apart, so that the
+// order of additions stays (two rows, 1,024 x 3,072: 10.9 us by a block a part, 9.2 by two; 6,144 x 1,024, whose 384 blocks are not: 11.4 and 16).
 struct F32Parts { int count, chunks, blocks; };      // parts, the chunks of each but the last, blocks (twice the parts: each shares one)
 static inline F32Parts gemm_parts(int n, int k) {
   const int chunks = (k + F32_CHUNK - 1) / F32_CHUNK, tiles = (n + F32_FEATURES - 1) / F32_FEATURES;
@@ -251,9 +253,9 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_unaligned + 1023) & ~(uintptr_t)1023);
   // of the buffers of shared memory: filled (in the issuing block), their products done; of the sums: taken out (in the issuing block)
   __shared__ __align__(8) unsigned long long full_bar[2], done_bar[2], sum_empty[2], drain_bar;
-  // the largest magnitude (as bits) of each row of A and of W, there 2^40 at most with the upper bit for rows that have notes
-  __shared__ unsigned x_most[S::X_ROWS], w_most, w_notes[F32_FEATURES];
-  __shared__ unsigned tile_x_most[PAIR ? TOKENS : 1], tile_w_most;                   // of all blocks that share the tile
+  // the largest magnitude (as bits) of each row of A and of W, there 2^40 at most with the upper bit for rows that have notes; whether one of
+  // them, of a pair in any block of the cluster, is 2^40 or more or not a number
+  __shared__ unsigned x_most[S::X_ROWS], w_most, w_notes[F32_FEATURES], large;
   __shared__ unsigned tmem_holder;
   __shared__ int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -277,6 +279,7 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
   for (int i = tid; i < F32_FEATURES; i += S::THREADS) w_notes[i] = 0;
   if (tid == 0) {
     abort_flag = 0;
+    large = 0;
     w_most = 0;
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&full_bar[b]), PAIRED * LOADER_WARPS);          // one lane of each warp, of both blocks
@@ -332,6 +335,12 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
 #pragma unroll
       for (int i = 0; i < X_LOADS; ++i) load_x(i, chunk + 1);
     };
+    auto tell_large = [&]() {
+      if (!PAIR) { large = 1; return; }
+      for (unsigned b = 0; b < 2 * gridDim.z; ++b)
+        asm volatile("{\n.reg .b32 remote;\nmapa.shared::cluster.u32 remote, %0, %1;\nst.shared::cluster.u32 [remote], %2;\n}\n"
+                     ::"r"(smem_u32(&large)), "r"(b), "r"(1u) : "memory");
+    };
     int chunk = 0;
     if (args.constant) {
       // Weights that no kernel ahead writes: both buffers' share of them is split ahead of the wait.
@@ -364,12 +373,16 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
 #pragma unroll
     for (int i = 0; i < X_LOADS; ++i) {                                  // (the sixteen lanes of a row are its only readers)
       const unsigned most = __reduce_max_sync(lane < 16 ? 0xffffu : 0xffff0000u, __float_as_uint(x_high[i]));
-      if (quad == 0) x_most[row + i * LINES] = most;
+      if (quad == 0) {
+        x_most[row + i * LINES] = most;
+        if (most >= F32_LIMIT) tell_large();
+      }
     }
     const unsigned most = __reduce_max_sync(0xffffffffu, min(__float_as_uint(w_high), F32_LIMIT));
     if (lane == 0) atomicMax(&w_most, most);
     if (!(w_high < 0x1p40f)) {                                           // which rows: in a second look
       atomicMax(&w_most, 0x80000000u | F32_LIMIT);
+      tell_large();
 #pragma unroll 1
       for (int i = 0; i < W_LOADS; ++i) {
         const int r = feature0 + row + i * LINES;
@@ -501,10 +514,13 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
   const bool two = blocks > 1 && (args.block_parts == 2 || (!PAIR && args.halved));
   float* tile = reinterpret_cast<float*>(smem);
   if (warp >= LOADER_WARPS && warp < ISSUE_WARP) {
+    const bool noted_here = large != 0;
 #pragma unroll
     for (int j = 0; j < OWN; ++j) {
       const int at = (group * OWN + j) * F32_FEATURES + quarter * 32 + lane;
       tile[at] = lost ? __int_as_float(0x7fffffff) : j & 1 ? high_of(part[j / 2]) : low_of(part[j / 2]);
+      // few rows: what has notes is not a number in this block's sums, whoever adds them (a pair's blocks are told)
+      if (!PAIR && noted_here && (x_most[(group * OWN + j) % S::X_ROWS] >= F32_LIMIT || w_notes[quarter * 32 + lane])) tile[at] = __int_as_float(0x7fffffff);
       if (!PAIR && two) level[at] = j & 1 ? high_of(held[PAIR ? 0 : j / 2]) : low_of(held[PAIR ? 0 : j / 2]);
       if (!PAIR && args.halved && half_chunks == 3)
         level[TOKENS * F32_FEATURES + at] = j & 1 ? high_of(middle[PAIR ? 0 : j / 2]) : low_of(middle[PAIR ? 0 : j / 2]);
@@ -523,11 +539,19 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
   };
   // Results below this may lack what the parts lose of small entries: 3 * 2^-126 an entry and 2^-126 a product.
   auto least = [&](unsigned x, unsigned w) { return args.unit * (__uint_as_float(x) + __uint_as_float(w & 0x7fffffffu) + 2.f); };
-  auto unsure = [&](unsigned x, unsigned w, float smallest) { return (w >> 31) || x >= F32_LIMIT || __any_sync(0xffffffffu, smallest < least(x, w)); };
-  // A result that may not be sure, by a whole warp with one row, whose largest magnitude is x, and 32 neighbouring columns.
-  auto reconsidered = [&](int r, int f, unsigned x, unsigned w, float v) {
+  // The first look, without the other blocks' notes: no entry is above 2^40 then.
+  const float at_most_least = args.unit * 0x1.1p41f;
+  auto unsure = [&](float smallest) { return (PAIR && large) || __any_sync(0xffffffffu, !(smallest >= at_most_least)); };
+  // A result that may not be sure, by a whole warp with one row and 32 neighbouring columns.
+  auto reconsidered = [&](int r, int f, float v) {
     const int row = token0 + r, col = feature0 + f;
-    unsigned notes = 0;
+    unsigned notes = 0, x = 0, w = 0;                                    // the largest magnitude of the row, and of W
+    if (lane < blocks) {
+      x = noted(&x_most[r % S::X_ROWS], first_rank + lane * PAIRED + r / S::X_ROWS);
+      w = noted(&w_most, first_rank + lane * PAIRED + (rank - leader));
+    }
+    x = __reduce_max_sync(0xffffffffu, x);
+    w = __reduce_max_sync(0xffffffffu, w);
     for (int b = 0; (w >> 31) && b < blocks; ++b) notes |= noted(&w_notes[f], first_rank + b * PAIRED + (rank - leader));
     const bool none = x > 0x7f800000u || (notes & F32_NAN);
     const bool again = row < args.m && col < args.n && !none && (x >= F32_LIMIT || notes || (x != 0 && fabsf(v) < least(x, w)));
@@ -539,18 +563,6 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
     }
     return v;
   };
-  if (PAIR) {
-    static_assert(!PAIR || TOKENS < S::THREADS, "a thread each");
-    if (tid <= TOKENS) {
-      unsigned most = 0;
-#pragma unroll
-      for (int b = 0; b < F32_MAX_BLOCKS / 2; ++b)
-        if (b < blocks) most = max(most, tid < TOKENS ? noted(&x_most[tid % S::X_ROWS], first_rank + b * PAIRED + tid / S::X_ROWS)
-                                                      : noted(&w_most, first_rank + b * PAIRED + (rank - leader)));
-      *(tid < TOKENS ? &tile_x_most[tid] : &tile_w_most) = most;
-    }
-    __syncthreads();
-  }
   constexpr int LINES_AT_ONCE = S::THREADS / F32_FEATURES;
   const int col = tid & (F32_FEATURES - 1), line = tid / F32_FEATURES, first_row = (int)blockIdx.z + line * blocks;
   const int limit = min(TOKENS, args.m - token0);
@@ -558,7 +570,6 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
   if (line < LINES_AT_ONCE && first_row < limit) {
     if (blocks == 1) {
       constexpr int AT_ONCE = 4;
-      const unsigned w = PAIR ? tile_w_most : w_most;
       for (int r0 = first_row; r0 < limit; r0 += LINES_AT_ONCE * AT_ONCE) {
         float v[AT_ONCE];
 #pragma unroll
@@ -566,16 +577,12 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
         float smallest = INFINITY;
 #pragma unroll
         for (int i = 0; i < AT_ONCE; ++i)
-          if (live && r0 + i * LINES_AT_ONCE < limit) smallest = fminf(smallest, fabsf(v[i]));
-        const unsigned* row_most = PAIR ? tile_x_most : x_most;
-        unsigned x = 0;
-#pragma unroll
-        for (int i = 0; i < AT_ONCE; ++i) x = max(x, row_most[min(r0 + i * LINES_AT_ONCE, limit - 1)]);
-        if (unsure(x, w, smallest)) {
+          if (live && r0 + i * LINES_AT_ONCE < limit) smallest = fabsf(v[i]) < smallest || v[i] != v[i] ? fabsf(v[i]) : smallest;
+        if (unsure(smallest)) {
 #pragma unroll 1
           for (int i = 0; i < AT_ONCE; ++i) {
             const int r = r0 + i * LINES_AT_ONCE;
-            if (r < limit) store(r, col, reconsidered(r, col, row_most[r], w, tile[r * F32_FEATURES + col]));
+            if (r < limit) store(r, col, reconsidered(r, col, tile[r * F32_FEATURES + col]));
           }
           continue;
         }
@@ -586,11 +593,6 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
     } else {
       constexpr int MOST = PAIR ? F32_MAX_BLOCKS / 2 : F32_MAX_BLOCKS;
       for (int r = first_row; r < limit; r += LINES_AT_ONCE * blocks) {
-        unsigned most = 0;
-        if (!PAIR) {                                                     // lanes b and 16 + b: the largest entry of the row and of W in range b of K
-          const unsigned range = first_rank + (lane & 15);
-          if ((lane & 15) < blocks) most = lane < 16 ? noted(&x_most[r % S::X_ROWS], range) : noted(&w_most, range);
-        }
         float v = 0.f;
         if (!PAIR && args.halved) {
           float half[F32_MAX_PARTS], one[F32_MAX_PARTS], more[F32_MAX_PARTS], last[F32_MAX_PARTS];
@@ -644,9 +646,7 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
           }
         }
         }
-        const unsigned x = PAIR ? tile_x_most[PAIR ? r : 0] : __reduce_max_sync(0xffffffffu, lane < 16 ? most : 0u);
-        const unsigned w = PAIR ? tile_w_most : __reduce_max_sync(0xffffffffu, lane < 16 ? 0u : most);
-        if (unsure(x, w, live ? fabsf(v) : INFINITY)) v = reconsidered(r, col, x, w, v);
+        if (unsure(live ? fabsf(v) : INFINITY)) v = reconsidered(r, col, v);
         store(r, col, v);
       }
     }
