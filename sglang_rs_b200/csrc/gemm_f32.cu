@@ -617,34 +617,34 @@ __global__ void __launch_bounds__(F32Shape<TOKENS, PAIR>::THREADS, F32Shape<TOKE
             for (int b = 0; b < F32_MAX_PARTS; ++b) v = b == 0 ? half[0] : b < args.parts ? v + half[b] : v;
           }
         } else {
-        float first[MOST], second[MOST];
+          float first[MOST], second[MOST];
 #pragma unroll
-        for (int b = 0; b < MOST; ++b) {
-          const unsigned peer = first_rank + b * PAIRED + (rank - leader);
-          first[b] = second[b] = 0.f;
-          if (b < blocks) {
-            if (two) first[b] = srb_load_peer_shared(level + r * F32_FEATURES + col, peer);
-            second[b] = srb_load_peer_shared(tile + r * F32_FEATURES + col, peer);
-          }
-        }
-        if (args.in_pairs) {
-          if (two) {
-#pragma unroll
-            for (int b = 0; b < MOST; ++b) v = b == 0 ? first[0] + second[0] : b < blocks ? v + (first[b] + second[b]) : v;
-          } else {
-#pragma unroll
-            for (int b = 0; b < MOST; b += 2) v = b == 0 ? second[0] + second[1] : b < blocks ? v + (second[b] + second[b + 1]) : v;
-          }
-        } else {
-          v = two ? first[0] + second[0] : second[0];
-#pragma unroll
-          for (int b = 1; b < MOST; ++b) {
+          for (int b = 0; b < MOST; ++b) {
+            const unsigned peer = first_rank + b * PAIRED + (rank - leader);
+            first[b] = second[b] = 0.f;
             if (b < blocks) {
-              if (two) v += first[b];
-              v += second[b];
+              if (two) first[b] = srb_load_peer_shared(level + r * F32_FEATURES + col, peer);
+              second[b] = srb_load_peer_shared(tile + r * F32_FEATURES + col, peer);
             }
           }
-        }
+          if (args.in_pairs) {
+            if (two) {
+#pragma unroll
+              for (int b = 0; b < MOST; ++b) v = b == 0 ? first[0] + second[0] : b < blocks ? v + (first[b] + second[b]) : v;
+            } else {
+#pragma unroll
+              for (int b = 0; b < MOST; b += 2) v = b == 0 ? second[0] + second[1] : b < blocks ? v + (second[b] + second[b + 1]) : v;
+            }
+          } else {
+            v = two ? first[0] + second[0] : second[0];
+#pragma unroll
+            for (int b = 1; b < MOST; ++b) {
+              if (b < blocks) {
+                if (two) v += first[b];
+                v += second[b];
+              }
+            }
+          }
         }
         if (unsure(live ? fabsf(v) : INFINITY)) v = reconsidered(r, col, v);
         store(r, col, v);

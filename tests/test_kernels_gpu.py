@@ -291,10 +291,11 @@ def test_gemm_f32_edges_of_segments_rounds_tiles_and_parts(n, k):
             assert torch.equal(ops.linear(rows[130 - m:], w_d, b_d), whole[130 - m:]), (m, offset)
 
 
-@pytest.mark.parametrize("n,k", [(4096, 1024), (6144, 1024), (1024, 3072), (1024, 6148), (12000, 4160), (20000, 1024), (2500, 4200)])
+@pytest.mark.parametrize("n,k", [(4096, 1024), (6144, 1024), (1024, 3072), (1024, 2048), (2304, 2048), (4000, 1536), (1024, 6148), (12000, 4160),
+                                 (20000, 1024), (2500, 4200)])
 def test_float_products_of_many_rows_give_the_bits_of_few(n, k):
-    """One pair of blocks that walks all parts of K (4,096 x 1,024 and more from 129 rows on), pairs with two parts, few-row blocks with one,
-    two and all: the order of additions is the same."""
+    """One pair of blocks that walks all parts of K (4,096 x 1,024 and more from 129 rows on), pairs with two parts, few-row blocks with half
+    a part, one, two and all: the order of additions is the same."""
     g = torch.Generator().manual_seed(n + k)
     x, w = torch.randn(450, k, generator=g).to(DEV), torch.randn(n, k, generator=g).to(DEV)
     whole = ops.linear(x, w)
